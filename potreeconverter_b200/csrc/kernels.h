@@ -23,6 +23,8 @@ struct ChunkingOut {
 // Decodes the LASzip chunks of one LAZ source into its point records
 // (chunks' byte offsets are file offsets; d_bytes holds the file from
 // `base` to the end of the last chunk). Throws on malformed data.
+// (d_bytes: laz_device_bytes(byte count) bytes of device memory, 4-byte aligned)
+inline size_t laz_device_bytes(uint64_t bytes) { return (size_t)((bytes + 3) & ~uint64_t(3)); }
 void launch_laz_decode(const uint8_t* d_bytes, uint64_t base, const std::vector<laz::Chunk>& chunks, const laz::Layout& L, uint8_t* d_out,
                        DeviceMem& mem);
 

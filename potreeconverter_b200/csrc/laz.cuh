@@ -1,6 +1,8 @@
 // LAZ point decoding for point formats 0-3 (LASzip "pointwise chunked"
-// compressor, items POINT10 v2, GPSTIME11 v2, RGB12 v2 and BYTE v2), written
-// for both the host (the chunk table) and the device (the point records).
+// compressor, items POINT10 v2, GPSTIME11 v2, RGB12 v2 and BYTE v2) by one
+// thread: the host reads the chunk table with it, and decode_chunk describes
+// the point records' steps and is what the device decoder (laz_warp.cuh) is
+// tested against.
 //
 // The method is LASzip's (M. Isenburg, "LASzip: lossless compression of LiDAR
 // data", PE&RS 79(2), 2013): an adaptive binary arithmetic coder with 32-bit

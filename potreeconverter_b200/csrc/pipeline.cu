@@ -607,7 +607,7 @@ struct Converter {
 				const auto& chunks = infos[k].laz_chunks;
 				if (chunks.empty()) continue;
 				const uint64_t base = chunks.front().start, nbytes = chunks.back().end - base;
-				uint8_t* d_laz = mem.alloc<uint8_t>(nbytes);
+				uint8_t* d_laz = mem.alloc<uint8_t>(pcg::laz_device_bytes(nbytes));
 				PCG_CUDA(cudaMemcpyAsync(d_laz, static_cast<const uint8_t*>(sources[k].las) + base, nbytes, cudaMemcpyHostToDevice, stream));
 				const auto t_dec = Clock::now();
 				launch_laz_decode(d_laz, base, chunks, infos[k].laz_layout, d_host + src_base[k], mem);
@@ -2384,7 +2384,7 @@ pcg_status pcg_kernel_decode_count(pcg_ctx* ctx, const void* las, uint64_t size,
 			const auto& chunks = info.laz_chunks;
 			if (!chunks.empty()) {
 				const uint64_t base = chunks.front().start, nbytes = chunks.back().end - base;
-				uint8_t* d_laz = mem.alloc<uint8_t>(nbytes);
+				uint8_t* d_laz = mem.alloc<uint8_t>(pcg::laz_device_bytes(nbytes));
 				PCG_CUDA(cudaMemcpyAsync(d_laz, static_cast<const uint8_t*>(las) + base, nbytes, cudaMemcpyHostToDevice, stream));
 				pcg::launch_laz_decode(d_laz, base, chunks, info.laz_layout, d_recs, mem);
 			}
@@ -2637,7 +2637,7 @@ pcg_status pcg_kernel_laz_decode(pcg_ctx* ctx, const void* laz_file, uint64_t si
 		pcg::DeviceMem mem(ctx->conv.stream, ctx->conv.arena.get());
 		const auto& chunks = info.laz_chunks;
 		const uint64_t base = chunks.front().start, nbytes = chunks.back().end - base;
-		uint8_t* d_laz = mem.alloc<uint8_t>(nbytes);
+		uint8_t* d_laz = mem.alloc<uint8_t>(pcg::laz_device_bytes(nbytes));
 		uint8_t* d_out = mem.alloc<uint8_t>(bytes);
 		PCG_CUDA(cudaMemcpyAsync(d_laz, static_cast<const uint8_t*>(laz_file) + base, nbytes, cudaMemcpyHostToDevice, mem.stream()));
 		pcg::launch_laz_decode(d_laz, base, chunks, info.laz_layout, d_out, mem);
