@@ -703,10 +703,7 @@ struct Converter {
 			for (auto& n : tree.nodes)
 				if (!n.has_children() && n.leaf_count > 0) { loff.push_back(n.leaf_start); lcnt.push_back(n.leaf_count); }
 			uint32_t* shuffled = mem.alloc<uint32_t>(N);
-			int32_t* scratch = mem.alloc<int32_t>(N);
-			int64_t* d_off = upload(loff, mem);
-			int64_t* d_cnt = upload(lcnt, mem);
-			launch_shuffle_leaves(d_off, d_cnt, (int)loff.size(), ids, shuffled, scratch, seed, mem);
+			launch_shuffle_leaves(loff, lcnt, ids, shuffled, seed, mem);
 			leaf_ids = shuffled;
 		}
 		if (method == PCG_POISSON_AVERAGE) {
@@ -1089,11 +1086,7 @@ struct Converter {
 				if (!t.has_children() && t.leaf_count > 0) { loff.push_back(t.leaf_start); lcnt.push_back(t.leaf_count); }
 			}
 			uint32_t* shuffled = mem.alloc<uint32_t>(std::max<int64_t>(n, 1));
-			int32_t* scratch = mem.alloc<int32_t>(std::max<int64_t>(n, 1));
-			int64_t* d_off = upload(loff, mem);
-			int64_t* d_cnt = upload(lcnt, mem);
-			launch_shuffle_leaves(d_off, d_cnt, (int)loff.size(), ids, shuffled, scratch, seed, mem);
-			mem.free(scratch);
+			launch_shuffle_leaves(loff, lcnt, ids, shuffled, seed, mem);
 			leaf_ids = shuffled;
 		}
 		if (method == PCG_POISSON_AVERAGE) {
@@ -1148,16 +1141,10 @@ struct Converter {
 		const cudaStream_t stream = mem.stream();
 		uint32_t* in = mem.alloc<uint32_t>(total);
 		uint32_t* out = mem.alloc<uint32_t>(total);
-		int32_t* scratch = mem.alloc<int32_t>(total);
 		for (size_t i = 0; i < sel.size(); i++)
 			PCG_CUDA(cudaMemcpyAsync(in + off[i], tree.nodes[sel[i]].buf_ids, cnt[i] * sizeof(uint32_t), cudaMemcpyDeviceToDevice, stream));
-		int64_t* d_off = upload(off, mem);
-		int64_t* d_cnt = upload(cnt, mem);
-		launch_shuffle_leaves(d_off, d_cnt, (int)sel.size(), in, out, scratch, seed, mem);
+		launch_shuffle_leaves(off, cnt, in, out, seed, mem);
 		for (size_t i = 0; i < sel.size(); i++) tree.nodes[sel[i]].buf_ids = out + off[i];
-		mem.free(d_cnt);
-		mem.free(d_off);
-		mem.free(scratch);
 		mem.free(in);
 	}
 

@@ -23,8 +23,6 @@
 //  * random_accept      -- sampler_random.h:146-178: a point is accepted if
 //    its child holds < 100 points, or if it is the first point of its
 //    128^3 cell that is eligible; first-eligible is an atomicMin per cell.
-//  * shuffle_leaves     -- std::shuffle(..., std::default_random_engine(seed))
-//    of sampler_random.h:97-118, libstdc++'s two-draws-per-call variant.
 
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -464,83 +462,6 @@ __global__ void random_accept_kernel(const LevelNode* __restrict__ nodes, const 
 __global__ void clear_hash_kernel(uint64_t* keys, int32_t* vals, int64_t n, int32_t fill) {
 	int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
 	if (i < n) { keys[i] = EMPTY_KEY; vals[i] = fill; }
-}
-
-// --------------------------------------------------------------- shuffle
-// std::default_random_engine = minstd_rand0 (16807, 0, 2^31 - 1)
-struct MinStd {
-	uint64_t x;
-	__device__ explicit MinStd(uint32_t seed) {
-		uint64_t s = (uint64_t)seed % 2147483647ull;
-		x = s == 0 ? 1 : s;
-	}
-	__device__ uint64_t operator()() {
-		x = (x * 16807ull) % 2147483647ull;
-		return x;
-	}
-};
-
-// uniform_int_distribution<unsigned long>{a, b}(minstd), downscaling branch
-__device__ __forceinline__ uint64_t uniform(MinStd& g, uint64_t a, uint64_t b) {
-	const uint64_t urngrange = 2147483646ull - 1ull;
-	const uint64_t urange = b - a;
-	uint64_t ret;
-	if (urngrange > urange) {
-		const uint64_t uerange = urange + 1;
-		const uint64_t scaling = urngrange / uerange;
-		const uint64_t past = uerange * scaling;
-		do ret = g() - 1ull; while (ret >= past);
-		ret /= scaling;
-	} else {
-		ret = g() - 1ull;  // urange == urngrange; larger ranges do not occur (n < 46341)
-	}
-	return ret + a;
-}
-
-__device__ void std_shuffle(int32_t* v, int64_t n, uint32_t seed) {
-	if (n == 0) return;
-	MinStd g(seed);
-	const uint64_t urngrange = 2147483645ull;
-	const uint64_t urange = (uint64_t)n;
-	if (urngrange / urange >= urange) {
-		int64_t i = 1;
-		if ((urange % 2) == 0) {
-			int64_t k = (int64_t)uniform(g, 0, 1);
-			int32_t t = v[i]; v[i] = v[k]; v[k] = t;
-			i++;
-		}
-		while (i != n) {
-			const uint64_t swap_range = (uint64_t)i + 1;
-			uint64_t xx = uniform(g, 0, swap_range * (swap_range + 1) - 1);
-			int64_t p1 = (int64_t)(xx / (swap_range + 1)), p2 = (int64_t)(xx % (swap_range + 1));
-			int32_t t = v[i]; v[i] = v[p1]; v[p1] = t;
-			i++;
-			t = v[i]; v[i] = v[p2]; v[p2] = t;
-			i++;
-		}
-	} else {
-		for (int64_t i = 1; i < n; i++) {
-			int64_t k = (int64_t)uniform(g, 0, (uint64_t)i);
-			int32_t t = v[i]; v[i] = v[k]; v[k] = t;
-		}
-	}
-}
-
-__global__ void shuffle_leaves_kernel(const int64_t* __restrict__ off, const int64_t* __restrict__ cnt, int num, const uint32_t* __restrict__ in,
-                                      uint32_t* __restrict__ out, int32_t* scratch, uint32_t seed) {
-	int l = blockIdx.x * blockDim.x + threadIdx.x;
-	if (l >= num) return;
-	const int64_t o = off[l], n = cnt[l];
-	int32_t* idx = scratch + o;
-	for (int64_t i = 0; i < n; i++) idx[i] = (int32_t)i;
-	std_shuffle(idx, n, seed);
-	// buffer[indices[i]] = points[i] (sampler_random.h:106-115)
-	for (int64_t i = 0; i < n; i++) out[o + idx[i]] = in[o + i];
-}
-
-__global__ void shuffle_single_kernel(int64_t n, uint32_t seed, int32_t* perm) {
-	for (int64_t i = 0; i < n; i++) perm[i] = (int32_t)i;
-	std_shuffle(perm, n, seed);
 }
 
 // ============================================ one CTA per large node
@@ -1825,21 +1746,6 @@ void launch_random_accept_sized(const LevelNode* nodes, const int32_t* X, const 
 	random_first_kernel<<<blocks, 256, 0, mem.stream()>>>(nodes, X, Y, Z, pp, lb, hash_keys, hash_vals, st);
 	PCG_LAUNCHED();
 	random_accept_kernel<<<blocks, 256, 0, mem.stream()>>>(nodes, X, Y, Z, pp, lb, hash_keys, hash_vals);
-	PCG_LAUNCHED();
-}
-
-void launch_shuffle_leaves(const int64_t* leaf_off, const int64_t* leaf_cnt, int num_leaves, const uint32_t* ids_in,
-                           uint32_t* ids_out, int32_t* scratch, uint32_t seed, DeviceMem& mem) {
-	if (num_leaves == 0) return;
-	shuffle_leaves_kernel<<<(unsigned)ceil_div(num_leaves, 64), 64, 0, mem.stream()>>>(leaf_off, leaf_cnt, num_leaves, ids_in, ids_out,
-	                                                                                    scratch, seed);
-	PCG_LAUNCHED();
-}
-
-
-void launch_shuffle_single(int64_t n, uint32_t seed, int32_t* perm, DeviceMem& mem) {
-	if (n <= 0) return;
-	shuffle_single_kernel<<<1, 1, 0, mem.stream()>>>(n, seed, perm);
 	PCG_LAUNCHED();
 }
 

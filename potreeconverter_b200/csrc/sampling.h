@@ -204,9 +204,9 @@ void launch_average_colors(const LevelNode* nodes, const int32_t* X, const int32
 void launch_random_accept_sized(const LevelNode* nodes, const int32_t* X, const int32_t* Y, const int32_t* Z, const PosParamsS& pp,
                                 LevelBuffers& lb, uint64_t* hash_keys, int32_t* hash_vals, int64_t hash_total, SampleStats* st,
                                 DeviceMem& mem);
-// leaf shuffle of the random sampler; leaves given as (offset, count) ranges of ids
-void launch_shuffle_leaves(const int64_t* leaf_off, const int64_t* leaf_cnt, int num_leaves, const uint32_t* ids_in,
-                           uint32_t* ids_out, int32_t* scratch, uint32_t seed, DeviceMem& mem);
+// leaf shuffle of the random sampler (shuffle.cu); leaves given as (offset, count) ranges of ids
+void launch_shuffle_leaves(const std::vector<int64_t>& off, const std::vector<int64_t>& cnt, const uint32_t* ids_in, uint32_t* ids_out,
+                           uint32_t seed, DeviceMem& mem);
 // stand-alone entry points for the parity tests
 void launch_sort_keys_single(double* keys, int32_t* vals, int64_t n, DeviceMem& mem, SampleStats* st, const SortedLevel* sorted = nullptr);
 void launch_shuffle_single(int64_t n, uint32_t seed, int32_t* perm, DeviceMem& mem);
