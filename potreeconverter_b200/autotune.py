@@ -1,6 +1,8 @@
 """Autotuner of the samplers' level schedule (csrc/sampling.h LevelSchedule):
-which nodes of a level get a CTA, a cluster of CTAs or a warp, and how many
-resident blocks per SM pull warp-sized nodes from the device work queue.
+from how many candidates a node's decisions get a block of 1,024 threads
+(cluster_min) or one of 16 x middle threads (cta_min, and small_level_cta_min
+on levels of few nodes) rather than one of 128, and middle, under the names
+that the table has for them.
 
 Run on the target GPU:
 

@@ -11,35 +11,57 @@
 // p, the earlier candidates q of its node with that property -- a
 // fixed-radius neighbour search, fully parallel over the level -- so the
 // acceptance kernel only has to look at those candidates' decisions.
+// poisson_average's colours use the same cells.
 //
-//  1. cell keys: cells of one spacing (x 1.000001) over the node box, so
-//     every point closer than the spacing lies in the 3 x 3 x 3 cells around
-//     a candidate's own;
-//  2. segmented radix sort of (cell, sorted position) per node;
-//  3. a hash table per node, cell -> range of the cell-sorted records;
-//  4. one thread per candidate in cell order (a warp shares neighbourhoods)
-//     scans the occupied cells among its 27 up to its own sorted position:
-//     the FP32 distance on node-relative coordinates decides every pair
-//     outside the band s^2 (1 -/+ 1e-3); pairs inside the band are decided
-//     by the reference's FP64 test and counted as escalated; then the
-//     early-exit bound. Error bound (u = 2^-24): a node-relative coordinate
-//     v lies in [0, L], L = 128 s, so its float differs from the FP64 value
-//     by at most L u = 128 s u; a coordinate difference d (|d| about s in the
-//     band) then carries at most 256 s u + |d| u, its square a relative
-//     error of 2 (257 u) + u, and the sum of three squares at most 517 u
-//     = 3.1e-5 of the squared distance D. The FP64 values the reference
-//     compares are themselves within 1.1e-16 |x| of the exact coordinates,
-//     below 1.1e-10 s when |x| < 1e6 s (checked per node; beyond it the
-//     node uses FP64 alone). So D32 >= s^2 (1 + 1e-3) (rounded up by at
-//     most u) implies D64 > s^2, and D32 < s^2 (1 - 1e-3) implies D64 < s^2:
-//     the margin is 30x the error.
-// A candidate with more than kListCap such predecessors marks its node
-// dense; dense nodes keep the grid-based acceptance kernel.
+//  1. cells of one spacing (x 1.000001) over the node box, so every point
+//     closer than the spacing lies in the 3 x 3 x 3 cells around a
+//     candidate's own; a bitmap of the occupied cells, 128 bits per row of
+//     cells along x, and per row how many occupied cells come before it: a
+//     cell's rank among the node's occupied ones is one 16-byte load, one
+//     4-byte load and a few population counts;
+//  2. a counting sort of the candidates by that rank (within a cell in any
+//     order: a list is a set). Everything up to here runs in gather order,
+//     in which neighbours in memory are neighbours in space, so the counters
+//     and the scattered records of a warp fall into a few lines. (A stable
+//     radix sort in the order of the distances and a hash table of the cells
+//     took 16.5 ms of a 50M-point conversion where this takes 7.6.)
+//  3. one thread per candidate in cell order: the cells x - 1 .. x + 1 of a
+//     row lie together in memory, so the 27 cells are nine runs of records,
+//     whose bounds are loaded at once. The FP32 distance on node-relative
+//     coordinates decides every pair outside the band s^2 (1 -/+ 1e-3);
+//     pairs inside the band are decided by the reference's FP64 test and
+//     counted as escalated; then the early-exit bound. (27 hash probes per
+//     candidate took 30.6 ms of a 50M-point conversion, this 17.2.)
+//
+// Error bound of the FP32 test (u = 2^-24): a node-relative coordinate v lies
+// in [0, L], L = 128 s, so its float differs from the FP64 value by at most
+// L u = 128 s u; a coordinate difference d (|d| about s in the band) then
+// carries at most 256 s u + |d| u, its square a relative error of 2 (257 u)
+// + u, and the sum of three squares at most 517 u = 3.1e-5 of the squared
+// distance D. The FP64 values the reference compares are themselves within
+// 1.1e-16 |x| of the exact coordinates, below 1.1e-10 s when |x| < 1e6 s
+// (checked per node; beyond it the node uses FP64 alone). So D32 >= s^2 (1 +
+// 1e-3) (rounded up by at most u) implies D64 > s^2, and D32 < s^2 (1 - 1e-3)
+// implies D64 < s^2: the margin is 30x the error.
+//
+// The early-exit bound needs the earlier candidate's key only where it can
+// fail. With c = sqrt(key(p)) >= 1.1 s and a pair the FP32 test puts inside
+// (distance d < 0.9995 s), the triangle inequality gives sqrt(key(q)) >= c - d
+// >= (c - s) + 5e-4 s, so key(q) exceeds (c - s)^2 by at least 5e-4 s * 0.1 s
+// = 5e-5 s^2, while the rounding of either side stays below 2e-8 s^2 (64 s *
+// 1.1e-10 s from the coordinates). Nearer the centre, and for pairs inside
+// the band, the keys are compared as the reference does.
+//
+// Lists of up to kListCap entries lie in the candidate's slot and a pool; a
+// longer one (points much denser than the spacing, as on a facade) is counted
+// here and written by a warp of its own once its room is known. Nodes whose
+// long lists would take more than kLongBudget entries in all keep the
+// lookup kernels (greedy_big_kernel).
 
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <cstdlib>
+#include <numeric>
 
 #include "devutil.cuh"
 #include "sampling.h"
@@ -48,18 +70,11 @@ namespace pcg {
 
 namespace {
 
-constexpr uint64_t kEmptyRun = ~0ull;
-constexpr int kListsVariant = 2;  // see lists_variant(); measured fastest on the benchmark's 50M cloud
-constexpr int kCellsPerAxis = 128;  // node box = 128 spacings
-
-struct alignas(16) RunSlot {  // run table entry, one 16-byte load per probe
-	uint64_t key;             // cell, kEmptyRun when free
-	int32_t start, count;     // first record in the node, records
-};
-
-__device__ __forceinline__ uint64_t run_hash(uint64_t k, int64_t cap) {
-	return ((k * 0x9E3779B97F4A7C15ull) >> 20) & (uint64_t)(cap - 1);
-}
+constexpr int kAxisBits = 7;
+constexpr int kCellsPerAxis = 1 << kAxisBits;  // node box = 128 spacings
+constexpr int64_t kRows = (int64_t)kCellsPerAxis * kCellsPerAxis;  // of a node
+// entries of all long lists of a level (1 GiB)
+constexpr int64_t kLongBudget = int64_t(1) << 28;
 
 __device__ __forceinline__ double qcoord(int32_t X, int a, const PosParamsS& pp) {
 	// (xyz[a] * scale) + offset, sampler_poisson.h:99-101
@@ -72,398 +87,545 @@ __device__ __forceinline__ int clamp_cell(double u) {
 	return (int)f;
 }
 
-__global__ void conf_cell_keys_kernel(const LevelNode* __restrict__ nodes, PosParamsS pp, LevelBuffers lb, uint64_t* __restrict__ keys) {
+// occupied cells of a row below x
+__device__ __forceinline__ int row_rank(const uint4& b, int x) {
+	const int w = x >> 5;
+	const uint32_t m = (1u << (x & 31)) - 1;
+	int r = __popc((w == 0 ? b.x : w == 1 ? b.y : w == 2 ? b.z : b.w) & m);
+	if (w > 0) r += __popc(b.x);
+	if (w > 1) r += __popc(b.y);
+	if (w > 2) r += __popc(b.z);
+	return r;
+}
+
+// every candidate's cell (z, y, x, seven bits each) and the occupancy bitmaps
+__global__ void cell_mark_kernel(const LevelNode* __restrict__ nodes, PosParamsS pp, LevelBuffers lb, uint32_t* __restrict__ cell,
+                                 uint32_t* __restrict__ rows) {
 	const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
 	if (j >= lb.M) return;
-	const LevelNode& nd = nodes[lb.node_of[j]];
-	const int4 r = lb.cq[j];
+	const int32_t node = lb.node_of[j];
+	const LevelNode& nd = nodes[node];
+	const int4 r = lb.rec[j];
 	const double inv = 1.0 / (nd.spacing * 1.000001);
 	const int cx = clamp_cell((qcoord(r.x, 0, pp) - nd.min[0]) * inv);
 	const int cy = clamp_cell((qcoord(r.y, 1, pp) - nd.min[1]) * inv);
 	const int cz = clamp_cell((qcoord(r.z, 2, pp) - nd.min[2]) * inv);
-	keys[j] = ((uint64_t)cz * kCellsPerAxis + (uint64_t)cy) * kCellsPerAxis + (uint64_t)cx;
+	const uint32_t row = (uint32_t)(cz << kAxisBits | cy);
+	cell[j] = row << kAxisBits | (uint32_t)cx;
+	uint32_t* word = rows + ((int64_t)node * kRows + row) * 4 + (cx >> 5);
+	const uint32_t bit = 1u << (cx & 31);
+	// most candidates find their cell marked already
+	if (!(*(volatile uint32_t*)word & bit)) atomicOr(word, bit);
 }
 
-// cell-sorted records: (X, Y, Z, sorted position) and, for the prefilter,
-// the position relative to the node's minimum corner in FP32 (w = sorted
-// position). Within a cell, records are in sorted order (the cell sort is
-// stable).
-__global__ void conf_gather_kernel(const LevelNode* __restrict__ nodes, PosParamsS pp, LevelBuffers lb, const uint32_t* __restrict__ cvals,
-                                   int4* __restrict__ crec, float4* __restrict__ crf) {
+constexpr int kRowThreads = 1024;
+constexpr int kRowsPerThread = (int)(kRows / kRowThreads);
+
+// occupied cells of the node before each row; one block per node
+__global__ void __launch_bounds__(kRowThreads) row_base_kernel(const uint4* __restrict__ rows, uint32_t* __restrict__ base) {
+	__shared__ uint32_t sums[32];
+	const int64_t r0 = (int64_t)blockIdx.x * kRows + (int64_t)threadIdx.x * kRowsPerThread;
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	uint32_t c[kRowsPerThread], sum = 0;
+#pragma unroll
+	for (int i = 0; i < kRowsPerThread; i++) {
+		const uint4 b = rows[r0 + i];
+		c[i] = (uint32_t)(__popc(b.x) + __popc(b.y) + __popc(b.z) + __popc(b.w));
+		sum += c[i];
+	}
+	uint32_t x = sum;
+#pragma unroll
+	for (int o = 1; o < 32; o <<= 1) {
+		const uint32_t y = __shfl_up_sync(FULL, x, o);
+		if (lane >= o) x += y;
+	}
+	if (lane == 31) sums[warp] = x;
+	__syncthreads();
+	if (warp == 0) {
+		uint32_t w = sums[lane];
+#pragma unroll
+		for (int o = 1; o < 32; o <<= 1) {
+			const uint32_t y = __shfl_up_sync(FULL, w, o);
+			if (lane >= o) w += y;
+		}
+		sums[lane] = w;
+	}
+	__syncthreads();
+	uint32_t run = x - sum + (warp ? sums[warp - 1] : 0u);
+#pragma unroll
+	for (int i = 0; i < kRowsPerThread; i++) {
+		base[r0 + i] = run;
+		run += c[i];
+	}
+}
+
+// (cell index of the level, place within the cell) of every candidate; the
+// node's cells are counted in count[cand_off ..). The lanes of a warp that
+// share a cell count once.
+__global__ void cell_count_kernel(const LevelNode* __restrict__ nodes, LevelBuffers lb, const uint32_t* __restrict__ cell,
+                                  const uint4* __restrict__ rows, const uint32_t* __restrict__ base, uint32_t* __restrict__ count,
+                                  uint2* __restrict__ place) {
+	const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+	uint32_t idx = 0xffffffffu;
+	if (j < lb.M) {
+		const int32_t node = lb.node_of[j];
+		const uint32_t c = cell[j];
+		const int64_t row = (int64_t)node * kRows + (c >> kAxisBits);
+		idx = (uint32_t)nodes[node].cand_off + base[row] + (uint32_t)row_rank(rows[row], (int)(c & (kCellsPerAxis - 1)));
+	}
+	const unsigned peers = __match_any_sync(FULL, idx);
+	const int leader = __ffs(peers) - 1;
+	uint32_t first = 0;
+	if (j < lb.M && (int)(threadIdx.x & 31) == leader) first = atomicAdd(&count[idx], (uint32_t)__popc(peers));
+	first = __shfl_sync(FULL, first, leader);
+	if (j < lb.M) place[j] = make_uint2(idx, first + (uint32_t)__popc(peers & lanemask_lt()));
+}
+
+// records in cell order: the position relative to the node's minimum corner in
+// FP32 and the sorted position; the cell; for poisson_average the colour
+__global__ void cell_scatter_kernel(const LevelNode* __restrict__ nodes, PosParamsS pp, LevelBuffers lb, const uint32_t* __restrict__ cell,
+                                    const uint2* __restrict__ place, LevelCells lc) {
 	const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
 	if (j >= lb.M) return;
 	const LevelNode& nd = nodes[lb.node_of[j]];
-	const uint32_t u = cvals[j];
-	int4 r = lb.cq[nd.cand_off + u];
-	r.w = (int32_t)u;
-	crec[j] = r;
-	crf[j] = make_float4((float)(qcoord(r.x, 0, pp) - nd.min[0]), (float)(qcoord(r.y, 1, pp) - nd.min[1]),
-	                     (float)(qcoord(r.z, 2, pp) - nd.min[2]), __int_as_float((int)u));
+	const uint2 pl = place[j];
+	const int64_t at = (int64_t)lc.start[pl.x] + pl.y;
+	const int4 r = lb.rec[j];
+	lc.rec[at] = make_float4((float)(qcoord(r.x, 0, pp) - nd.min[0]), (float)(qcoord(r.y, 1, pp) - nd.min[1]),
+	                         (float)(qcoord(r.z, 2, pp) - nd.min[2]), __int_as_float(lb.pos[j]));
+	lc.cell[at] = cell[j];
+	if (lc.col) lc.col[at] = lb.cols[j];
 }
 
-// occupancy bitmap of a node's cells: 128 bits per (z, y) row, 4 words
-constexpr int kRowWords = kCellsPerAxis / 32;
-constexpr int64_t kBitmapWords = (int64_t)kCellsPerAxis * kCellsPerAxis * kRowWords;
-constexpr int64_t kBitmapMinCandidates = 2048;  // smaller nodes probe the hash for every cell
-
-__global__ void conf_bitmap_kernel(const int32_t* __restrict__ node_of, const uint64_t* __restrict__ ck, int64_t M,
-                                   const int64_t* __restrict__ bm_off, uint32_t* __restrict__ bm) {
-	const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-	if (j >= M) return;
-	const int64_t off = bm_off[node_of[j]];
-	if (off < 0) return;
-	const uint64_t c = ck[j];
-	const int cx = (int)(c % kCellsPerAxis);
-	atomicOr(&bm[off + (int64_t)(c / kCellsPerAxis) * kRowWords + (cx >> 5)], 1u << (cx & 31));
-}
-
-__device__ __forceinline__ bool run_head(const LevelNode* nodes, const int32_t* node_of, const uint64_t* ck, int64_t j) {
-	return j == nodes[node_of[j]].cand_off || ck[j] != ck[j - 1];
-}
-
-// occupied cells (runs) per node
-__global__ void conf_count_runs_kernel(const LevelNode* __restrict__ nodes, const int32_t* __restrict__ node_of, const uint64_t* __restrict__ ck,
-                                       int64_t M, unsigned long long* __restrict__ node_runs) {
-	const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-	const bool h = j < M && run_head(nodes, node_of, ck, j);
-	const int32_t node = j < M ? node_of[j] : -1;
-	const unsigned peers = __match_any_sync(FULL, node);
-	const unsigned heads = __ballot_sync(FULL, h) & peers;
-	if (node >= 0 && heads && (int)(threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&node_runs[node], (unsigned long long)__popc(heads));
-}
-
-// run tables, one per node: cell -> (first record, count). A node's table
-// is its own region (tab_off, power-of-two tab_cap), so the probes of the
-// candidates in flight stay within the few nodes being searched and hit L2.
-__global__ void conf_insert_runs_kernel(const LevelNode* __restrict__ nodes, const uint8_t* __restrict__ use, const int32_t* __restrict__ node_of,
-                                        const uint64_t* __restrict__ ck, int64_t M, RunSlot* __restrict__ table,
-                                        const int64_t* __restrict__ tab_off, const int64_t* __restrict__ tab_cap, SampleStats* st) {
-	const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-	if (j >= M) return;
-	const int32_t node = node_of[j];
-	if (!use[node] || !run_head(nodes, node_of, ck, j)) return;
-	const int64_t end = nodes[node].cand_off + nodes[node].count;
-	int64_t e = j + 1;
-	while (e < end && ck[e] == ck[j]) e++;
-	const uint64_t key = ck[j];
-	RunSlot* tb = table + tab_off[node];
-	const int64_t cap = tab_cap[node];
-	uint64_t s = run_hash(key, cap);
-	for (int64_t probe = 0; probe < cap; probe++) {
-		const unsigned long long prev = atomicCAS((unsigned long long*)&tb[s].key, (unsigned long long)kEmptyRun, (unsigned long long)key);
-		if (prev == kEmptyRun) {
-			tb[s].start = (int32_t)(j - nodes[node].cand_off);
-			tb[s].count = (int32_t)(e - j);
-			return;
-		}
-		s = (s + 1) & (uint64_t)(cap - 1);
-	}
-	atomicAdd(&st->timeouts, 1ull);
-}
-
-__device__ __forceinline__ int2 find_run(const RunSlot* table, int64_t cap, uint64_t key) {
-	uint64_t s = run_hash(key, cap);
-	for (int64_t probe = 0; probe < cap; probe++) {
-		const RunSlot r = table[s];
-		if (r.key == key) return make_int2(r.start, r.count);
-		if (r.key == kEmptyRun) break;
-		s = (s + 1) & (uint64_t)(cap - 1);
-	}
-	return make_int2(0, 0);
-}
-
-// The search waits on dependent loads (bitmap row, run table, runs) and is
-// near its issue limit: MINB resident blocks of 256 threads per SM (5: 48
-// registers, 4: 64), GAPS skips the neighbour cells beyond the band. The
-// variant is chosen by lists_variant() (measured; PCG_LISTS overrides).
-template <int MODE, int MINB, bool GAPS>
-__global__ void __launch_bounds__(256, MINB) conf_lists_kernel(const LevelNode* __restrict__ nodes, const uint8_t* __restrict__ use, PosParamsS pp,
-                                                        LevelBuffers lb, const uint64_t* __restrict__ ck, const int4* __restrict__ crec,
-                                                        const float4* __restrict__ crf, const RunSlot* __restrict__ table,
-                                                        const int64_t* __restrict__ tab_off, const int64_t* __restrict__ tab_cap,
-                                                        const int64_t* __restrict__ bm_off, const uint32_t* __restrict__ bm,
-                                                        ConflictLists cl, SampleStats* st) {
-	const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-	if (j >= lb.M) return;
-	const int32_t node = lb.node_of[j];
-	if (!use[node]) return;
-	const LevelNode& nd = nodes[node];
-	const int64_t co = nd.cand_off;
-	const float4 mf = crf[j];
-	const int32_t t = __float_as_int(mf.w);
-	const double sp = nd.spacing, s2 = sp * sp;
-	double lim = 0.0;
-	if (MODE == 0) {
-		// the early-exit bound of the acceptance kernels, same expression
-		const double cd = sqrt(lb.keys[co + t]);
-		const double limit = cd - sp;
-		lim = limit * limit;
-	}
-	// node-relative FP32 coordinates: error far below the 1e-3 margin on s^2
-	// (the bound on its error, derived for node-relative coordinates below
-	// 128 spacings, holds while the FP64 coordinates themselves carry a
-	// rounding error far below the spacing: |coordinate| < 1e6 spacings)
-	double amax = 0.0;
-	for (int a = 0; a < 3; a++) amax = fmax(amax, fmax(fabs(nd.min[a]), fabs(nd.max[a])));
-	const bool pre32 = s2 > 1e-30 && s2 < 1e30 && amax < 1e6 * sp;
-	const float s2hi = (float)(s2 * 1.001), s2lo = (float)(s2 * 0.999);
-	unsigned escalated = 0;  // pairs inside the band, decided in FP64
-	const uint64_t c = ck[j];
-	const int cx = (int)(c % kCellsPerAxis), cy = (int)((c / kCellsPerAxis) % kCellsPerAxis), cz = (int)(c / (kCellsPerAxis * kCellsPerAxis));
-	// the first kListInline entries go to the candidate's own slot (positions
-	// past the list read as 0); the rest (rare) wait in a per-thread array
-	// and take exactly their room in the pool once the search is done
-	int32_t* inl = reinterpret_cast<int32_t*>(cl.inl + co + t);
-	cl.inl[co + t] = make_int4(0, 0, 0, 0);
-	int32_t rest[kListCap - kListInline];
+// The runs of records around cell c of a node (rows, base: the node's; co: its
+// cand_off): up to nine, written to runs[0], runs[stride], ... as [first, end).
+// Returns how many.
+__device__ __forceinline__ int find_runs(uint32_t c, uint32_t co, const uint4* __restrict__ rows, const uint32_t* __restrict__ base,
+                                         const uint32_t* __restrict__ start, uint2* runs, int stride) {
+	const int cx = (int)(c & (kCellsPerAxis - 1)), cy = (int)(c >> kAxisBits & (kCellsPerAxis - 1)), cz = (int)(c >> (2 * kAxisBits));
+	const int x0 = cx > 0 ? cx - 1 : 0, x1 = cx + 1 < kCellsPerAxis ? cx + 1 : cx;
 	int n = 0;
-	const int64_t boff = bm_off[node];
-	const RunSlot* tb = table + tab_off[node];
-	const int64_t cap = tab_cap[node];
-	// gaps from the candidate to the faces it shares with the cells below
-	// and above it on each axis: a neighbour cell whose nearest point is
-	// at least the band's upper edge away holds no pair (with the
-	// prefilter's margin over the FP32 error; nodes without the prefilter
-	// visit every cell)
-	const float cs = (float)(sp * 1.000001);
-	auto gap2 = [&](int d, float v, int c) {
-		const float g = d < 0 ? v - (float)c * cs : (float)(c + 1) * cs - v;
-		return GAPS && pre32 && d != 0 && g > 0.f ? g * g : 0.f;
-	};
-#pragma unroll 1
-	for (int dz = -1; dz <= 1; dz++) {
-		const int qz = cz + dz;
-		if (qz < 0 || qz >= kCellsPerAxis) continue;
-		const float dz2 = gap2(dz, mf.z, cz);
-		if (dz2 >= s2hi) continue;
-#pragma unroll 1
-		for (int dy = -1; dy <= 1; dy++) {
-			const int qy = cy + dy;
-			if (qy < 0 || qy >= kCellsPerAxis) continue;
-			const float dzy2 = dz2 + gap2(dy, mf.y, cy);
-			if (dzy2 >= s2hi) continue;
-			// occupied cells among x = cx-1 .. cx+1 of this row
-			uint32_t occ = 7u;
-			if (boff >= 0) {
-				const uint32_t* row = bm + boff + ((int64_t)qz * kCellsPerAxis + qy) * kRowWords;
-				const int x0 = cx - 1;
-				occ = 0;
-				for (int b = 0; b < 3; b++) {
-					const int qx = x0 + b;
-					if (qx >= 0 && qx < kCellsPerAxis && ((row[qx >> 5] >> (qx & 31)) & 1u)) occ |= 1u << b;
-				}
-			}
-			for (int dx = -1; dx <= 1; dx++) {
-				const int qx = cx + dx;
-				if (qx < 0 || qx >= kCellsPerAxis || !((occ >> (dx + 1)) & 1u)) continue;
-				if (dzy2 + gap2(dx, mf.x, cx) >= s2hi) continue;
-				const uint64_t cell = ((uint64_t)qz * kCellsPerAxis + (uint64_t)qy) * kCellsPerAxis + (uint64_t)qx;
-				const int2 run = find_run(tb, cap, cell);
-				const int4* rp = crec + co + run.x;
-				const float4* rf = crf + co + run.x;
-				for (int i = 0; i < run.y; i++) {
-					const float4 qf = rf[i];
-					const int32_t u = __float_as_int(qf.w);
-					if (u >= t) break;  // a cell's records are in sorted order: only earlier candidates
-					bool inside = false;
-					if (pre32) {
-						// FP32 decides outside the band s^2 (1 -/+ 1e-3), well clear
-						// of its rounding error; pairs in the band go to FP64
-						const float fx = qf.x - mf.x, fy = qf.y - mf.y, fz = qf.z - mf.z;
-						const float d2 = fx * fx + fy * fy + fz * fz;
-						if (d2 >= s2hi) continue;
-						inside = d2 < s2lo;
-					}
-					if (!inside) {
-						// the FP64 positions are recomputed here, not held in
-						// registers through the search (pairs in the band are rare)
-						const int4 q = rp[i];
-						const int4 me = crec[j];
-						const double ax = qcoord(q.x, 0, pp), ay = qcoord(q.y, 1, pp), az = qcoord(q.z, 2, pp);
-						const double x = qcoord(me.x, 0, pp), y = qcoord(me.y, 1, pp), z = qcoord(me.z, 2, pp);
-						// squaredDistance(point, candidate), sampler_poisson.h:117-125
-						const double dx_ = ax - x, dy_ = ay - y, dz_ = az - z;
-						escalated++;
-						if (!(dx_ * dx_ + dy_ * dy_ + dz_ * dz_ < s2)) continue;
-					}
-					if (MODE == 0 && !(lb.keys[co + u] >= lim)) continue;
-					if (n < kListInline) inl[n] = u;
-					else if (n < kListCap) rest[n - kListInline] = u;
-					n++;
-				}
+#pragma unroll
+	for (int q = 0; q < 9; q++) {
+		const int y = cy + q % 3 - 1, z = cz + q / 3 - 1;
+		if (y >= 0 && y < kCellsPerAxis && z >= 0 && z < kCellsPerAxis) {
+			const int row = z << kAxisBits | y;
+			const uint4 b = rows[row];
+			// the occupied ones among x0 .. x1
+			const int w = x0 >> 5;
+			const uint32_t lo = w == 0 ? b.x : w == 1 ? b.y : w == 2 ? b.z : b.w;
+			const uint32_t up = w == 0 ? b.y : w == 1 ? b.z : w == 2 ? b.w : 0u;
+			const uint32_t bits = __funnelshift_r(lo, up, x0 & 31) & ((2u << (x1 - x0)) - 1);
+			if (bits) {
+				const uint32_t first = co + base[row] + (uint32_t)row_rank(b, x0);
+				runs[n * stride] = make_uint2(start[first], start[first + __popc(bits)]);
+				n++;
 			}
 		}
 	}
-	bool dense = n > kListCap;
-	if (!dense && n > kListInline) {
-		const int extra = n - kListInline;
-		const unsigned long long at = atomicAdd(cl.pool_used, (unsigned long long)extra);
-		if ((int64_t)(at + extra) <= cl.pool_cap) {
-			cl.ovf_off[co + t] = (int32_t)at;
-			for (int e = 0; e < extra; e++) cl.pool[at + e] = rest[e];
-		} else {
-			dense = true;  // the pool is full: the level builds its lists again with a larger pool
+	return n;
+}
+
+// What a candidate p is compared with: whether a record q could reject it.
+template <int MODE>
+struct PairTest {
+	float4 mf;
+	int32_t t;
+	double s2, lim;
+	float s2hi, s2lo;
+	bool pre32, far_from_centre;
+	int64_t co;
+	unsigned escalated;
+
+	__device__ __forceinline__ PairTest(const LevelNode& nd, const LevelBuffers& lb, const float4& rec) {
+		mf = rec;
+		t = __float_as_int(rec.w);
+		co = nd.cand_off;
+		const double sp = nd.spacing;
+		s2 = sp * sp;
+		lim = 0.0;
+		far_from_centre = true;
+		if (MODE == 0) {
+			// the early-exit bound of the acceptance kernels, same expression
+			const double cd = sqrt(lb.keys[co + t]);
+			const double limit = cd - sp;
+			lim = limit * limit;
+			far_from_centre = cd > 1.1 * sp;
+		}
+		double amax = 0.0;
+		for (int a = 0; a < 3; a++) amax = fmax(amax, fmax(fabs(nd.min[a]), fabs(nd.max[a])));
+		pre32 = s2 > 1e-30 && s2 < 1e30 && amax < 1e6 * sp;
+		s2hi = (float)(s2 * 1.001);
+		s2lo = (float)(s2 * 0.999);
+		escalated = 0;
+	}
+	// squaredDistance(point, candidate), sampler_poisson.h:117-125
+	__device__ __forceinline__ bool exact(const LevelBuffers& lb, const PosParamsS& pp, int32_t u) const {
+		const int4 q = lb.rec[co + lb.perm[co + u]], me = lb.rec[co + lb.perm[co + t]];
+		const double dx = qcoord(q.x, 0, pp) - qcoord(me.x, 0, pp), dy = qcoord(q.y, 1, pp) - qcoord(me.y, 1, pp),
+		             dz = qcoord(q.z, 2, pp) - qcoord(me.z, 2, pp);
+		return dx * dx + dy * dy + dz * dz < s2;
+	}
+	// the record's sorted position is u < t
+	__device__ __forceinline__ bool operator()(const float4& qf, int32_t u, const LevelBuffers& lb, const PosParamsS& pp) {
+		const float fx = qf.x - mf.x, fy = qf.y - mf.y, fz = qf.z - mf.z;
+		const float d2 = fx * fx + fy * fy + fz * fz;
+		if (pre32 && d2 >= s2hi) return false;
+		const bool inside = pre32 && d2 < s2lo;
+		if (!inside) {
+			escalated++;
+			if (!exact(lb, pp, u)) return false;
+		}
+		if (MODE == 0 && !(inside && far_from_centre) && !(lb.keys[co + u] >= lim)) return false;
+		return true;
+	}
+};
+
+// One thread per record in cell order; a thread's runs wait in shared memory.
+template <int MODE>
+__global__ void __launch_bounds__(256, 5) conf_lists_kernel(const LevelNode* __restrict__ nodes, PosParamsS pp, LevelBuffers lb, LevelCells lc,
+                                                            ConflictLists cl, SampleStats* st) {
+	__shared__ uint2 runs[9][256];
+	const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+	const int lane = threadIdx.x & 31;
+	unsigned escalated = 0;
+	int n = 0;
+	bool distant = false;
+	int64_t slot = 0;
+	int32_t rest[kListCap - kListInline];
+	if (i < lb.M) {
+		const int32_t node = lb.node_of[i];  // a node's records keep its range
+		const LevelNode& nd = nodes[node];
+		const int64_t co = nd.cand_off;
+		const int nr = find_runs(lc.cell[i], (uint32_t)co, lc.rows + (int64_t)node * kRows, lc.base + (int64_t)node * kRows, lc.start,
+		                         &runs[0][threadIdx.x], 256);
+		PairTest<MODE> test(nd, lb, lc.rec[i]);
+		const int32_t t = test.t;
+		int4 inl = make_int4(0, 0, 0, 0);
+#pragma unroll 1
+		for (int q = 0; q < nr; q++) {
+			const uint2 run = runs[q][threadIdx.x];
+#pragma unroll 2
+			for (uint32_t k = run.x; k < run.y; k++) {
+				const float4 qf = lc.rec[k];
+				const int32_t u = __float_as_int(qf.w);
+				if (u >= t || !test(qf, u, lb, pp)) continue;
+				if (n == 0) inl.x = u;
+				else if (n == 1) inl.y = u;
+				else if (n == 2) inl.z = u;
+				else if (n == 3) inl.w = u;
+				else if (n < kListCap) rest[n - kListInline] = u;
+				n++;
+				if (MODE == 0) distant |= t - u > 10001;
+			}
+		}
+		slot = co + t;
+		cl.inl[slot] = inl;
+		cl.count[slot] = (uint8_t)(n > kListCap ? kListLong : n | (distant ? kListDistant : 0));
+		escalated = test.escalated;
+		if (n > kListCap) {
+			const unsigned long long at = atomicAdd(cl.long_used, 1ull);
+			const unsigned long long off = atomicAdd(cl.long_entries, (unsigned long long)n);
+			atomicAdd(cl.node_long + node, (unsigned long long)n);
+			if ((int64_t)at < cl.long_cap) {
+				cl.longs[at] = LongList{(int64_t)off, (int32_t)i, n};
+				cl.ovf_off[slot] = (int32_t)at;
+			}
 		}
 	}
-	cl.count[co + t] = (uint8_t)(dense ? kListDense : n);
-	if (dense) cl.node_dense[node] = 1;
-	const unsigned active = __activemask();
-	const unsigned sum = __reduce_add_sync(active, (unsigned)(dense ? 0 : n));
-	const unsigned esc = __reduce_add_sync(active, escalated);
-	if ((int)(threadIdx.x & 31) == __ffs(active) - 1) {
-		atomicAdd(&st->list_entries, (unsigned long long)sum);
-		if (esc) atomicAdd(&st->escalated, (unsigned long long)esc);
+	// room in the pool for the warp's lists at once
+	const uint32_t extra = n > kListInline && n <= kListCap ? (uint32_t)(n - kListInline) : 0u;
+	if (__any_sync(FULL, extra != 0)) {
+		uint32_t x = extra;
+#pragma unroll
+		for (int o = 1; o < 32; o <<= 1) {
+			const uint32_t y = __shfl_up_sync(FULL, x, o);
+			if (lane >= o) x += y;
+		}
+		unsigned long long at = 0;
+		if (lane == 31) at = atomicAdd(cl.pool_used, (unsigned long long)x);
+		at = __shfl_sync(FULL, at, 31) + x - extra;
+		if (extra && (int64_t)(at + extra) <= cl.pool_cap) {
+			cl.ovf_off[slot] = (int32_t)at;
+			for (uint32_t e = 0; e < extra; e++) cl.pool[at + e] = rest[e];
+		}
+	}
+	const unsigned entries = __reduce_add_sync(FULL, (unsigned)n);
+	escalated = __reduce_add_sync(FULL, escalated);
+	if (lane == 0) {
+		if (entries) atomicAdd(&st->list_entries, (unsigned long long)entries);
+		if (escalated) atomicAdd(&st->escalated, (unsigned long long)escalated);
 	}
 }
 
-// 0: five blocks per SM with the cell skip, 1: four blocks with it, 2: five
-// blocks without it; PCG_LISTS=<n> overrides the measured default
-int lists_variant() {
-	static const int v = [] {
-		const char* e = std::getenv("PCG_LISTS");
-		return e ? std::atoi(e) : kListsVariant;
-	}();
-	return v;
+// the entries of the long lists, one warp each
+template <int MODE>
+__global__ void __launch_bounds__(128) conf_long_kernel(const LevelNode* __restrict__ nodes, PosParamsS pp, LevelBuffers lb, LevelCells lc,
+                                                        ConflictLists cl, const uint8_t* __restrict__ dense, int64_t num) {
+	__shared__ uint2 runs[9][128];
+	const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+	const int lane = threadIdx.x & 31;
+	if (w >= num) return;
+	const LongList l = cl.longs[w];
+	const int64_t i = l.record;
+	const int32_t node = lb.node_of[i];
+	if (dense[node]) return;
+	const LevelNode& nd = nodes[node];
+	const int nr = find_runs(lc.cell[i], (uint32_t)nd.cand_off, lc.rows + (int64_t)node * kRows, lc.base + (int64_t)node * kRows, lc.start,
+	                         &runs[0][threadIdx.x], 128);
+	PairTest<MODE> test(nd, lb, lc.rec[i]);
+	int32_t* out = cl.long_pool + l.off;
+	int n = 0;
+#pragma unroll 1
+	for (int q = 0; q < nr; q++) {
+		const uint2 run = runs[q][threadIdx.x];  // the same for every lane
+		for (uint32_t k0 = run.x; k0 < run.y; k0 += 32) {
+			const uint32_t k = k0 + lane;
+			bool hit = false;
+			int32_t u = 0;
+			if (k < run.y) {
+				const float4 qf = lc.rec[k];
+				u = __float_as_int(qf.w);
+				hit = u < test.t && test(qf, u, lb, pp);
+			}
+			const unsigned hits = __ballot_sync(FULL, hit);
+			const int at = n + __popc(hits & lanemask_lt());
+			if (hit && at < l.count) out[at] = u;
+			n += __popc(hits);
+		}
+	}
+}
+
+// places of the long lists of the nodes that keep them, from 0 on again
+__global__ void long_places_kernel(LevelBuffers lb, ConflictLists cl, const uint8_t* __restrict__ dense, int64_t num,
+                                   unsigned long long* __restrict__ next) {
+	const int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+	if (w >= num || dense[lb.node_of[cl.longs[w].record]]) return;
+	cl.longs[w].off = (int64_t)atomicAdd(next, (unsigned long long)cl.longs[w].count);
+}
+
+constexpr int kCompact = 256;
+
+// records of accepted candidates of the nodes that are not dense
+__global__ void __launch_bounds__(kCompact) accepted_records_kernel(const LevelNode* __restrict__ nodes, const uint8_t* __restrict__ dense, LevelBuffers lb,
+                                                                    LevelCells lc, const uint32_t* __restrict__ accepted_bits,
+                                                                    uint32_t* __restrict__ list, unsigned int* __restrict__ num) {
+	__shared__ uint32_t sums[kCompact / 32], first;
+	const int64_t i = (int64_t)blockIdx.x * kCompact + threadIdx.x;
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	bool acc = false;
+	if (i < lb.M) {
+		const int32_t node = lb.node_of[i];
+		const int32_t t = __float_as_int(lc.rec[i].w);
+		if (!(dense && dense[node])) acc = accepted_bits[accept_word(nodes[node].cand_off, node) + (t >> 5)] >> (t & 31) & 1;
+	}
+	const uint32_t votes = __ballot_sync(FULL, acc);
+	if (lane == 0) sums[warp] = (uint32_t)__popc(votes);
+	__syncthreads();
+	if (threadIdx.x == 0) {
+		uint32_t total = 0;
+		for (int w = 0; w < kCompact / 32; w++) {
+			const uint32_t c = sums[w];
+			sums[w] = total;
+			total += c;
+		}
+		first = total ? atomicAdd(num, total) : 0u;
+	}
+	__syncthreads();
+	if (acc) list[first + sums[warp] + (uint32_t)__popc(votes & lanemask_lt())] = (uint32_t)i;
+}
+
+// poisson_average's colours (sampler_poisson_average.h:357-416) in closed
+// form: every rejected candidate adds its colour to each accepted point within
+// the spacing, twice when it precedes that point in sorted order (the
+// reference doubles an accepted point's running sum when its own turn comes),
+// and every accepted point adds twice its own colour. A thread per accepted
+// point sums over the records around it (no two accepted points lie within
+// the spacing); colours lie in cell order, beside the records. Bound by the
+// records and colours read; scattered atomics from the rejected side through
+// a hash of the accepted points took 4.04 ms for 31M candidates, this 2.25.
+__global__ void __launch_bounds__(128) cell_colors_kernel(const LevelNode* __restrict__ nodes, PosParamsS pp, LevelBuffers lb, LevelCells lc,
+                                                          const uint32_t* __restrict__ list, const unsigned int* __restrict__ num) {
+	__shared__ uint2 runs[9][128];
+	for (uint32_t a = blockIdx.x * 128 + threadIdx.x; a < *num; a += gridDim.x * 128) {
+		const int64_t i = list[a];
+		const int32_t node = lb.node_of[i];
+		const LevelNode& nd = nodes[node];
+		const int64_t co = nd.cand_off;
+		const int nr = find_runs(lc.cell[i], (uint32_t)co, lc.rows + (int64_t)node * kRows, lc.base + (int64_t)node * kRows, lc.start,
+		                         &runs[0][threadIdx.x], 128);
+		PairTest<1> test(nd, lb, lc.rec[i]);
+		unsigned long long r = 0, g = 0, b = 0, w = 0;
+		auto add = [&](uint64_t col, unsigned f) {
+			r += (unsigned long long)(f * (uint32_t)(col & 0xffff));
+			g += (unsigned long long)(f * (uint32_t)(col >> 16 & 0xffff));
+			b += (unsigned long long)(f * (uint32_t)(col >> 32 & 0xffff));
+			w += f;
+		};
+		add(lc.col[i], 2);
+#pragma unroll 1
+		for (int q = 0; q < nr; q++) {
+			const uint2 run = runs[q][threadIdx.x];
+			for (uint32_t k = run.x; k < run.y; k++) {
+				const float4 qf = lc.rec[k];
+				const int32_t u = __float_as_int(qf.w);
+				if (u != test.t && test(qf, u, lb, pp)) add(lc.col[k], u < test.t ? 2u : 1u);
+			}
+		}
+		// rgbTarget = p.r / p.w (sampler_poisson_average.h:443-445)
+		lb.cols[co + lb.perm[co + test.t]] = (uint64_t)(uint16_t)(r / w) | (uint64_t)(uint16_t)(g / w) << 16 | (uint64_t)(uint16_t)(b / w) << 32;
+	}
 }
 
 // st += the list build's own counters
 __global__ void add_list_stats_kernel(SampleStats* st, const SampleStats* lst) {
 	atomicAdd(&st->list_entries, lst->list_entries);
 	atomicAdd(&st->escalated, lst->escalated);
-	atomicAdd(&st->timeouts, lst->timeouts);
 }
 
 }  // namespace
 
-void build_conflict_lists(int mode, const LevelNode* d_nodes, const std::vector<LevelNode>& ln, const std::vector<uint8_t>& use,
-                          const PosParamsS& pp, LevelBuffers& lb, ConflictLists& cl, std::vector<uint8_t>& dense, SampleStats* st,
-                          DeviceMem& mem) {
-	const int K = (int)ln.size();
+void build_level_cells(const LevelNode* d_nodes, const PosParamsS& pp, LevelBuffers& lb, LevelCells& lc, DeviceMem& mem) {
+	const int64_t M = lb.M;
+	if (M >= (int64_t(1) << 32)) throw PcgError(5, "more candidates in a level than the cell index holds");
+	cudaStream_t s = mem.stream();
+	const unsigned blocks = (unsigned)ceil_div(M, 256);
+	const int64_t rows = (int64_t)lb.K * kRows;
+	lc.rows = mem.alloc<uint4>(rows);
+	lc.base = mem.alloc<uint32_t>(rows);
+	lc.start = mem.alloc<uint32_t>(M + 1);
+	lc.rec = mem.alloc<float4>(M);
+	lc.cell = mem.alloc<uint32_t>(M);
+	lc.col = lb.cols ? mem.alloc<uint64_t>(M) : nullptr;
+	uint32_t* cell = mem.alloc<uint32_t>(M);
+	uint32_t* count = mem.alloc<uint32_t>(M);
+	uint2* place = mem.alloc<uint2>(M);
+	PCG_CUDA(cudaMemsetAsync(lc.rows, 0, rows * sizeof(uint4), s));
+	PCG_CUDA(cudaMemsetAsync(count, 0, M * sizeof(uint32_t), s));
+	cell_mark_kernel<<<blocks, 256, 0, s>>>(d_nodes, pp, lb, cell, reinterpret_cast<uint32_t*>(lc.rows));
+	PCG_LAUNCHED();
+	row_base_kernel<<<(unsigned)lb.K, kRowThreads, 0, s>>>(lc.rows, lc.base);
+	PCG_LAUNCHED();
+	cell_count_kernel<<<blocks, 256, 0, s>>>(d_nodes, lb, cell, lc.rows, lc.base, count, place);
+	PCG_LAUNCHED();
+	exclusive_scan_u32(count, lc.start, M, true, mem);
+	cell_scatter_kernel<<<blocks, 256, 0, s>>>(d_nodes, pp, lb, cell, place, lc);
+	PCG_LAUNCHED();
+	mem.free(place);
+	mem.free(count);
+	mem.free(cell);
+}
+
+void free_level_cells(LevelCells& lc, DeviceMem& mem) {
+	if (lc.rows) mem.free(lc.rows);
+	if (lc.base) mem.free(lc.base);
+	if (lc.start) mem.free(lc.start);
+	if (lc.rec) mem.free(lc.rec);
+	if (lc.cell) mem.free(lc.cell);
+	if (lc.col) mem.free(lc.col);
+	lc = LevelCells{};
+}
+
+void build_conflict_lists(int mode, const LevelNode* d_nodes, int K, const PosParamsS& pp, LevelBuffers& lb, const LevelCells& lc,
+                          ConflictLists& cl, std::vector<uint8_t>& dense, SampleStats* st, DeviceMem& mem) {
 	const int64_t M = lb.M;
 	dense.assign(K, 0);
 	if (M == 0 || K == 0) return;
 	cudaStream_t s = mem.stream();
 	const unsigned blocks = (unsigned)ceil_div(M, 256);
-	uint64_t* keys = mem.alloc<uint64_t>(M);
-	conf_cell_keys_kernel<<<blocks, 256, 0, s>>>(d_nodes, pp, lb, keys);
-	PCG_LAUNCHED();
-	uint64_t* ck = mem.alloc<uint64_t>(M);
-	uint32_t* cv = mem.alloc<uint32_t>(M);
-	segmented_sort_pairs(ln, M, keys, nullptr, ck, cv, 0, 21, mem);
-	mem.free(keys);
-	int4* crec = mem.alloc<int4>(M);
-	float4* crf = mem.alloc<float4>(M);
-	conf_gather_kernel<<<blocks, 256, 0, s>>>(d_nodes, pp, lb, cv, crec, crf);
-	PCG_LAUNCHED();
-	mem.free(cv);
-	unsigned long long* d_runs = mem.alloc<unsigned long long>(K);
-	PCG_CUDA(cudaMemsetAsync(d_runs, 0, K * sizeof(unsigned long long), s));
-	conf_count_runs_kernel<<<blocks, 256, 0, s>>>(d_nodes, lb.node_of, ck, M, d_runs);
-	PCG_LAUNCHED();
-	std::vector<unsigned long long> runs(K);
-	PCG_CUDA(cudaMemcpyAsync(runs.data(), d_runs, K * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-	PCG_CUDA(cudaStreamSynchronize(s));
-	mem.free(d_runs);
-	// per-node tables at most half full
-	std::vector<int64_t> tab(2 * (size_t)K, 0);  // offsets, then capacities
-	int64_t slots = 0;
-	for (int k = 0; k < K; k++) {
-		int64_t cap = 0;
-		if (use[k] && runs[k] > 0) {
-			cap = 16;
-			while (cap < 2 * (int64_t)runs[k]) cap <<= 1;
-		}
-		tab[k] = slots;
-		tab[K + k] = cap;
-		slots += cap;
-	}
-	int64_t* d_tab = mem.alloc<int64_t>(2 * (size_t)K);
-	PCG_CUDA(cudaMemcpyAsync(d_tab, tab.data(), tab.size() * sizeof(int64_t), cudaMemcpyHostToDevice, s));
-	const int64_t* tab_off = d_tab;
-	const int64_t* tab_cap = d_tab + K;
-	RunSlot* table = mem.alloc<RunSlot>(slots > 0 ? slots : 1);
-	if (slots > 0) PCG_CUDA(cudaMemsetAsync(table, 0xff, slots * sizeof(RunSlot), s));
-	uint8_t* d_use = mem.alloc<uint8_t>(K);
-	PCG_CUDA(cudaMemcpyAsync(d_use, use.data(), K, cudaMemcpyHostToDevice, s));
-	conf_insert_runs_kernel<<<blocks, 256, 0, s>>>(d_nodes, d_use, lb.node_of, ck, M, table, tab_off, tab_cap, st);
-	PCG_LAUNCHED();
-	// occupancy bitmaps of the larger nodes
-	std::vector<int64_t> bm_off(K, -1);
-	int64_t bm_words = 0;
-	for (int k = 0; k < K; k++)
-		if (use[k] && ln[k].count >= kBitmapMinCandidates) { bm_off[k] = bm_words; bm_words += kBitmapWords; }
-	int64_t* d_bm_off = mem.alloc<int64_t>(K);
-	PCG_CUDA(cudaMemcpyAsync(d_bm_off, bm_off.data(), K * sizeof(int64_t), cudaMemcpyHostToDevice, s));
-	uint32_t* bm = mem.alloc<uint32_t>(bm_words > 0 ? bm_words : 1);
-	if (bm_words > 0) {
-		PCG_CUDA(cudaMemsetAsync(bm, 0, bm_words * sizeof(uint32_t), s));
-		conf_bitmap_kernel<<<blocks, 256, 0, s>>>(lb.node_of, ck, M, d_bm_off, bm);
-		PCG_LAUNCHED();
-	}
 	cl.inl = mem.alloc<int4>(M);
 	cl.ovf_off = mem.alloc<int32_t>(M);
-	// entries past the inline ones: room for 8 more per candidate on
-	// average (lists average about one entry; the top levels' dense nodes
-	// need more than 4). When the lists need more, the build runs again
-	// with a pool of the exact size they asked for. A pool the device cannot
-	// hold is made smaller: the candidates it cannot take mark their nodes
-	// dense, which keep the lookup kernels.
-	auto alloc_pool = [&](int64_t want) {
-		int64_t cap = std::max<int64_t>(want, 1);
-		while (true) {
-			try {
-				cl.pool = mem.alloc<int32_t>(cap);
-				cl.pool_cap = cap;
-				return;
-			} catch (const PcgError& e) {
-				if (e.status != 3 || cap <= 4096) throw;  // 3: PCG_OOM
-				cap /= 2;
-			}
-		}
-	};
-	alloc_pool(std::min<int64_t>((int64_t)M * 2 * kListInline, (int64_t)INT32_MAX));
-	cl.pool_used = mem.alloc<unsigned long long>(1);
 	cl.count = mem.alloc<uint8_t>(M);
-	cl.node_dense = mem.alloc<uint8_t>(K);
+	// room for 8 pooled entries per candidate (lists average about one entry)
+	// and one long list in 16; a level that needs more is searched again with
+	// the room it asked for
+	unsigned long long* used = mem.alloc<unsigned long long>(3 + (size_t)K);
+	cl.pool_used = used;
+	cl.long_used = used + 1;
+	cl.long_entries = used + 2;
+	cl.node_long = used + 3;
+	cl.pool_cap = std::min<int64_t>(M * 2 * kListInline, (int64_t)INT32_MAX);
+	cl.long_cap = std::min<int64_t>(M, M / 16 + 4096);
+	cl.pool = mem.alloc<int32_t>(cl.pool_cap);
+	cl.longs = mem.alloc<LongList>(cl.long_cap);
 	SampleStats* lst = mem.alloc<SampleStats>(1);
+	std::vector<unsigned long long> h(3 + (size_t)K);
 	for (int attempt = 0; attempt < 2; attempt++) {
-		PCG_CUDA(cudaMemsetAsync(cl.pool_used, 0, sizeof(unsigned long long), s));
-		PCG_CUDA(cudaMemsetAsync(cl.node_dense, 0, K, s));
+		PCG_CUDA(cudaMemsetAsync(used, 0, (3 + (size_t)K) * sizeof(unsigned long long), s));
 		PCG_CUDA(cudaMemsetAsync(lst, 0, sizeof(SampleStats), s));
-		auto run = [&](auto kernel) {
-			kernel<<<blocks, 256, 0, s>>>(d_nodes, d_use, pp, lb, ck, crec, crf, table, tab_off, tab_cap, d_bm_off, bm, cl, lst);
-		};
-		const int v = lists_variant();
-		if (mode == 0) {
-			if (v == 1) run(conf_lists_kernel<0, 4, true>);
-			else if (v == 2) run(conf_lists_kernel<0, 5, false>);
-			else run(conf_lists_kernel<0, 5, true>);
-		} else {
-			if (v == 1) run(conf_lists_kernel<1, 4, true>);
-			else if (v == 2) run(conf_lists_kernel<1, 5, false>);
-			else run(conf_lists_kernel<1, 5, true>);
-		}
+		if (mode == 0) conf_lists_kernel<0><<<blocks, 256, 0, s>>>(d_nodes, pp, lb, lc, cl, lst);
+		else conf_lists_kernel<1><<<blocks, 256, 0, s>>>(d_nodes, pp, lb, lc, cl, lst);
 		PCG_LAUNCHED();
-		unsigned long long used = 0;
-		PCG_CUDA(cudaMemcpyAsync(&used, cl.pool_used, sizeof(used), cudaMemcpyDeviceToHost, s));
+		PCG_CUDA(cudaMemcpyAsync(h.data(), used, h.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
 		PCG_CUDA(cudaStreamSynchronize(s));
-		if ((int64_t)used <= cl.pool_cap || attempt == 1 || (int64_t)used > (int64_t)INT32_MAX) break;
-		mem.free(cl.pool);
-		alloc_pool((int64_t)used);
+		if ((int64_t)h[0] > (int64_t)INT32_MAX) throw PcgError(3, "conflict lists of a level exceed 2^31 entries");
+		const bool fits = (int64_t)h[0] <= cl.pool_cap && (int64_t)h[1] <= cl.long_cap;
+		if (fits) break;
+		if (attempt == 1) throw PcgError(5, "conflict lists changed between two searches");
+		if ((int64_t)h[0] > cl.pool_cap) {
+			mem.free(cl.pool);
+			cl.pool_cap = (int64_t)h[0];
+			cl.pool = mem.alloc<int32_t>(cl.pool_cap);
+		}
+		if ((int64_t)h[1] > cl.long_cap) {
+			mem.free(cl.longs);
+			cl.long_cap = (int64_t)h[1];
+			cl.longs = mem.alloc<LongList>(cl.long_cap);
+		}
 	}
 	add_list_stats_kernel<<<1, 1, 0, s>>>(st, lst);
 	PCG_LAUNCHED();
-	PCG_CUDA(cudaMemcpyAsync(dense.data(), cl.node_dense, K, cudaMemcpyDeviceToHost, s));
-	PCG_CUDA(cudaStreamSynchronize(s));
+	if (h[1]) {
+		// past the budget the nodes with the most entries go to the lookup kernels
+		int64_t kept = (int64_t)h[2];
+		if (kept > kLongBudget) {
+			std::vector<int> order(K);
+			std::iota(order.begin(), order.end(), 0);
+			std::sort(order.begin(), order.end(), [&](int a, int b) { return h[3 + a] > h[3 + b]; });
+			for (int k : order) {
+				if (kept <= kLongBudget) break;
+				dense[k] = 1;
+				kept -= (int64_t)h[3 + k];
+			}
+		}
+		uint8_t* d_dense = mem.alloc<uint8_t>(K);
+		PCG_CUDA(cudaMemcpyAsync(d_dense, dense.data(), K, cudaMemcpyHostToDevice, s));
+		if ((int64_t)h[2] > kLongBudget) {
+			PCG_CUDA(cudaMemsetAsync(cl.long_entries, 0, sizeof(unsigned long long), s));
+			long_places_kernel<<<(unsigned)ceil_div((int64_t)h[1], 256), 256, 0, s>>>(lb, cl, d_dense, (int64_t)h[1], cl.long_entries);
+			PCG_LAUNCHED();
+		}
+		cl.long_pool = mem.alloc<int32_t>(std::max<int64_t>(kept, 1));
+		const unsigned lblocks = (unsigned)ceil_div((int64_t)h[1] * 32, 128);
+		if (mode == 0) conf_long_kernel<0><<<lblocks, 128, 0, s>>>(d_nodes, pp, lb, lc, cl, d_dense, (int64_t)h[1]);
+		else conf_long_kernel<1><<<lblocks, 128, 0, s>>>(d_nodes, pp, lb, lc, cl, d_dense, (int64_t)h[1]);
+		PCG_LAUNCHED();
+		mem.free(d_dense);
+	}
 	mem.free(lst);
-	mem.free(d_use);
-	mem.free(d_bm_off);
-	mem.free(bm);
-	mem.free(table);
-	mem.free(d_tab);
-	mem.free(crec);
-	mem.free(crf);
-	mem.free(ck);
+}
+
+void launch_cell_colors(const LevelNode* d_nodes, const std::vector<uint8_t>& dense, const PosParamsS& pp, LevelBuffers& lb,
+                        const LevelCells& lc, const uint32_t* accepted_bits, DeviceMem& mem) {
+	const int64_t M = lb.M;
+	if (M == 0) return;
+	cudaStream_t s = mem.stream();
+	uint8_t* d_dense = nullptr;
+	if (std::find(dense.begin(), dense.end(), 1) != dense.end()) {
+		d_dense = mem.alloc<uint8_t>(dense.size());
+		PCG_CUDA(cudaMemcpyAsync(d_dense, dense.data(), dense.size(), cudaMemcpyHostToDevice, s));
+	}
+	uint32_t* list = mem.alloc<uint32_t>(M);
+	unsigned int* num = mem.alloc<unsigned int>(1);
+	PCG_CUDA(cudaMemsetAsync(num, 0, sizeof(unsigned int), s));
+	accepted_records_kernel<<<(unsigned)ceil_div(M, kCompact), kCompact, 0, s>>>(d_nodes, d_dense, lb, lc, accepted_bits, list, num);
+	PCG_LAUNCHED();
+	// about a quarter of the candidates are accepted; the grid strides over the rest
+	cell_colors_kernel<<<(unsigned)ceil_div(M, 128 * 4), 128, 0, s>>>(d_nodes, pp, lb, lc, list, num);
+	PCG_LAUNCHED();
+	mem.free(num);
+	mem.free(list);
+	if (d_dense) mem.free(d_dense);
 }
 
 void free_conflict_lists(ConflictLists& cl, DeviceMem& mem) {
@@ -472,7 +634,8 @@ void free_conflict_lists(ConflictLists& cl, DeviceMem& mem) {
 	if (cl.pool) mem.free(cl.pool);
 	if (cl.pool_used) mem.free(cl.pool_used);
 	if (cl.count) mem.free(cl.count);
-	if (cl.node_dense) mem.free(cl.node_dense);
+	if (cl.longs) mem.free(cl.longs);
+	if (cl.long_pool) mem.free(cl.long_pool);
 	cl = ConflictLists{};
 }
 

@@ -1641,47 +1641,75 @@ struct Converter {
 		LevelNode* d_nodes = upload(ln, mem);
 		GatherItem* d_items = upload(items, mem);
 		launch_gather(items, d_items, lb, mem);
-		// node order for the warp-per-node kernels: largest first
-		std::vector<int32_t> order(K);
-		for (int k = 0; k < K; k++) order[k] = k;
-		std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return ln[a].count > ln[b].count; });
-		int32_t* d_order = upload(order, mem);
-		uint64_t* hkeys = mem.alloc<uint64_t>(H);
-		int32_t* hvals = mem.alloc<int32_t>(H);
 		if (method == PCG_RANDOM) {
+			uint64_t* hkeys = mem.alloc<uint64_t>(H);
+			int32_t* hvals = mem.alloc<int32_t>(H);
 			launch_random_accept_sized(d_nodes, co.X, co.Y, co.Z, pps, lb, hkeys, hvals, H, d_st, mem);
+			mem.free(hkeys);
+			mem.free(hvals);
 		} else {
 			lb.keys = mem.alloc<double>(M);
 			lb.perm = mem.alloc<int32_t>(M);
 			lb.pos = mem.alloc<int32_t>(M);
-			lb.acc_rank = mem.alloc<int32_t>(M);
-			lb.cq = mem.alloc<int4>(M);
 			launch_keys(d_nodes, pps, lb, mem);
-			double* axyz = mem.alloc<double>(3 * M);
-			double* akey = mem.alloc<double>(M);
-			int32_t* anext = mem.alloc<int32_t>(M);
-			int32_t* apos = mem.alloc<int32_t>(M);
 			const int mode = method == PCG_POISSON ? 0 : 1;
-			const bool guard = form == PCG_FORM_BATCHED;
-			// large nodes get a CTA each; on levels with few nodes every node
-			// of some size does, so the GPU is not left to a handful of warps
-			int num_big = 0;
+			// what the lookup kernels (plain form, dense nodes) work with
+			struct Lookup {
+				uint64_t* hkeys;
+				int32_t* hvals;
+				double *axyz, *akey;
+				int32_t *anext, *apos, *d_order;
+				long long* sums;
+			} lk{};
+			auto lookup_begin = [&](const std::vector<int32_t>& order) {
+				lb.acc_rank = mem.alloc<int32_t>(M);
+				lb.cq = mem.alloc<int4>(M);
+				lk.hkeys = mem.alloc<uint64_t>(H);
+				lk.hvals = mem.alloc<int32_t>(H);
+				lk.axyz = mem.alloc<double>(3 * M);
+				lk.akey = mem.alloc<double>(M);
+				lk.anext = mem.alloc<int32_t>(M);
+				lk.apos = mem.alloc<int32_t>(M);
+				lk.d_order = upload(order, mem);
+			};
+			auto lookup_end = [&](const uint8_t* only) {
+				if (method == PCG_POISSON_AVERAGE) {
+					lk.sums = mem.alloc<long long>(4 * M);
+					launch_average_colors(d_nodes, co.X, co.Y, co.Z, pps, lb, lk.hkeys, lk.hvals, lk.axyz, lk.anext, lk.apos, only, lk.sums, mem);
+					mem.free(lk.sums);
+				}
+				mem.free(lk.hkeys); mem.free(lk.hvals); mem.free(lk.axyz); mem.free(lk.akey); mem.free(lk.anext); mem.free(lk.apos);
+				mem.free(lk.d_order);
+				mem.free(lb.acc_rank); mem.free(lb.cq);
+			};
+			// node order for the lookup kernels: largest first; the large ones
+			// (on levels with few nodes every node of some size) get a CTA each
+			std::vector<int32_t> order(K);
+			for (int k = 0; k < K; k++) order[k] = k;
+			std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return ln[a].count > ln[b].count; });
 			const LevelSchedule sch = level_schedule();
 			const int64_t big_min = K < 2 * sms ? sch.small_level_cta_min : sch.cta_min;
-			while (num_big < K && ln[order[num_big]].count >= big_min) num_big++;
-			int list_nodes = 0;
-			cudaEvent_t ev_lists;
-			PCG_CUDA(cudaEventCreate(&ev_lists));
-			cudaEvent_t ev[3];
+			auto big_nodes = [&](const std::vector<int32_t>& o) {
+				int n = 0;
+				while (n < (int)o.size() && ln[o[n]].count >= big_min) n++;
+				return n;
+			};
+			int dense_nodes = 0;
+			cudaEvent_t ev[4];  // start, sorted, lists built, accepted
 			for (auto& e : ev) PCG_CUDA(cudaEventCreate(&e));
 			PCG_CUDA(cudaEventRecord(ev[0], s));
 			if (form == PCG_FORM_PLAIN) {
-				for (int k = 0; k < K; k++) launch_node_sort(d_nodes, d_order, K, lb, d_st, mem, k, k + 1, num_big);
+				lookup_begin(order);
+				const int num_big = big_nodes(order);
+				for (int k = 0; k < K; k++) launch_node_sort(d_nodes, lk.d_order, K, lb, d_st, mem, k, k + 1, num_big);
 				launch_cand_records(d_nodes, co.X, co.Y, co.Z, lb, mem);
 				PCG_CUDA(cudaEventRecord(ev[1], s));
+				PCG_CUDA(cudaEventRecord(ev[2], s));
 				for (int k = 0; k < K; k++)
-					launch_greedy(mode, false, d_nodes, d_order, K, co.X, co.Y, co.Z, pps, lb, hkeys, hvals, axyz, akey, anext, apos, d_st, mem, &grid_arena, k, k + 1,
-					              num_big);
+					launch_greedy(mode, false, d_nodes, lk.d_order, K, co.X, co.Y, co.Z, pps, lb, lk.hkeys, lk.hvals, lk.axyz, lk.akey, lk.anext,
+					              lk.apos, d_st, mem, &grid_arena, k, k + 1, num_big);
+				PCG_CUDA(cudaEventRecord(ev[3], s));
+				lookup_end(nullptr);
 			} else {
 				// distinct keys: one exact radix sort of the level; equal keys:
 				// the introsort replay, for those nodes only
@@ -1702,69 +1730,56 @@ struct Converter {
 					launch_node_pos(d_nodes, tie, lb, mem);
 				}
 				free_sorted_level(sorted, mem);
-				launch_cand_records(d_nodes, co.X, co.Y, co.Z, lb, mem);
 				PCG_CUDA(cudaEventRecord(ev[1], s));
-				// conflict lists for every node; a node where some candidate has
-				// too many close predecessors keeps the lookup kernels
+				// conflict lists and their acceptance; a dense node keeps the
+				// lookup kernels
+				LevelCells lc;
+				build_level_cells(d_nodes, pps, lb, lc, mem);
 				ConflictLists cl;
-				std::vector<int32_t> cta_list, warp_list, order2;
-				{
-					std::vector<uint8_t> use(K, 1), dense;
-					build_conflict_lists(mode, d_nodes, ln, use, pps, lb, cl, dense, d_st, mem);
-					PCG_CUDA(cudaEventRecord(ev_lists, s));
-					for (int i = 0; i < num_big; i++) (dense[order[i]] ? order2 : cta_list).push_back(order[i]);
-					const int num_grid = (int)order2.size();
-					for (int i = num_big; i < K; i++) (dense[order[i]] ? order2 : warp_list).push_back(order[i]);
-					list_nodes = (int)(cta_list.size() + warp_list.size());
-					launch_greedy_lists(mode, d_nodes, cta_list, warp_list, pps, lb, hkeys, hvals, axyz, akey, anext, apos, cl, d_st, mem, ln);
-					if (!order2.empty()) {
-						int32_t* d_order2 = upload(order2, mem);
-						launch_greedy(mode, guard, d_nodes, d_order2, (int)order2.size(), co.X, co.Y, co.Z, pps, lb, hkeys, hvals, axyz, akey,
-						              anext, apos, d_st, mem, &grid_arena, 0, -1, num_grid);
-						mem.free(d_order2);
-					}
-				}
+				std::vector<uint8_t> dense;
+				build_conflict_lists(mode, d_nodes, K, pps, lb, lc, cl, dense, d_st, mem);
+				PCG_CUDA(cudaEventRecord(ev[2], s));
+				uint32_t* accepted_bits = mem.alloc<uint32_t>((size_t)accept_words(M, K));
+				launch_accept(mode, d_nodes, ln, dense, lb, cl, accepted_bits, d_st, mem);
 				free_conflict_lists(cl, mem);
+				if (mode == 1) launch_cell_colors(d_nodes, dense, pps, lb, lc, accepted_bits, mem);
+				mem.free(accepted_bits);
+				free_level_cells(lc, mem);
+				std::vector<int32_t> dense_order;
+				for (int32_t k : order)
+					if (dense[k]) dense_order.push_back(k);
+				dense_nodes = (int)dense_order.size();
+				if (dense_nodes) {
+					lookup_begin(dense_order);
+					uint8_t* d_dense = upload(dense, mem);
+					launch_cand_records(d_nodes, co.X, co.Y, co.Z, lb, mem);
+					launch_greedy(mode, true, d_nodes, lk.d_order, dense_nodes, co.X, co.Y, co.Z, pps, lb, lk.hkeys, lk.hvals, lk.axyz, lk.akey,
+					              lk.anext, lk.apos, d_st, mem, &grid_arena, 0, -1, big_nodes(dense_order));
+					lookup_end(d_dense);
+					mem.free(d_dense);
+				}
+				PCG_CUDA(cudaEventRecord(ev[3], s));
 			}
-			PCG_CUDA(cudaEventRecord(ev[2], s));
-			PCG_CUDA(cudaEventSynchronize(ev[2]));
-			float t_sort = 0, t_greedy = 0;
+			PCG_CUDA(cudaEventSynchronize(ev[3]));
+			float t_sort = 0, t_greedy = 0, t_lists = 0;
 			PCG_CUDA(cudaEventElapsedTime(&t_sort, ev[0], ev[1]));
-			PCG_CUDA(cudaEventElapsedTime(&t_greedy, ev[1], ev[2]));
+			PCG_CUDA(cudaEventElapsedTime(&t_lists, ev[1], ev[2]));
+			PCG_CUDA(cudaEventElapsedTime(&t_greedy, ev[1], ev[3]));
 			res.stats.ms_sort += t_sort;
 			res.stats.ms_greedy += t_greedy;
-			float t_lists = 0;
-			if (form != PCG_FORM_PLAIN) PCG_CUDA(cudaEventElapsedTime(&t_lists, ev[1], ev_lists));
 			res.stats.ms_lists += t_lists;
-			cudaEventDestroy(ev_lists);
 			if (trace_levels()) {
 				int64_t mx = 0;
 				for (auto& l : ln) mx = std::max<int64_t>(mx, l.count);
-				static thread_local SampleStats prev{};
-				SampleStats now = download(d_st, 1, s)[0];
-				if (now.rounds < prev.rounds) prev = SampleStats{};
 				fprintf(stderr,
-				        "[pcg] level %d: nodes %d (cta %d, lists %d), candidates %lld, largest %lld, sort %.3f ms, greedy %.3f ms (lists %.3f), "
-				        "host %.3f ms (alloc %.3f), cta rounds %llu, passes %llu, serial rounds %llu, kcycles/round A %.1f C1 %.1f C2 %.1f D %.1f\n",
-				        K ? ln[0].level : -1, K, num_big, list_nodes, (long long)M, (long long)mx, t_sort, t_greedy, t_lists, ms_since(t_level), mem.alloc_ms() - alloc0,
-				        now.rounds - prev.rounds, now.passes - prev.passes, now.serial - prev.serial,
-				        [&](int i) { return (double)(now.cycles[i] - prev.cycles[i]) / 1e3 / std::max(1ull, now.rounds - prev.rounds); }(0),
-				        [&](int i) { return (double)(now.cycles[i] - prev.cycles[i]) / 1e3 / std::max(1ull, now.rounds - prev.rounds); }(2),
-				        [&](int i) { return (double)(now.cycles[i] - prev.cycles[i]) / 1e3 / std::max(1ull, now.rounds - prev.rounds); }(3),
-				        [&](int i) { return (double)(now.cycles[i] - prev.cycles[i]) / 1e3 / std::max(1ull, now.rounds - prev.rounds); }(4));
-				prev = now;
+				        "[pcg] level %d: nodes %d (dense %d), candidates %lld, largest %lld, sort %.3f ms, greedy %.3f ms (lists %.3f), "
+				        "host %.3f ms (alloc %.3f)\n",
+				        K ? ln[0].level : -1, K, dense_nodes, (long long)M, (long long)mx, t_sort, t_greedy, t_lists, ms_since(t_level),
+				        mem.alloc_ms() - alloc0);
 			}
 			for (auto& e : ev) cudaEventDestroy(e);
-			if (method == PCG_POISSON_AVERAGE) {
-				long long* sums = mem.alloc<long long>(4 * M);
-				launch_average_colors(d_nodes, co.X, co.Y, co.Z, pps, lb, hkeys, hvals, axyz, anext, apos, nullptr, sums, mem);
-				mem.free(sums);
-			}
-			mem.free(axyz); mem.free(akey); mem.free(anext); mem.free(apos);
-			mem.free(lb.keys); mem.free(lb.perm); mem.free(lb.pos); mem.free(lb.acc_rank); mem.free(lb.cq);
+			mem.free(lb.keys); mem.free(lb.perm); mem.free(lb.pos);
 		}
-		mem.free(hkeys);
-		mem.free(hvals);
 		// split candidates into the parents' buffers and the children's payloads
 		uint32_t* pre = mem.alloc<uint32_t>(M + 1);
 		uint32_t* acc_ids = mem.alloc<uint32_t>(M);
@@ -1823,7 +1838,6 @@ struct Converter {
 		mem.free(pre);
 		mem.free(d_nodes);
 		mem.free(d_items);
-		mem.free(d_order);
 		mem.free(lb.child);
 		mem.free(lb.node_of);
 		mem.free(lb.count_in_child);

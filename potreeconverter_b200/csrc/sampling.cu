@@ -24,16 +24,11 @@
 //    its child holds < 100 points, or if it is the first point of its
 //    128^3 cell that is eligible; first-eligible is an atomicMin per cell.
 
-#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <math_constants.h>
 
-#include <cstdio>
-#include <cstdlib>
-
 #include "devutil.cuh"
 #include "sampling.h"
-#include "tuned_schedule.h"
 
 namespace pcg {
 
@@ -331,9 +326,9 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) greedy_kernel(const Level
 // --------------------------------------------------- poisson_average colours
 __global__ void average_colors_kernel(const LevelNode* __restrict__ nodes, const int32_t* __restrict__ X, const int32_t* __restrict__ Y,
                                       const int32_t* __restrict__ Z, PosParamsS pp, LevelBuffers lb, GreedyArgs ga,
-                                      long long* __restrict__ sums) {
+                                      const uint8_t* __restrict__ only, long long* __restrict__ sums) {
 	int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-	if (j >= lb.M) return;
+	if (j >= lb.M || (only && !only[lb.node_of[j]])) return;
 	const LevelNode& nd = nodes[lb.node_of[j]];
 	const int64_t co = nd.cand_off;
 	const uint64_t col = lb.cols[j];
@@ -379,9 +374,10 @@ __global__ void average_colors_kernel(const LevelNode* __restrict__ nodes, const
 	}
 }
 
-__global__ void average_finish_kernel(const LevelNode* __restrict__ nodes, LevelBuffers lb, const long long* __restrict__ sums) {
+__global__ void average_finish_kernel(const LevelNode* __restrict__ nodes, LevelBuffers lb, const uint8_t* __restrict__ only,
+                                      const long long* __restrict__ sums) {
 	int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-	if (j >= lb.M || !lb.accepted[j]) return;
+	if (j >= lb.M || (only && !only[lb.node_of[j]]) || !lb.accepted[j]) return;
 	const int64_t slot = nodes[lb.node_of[j]].cand_off + lb.acc_rank[j];
 	const long long* s = sums + 4 * slot;
 	// rgbTarget = p.r / p.w (sampler_poisson_average.h:443-445)
@@ -874,636 +870,6 @@ __global__ void __launch_bounds__(kBigThreads) greedy_big_kernel(const LevelNode
 	}
 }
 
-
-// Pulls the list row, list length and record of sorted position u into L2
-// ahead of the round that reads them (they were written by an earlier kernel
-// and usually sit in DRAM).
-__device__ __forceinline__ void prefetch_list(const ConflictLists& cl, const LevelBuffers& lb, int64_t co, int64_t u) {
-	asm volatile("prefetch.global.L2 [%0];" ::"l"(cl.inl + co + u));
-	asm volatile("prefetch.global.L2 [%0];" ::"l"(cl.count + co + u));
-	asm volatile("prefetch.global.L2 [%0];" ::"l"(lb.cq + co + u));
-}
-
-// Rounds of 1024 candidates, one per thread of a 1024-thread CTA.
-constexpr int kListThreads = 1024;
-constexpr int kListWarps = kListThreads / 32;
-constexpr int kListRound = kListThreads;
-
-// exclusive scan over the CTA of one count per thread
-__device__ __forceinline__ uint32_t list_block_scan(uint32_t v, uint32_t& total, uint32_t* warp_sums) {
-	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-	uint32_t x = v;
-#pragma unroll
-	for (int o = 1; o < 32; o <<= 1) {
-		const uint32_t y = __shfl_up_sync(FULL, x, o);
-		if (lane >= o) x += y;
-	}
-	if (lane == 31) warp_sums[warp] = x;
-	__syncthreads();
-	if (warp == 0) {
-		uint32_t w = warp_sums[lane];
-#pragma unroll
-		for (int o = 1; o < 32; o <<= 1) {
-			const uint32_t y = __shfl_up_sync(FULL, w, o);
-			if (lane >= o) w += y;
-		}
-		warp_sums[lane] = w;
-	}
-	__syncthreads();
-	const uint32_t before = warp > 0 ? warp_sums[warp - 1] : 0u;
-	total = warp_sums[kListWarps - 1];
-	__syncthreads();
-	return before + x - v;
-}
-static_assert(kListWarps == 32, "one warp-sum per lane of warp 0");
-
-// Greedy acceptance for a large node from its conflict lists (conflicts.cu),
-// one CTA, 1024 candidates per round. A candidate's list names every earlier
-// candidate that would reject it if accepted, so the round needs no spatial
-// lookups: earlier rounds' decisions are read from srank (rank, or -1 for
-// rejected), this round's are resolved by the same parallel passes and
-// in-order warp as the grid kernel.
-struct ListRound {
-	int32_t maxrank[kListRound];
-	int32_t local[kListRound];
-	int16_t conf[kListRound][kListCap];
-	uint8_t nconf[kListRound];
-	uint8_t state[kListRound];   // 0 undecided, 1 accepted, 2 rejected
-	uint8_t old[kListRound];     // old-window status: 0 no conflict, 1 conflict, 2 depends on the count
-	int32_t cnt;             // accepted before this round
-	uint32_t warp_sums[kListWarps];
-};
-
-template <int MODE>
-__global__ void __launch_bounds__(kListThreads) greedy_list_kernel(const LevelNode* __restrict__ nodes, const int32_t* __restrict__ order,
-                                                                 int node_begin, PosParamsS pp, LevelBuffers lb, GreedyArgs ga,
-                                                                 ConflictLists cl, int32_t* __restrict__ srank, SampleStats* st) {
-	extern __shared__ __align__(16) unsigned char smem_raw[];
-	ListRound& R = *reinterpret_cast<ListRound*>(smem_raw);
-	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-	const LevelNode nd = nodes[order[node_begin + blockIdx.x]];
-	const int64_t n = nd.count, co = nd.cand_off;
-	uint64_t* hk = ga.hkeys + nd.hash_off;
-	int32_t* hh = ga.hheads + nd.hash_off;
-	if (MODE == 1) {
-		// poisson_average's colour pass finds accepted points through the hash
-		for (int64_t i = tid; i < nd.hash_cap; i += kListThreads) { hk[i] = EMPTY_KEY; hh[i] = -1; }
-	}
-	if (tid == 0) R.cnt = 0;
-	__syncthreads();
-	CellGrid g;
-	g.min[0] = nd.min[0]; g.min[1] = nd.min[1]; g.min[2] = nd.min[2];
-	g.inv = 1.0 / (2.0 * nd.spacing * 1.000001);
-	for (int64_t r0 = 0; r0 < n; r0 += kListRound) {
-		const int64_t t = r0 + tid;
-		const bool valid = t < n;
-		const int nr = (int)((n - r0) < kListRound ? (n - r0) : kListRound);
-		const int32_t cnt0 = R.cnt;
-		// ---- A: the candidate's list
-		long long clk0 = clock64();
-		if (t + kListRound < n) prefetch_list(cl, lb, co, t + kListRound);
-		int32_t maxrank = -1, local = 0;
-		int nc = 0, nl = 0;
-		int4 me = make_int4(0, 0, 0, 0);
-		if (valid) {
-			me = lb.cq[co + t];
-			local = me.w;
-			nl = cl.count[co + t];
-		}
-		{
-			// lists are short (about one entry on average): loop to the
-			// warp's longest list, four entries at a time (the first four in one
-			// 16-byte load)
-			const int wmax = (int)__reduce_max_sync(FULL, (unsigned)nl);
-			for (int w = 0; 4 * w < wmax; w++) {
-				const int4 v = 4 * w < nl ? list_quad(cl, co + t, nl, w) : make_int4(0, 0, 0, 0);
-				const int32_t u4[4] = {v.x, v.y, v.z, v.w};
-				int32_t rk4[4];
-#pragma unroll
-				for (int k = 0; k < 4; k++) rk4[k] = (4 * w + k < nl && u4[k] < r0) ? srank[co + u4[k]] : -1;
-#pragma unroll
-				for (int k = 0; k < 4; k++) {
-					if (4 * w + k < nl) {
-						if (u4[k] < r0) maxrank = rk4[k] > maxrank ? rk4[k] : maxrank;
-						else R.conf[tid][nc++] = (int16_t)(u4[k] - r0);
-					}
-				}
-			}
-		}
-		R.maxrank[tid] = maxrank;
-		R.local[tid] = local;
-		R.nconf[tid] = (uint8_t)nc;
-		R.state[tid] = valid ? 0 : 2;
-		{
-			uint8_t os = 0;
-			if (maxrank >= 0) {
-				if (MODE == 1) os = 1;
-				else if (maxrank >= cnt0 + tid - 10001) os = 1;       // conflicts whatever was accepted before it
-				else if (maxrank < cnt0 - 10001) os = 0;              // outside the window in any case
-				else os = 2;
-			}
-			R.old[tid] = os;
-		}
-		__syncthreads();
-		long long clk1 = clock64();
-		long long clk2 = clk1;
-		// ---- C1: parallel passes
-		volatile uint8_t* vstate = R.state;
-		for (int pass = 0; pass < 64; pass++) {
-			bool changed = false;
-			if (valid && vstate[tid] == 0) {
-				const uint8_t os = R.old[tid];
-				uint8_t dec = 0;
-				if (os == 1) {
-					dec = 2;
-				} else {
-					bool any_acc = false, all_done = true;
-					for (int e = 0; e < R.nconf[tid]; e++) {
-						uint8_t sj = vstate[R.conf[tid][e]];
-						any_acc |= sj == 1;
-						all_done &= sj != 0;
-					}
-					if (any_acc) dec = 2;
-					else if (all_done && os == 0) dec = 1;
-				}
-				if (dec) { vstate[tid] = dec; changed = true; }
-			}
-			if (!__syncthreads_or(changed)) {
-				if (tid == 0) atomicAdd(&st->passes, (unsigned long long)pass + 1);
-				break;
-			}
-		}
-		const bool left = __syncthreads_or(valid && vstate[tid] == 0);
-		if (tid == 0) {
-			atomicAdd(&st->rounds, 1ull);
-			if (left) atomicAdd(&st->serial, 1ull);
-		}
-		long long clk3 = clock64();
-		// ---- C2: warp 0 decides the rest in sorted order
-		if (left && warp == 0) {
-			int32_t cnt = cnt0;
-			const uint32_t ltm = lanemask_lt();
-			for (int cb = 0; cb < nr; cb += 32) {
-				const int i = cb + lane;
-				const bool v = i < nr;
-				const uint8_t si = v ? vstate[i] : 2;
-				const bool undec = v && si == 0;
-				uint32_t accmask = __ballot_sync(FULL, v && si == 1);
-				if (__ballot_sync(FULL, undec) != 0) {
-					bool prev_conflict = false;
-					uint32_t mask = 0;
-					if (undec) {
-						const int ncf = R.nconf[i];
-						for (int e = 0; e < ncf; e++) {
-							int j = R.conf[i][e];
-							if (j < cb) prev_conflict |= vstate[j] == 1;
-							else mask |= 1u << (j - cb);
-						}
-					}
-					const int nvalid = nr - cb < 32 ? nr - cb : 32;
-					for (int b = 0; b < nvalid; b++) {
-						bool dec = false;
-						const bool ub = __shfl_sync(FULL, undec, b);
-						if (!ub) continue;
-						if (lane == b) {
-							int32_t m_i = cnt + __popc(accmask & ltm);
-							bool old_conflict = R.maxrank[i] >= 0 && (MODE == 1 || R.maxrank[i] >= m_i - 10001);
-							dec = !old_conflict && !prev_conflict && !(mask & accmask);
-							vstate[i] = dec ? 1 : 2;
-						}
-						dec = __shfl_sync(FULL, dec, b);
-						if (dec) accmask |= 1u << b;
-					}
-				}
-				cnt += __popc(accmask);
-				__syncwarp();
-			}
-		}
-		__syncthreads();
-		// ---- D: publish
-		long long clk4 = clock64();
-		const bool acc = valid && vstate[tid] == 1;
-		uint32_t total;
-		uint32_t pre;
-		{
-			pre = list_block_scan(acc ? 1u : 0u, total, R.warp_sums);
-		}
-		if (valid) {
-			const int32_t rank = cnt0 + (int32_t)pre;
-			srank[co + t] = acc ? rank : -1;
-			lb.accepted[co + local] = acc ? 1 : 0;
-			if (acc) {
-				lb.acc_rank[co + local] = rank;
-				if (MODE == 1) {
-					// the colour pass walks the hash lists (linked through anext)
-					const int64_t slot = co + rank;
-					const double x = ((double)me.x * pp.scale[0]) + pp.offset[0];
-					const double y = ((double)me.y * pp.scale[1]) + pp.offset[1];
-					const double z = ((double)me.z * pp.scale[2]) + pp.offset[2];
-					ga.axyz[3 * slot] = x;
-					ga.axyz[3 * slot + 1] = y;
-					ga.axyz[3 * slot + 2] = z;
-					ga.akey[slot] = lb.keys[co + t];
-					ga.apos[slot] = (int32_t)t;
-					int c[3];
-					double fr[3];
-					cell_of(g, x, y, z, c, fr);
-					if (!hash_push(hk, hh, ga.anext + co, nd.hash_cap, cell_key(c[0], c[1], c[2]), rank)) atomicAdd(&st->timeouts, 1ull);
-				}
-			}
-		}
-		__syncthreads();
-		if (tid == 0) {
-			R.cnt = cnt0 + (int32_t)total;
-			const long long clk5 = clock64();
-			atomicAdd(&st->cycles[0], (unsigned long long)(clk1 - clk0));
-			atomicAdd(&st->cycles[1], (unsigned long long)(clk2 - clk1));
-			atomicAdd(&st->cycles[2], (unsigned long long)(clk3 - clk2));
-			atomicAdd(&st->cycles[3], (unsigned long long)(clk4 - clk3));
-			atomicAdd(&st->cycles[4], (unsigned long long)(clk5 - clk4));
-		}
-		__syncthreads();
-	}
-}
-
-
-// Greedy acceptance for the largest nodes on a cluster of CS CTAs (CS x
-// 1024 threads, CS = 4, or 8 for the few largest nodes of a level): a
-// super-round decides CS x 1024 candidates, CTA k holding candidates
-// [1024k, 1024k + 1024) of it. Each CTA keeps its candidates' states in its
-// own shared memory; a candidate's conflicts inside the super-round (always
-// with lower indices) are read from the owning CTA's shared memory through
-// the cluster's distributed shared memory. Passes, the in-order warp (CTA
-// 0, warp 0, reading and writing all CTAs' states) and the rank prefix are
-// separated by cluster barriers, which every CTA reaches the same number of
-// times. A node's serial chain of super-rounds sets a level's acceptance
-// time, so its largest nodes take the wider cluster: half the super-rounds.
-constexpr int kClusterCtas = 4;
-constexpr int kWideClusterCtas = 8;  // portable maximum cluster size
-constexpr int64_t kClusterMinCandidates = 65536;  // smallest cluster node the shared-memory layout is sized for
-static_assert(kListRound * kWideClusterCtas <= 32767, "conflict indices are int16");
-// A level's cluster nodes take 8-CTA clusters only when there are at most
-// this many of them (the top levels): an 8-CTA cluster needs eight free SMs
-// of one GPC at once, and beside many other nodes' CTAs it waits for them
-// (measured: the 50M cloud's levels 3-5 lost 2-4x).
-constexpr int kMaxWideClusterNodes = 4;
-
-struct ClusterRound {
-	int32_t maxrank[kListRound];
-	int32_t local[kListRound];
-	int16_t conf[kListRound][kListCap];  // indices inside the super-round
-	uint8_t nconf[kListRound];
-	uint8_t state[kListRound];   // 0 undecided, 1 accepted, 2 rejected
-	uint8_t old[kListRound];     // old-window status as in ListRound
-	uint32_t warp_sums[kListWarps];
-	int32_t changed[2];          // per pass parity: this CTA changed a state
-	int32_t left;                // this CTA has undecided candidates
-	int32_t total;               // accepted in this CTA's part of the super-round
-};
-
-template <int MODE, int CS>
-__global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(kListThreads, 1)
-    greedy_list_cluster_kernel(const LevelNode* __restrict__ nodes, const int32_t* __restrict__ order, PosParamsS pp, LevelBuffers lb,
-                               GreedyArgs ga, ConflictLists cl, int32_t* __restrict__ srank, SampleStats* st) {
-	constexpr int kSuper = kListRound * CS;
-	namespace cgr = cooperative_groups;
-	cgr::cluster_group cluster = cgr::this_cluster();
-	extern __shared__ __align__(16) unsigned char smem_raw[];
-	ClusterRound& R = *reinterpret_cast<ClusterRound*>(smem_raw);
-	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-	const int crank = (int)cluster.block_rank();
-	// another CTA's round state (distributed shared memory)
-	auto peer = [&](int r) { return cluster.map_shared_rank(&R, r); };
-	const LevelNode nd = nodes[order[blockIdx.x / CS]];
-	const int64_t n = nd.count, co = nd.cand_off;
-	uint64_t* hk = ga.hkeys + nd.hash_off;
-	int32_t* hh = ga.hheads + nd.hash_off;
-	if (MODE == 1) {
-		for (int64_t i = crank * kListThreads + tid; i < nd.hash_cap; i += kSuper) { hk[i] = EMPTY_KEY; hh[i] = -1; }
-	}
-	CellGrid g;
-	g.min[0] = nd.min[0]; g.min[1] = nd.min[1]; g.min[2] = nd.min[2];
-	g.inv = 1.0 / (2.0 * nd.spacing * 1.000001);
-	int32_t cnt0 = 0;  // accepted before the super-round, the same in every CTA
-	if (crank == 0 && tid == 0) atomicAdd(&st->cluster_nodes, 1ull);
-	cluster.sync();
-	for (int64_t r0 = 0; r0 < n; r0 += kSuper) {
-		const int idx = crank * kListThreads + tid;  // index inside the super-round
-		const int64_t t = r0 + idx;
-		const bool valid = t < n;
-		const int nr = (int)((n - r0) < kSuper ? (n - r0) : kSuper);
-		// ---- A: the candidate's list
-		const long long clk0 = clock64();
-		if (t + kSuper < n) prefetch_list(cl, lb, co, t + kSuper);
-		int32_t maxrank = -1, local = 0;
-		int nc = 0, nl = 0;
-		int4 me = make_int4(0, 0, 0, 0);
-		if (valid) {
-			me = lb.cq[co + t];
-			local = me.w;
-			nl = cl.count[co + t];
-		}
-		{
-			const int wmax = (int)__reduce_max_sync(FULL, (unsigned)nl);
-			for (int w = 0; 4 * w < wmax; w++) {
-				const int4 v = 4 * w < nl ? list_quad(cl, co + t, nl, w) : make_int4(0, 0, 0, 0);
-				const int32_t u4[4] = {v.x, v.y, v.z, v.w};
-				int32_t rk4[4];
-#pragma unroll
-				for (int k = 0; k < 4; k++) rk4[k] = (4 * w + k < nl && u4[k] < r0) ? srank[co + u4[k]] : -1;
-#pragma unroll
-				for (int k = 0; k < 4; k++) {
-					if (4 * w + k < nl) {
-						if (u4[k] < r0) maxrank = rk4[k] > maxrank ? rk4[k] : maxrank;
-						else R.conf[tid][nc++] = (int16_t)(u4[k] - r0);
-					}
-				}
-			}
-		}
-		R.maxrank[tid] = maxrank;
-		R.local[tid] = local;
-		R.nconf[tid] = (uint8_t)nc;
-		R.state[tid] = valid ? 0 : 2;
-		{
-			uint8_t os = 0;
-			if (maxrank >= 0) {
-				if (MODE == 1) os = 1;
-				else if (maxrank >= cnt0 + idx - 10001) os = 1;       // conflicts whatever was accepted before it
-				else if (maxrank < cnt0 - 10001) os = 0;              // outside the window in any case
-				else os = 2;
-			}
-			R.old[tid] = os;
-		}
-		cluster.sync();
-		const long long clk1 = clock64();
-		// ---- C1: parallel passes. Decisions only go from undecided to final,
-		// so a stale read of another CTA's state only delays a decision:
-		// each CTA repeats local passes (block barriers) while it makes
-		// progress, then the cluster barrier publishes whether any CTA did;
-		// the fixpoint is a cluster round in which none did.
-		int passes = 0;
-		for (int gpass = 0; gpass < 64; gpass++) {
-			int progressed = 0;
-			for (int lp = 0; lp < 64; lp++) {
-				bool changed = false;
-				if (valid && R.state[tid] == 0) {
-					const uint8_t os = R.old[tid];
-					uint8_t dec = 0;
-					if (os == 1) {
-						dec = 2;
-					} else {
-						bool any_acc = false, all_done = true;
-						for (int e = 0; e < R.nconf[tid]; e++) {
-							const int j = R.conf[tid][e];
-							const uint8_t sj = *(volatile uint8_t*)&peer(j / kListRound)->state[j % kListRound];
-							any_acc |= sj == 1;
-							all_done &= sj != 0;
-						}
-						if (any_acc) dec = 2;
-						else if (all_done && os == 0) dec = 1;
-					}
-					if (dec) {
-						*(volatile uint8_t*)&R.state[tid] = dec;
-						changed = true;
-					}
-				}
-				passes++;
-				if (!__syncthreads_or(changed)) break;
-				progressed = 1;
-			}
-			if (tid == 0) R.changed[gpass & 1] = progressed;
-			cluster.sync();
-			int all = 0;
-#pragma unroll
-			for (int r = 0; r < CS; r++) all |= *(volatile int32_t*)&peer(r)->changed[gpass & 1];
-			if (!all) break;
-		}
-		if (tid == 0 && crank == 0) atomicAdd(&st->passes, (unsigned long long)passes);
-		const int left_here = __syncthreads_or(valid && R.state[tid] == 0);
-		if (tid == 0) R.left = left_here;
-		cluster.sync();
-		int left = 0;
-#pragma unroll
-		for (int r = 0; r < CS; r++) left |= *(volatile int32_t*)&peer(r)->left;
-		if (crank == 0 && tid == 0) {
-			atomicAdd(&st->rounds, 1ull);
-			if (left) atomicAdd(&st->serial, 1ull);
-		}
-		const long long clk2 = clock64();
-		// ---- C2: one warp decides the rest in order
-		if (left && crank == 0 && warp == 0) {
-			int32_t cnt = cnt0;
-			const uint32_t ltm = lanemask_lt();
-			for (int cb = 0; cb < nr; cb += 32) {
-				const int i = cb + lane;
-				const bool v = i < nr;
-				ClusterRound* Ri = peer((v ? i : 0) / kListRound);
-				const int li = (v ? i : 0) % kListRound;
-				const uint8_t si = v ? *(volatile uint8_t*)&Ri->state[li] : 2;
-				const bool undec = v && si == 0;
-				uint32_t accmask = __ballot_sync(FULL, v && si == 1);
-				if (__ballot_sync(FULL, undec) != 0) {
-					bool prev_conflict = false;
-					uint32_t mask = 0;
-					if (undec) {
-						const int ncf = Ri->nconf[li];
-						for (int e = 0; e < ncf; e++) {
-							const int j = Ri->conf[li][e];
-							if (j < cb) prev_conflict |= *(volatile uint8_t*)&peer(j / kListRound)->state[j % kListRound] == 1;
-							else mask |= 1u << (j - cb);
-						}
-					}
-					const int nvalid = nr - cb < 32 ? nr - cb : 32;
-					for (int b = 0; b < nvalid; b++) {
-						bool dec = false;
-						const bool ub = __shfl_sync(FULL, undec, b);
-						if (!ub) continue;
-						if (lane == b) {
-							const int32_t m_i = cnt + __popc(accmask & ltm);
-							const int32_t mr = Ri->maxrank[li];
-							const bool old_conflict = mr >= 0 && (MODE == 1 || mr >= m_i - 10001);
-							dec = !old_conflict && !prev_conflict && !(mask & accmask);
-							*(volatile uint8_t*)&Ri->state[li] = dec ? 1 : 2;
-						}
-						dec = __shfl_sync(FULL, dec, b);
-						if (dec) accmask |= 1u << b;
-					}
-				}
-				cnt += __popc(accmask);
-				__syncwarp();
-			}
-		}
-		cluster.sync();
-		const long long clk3 = clock64();
-		// ---- D: ranks across the cluster, publish
-		const bool acc = valid && R.state[tid] == 1;
-		uint32_t total;
-		const uint32_t pre = list_block_scan(acc ? 1u : 0u, total, R.warp_sums);
-		if (tid == 0) R.total = (int32_t)total;
-		cluster.sync();
-		int32_t before = 0, all_acc = 0;
-#pragma unroll
-		for (int r = 0; r < CS; r++) {
-			const int32_t tr = *(volatile int32_t*)&peer(r)->total;
-			if (r < crank) before += tr;
-			all_acc += tr;
-		}
-		if (valid) {
-			const int32_t rank = cnt0 + before + (int32_t)pre;
-			srank[co + t] = acc ? rank : -1;
-			lb.accepted[co + local] = acc ? 1 : 0;
-			if (acc) {
-				lb.acc_rank[co + local] = rank;
-				if (MODE == 1) {
-					const int64_t slot = co + rank;
-					const double x = ((double)me.x * pp.scale[0]) + pp.offset[0];
-					const double y = ((double)me.y * pp.scale[1]) + pp.offset[1];
-					const double z = ((double)me.z * pp.scale[2]) + pp.offset[2];
-					ga.axyz[3 * slot] = x;
-					ga.axyz[3 * slot + 1] = y;
-					ga.axyz[3 * slot + 2] = z;
-					ga.akey[slot] = lb.keys[co + t];
-					ga.apos[slot] = (int32_t)t;
-					int c[3];
-					double fr[3];
-					cell_of(g, x, y, z, c, fr);
-					if (!hash_push(hk, hh, ga.anext + co, nd.hash_cap, cell_key(c[0], c[1], c[2]), rank)) atomicAdd(&st->timeouts, 1ull);
-				}
-			}
-		}
-		cnt0 += all_acc;
-		// the next super-round rewrites states, flags and totals other CTAs read
-		cluster.sync();
-		if (crank == 0 && tid == 0) {
-			const long long clk4 = clock64();
-			atomicAdd(&st->cycles[0], (unsigned long long)(clk1 - clk0));
-			atomicAdd(&st->cycles[2], (unsigned long long)(clk2 - clk1));
-			atomicAdd(&st->cycles[3], (unsigned long long)(clk3 - clk2));
-			atomicAdd(&st->cycles[4], (unsigned long long)(clk4 - clk3));
-		}
-	}
-}
-
-// Greedy acceptance from conflict lists for the smaller nodes, one warp per
-// node, 32 candidates per step. Conflicts with earlier steps come from
-// srank; inside a step they are a lane mask, resolved by ballot passes (a
-// lane decides once its earlier conflicting lanes have) or, when a lane's
-// old conflict sits at the edge of the 10,001-check window, in lane order.
-template <int MODE>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32) greedy_list_warp_kernel(const LevelNode* __restrict__ nodes,
-                                                                              const int32_t* __restrict__ order, int num, PosParamsS pp,
-                                                                              LevelBuffers lb, GreedyArgs ga, ConflictLists cl,
-                                                                              int32_t* __restrict__ srank, SampleStats* st,
-                                                                              int* next_node) {
-	const int lane = threadIdx.x & 31;
-	const uint32_t lt = lanemask_lt();
-	while (true) {
-		int idx = 0;
-		if (lane == 0) idx = atomicAdd(next_node, 1);
-		idx = __shfl_sync(FULL, idx, 0);
-		if (idx >= num) break;
-		const LevelNode nd = nodes[order[idx]];
-		const int64_t n = nd.count, co = nd.cand_off;
-		uint64_t* hk = ga.hkeys + nd.hash_off;
-		int32_t* hh = ga.hheads + nd.hash_off;
-		CellGrid g;
-		g.min[0] = nd.min[0]; g.min[1] = nd.min[1]; g.min[2] = nd.min[2];
-		g.inv = 1.0 / (2.0 * nd.spacing * 1.000001);
-		if (MODE == 1) {
-			for (int64_t s = lane; s < nd.hash_cap; s += 32) { hk[s] = EMPTY_KEY; hh[s] = -1; }
-			__syncwarp();
-		}
-		int32_t cnt = 0;  // accepted so far
-		for (int64_t b0 = 0; b0 < n; b0 += 32) {
-			const int64_t t = b0 + lane;
-			const bool valid = t < n;
-			if (t + 64 < n) prefetch_list(cl, lb, co, t + 64);
-			int4 me = make_int4(0, 0, 0, 0);
-			int32_t maxrank = -1;
-			uint32_t mask = 0;  // earlier lanes of this step that conflict
-			int nl = 0;
-			if (valid) {
-				me = lb.cq[co + t];
-				nl = cl.count[co + t];
-			}
-			{
-				const int wmax = (int)__reduce_max_sync(FULL, (unsigned)nl);
-				for (int w = 0; 4 * w < wmax; w++) {
-					const int4 v = 4 * w < nl ? list_quad(cl, co + t, nl, w) : make_int4(0, 0, 0, 0);
-					const int32_t u4[4] = {v.x, v.y, v.z, v.w};
-					int32_t rk4[4];
-#pragma unroll
-					for (int k = 0; k < 4; k++) rk4[k] = (4 * w + k < nl && u4[k] < b0) ? srank[co + u4[k]] : -1;
-#pragma unroll
-					for (int k = 0; k < 4; k++) {
-						if (4 * w + k < nl) {
-							if (u4[k] < b0) maxrank = rk4[k] > maxrank ? rk4[k] : maxrank;
-							else mask |= 1u << (u4[k] - b0);
-						}
-					}
-				}
-			}
-			int os = 0;
-			if (maxrank >= 0) {
-				if (MODE == 1) os = 1;
-				else if (maxrank >= cnt + lane - 10001) os = 1;  // conflicts whatever was accepted before it
-				else if (maxrank < cnt - 10001) os = 0;          // outside the window in any case
-				else os = 2;
-			}
-			const uint32_t validmask = __ballot_sync(FULL, valid);
-			uint32_t accmask = 0;
-			if (__ballot_sync(FULL, valid && os == 2) == 0) {
-				uint32_t undec = validmask & ~__ballot_sync(FULL, valid && os == 1);
-				for (int it = 0; it < 33 && undec; it++) {
-					const bool mine = (undec >> lane) & 1u;
-					const bool ready = mine && (mask & undec) == 0;
-					const bool a = ready && (mask & accmask) == 0;
-					accmask |= __ballot_sync(FULL, a);
-					undec &= ~__ballot_sync(FULL, ready);
-				}
-			} else {
-				for (int b = 0; b < 32; b++) {
-					if (!((validmask >> b) & 1u)) continue;
-					bool dec = false;
-					if (lane == b && os != 1) {
-						const int32_t m_i = cnt + __popc(accmask & lt);
-						const bool old_conflict = maxrank >= 0 && (MODE == 1 || maxrank >= m_i - 10001);
-						dec = !old_conflict && !(mask & accmask);
-					}
-					dec = __shfl_sync(FULL, dec, b);
-					if (dec) accmask |= 1u << b;
-				}
-			}
-			const bool acc = (accmask >> lane) & 1u;
-			if (valid) {
-				const int32_t rank = cnt + __popc(accmask & lt);
-				const int32_t local = me.w;
-				srank[co + t] = acc ? rank : -1;
-				lb.accepted[co + local] = acc ? 1 : 0;
-				if (acc) {
-					lb.acc_rank[co + local] = rank;
-					if (MODE == 1) {
-						const int64_t slot = co + rank;
-						const double x = ((double)me.x * pp.scale[0]) + pp.offset[0];
-						const double y = ((double)me.y * pp.scale[1]) + pp.offset[1];
-						const double z = ((double)me.z * pp.scale[2]) + pp.offset[2];
-						ga.axyz[3 * slot] = x;
-						ga.axyz[3 * slot + 1] = y;
-						ga.axyz[3 * slot + 2] = z;
-						ga.akey[slot] = lb.keys[co + t];
-						ga.apos[slot] = (int32_t)t;
-						int c[3];
-						double fr[3];
-						cell_of(g, x, y, z, c, fr);
-						if (!hash_push(hk, hh, ga.anext + co, nd.hash_cap, cell_key(c[0], c[1], c[2]), rank)) atomicAdd(&st->timeouts, 1ull);
-					}
-				}
-			}
-			cnt += __popc(accmask);
-		}
-	}
-}
-
 }  // namespace
 
 // ----------------------------------------------------------------- launchers
@@ -1617,122 +983,17 @@ void launch_greedy(int mode, bool fp32_guard, const LevelNode* nodes, const int3
 	}
 }
 
-LevelSchedule level_schedule() {
-	// read at every level, so the autotuner can sweep in one process
-	LevelSchedule v{PCG_TUNED_CTA_MIN, PCG_TUNED_SMALL_LEVEL_CTA_MIN, PCG_TUNED_CLUSTER_MIN, PCG_TUNED_WARP_BLOCKS_PER_SM};
-	if (const char* e = std::getenv("PCG_SCHEDULE")) {
-		long long a = 0, b = 0, c = 0, d = 0;
-		if (std::sscanf(e, "%lld,%lld,%lld,%lld", &a, &b, &c, &d) == 4 && a > 0 && b > 0 && c > 0 && d > 0 && d <= 64)
-			v = LevelSchedule{a, b, c, (int)d};
-	}
-	return v;
-}
-
-void launch_greedy_lists(int mode, const LevelNode* nodes, const std::vector<int32_t>& cta_nodes, const std::vector<int32_t>& warp_nodes,
-                         const PosParamsS& pp, LevelBuffers& lb, uint64_t* hash_keys, int32_t* hash_heads, double* acc_xyz,
-                         double* acc_key, int32_t* acc_next, int32_t* acc_pos, const ConflictLists& cl, SampleStats* st, DeviceMem& mem,
-                         const std::vector<LevelNode>& ln) {
-	if (lb.M == 0 || (cta_nodes.empty() && warp_nodes.empty())) return;
-	GreedyArgs ga{hash_keys, hash_heads, acc_xyz, acc_key, acc_next, acc_pos};
-	cudaStream_t s = mem.stream();
-	// the largest nodes (cta_nodes is largest first) on a cluster each, the
-	// other CTA nodes on one CTA, the rest on a warp
-	std::vector<int32_t> wide, clu, one;
-	const int64_t cluster_min = std::max(level_schedule().cluster_min, kClusterMinCandidates);
-	for (int32_t k : cta_nodes) (ln[k].count >= cluster_min ? clu : one).push_back(k);
-	if (!clu.empty() && (int)clu.size() <= kMaxWideClusterNodes) wide.swap(clu);
-	int32_t* srank = mem.alloc<int32_t>((size_t)lb.M);
-	int32_t* d_wide = wide.empty() ? nullptr : mem.alloc<int32_t>(wide.size());
-	int32_t* d_clu = clu.empty() ? nullptr : mem.alloc<int32_t>(clu.size());
-	int32_t* d_one = one.empty() ? nullptr : mem.alloc<int32_t>(one.size());
-	int32_t* d_warp = warp_nodes.empty() ? nullptr : mem.alloc<int32_t>(warp_nodes.size());
-	int* counter = mem.alloc<int>(1);
-	if (d_wide) PCG_CUDA(cudaMemcpyAsync(d_wide, wide.data(), wide.size() * sizeof(int32_t), cudaMemcpyHostToDevice, s));
-	if (d_clu) PCG_CUDA(cudaMemcpyAsync(d_clu, clu.data(), clu.size() * sizeof(int32_t), cudaMemcpyHostToDevice, s));
-	if (d_one) PCG_CUDA(cudaMemcpyAsync(d_one, one.data(), one.size() * sizeof(int32_t), cudaMemcpyHostToDevice, s));
-	if (d_warp) PCG_CUDA(cudaMemcpyAsync(d_warp, warp_nodes.data(), warp_nodes.size() * sizeof(int32_t), cudaMemcpyHostToDevice, s));
-	PCG_CUDA(cudaMemsetAsync(counter, 0, sizeof(int), s));
-	// the node sets are independent: the first runs on the job's stream, the
-	// second on one forked stream, the others on a second one
-	constexpr int kSides = DeviceArena::kSides;
-	cudaStream_t side[kSides] = {nullptr, nullptr};
-	cudaEvent_t fork[kSides] = {nullptr, nullptr}, join[kSides] = {nullptr, nullptr};
-	const int sets = (d_wide ? 1 : 0) + (d_clu ? 1 : 0) + (d_one ? 1 : 0) + (d_warp ? 1 : 0);
-	const int nsides = mem.arena() ? std::min(sets - 1, kSides) : 0;
-	for (int k = 0; k < nsides; k++) {
-		side[k] = mem.arena()->side_stream(fork[k], join[k], k);
-		PCG_CUDA(cudaEventRecord(fork[k], s));
-		PCG_CUDA(cudaStreamWaitEvent(side[k], fork[k], 0));
-	}
-	int next_set = 0;
-	auto stream_for_set = [&]() {
-		const int i = next_set++;
-		if (i == 0 || nsides == 0) return s;
-		return side[std::min(i, nsides) - 1];
-	};
-	auto launch_cluster = [&](auto kernel, int cs_ctas, const int32_t* d_set, size_t count, cudaStream_t cs) {
-		const size_t smem = sizeof(ClusterRound);
-		PCG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-		kernel<<<(unsigned)(count * cs_ctas), kListThreads, smem, cs>>>(nodes, d_set, pp, lb, ga, cl, srank, st);
-		PCG_LAUNCHED();
-	};
-	if (d_wide) {
-		cudaStream_t cs = stream_for_set();
-		if (mode == 0) launch_cluster(greedy_list_cluster_kernel<0, kWideClusterCtas>, kWideClusterCtas, d_wide, wide.size(), cs);
-		else launch_cluster(greedy_list_cluster_kernel<1, kWideClusterCtas>, kWideClusterCtas, d_wide, wide.size(), cs);
-	}
-	if (d_clu) {
-		cudaStream_t cs = stream_for_set();
-		if (mode == 0) launch_cluster(greedy_list_cluster_kernel<0, kClusterCtas>, kClusterCtas, d_clu, clu.size(), cs);
-		else launch_cluster(greedy_list_cluster_kernel<1, kClusterCtas>, kClusterCtas, d_clu, clu.size(), cs);
-	}
-	if (d_one) {
-		const size_t smem = sizeof(ListRound);
-		const int nc = (int)one.size();
-		cudaStream_t cs = stream_for_set();
-		if (mode == 0) {
-			PCG_CUDA(cudaFuncSetAttribute(greedy_list_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-			greedy_list_kernel<0><<<nc, kListThreads, smem, cs>>>(nodes, d_one, 0, pp, lb, ga, cl, srank, st);
-		} else {
-			PCG_CUDA(cudaFuncSetAttribute(greedy_list_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-			greedy_list_kernel<1><<<nc, kListThreads, smem, cs>>>(nodes, d_one, 0, pp, lb, ga, cl, srank, st);
-		}
-		PCG_LAUNCHED();
-	}
-	if (d_warp) {
-		cudaStream_t ws = stream_for_set();
-		const int nw = (int)warp_nodes.size();
-		int blocks = (int)ceil_div(nw, kWarpsPerBlock);
-		const int cap = sm_count() * level_schedule().warp_blocks_per_sm;
-		if (blocks > cap) blocks = cap;
-		if (mode == 0) greedy_list_warp_kernel<0><<<blocks, kWarpsPerBlock * 32, 0, ws>>>(nodes, d_warp, nw, pp, lb, ga, cl, srank, st, counter);
-		else greedy_list_warp_kernel<1><<<blocks, kWarpsPerBlock * 32, 0, ws>>>(nodes, d_warp, nw, pp, lb, ga, cl, srank, st, counter);
-		PCG_LAUNCHED();
-	}
-	for (int k = 0; k < nsides; k++) {
-		PCG_CUDA(cudaEventRecord(join[k], side[k]));
-		PCG_CUDA(cudaStreamWaitEvent(s, join[k], 0));
-	}
-	mem.free(srank);
-	if (d_wide) mem.free(d_wide);
-	if (d_clu) mem.free(d_clu);
-	if (d_one) mem.free(d_one);
-	if (d_warp) mem.free(d_warp);
-	mem.free(counter);
-}
-
 void launch_average_colors(const LevelNode* nodes, const int32_t* X, const int32_t* Y, const int32_t* Z, const PosParamsS& pp,
                            LevelBuffers& lb, const uint64_t* hash_keys, const int32_t* hash_heads, const double* acc_xyz,
-                           const int32_t* acc_next, const int32_t* acc_pos, const int64_t* /*acc_base*/, long long* sums,
-                           DeviceMem& mem) {
+                           const int32_t* acc_next, const int32_t* acc_pos, const uint8_t* only, long long* sums, DeviceMem& mem) {
 	if (lb.M == 0) return;
 	GreedyArgs ga{const_cast<uint64_t*>(hash_keys), const_cast<int32_t*>(hash_heads), const_cast<double*>(acc_xyz), nullptr,
 	              const_cast<int32_t*>(acc_next), const_cast<int32_t*>(acc_pos)};
 	PCG_CUDA(cudaMemsetAsync(sums, 0, sizeof(long long) * 4 * lb.M, mem.stream()));
 	unsigned blocks = (unsigned)ceil_div(lb.M, 256);
-	average_colors_kernel<<<blocks, 256, 0, mem.stream()>>>(nodes, X, Y, Z, pp, lb, ga, sums);
+	average_colors_kernel<<<blocks, 256, 0, mem.stream()>>>(nodes, X, Y, Z, pp, lb, ga, only, sums);
 	PCG_LAUNCHED();
-	average_finish_kernel<<<blocks, 256, 0, mem.stream()>>>(nodes, lb, sums);
+	average_finish_kernel<<<blocks, 256, 0, mem.stream()>>>(nodes, lb, only, sums);
 	PCG_LAUNCHED();
 }
 

@@ -62,11 +62,11 @@ struct SampleStats {
 	unsigned long long escalated;  // FP32 decisions re-made in FP64
 	unsigned long long heapsorts;  // introsort depth-limit fallbacks
 	unsigned long long timeouts;   // bounded loops that gave up
-	unsigned long long rounds;     // CTA greedy rounds
-	unsigned long long passes;     // parallel decision passes over all rounds
-	unsigned long long serial;     // rounds that needed the in-order decision warp
+	unsigned long long rounds;     // rounds of the grid-based acceptance
+	unsigned long long passes;     // its parallel decision passes
+	unsigned long long serial;     // its rounds that needed the in-order decision warp
 	unsigned long long list_entries; // conflict-list entries written
-	unsigned long long cluster_nodes; // nodes accepted by a CTA cluster
+	unsigned long long cluster_nodes; // nodes decided by 1,024 threads
 	unsigned long long cycles[7];  // CTA greedy: SM cycles of thread 0 in phases A, B, C1, C2, D; cells read past 3 and 7 points
 };
 
@@ -80,20 +80,19 @@ void launch_gather_records(const uint32_t* ids, int64_t n, const int32_t* X, con
                            int64_t n_src = 0);
 // std::sort emulation per node; `order` lists node indices, largest first.
 // Nodes order[0..num_big) (the largest) get one CTA each, the rest one warp.
-// Which kernel shape samples which node of a level: nodes of at least
-// cta_min candidates get a CTA each (small_level_cta_min on levels with
-// fewer nodes than 2 x SMs), those of at least cluster_min a cluster of
-// CTAs, the rest a warp each, pulled from a device work queue by
-// warp_blocks_per_sm resident blocks per SM. The compiled-in values come from
-// the autotuner's table (tuned_schedule.h, written by
-// potreeconverter_b200/autotune.py); PCG_SCHEDULE="cta_min,small_level_cta_min,
-// cluster_min,warp_blocks_per_sm" in the environment overrides them (read at
-// every level, for the autotuner's sweep).
+// How many threads decide which node of a level (accept.cu): nodes of at
+// least cluster_min candidates get 1,024, those of at least cta_min
+// (small_level_cta_min on levels with fewer nodes than 2 x SMs) 16 x middle
+// (128, 256 or 512), smaller ones 128. The compiled-in values come from the
+// autotuner's table (tuned_schedule.h, written by
+// potreeconverter_b200/autotune.py); PCG_SCHEDULE="cta_min,
+// small_level_cta_min,cluster_min,middle" in the environment overrides them
+// (read at every level, for the autotuner's sweep).
 struct LevelSchedule {
 	int64_t cta_min;
 	int64_t small_level_cta_min;
 	int64_t cluster_min;
-	int warp_blocks_per_sm;
+	int middle;
 };
 LevelSchedule level_schedule();
 void launch_node_sort(const LevelNode* nodes, const int32_t* order, int K, LevelBuffers& lb, SampleStats* st, DeviceMem& mem,
@@ -141,38 +140,63 @@ void replay_segments(double* key, int32_t* val, int64_t M, const std::vector<Sor
 int sort_depth_budget(int64_t n);
 // lb.pos of the nodes k with pick[k] != 0, from their sorted lb.perm
 void launch_node_pos(const LevelNode* nodes, const std::vector<uint8_t>& pick, LevelBuffers& lb, DeviceMem& mem);
+// The candidates of a level sorted by cell (conflicts.cu): cells of one
+// spacing, a node's records in its own range [cand_off, cand_off + count).
+struct LevelCells {
+	uint4* rows = nullptr;      // [K x 128 x 128] occupied cells of the row (z, y), a bit per x
+	uint32_t* base = nullptr;   // [K x 128 x 128] the node's occupied cells before the row
+	uint32_t* start = nullptr;  // [M + 1] first record of occupied cell r of a node, at cand_off + r
+	float4* rec = nullptr;      // [M] position relative to the node's minimum corner, sorted position
+	uint32_t* cell = nullptr;   // [M] the record's cell, z << 14 | y << 7 | x
+	uint64_t* col = nullptr;    // [M] the record's colour (poisson_average)
+};
+// from lb.rec, lb.pos and lb.cols
+void build_level_cells(const LevelNode* d_nodes, const PosParamsS& pp, LevelBuffers& lb, LevelCells& lc, DeviceMem& mem);
+void free_level_cells(LevelCells& lc, DeviceMem& mem);
 // Earlier candidates of the same node that would reject a candidate if
 // accepted (within the spacing and, for poisson, not before the early-exit
-// bound), by sorted position; built for the nodes flagged in `use`.
-// A list holds at most kListCap entries: the first kListInline in the
-// candidate's own 16-byte slot, the rest in a pool shared by the level
-// (lists average about one entry, so a fixed row per candidate would be
-// mostly empty).
+// bound), by sorted position, in any order. A list of up to kListCap entries
+// lies in the candidate's own 16-byte slot (the first kListInline) and in a
+// pool shared by the level (lists average about one entry, so a fixed row per
+// candidate would be mostly empty); a longer one in a second pool.
 constexpr int kListCap = 32;
 constexpr int kListInline = 4;
-constexpr uint8_t kListDense = 255;
+constexpr int kListCount = 63;           // bits of ConflictLists::count that hold the length
+constexpr uint8_t kListDistant = 64;     // poisson: an entry lies more than 10,001 positions back
+constexpr uint8_t kListLong = 255;
+struct LongList {
+	int64_t off;     // first entry in long_pool
+	int32_t record;  // the candidate's record in cell order
+	int32_t count;
+};
 struct ConflictLists {
 	int4* inl = nullptr;            // [M] first entries (node-local sorted positions)
-	int32_t* ovf_off = nullptr;     // [M] where entries kListInline.. start in pool
+	int32_t* ovf_off = nullptr;     // [M] where entries kListInline.. start in pool; a long list's index
 	int32_t* pool = nullptr;        // [pool_cap] the longer lists' remaining entries
-	unsigned long long* pool_used = nullptr;  // entries handed out of pool
 	int64_t pool_cap = 0;
-	uint8_t* count = nullptr;       // [M] by sorted position: entries, or kListDense past kListCap
-	uint8_t* node_dense = nullptr;  // [K] some candidate has more than kListCap
+	LongList* longs = nullptr;      // [long_cap]
+	int64_t long_cap = 0;
+	int32_t* long_pool = nullptr;
+	uint8_t* count = nullptr;       // [M] by sorted position: entries (| kListDistant), or kListLong past kListCap
+	unsigned long long* pool_used = nullptr;  // entries of pool handed out (one allocation with the next three)
+	unsigned long long* long_used = nullptr;     // long lists
+	unsigned long long* long_entries = nullptr;  // their entries
+	unsigned long long* node_long = nullptr;     // [K] their entries by node
 };
-
-// entries 4w .. 4w + 3 of the list of candidate slot `idx` (nl entries);
-// positions past the list read as 0
-__device__ __forceinline__ int4 list_quad(const ConflictLists& cl, int64_t idx, int nl, int w) {
-	if (w == 0) return cl.inl[idx];
-	const int32_t* p = cl.pool + cl.ovf_off[idx] + 4 * (w - 1);
-	const int e = 4 * w;
-	return make_int4(e < nl ? p[0] : 0, e + 1 < nl ? p[1] : 0, e + 2 < nl ? p[2] : 0, e + 3 < nl ? p[3] : 0);
-}
-void build_conflict_lists(int mode, const LevelNode* d_nodes, const std::vector<LevelNode>& ln, const std::vector<uint8_t>& use,
-                          const PosParamsS& pp, LevelBuffers& lb, ConflictLists& cl, std::vector<uint8_t>& dense, SampleStats* st,
-                          DeviceMem& mem);
+// Nodes flagged in `dense` have no lists (conflicts.cu kLongBudget).
+void build_conflict_lists(int mode, const LevelNode* d_nodes, int K, const PosParamsS& pp, LevelBuffers& lb, const LevelCells& lc,
+                          ConflictLists& cl, std::vector<uint8_t>& dense, SampleStats* st, DeviceMem& mem);
 void free_conflict_lists(ConflictLists& cl, DeviceMem& mem);
+// Acceptance from conflict lists (accept.cu): a bit per candidate by sorted
+// position, node k's words from accept_word(cand_off, k) on (a multiple of 4).
+__host__ __device__ inline int64_t accept_word(int64_t cand_off, int node) { return ((cand_off >> 7) + node) * 4; }
+inline int64_t accept_words(int64_t M, int K) { return ((M >> 7) + K + 1) * 4; }
+// decides every node that is not dense; lb.accepted of their candidates
+void launch_accept(int mode, const LevelNode* d_nodes, const std::vector<LevelNode>& ln, const std::vector<uint8_t>& dense, LevelBuffers& lb,
+                   const ConflictLists& cl, uint32_t* accepted_bits, SampleStats* st, DeviceMem& mem);
+// poisson_average's colours of those nodes, into lb.cols
+void launch_cell_colors(const LevelNode* d_nodes, const std::vector<uint8_t>& dense, const PosParamsS& pp, LevelBuffers& lb,
+                        const LevelCells& lc, const uint32_t* accepted_bits, DeviceMem& mem);
 // sorted candidate records lb.cq from lb.perm
 void launch_cand_records(const LevelNode* nodes, const int32_t* X, const int32_t* Y, const int32_t* Z, LevelBuffers& lb, DeviceMem& mem);
 // Acceptance grids of the CTA-per-node greedy, one per resident CTA. They
@@ -189,18 +213,11 @@ void launch_greedy(int mode, bool fp32_guard, const LevelNode* nodes, const int3
                    const int32_t* Z, const PosParamsS& pp, LevelBuffers& lb, uint64_t* hash_keys, int32_t* hash_heads,
                    double* acc_xyz, double* acc_key, int32_t* acc_next, int32_t* acc_pos, SampleStats* st, DeviceMem& mem,
                    GreedyArena* grid, int node_begin = 0, int node_end = -1, int num_big = 0);
-// acceptance from conflict lists: cta_nodes (largest first) get a cluster of
-// CTAs each when they hold at least 65,536 candidates, else one CTA;
-// warp_nodes a warp each
-void launch_greedy_lists(int mode, const LevelNode* nodes, const std::vector<int32_t>& cta_nodes, const std::vector<int32_t>& warp_nodes,
-                         const PosParamsS& pp, LevelBuffers& lb, uint64_t* hash_keys, int32_t* hash_heads, double* acc_xyz,
-                         double* acc_key, int32_t* acc_next, int32_t* acc_pos, const ConflictLists& cl, SampleStats* st, DeviceMem& mem,
-                         const std::vector<LevelNode>& ln);
 // poisson_average colour sums: new packed colour per accepted candidate
+// (of the nodes flagged in `only`, device memory, or of all)
 void launch_average_colors(const LevelNode* nodes, const int32_t* X, const int32_t* Y, const int32_t* Z, const PosParamsS& pp,
                            LevelBuffers& lb, const uint64_t* hash_keys, const int32_t* hash_heads, const double* acc_xyz,
-                           const int32_t* acc_next, const int32_t* acc_pos, const int64_t* acc_base, long long* sums,
-                           DeviceMem& mem);
+                           const int32_t* acc_next, const int32_t* acc_pos, const uint8_t* only, long long* sums, DeviceMem& mem);
 void launch_random_accept_sized(const LevelNode* nodes, const int32_t* X, const int32_t* Y, const int32_t* Z, const PosParamsS& pp,
                                 LevelBuffers& lb, uint64_t* hash_keys, int32_t* hash_vals, int64_t hash_total, SampleStats* st,
                                 DeviceMem& mem);
