@@ -31,7 +31,7 @@
 //     coordinates decides every pair outside the band s^2 (1 -/+ 1e-3);
 //     pairs inside the band are decided by the reference's FP64 test and
 //     counted as escalated; then the early-exit bound. (27 hash probes per
-//     candidate took 30.6 ms of a 50M-point conversion, this 17.2.)
+//     candidate took 30.6 ms of a 50M-point conversion, this 13.3.)
 //
 // Error bound of the FP32 test (u = 2^-24): a node-relative coordinate v lies
 // in [0, L], L = 128 s, so its float differs from the FP64 value by at most
@@ -41,7 +41,7 @@
 // distance D. The FP64 values the reference compares are themselves within
 // 1.1e-16 |x| of the exact coordinates, below 1.1e-10 s when |x| < 1e6 s
 // (checked per node; beyond it the node uses FP64 alone). So D32 >= s^2 (1 +
-// 1e-3) (rounded up by at most u) implies D64 > s^2, and D32 < s^2 (1 - 1e-3)
+// 1e-3) (rounded up by at most u; fused multiply-adds only drop roundings) implies D64 > s^2, and D32 < s^2 (1 - 1e-3)
 // implies D64 < s^2: the margin is 30x the error.
 //
 // The early-exit bound needs the earlier candidate's key only where it can
@@ -75,6 +75,9 @@ constexpr int kCellsPerAxis = 1 << kAxisBits;  // node box = 128 spacings
 constexpr int64_t kRows = (int64_t)kCellsPerAxis * kCellsPerAxis;  // of a node
 // entries of all long lists of a level (1 GiB)
 constexpr int64_t kLongBudget = int64_t(1) << 28;
+// six blocks an SM: 40 registers, a few spills outside the loop (50M points:
+// a loop per run: four blocks 17.0 ms, five 15.1, six 14.6, seven 19.4)
+constexpr int kListThreads = 256, kListBlocks = 6;
 
 __device__ __forceinline__ double qcoord(int32_t X, int a, const PosParamsS& pp) {
 	// (xyz[a] * scale) + offset, sampler_poisson.h:99-101
@@ -226,101 +229,122 @@ __device__ __forceinline__ int find_runs(uint32_t c, uint32_t co, const uint4* _
 	return n;
 }
 
+// A thread's way through its runs, one record after the other and the next one
+// loaded ahead. (A loop per run costs a warp the longest of its lanes' runs
+// nine times over: 14 of 32 lanes were at work, so it is 20, and the search of
+// 162M candidates' lists fell from 17.4 ms to 13.3.)
+struct RunWalk {
+	uint2* runs;
+	const float4* rec;
+	uint2 run;
+	float4 next;
+	uint32_t left;
+	int stride;
+
+	// runs: this thread's n runs, and room for one more
+	__device__ __forceinline__ RunWalk(uint2* r, int n, int stride_, const float4* rec_) : runs(r), rec(rec_), left(0), stride(stride_) {
+		for (int q = 0; q < n; q++) left += runs[q * stride].y - runs[q * stride].x;
+		run = runs[0];
+		runs[n * stride] = run;  // what is loaded after the last record
+		next = rec[run.x];
+	}
+	// the record, and in k its index; left is above 0
+	__device__ __forceinline__ float4 take(uint32_t& k) {
+		const float4 r = next;
+		k = run.x;
+		if (++run.x == run.y) run = *(runs += stride);
+		next = rec[run.x];
+		left--;
+		return r;
+	}
+};
+
 // What a candidate p is compared with: whether a record q could reject it.
 template <int MODE>
 struct PairTest {
 	float4 mf;
 	int32_t t;
-	double s2, lim;
-	float s2hi, s2lo;
-	bool pre32, far_from_centre;
-	int64_t co;
+	float s2hi, s2lo;  // NaN and -1 where FP64 alone decides
+	bool far_from_centre;
 	unsigned escalated;
+	const LevelNode& nd;
 
-	__device__ __forceinline__ PairTest(const LevelNode& nd, const LevelBuffers& lb, const float4& rec) {
+	__device__ __forceinline__ PairTest(const LevelNode& node, const float4& rec) : nd(node) {
 		mf = rec;
 		t = __float_as_int(rec.w);
-		co = nd.cand_off;
-		const double sp = nd.spacing;
-		s2 = sp * sp;
-		lim = 0.0;
-		far_from_centre = true;
-		if (MODE == 0) {
-			// the early-exit bound of the acceptance kernels, same expression
-			const double cd = sqrt(lb.keys[co + t]);
-			const double limit = cd - sp;
-			lim = limit * limit;
-			far_from_centre = cd > 1.1 * sp;
-		}
+		escalated = 0;
+		const double sp = nd.spacing, s2 = sp * sp;
 		double amax = 0.0;
 		for (int a = 0; a < 3; a++) amax = fmax(amax, fmax(fabs(nd.min[a]), fabs(nd.max[a])));
-		pre32 = s2 > 1e-30 && s2 < 1e30 && amax < 1e6 * sp;
-		s2hi = (float)(s2 * 1.001);
-		s2lo = (float)(s2 * 0.999);
-		escalated = 0;
+		const bool pre32 = s2 > 1e-30 && s2 < 1e30 && amax < 1e6 * sp;
+		s2hi = pre32 ? (float)(s2 * 1.001) : __int_as_float(0x7fffffff);
+		s2lo = pre32 ? (float)(s2 * 0.999) : -1.0f;
+		// c >= 1.1 s: 1.25 s^2 leaves 3 % for the roundings of FP32
+		const float cx = mf.x - (float)(0.5 * (nd.max[0] - nd.min[0])), cy = mf.y - (float)(0.5 * (nd.max[1] - nd.min[1])),
+		            cz = mf.z - (float)(0.5 * (nd.max[2] - nd.min[2]));
+		far_from_centre = MODE != 0 || cx * cx + cy * cy + cz * cz > 1.25f * (float)s2;
 	}
-	// squaredDistance(point, candidate), sampler_poisson.h:117-125
-	__device__ __forceinline__ bool exact(const LevelBuffers& lb, const PosParamsS& pp, int32_t u) const {
-		const int4 q = lb.rec[co + lb.perm[co + u]], me = lb.rec[co + lb.perm[co + t]];
-		const double dx = qcoord(q.x, 0, pp) - qcoord(me.x, 0, pp), dy = qcoord(q.y, 1, pp) - qcoord(me.y, 1, pp),
-		             dz = qcoord(q.z, 2, pp) - qcoord(me.z, 2, pp);
-		return dx * dx + dy * dy + dz * dz < s2;
-	}
-	// the record's sorted position is u < t
-	__device__ __forceinline__ bool operator()(const float4& qf, int32_t u, const LevelBuffers& lb, const PosParamsS& pp) {
-		const float fx = qf.x - mf.x, fy = qf.y - mf.y, fz = qf.z - mf.z;
-		const float d2 = fx * fx + fy * fy + fz * fz;
-		if (pre32 && d2 >= s2hi) return false;
-		const bool inside = pre32 && d2 < s2lo;
+	// as the reference compares: squaredDistance(point, candidate),
+	// sampler_poisson.h:117-125, and the early-exit bound
+	__device__ __forceinline__ bool exact(const LevelBuffers& lb, const PosParamsS& pp, int32_t u, bool inside) {
+		const int64_t co = nd.cand_off;
+		const double sp = nd.spacing;
 		if (!inside) {
 			escalated++;
-			if (!exact(lb, pp, u)) return false;
+			const int4 q = lb.rec[co + lb.perm[co + u]], me = lb.rec[co + lb.perm[co + t]];
+			const double dx = qcoord(q.x, 0, pp) - qcoord(me.x, 0, pp), dy = qcoord(q.y, 1, pp) - qcoord(me.y, 1, pp),
+			             dz = qcoord(q.z, 2, pp) - qcoord(me.z, 2, pp);
+			if (!(dx * dx + dy * dy + dz * dz < sp * sp)) return false;
 		}
-		if (MODE == 0 && !(inside && far_from_centre) && !(lb.keys[co + u] >= lim)) return false;
-		return true;
+		if (MODE != 0) return true;
+		const double limit = sqrt(lb.keys[co + t]) - sp;
+		return lb.keys[co + u] >= limit * limit;
+	}
+	// qf: the record, u: its sorted position; a wanted one could reject
+	__device__ __forceinline__ bool operator()(const float4& qf, int32_t u, bool wanted, const LevelBuffers& lb, const PosParamsS& pp) {
+		const float fx = qf.x - mf.x, fy = qf.y - mf.y, fz = qf.z - mf.z;
+		const float d2 = __fmaf_rn(fz, fz, __fmaf_rn(fy, fy, fx * fx));
+		bool hit = wanted && !(d2 >= s2hi);
+		const bool inside = d2 < s2lo;
+		if (hit && !(inside && far_from_centre)) hit = exact(lb, pp, u, inside);
+		return hit;
 	}
 };
 
 // One thread per record in cell order; a thread's runs wait in shared memory.
 template <int MODE>
-__global__ void __launch_bounds__(256, 5) conf_lists_kernel(const LevelNode* __restrict__ nodes, PosParamsS pp, LevelBuffers lb, LevelCells lc,
-                                                            ConflictLists cl, SampleStats* st) {
-	__shared__ uint2 runs[9][256];
+__global__ void __launch_bounds__(kListThreads, kListBlocks) conf_lists_kernel(const LevelNode* __restrict__ nodes, PosParamsS pp, LevelBuffers lb,
+                                                                               LevelCells lc, ConflictLists cl, SampleStats* st) {
+	__shared__ uint2 runs[10][kListThreads];
 	const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
 	const int lane = threadIdx.x & 31;
 	unsigned escalated = 0;
 	int n = 0;
 	bool distant = false;
 	int64_t slot = 0;
-	int32_t rest[kListCap - kListInline];
+	int32_t list[kListCap + 1];
 	if (i < lb.M) {
 		const int32_t node = lb.node_of[i];  // a node's records keep its range
 		const LevelNode& nd = nodes[node];
 		const int64_t co = nd.cand_off;
 		const int nr = find_runs(lc.cell[i], (uint32_t)co, lc.rows + (int64_t)node * kRows, lc.base + (int64_t)node * kRows, lc.start,
-		                         &runs[0][threadIdx.x], 256);
-		PairTest<MODE> test(nd, lb, lc.rec[i]);
+		                         &runs[0][threadIdx.x], kListThreads);
+		PairTest<MODE> test(nd, lc.rec[i]);
 		const int32_t t = test.t;
-		int4 inl = make_int4(0, 0, 0, 0);
+		RunWalk walk(&runs[0][threadIdx.x], nr, kListThreads, lc.rec);
 #pragma unroll 1
-		for (int q = 0; q < nr; q++) {
-			const uint2 run = runs[q][threadIdx.x];
-#pragma unroll 2
-			for (uint32_t k = run.x; k < run.y; k++) {
-				const float4 qf = lc.rec[k];
-				const int32_t u = __float_as_int(qf.w);
-				if (u >= t || !test(qf, u, lb, pp)) continue;
-				if (n == 0) inl.x = u;
-				else if (n == 1) inl.y = u;
-				else if (n == 2) inl.z = u;
-				else if (n == 3) inl.w = u;
-				else if (n < kListCap) rest[n - kListInline] = u;
-				n++;
-				if (MODE == 0) distant |= t - u > 10001;
-			}
+		while (walk.left) {
+			uint32_t k;
+			const float4 qf = walk.take(k);
+			const int32_t u = __float_as_int(qf.w);
+			const bool hit = test(qf, u, u < t, lb, pp);
+			if (hit) list[n < kListCap ? n : kListCap] = u;
+			n += hit;
 		}
+		if (MODE == 0 && n <= kListCap)
+			for (int e = 0; e < n; e++) distant |= t - list[e] > 10001;
 		slot = co + t;
-		cl.inl[slot] = inl;
+		cl.inl[slot] = make_int4(n > 0 ? list[0] : 0, n > 1 ? list[1] : 0, n > 2 ? list[2] : 0, n > 3 ? list[3] : 0);
 		cl.count[slot] = (uint8_t)(n > kListCap ? kListLong : n | (distant ? kListDistant : 0));
 		escalated = test.escalated;
 		if (n > kListCap) {
@@ -347,7 +371,7 @@ __global__ void __launch_bounds__(256, 5) conf_lists_kernel(const LevelNode* __r
 		at = __shfl_sync(FULL, at, 31) + x - extra;
 		if (extra && (int64_t)(at + extra) <= cl.pool_cap) {
 			cl.ovf_off[slot] = (int32_t)at;
-			for (uint32_t e = 0; e < extra; e++) cl.pool[at + e] = rest[e];
+			for (uint32_t e = 0; e < extra; e++) cl.pool[at + e] = list[kListInline + e];
 		}
 	}
 	const unsigned entries = __reduce_add_sync(FULL, (unsigned)n);
@@ -373,7 +397,7 @@ __global__ void __launch_bounds__(128) conf_long_kernel(const LevelNode* __restr
 	const LevelNode& nd = nodes[node];
 	const int nr = find_runs(lc.cell[i], (uint32_t)nd.cand_off, lc.rows + (int64_t)node * kRows, lc.base + (int64_t)node * kRows, lc.start,
 	                         &runs[0][threadIdx.x], 128);
-	PairTest<MODE> test(nd, lb, lc.rec[i]);
+	PairTest<MODE> test(nd, lc.rec[i]);
 	int32_t* out = cl.long_pool + l.off;
 	int n = 0;
 #pragma unroll 1
@@ -386,7 +410,7 @@ __global__ void __launch_bounds__(128) conf_long_kernel(const LevelNode* __restr
 			if (k < run.y) {
 				const float4 qf = lc.rec[k];
 				u = __float_as_int(qf.w);
-				hit = u < test.t && test(qf, u, lb, pp);
+				hit = test(qf, u, u < test.t, lb, pp);
 			}
 			const unsigned hits = __ballot_sync(FULL, hit);
 			const int at = n + __popc(hits & lanemask_lt());
@@ -443,7 +467,7 @@ __global__ void __launch_bounds__(kCompact) accepted_records_kernel(const LevelN
 // point sums over the records around it (no two accepted points lie within
 // the spacing); colours lie in cell order, beside the records. Bound by the
 // records and colours read; scattered atomics from the rejected side through
-// a hash of the accepted points took 4.04 ms for 31M candidates, this 2.25.
+// a hash of the accepted points took 4.04 ms for 31M candidates, this 2.07.
 __global__ void __launch_bounds__(128) cell_colors_kernel(const LevelNode* __restrict__ nodes, PosParamsS pp, LevelBuffers lb, LevelCells lc,
                                                           const uint32_t* __restrict__ list, const unsigned int* __restrict__ num) {
 	__shared__ uint2 runs[9][128];
@@ -454,7 +478,7 @@ __global__ void __launch_bounds__(128) cell_colors_kernel(const LevelNode* __res
 		const int64_t co = nd.cand_off;
 		const int nr = find_runs(lc.cell[i], (uint32_t)co, lc.rows + (int64_t)node * kRows, lc.base + (int64_t)node * kRows, lc.start,
 		                         &runs[0][threadIdx.x], 128);
-		PairTest<1> test(nd, lb, lc.rec[i]);
+		PairTest<1> test(nd, lc.rec[i]);
 		unsigned long long r = 0, g = 0, b = 0, w = 0;
 		auto add = [&](uint64_t col, unsigned f) {
 			r += (unsigned long long)(f * (uint32_t)(col & 0xffff));
@@ -463,13 +487,14 @@ __global__ void __launch_bounds__(128) cell_colors_kernel(const LevelNode* __res
 			w += f;
 		};
 		add(lc.col[i], 2);
+		// (a loop per run: with a RunWalk 31M candidates took 2.29 ms)
 #pragma unroll 1
 		for (int q = 0; q < nr; q++) {
 			const uint2 run = runs[q][threadIdx.x];
 			for (uint32_t k = run.x; k < run.y; k++) {
 				const float4 qf = lc.rec[k];
 				const int32_t u = __float_as_int(qf.w);
-				if (u != test.t && test(qf, u, lb, pp)) add(lc.col[k], u < test.t ? 2u : 1u);
+				if (test(qf, u, u != test.t, lb, pp)) add(lc.col[k], u < test.t ? 2u : 1u);
 			}
 		}
 		// rgbTarget = p.r / p.w (sampler_poisson_average.h:443-445)
@@ -533,6 +558,7 @@ void build_conflict_lists(int mode, const LevelNode* d_nodes, int K, const PosPa
 	if (M == 0 || K == 0) return;
 	cudaStream_t s = mem.stream();
 	const unsigned blocks = (unsigned)ceil_div(M, 256);
+	const unsigned list_blocks = (unsigned)ceil_div(M, kListThreads);
 	cl.inl = mem.alloc<int4>(M);
 	cl.ovf_off = mem.alloc<int32_t>(M);
 	cl.count = mem.alloc<uint8_t>(M);
@@ -553,8 +579,8 @@ void build_conflict_lists(int mode, const LevelNode* d_nodes, int K, const PosPa
 	for (int attempt = 0; attempt < 2; attempt++) {
 		PCG_CUDA(cudaMemsetAsync(used, 0, (3 + (size_t)K) * sizeof(unsigned long long), s));
 		PCG_CUDA(cudaMemsetAsync(lst, 0, sizeof(SampleStats), s));
-		if (mode == 0) conf_lists_kernel<0><<<blocks, 256, 0, s>>>(d_nodes, pp, lb, lc, cl, lst);
-		else conf_lists_kernel<1><<<blocks, 256, 0, s>>>(d_nodes, pp, lb, lc, cl, lst);
+		if (mode == 0) conf_lists_kernel<0><<<list_blocks, kListThreads, 0, s>>>(d_nodes, pp, lb, lc, cl, lst);
+		else conf_lists_kernel<1><<<list_blocks, kListThreads, 0, s>>>(d_nodes, pp, lb, lc, cl, lst);
 		PCG_LAUNCHED();
 		PCG_CUDA(cudaMemcpyAsync(h.data(), used, h.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
 		PCG_CUDA(cudaStreamSynchronize(s));

@@ -4,6 +4,6 @@
 // hand-set defaults until a sweep has run.
 #pragma once
 #define PCG_TUNED_CTA_MIN 8192
-#define PCG_TUNED_SMALL_LEVEL_CTA_MIN 1024
+#define PCG_TUNED_SMALL_LEVEL_CTA_MIN 4096
 #define PCG_TUNED_CLUSTER_MIN 131072
 #define PCG_TUNED_WARP_BLOCKS_PER_SM 32
