@@ -18,6 +18,20 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
 	return m;
 }
 
+// The lanes whose 8-bit digit equals this lane's, of all 32. (Eight ballots:
+// __match_any_sync, which works through a warp's distinct values one by one,
+// took a radix scatter of 162M candidates 4.03 ms for 3.19.)
+__device__ __forceinline__ uint32_t digit_peers(int digit) {
+	uint32_t p = FULL;
+#pragma unroll
+	for (int b = 0; b < 8; b++) {
+		const bool bit = digit >> b & 1;
+		const uint32_t m = __ballot_sync(FULL, bit);
+		p &= bit ? m : ~m;
+	}
+	return p;
+}
+
 constexpr int kWarpsPerBlock = 4;            // warp-per-node kernels: warps per CTA
 constexpr int kBigThreads = 512;             // CTA-per-node kernels
 constexpr int kBigWarps = kBigThreads / 32;

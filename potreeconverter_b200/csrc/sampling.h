@@ -97,16 +97,9 @@ struct LevelSchedule {
 LevelSchedule level_schedule();
 void launch_node_sort(const LevelNode* nodes, const int32_t* order, int K, LevelBuffers& lb, SampleStats* st, DeviceMem& mem,
                       int node_begin = 0, int node_end = -1, int num_big = 0);
-// Exact ascending sort of every node's keys (segmented LSD radix sort of the
-// key bits). Nodes whose keys are pairwise distinct end sorted in lb.keys,
+// Exact ascending sort of every node's keys (segmented LSD radix sort). Nodes whose keys are pairwise distinct end sorted in lb.keys,
 // lb.perm and lb.pos, which is std::sort's unique result for them; nodes with
 // equal keys are left as they were and flagged in tie[k] for the replay.
-// Stable sort of every node's (key, value) pairs by key bits [begin_bit, end_bit) into
-// (keys_out, vals_out), each node within its own range [cand_off,
-// cand_off + count). vals_in == nullptr means value = index in the node.
-// keys_in must not alias keys_out.
-void segmented_sort_pairs(const std::vector<LevelNode>& ln, int64_t M, const uint64_t* keys_in, const uint32_t* vals_in,
-                          uint64_t* keys_out, uint32_t* vals_out, int begin_bit, int end_bit, DeviceMem& mem);
 // The radix-sorted keys of a level, kept for the replay of the nodes with
 // equal keys. A segment of the replay whose keys are pairwise distinct ends
 // in ascending order whatever its partitions do (the unique sorted order of

@@ -9,21 +9,32 @@
 // order among equal keys is an artefact of the partitions.
 //
 // This unit sorts every node of a level at once with a segmented LSD radix
-// sort of the high 32 key bits (keys are finite and >= +0, so their IEEE bit
-// patterns order like the values), puts each short run of equal high words
-// in full-key order in place (a node with a run longer than 32 gets all 64
-// bits by radix instead), then flags the nodes that hold two equal adjacent
-// keys. Segmentation comes from the tiling: tiles never straddle a
-// node, and the per-tile digit counts are laid out node-major, digit-major,
-// tile-minor, so one flat exclusive scan of the count matrix yields, for
-// every (node, digit, tile), the output position inside the node's own range
-// [cand_off, cand_off + count). Elements therefore never leave their node, and
-// no pass over the node index is needed.
+// sort. Only 24 bits go through it, three passes of 8 bytes (quantised key,
+// index) per candidate: the key times a constant of the node that takes its
+// largest possible distance to 2^24, rounded down, which never reverses an
+// order. 20 mantissa bits of the FP64 pattern resolve less for all but the
+// candidates in the inner 27 of a node's 64 spacings. The fix kernel then
+// reads the full keys in the order found, puts each short run of equal
+// quantised keys in full-key order, and flags the nodes that hold two equal
+// keys; a node with a run longer than kLowRunMax (but for one of equal keys)
+// is sorted again on all 64 bits of its keys (finite and >= +0, so their
+// IEEE bit patterns order like the values).
 //
-// A pass reads 12 bytes (key, value) and writes 12 bytes per candidate; the
-// counting pass reads the 8-byte key. Within a tile, ranks come from
-// __match_any_sync peer masks in warp order (stable), the tile is reordered in
-// shared memory, and each digit's run is written out contiguously.
+// Segmentation comes from the tiling: tiles never straddle a node. A pass
+// counts each tile's digits, one block per node turns the counts into
+// positions (per digit over the tiles, then over the digits), and the scatter
+// places the tile. The counts lie tile by tile, 256 words together, so all
+// three kernels read and write them in whole lines. Within a tile, ranks come
+// from ballots of the digit's bits in warp order (stable), the tile is
+// reordered in shared memory, and each digit's run is written out
+// contiguously.
+//
+// Measured, 162M candidates of a 50M-point conversion: counts 1.1 ms (shared
+// atomics: the digits of a tile spread; by peer masks 3.4), positions 0.4,
+// scatters 3.0, fixing 2.1. Four passes over the high 32 bits of the FP64 keys,
+// 12 bytes per candidate each, with one scan over the level's counts in
+// digit order, then separate kernels for the low bits, the ties and the
+// results took 14.
 
 #include <cuda_runtime.h>
 
@@ -39,80 +50,173 @@ namespace {
 
 constexpr int kSegThreads = 256;
 constexpr int kSegWarps = kSegThreads / 32;
-// 2048-element tiles: the downsweep keeps a tile's keys, values and ranks in
-// registers, and at 8 per thread it fits 64 registers, four blocks per SM
-// (16 per thread took 106 registers, two blocks, and waited on memory)
-constexpr int kSegSteps = 8;
-constexpr int kSegTile = kSegThreads * kSegSteps;  // 2048
 constexpr int kSegDigits = 256;
 static_assert(kSegThreads == kSegDigits, "one thread per digit");
+constexpr int kQuantBits = 24;
 
-struct SegTile {
-	int64_t start;     // first candidate (level-wide index)
-	int64_t node_off;  // cand_off of the tile's node
-	int64_t adjust;    // node_off minus the candidates of the nodes before it in the count matrix
-	int64_t cnt_base;  // count-matrix index of (digit 0, this tile)
-	int32_t count;     // candidates in the tile, <= kSegTile
-	int32_t stride;    // tiles of the node = count-matrix stride between digits
+// Tiles of 2,048: a warp ranks 8 x 32 candidates, all kept in registers, and
+// four blocks fit an SM. (32-bit keys, 162M candidates, three passes: 8 steps
+// and four blocks 3.14 ms, five blocks 3.24, 12 steps 3.17, 16 steps 4.9;
+// 64-bit keys at 16 steps took 106 registers, two blocks, and waited on
+// memory.)
+constexpr int kSegSteps = 8;
+constexpr int kSegTile = kSegThreads * kSegSteps;
+
+struct SegNode {
+	int64_t off;    // first candidate (level-wide index)
+	int64_t count;
+	double scale;   // key -> quantised key
+	int32_t tile0;  // its first tile
+	int32_t tiles;
 };
 
+struct SegTile {
+	int64_t start;     // first candidate
+	int64_t node_off;  // of the tile's node
+	double scale;
+	int32_t count;     // candidates in the tile
+	int32_t node;
+};
+
+__device__ __forceinline__ uint32_t quantised(uint64_t key, double scale) {
+	const uint32_t q = __double2uint_rd(__longlong_as_double((long long)key) * scale);
+	return q < (1u << kQuantBits) - 1 ? q : (1u << kQuantBits) - 1;
+}
+
+template <class K>
 struct SegShared {
-	uint64_t key[kSegTile];
+	K key[kSegTile];
 	uint32_t val[kSegTile];
 	uint32_t whist[kSegWarps][kSegDigits];
 	int64_t gbase[kSegDigits];
 	uint32_t wsum[kSegWarps];
 };
 
-__global__ void __launch_bounds__(kSegThreads) seg_upsweep(const SegTile* __restrict__ tiles, const uint64_t* __restrict__ keys, int shift,
-                                                         uint32_t* __restrict__ counts) {
+__global__ void seg_tiles_kernel(const SegNode* __restrict__ nodes, int K, int num_tiles, SegTile* __restrict__ tiles) {
+	const int i = blockIdx.x * blockDim.x + threadIdx.x;
+	if (i >= num_tiles) return;
+	int lo = 0, hi = K - 1;  // the last node whose first tile is <= i (empty ones have the next one's)
+	while (lo < hi) {
+		const int mid = (lo + hi + 1) >> 1;
+		if (nodes[mid].tile0 <= i) lo = mid;
+		else hi = mid - 1;
+	}
+	const SegNode n = nodes[lo];
+	const int64_t first = (int64_t)(i - n.tile0) * kSegTile;
+	SegTile t;
+	t.start = n.off + first;
+	t.node_off = n.off;
+	t.scale = n.scale;
+	t.count = (int32_t)(n.count - first < kSegTile ? n.count - first : kSegTile);
+	t.node = lo;
+	tiles[i] = t;
+}
+
+// FIRST: the keys are the node's, to be quantised when K has 32 bits
+template <class K, bool FIRST>
+__device__ __forceinline__ K seg_key(const void* keys, int64_t p, double scale) {
+	if (sizeof(K) == 4 && FIRST) return (K)quantised(static_cast<const uint64_t*>(keys)[p], scale);
+	return static_cast<const K*>(keys)[p];
+}
+
+template <class K, bool FIRST>
+__global__ void __launch_bounds__(kSegThreads) seg_count_kernel(const SegTile* __restrict__ tiles, const void* __restrict__ keys, int shift,
+                                                              uint32_t* __restrict__ counts) {
 	__shared__ uint32_t hist[kSegDigits];
 	const SegTile t = tiles[blockIdx.x];
 	hist[threadIdx.x] = 0;
 	__syncthreads();
-	const int lane = threadIdx.x & 31;
-	for (int base = 0; base < t.count; base += kSegThreads) {
-		const int i = base + (int)threadIdx.x;
-		const int digit = i < t.count ? (int)((keys[t.start + i] >> shift) & 0xff) : kSegDigits;
-		const uint32_t peers = __match_any_sync(FULL, digit);
-		if (digit < kSegDigits && lane == __ffs(peers) - 1) atomicAdd(&hist[digit], (uint32_t)__popc(peers));
+#pragma unroll
+	for (int s = 0; s < kSegSteps; s++) {
+		const int i = s * kSegThreads + (int)threadIdx.x;
+		if (i < t.count) atomicAdd(&hist[(seg_key<K, FIRST>(keys, t.start + i, t.scale) >> shift) & 0xff], 1u);
 	}
 	__syncthreads();
-	counts[t.cnt_base + (int64_t)threadIdx.x * t.stride] = hist[threadIdx.x];
+	counts[(int64_t)blockIdx.x * kSegDigits + threadIdx.x] = hist[threadIdx.x];
 }
 
-// vals_in == nullptr: first pass, the value is the candidate's index in its node
-__global__ void __launch_bounds__(kSegThreads, 4) seg_downsweep(const SegTile* __restrict__ tiles, const uint64_t* __restrict__ keys_in,
-                                                           const uint32_t* __restrict__ vals_in, uint64_t* __restrict__ keys_out,
-                                                           uint32_t* __restrict__ vals_out, int shift, const uint32_t* __restrict__ offsets) {
+// One block per node: a tile's count of a digit becomes the node's count of
+// that digit in the tiles before it; base: where the digit begins in the node.
+// kParts threads share a digit's tiles, each its own stretch of them.
+constexpr int kParts = 4;
+
+__global__ void __launch_bounds__(kSegDigits* kParts) seg_offsets_kernel(const SegNode* __restrict__ nodes, uint32_t* __restrict__ counts,
+                                                                         uint32_t* __restrict__ base) {
+	__shared__ uint32_t part[kParts][kSegDigits];
+	__shared__ uint32_t wsum[kSegDigits / 32];
+	const SegNode n = nodes[blockIdx.x];
+	if (n.tiles == 0) return;
+	const int d = threadIdx.x & (kSegDigits - 1), p = threadIdx.x / kSegDigits, lane = threadIdx.x & 31;
+	uint32_t* c = counts + (int64_t)n.tile0 * kSegDigits + d;
+	const int t0 = (int)((int64_t)n.tiles * p / kParts), t1 = (int)((int64_t)n.tiles * (p + 1) / kParts);
+	uint32_t sum = 0;
+#pragma unroll 8
+	for (int t = t0; t < t1; t++) sum += c[(int64_t)t * kSegDigits];
+	part[p][d] = sum;
+	__syncthreads();
+	uint32_t run = 0, total = 0;
+#pragma unroll
+	for (int k = 0; k < kParts; k++) {
+		run += k < p ? part[k][d] : 0;
+		total += part[k][d];
+	}
+	uint32_t x = total;
+#pragma unroll
+	for (int o = 1; o < 32; o <<= 1) {
+		const uint32_t y = __shfl_up_sync(FULL, x, o);
+		if (lane >= o) x += y;
+	}
+	if (p == 0 && lane == 31) wsum[d >> 5] = x;
+	__syncthreads();
+	if (p == 0) {
+		uint32_t before = 0;
+		for (int w = 0; w < d >> 5; w++) before += wsum[w];
+		base[(int64_t)blockIdx.x * kSegDigits + d] = before + x - total;
+	}
+#pragma unroll 8
+	for (int t = t0; t < t1; t++) {
+		const uint32_t v = c[(int64_t)t * kSegDigits];
+		c[(int64_t)t * kSegDigits] = run;
+		run += v;
+	}
+}
+
+// vals_in == nullptr: the value is the candidate's index in its node
+template <class K, bool FIRST>
+__global__ void __launch_bounds__(kSegThreads, 4) seg_scatter_kernel(const SegTile* __restrict__ tiles, const void* __restrict__ keys_in,
+                                                                     const uint32_t* __restrict__ vals_in, K* __restrict__ keys_out,
+                                                                     uint32_t* __restrict__ vals_out, int shift,
+                                                                     const uint32_t* __restrict__ counts, const uint32_t* __restrict__ base) {
 	extern __shared__ __align__(16) unsigned char seg_smem[];
-	SegShared& sh = *reinterpret_cast<SegShared*>(seg_smem);
+	SegShared<K>& sh = *reinterpret_cast<SegShared<K>*>(seg_smem);
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 	const SegTile t = tiles[blockIdx.x];
+	const uint32_t before_tile = counts[(int64_t)blockIdx.x * kSegDigits + tid] + base[(int64_t)t.node * kSegDigits + tid];
 	for (int i = tid; i < kSegWarps * kSegDigits; i += kSegThreads) (&sh.whist[0][0])[i] = 0;
 	__syncthreads();
-	uint64_t kr[kSegSteps];
+	K kr[kSegSteps];
 	uint32_t vr[kSegSteps], rr[kSegSteps];
 	const uint32_t lt = lanemask_lt();
 #pragma unroll
 	for (int s = 0; s < kSegSteps; s++) {
 		const int li = warp * (kSegSteps * 32) + s * 32 + lane;
-		uint64_t key = 0;
-		uint32_t val = 0;
-		int digit = kSegDigits;  // sentinel past the tile's end
+		kr[s] = 0;
+		vr[s] = 0;
 		if (li < t.count) {
 			const int64_t p = t.start + li;
-			key = keys_in[p];
-			val = vals_in ? vals_in[p] : (uint32_t)(p - t.node_off);
-			digit = (int)((key >> shift) & 0xff);
+			kr[s] = seg_key<K, FIRST>(keys_in, p, t.scale);
+			vr[s] = vals_in ? vals_in[p] : (uint32_t)(p - t.node_off);
 		}
-		const uint32_t peers = __match_any_sync(FULL, digit);
-		uint32_t before = digit < kSegDigits ? sh.whist[warp][digit] : 0u;
+	}
+#pragma unroll
+	for (int s = 0; s < kSegSteps; s++) {
+		const int li = warp * (kSegSteps * 32) + s * 32 + lane;
+		const int digit = li < t.count ? (int)((kr[s] >> shift) & 0xff) : kSegDigits;  // sentinel past the tile's end
+		const uint32_t peers = __ballot_sync(FULL, li < t.count) & digit_peers(digit);
+		const uint32_t before = digit < kSegDigits ? sh.whist[warp][digit] : 0u;
 		__syncwarp();
 		if (digit < kSegDigits && lane == __ffs(peers) - 1) sh.whist[warp][digit] = before + __popc(peers);
 		__syncwarp();
-		kr[s] = key;
-		vr[s] = val;
 		rr[s] = digit < kSegDigits ? before + __popc(peers & lt) : 0xffffffffu;
 	}
 	__syncthreads();
@@ -138,7 +242,7 @@ __global__ void __launch_bounds__(kSegThreads, 4) seg_downsweep(const SegTile* _
 	const uint32_t lbase = wbefore + x - run;  // exclusive over digits
 #pragma unroll
 	for (int w = 0; w < kSegWarps; w++) sh.whist[w][d] += lbase;
-	sh.gbase[d] = t.adjust + (int64_t)offsets[t.cnt_base + (int64_t)d * t.stride] - (int64_t)lbase;
+	sh.gbase[d] = t.node_off + (int64_t)before_tile - (int64_t)lbase;
 	__syncthreads();
 #pragma unroll
 	for (int s = 0; s < kSegSteps; s++) {
@@ -151,127 +255,156 @@ __global__ void __launch_bounds__(kSegThreads, 4) seg_downsweep(const SegTile* _
 	}
 	__syncthreads();
 	for (int L = tid; L < t.count; L += kSegThreads) {
-		const uint64_t key = sh.key[L];
+		const K key = sh.key[L];
 		const int64_t pos = sh.gbase[(key >> shift) & 0xff] + L;
 		keys_out[pos] = key;
 		vals_out[pos] = sh.val[L];
 	}
 }
 
-// After a sort on the high 32 key bits: every run of equal high words is
-// put in full-key order by its first element's thread (stable insertion
-// sort). Runs longer than kLowRunMax flag their node (bit 1) for a full sort.
-constexpr int kLowRunMax = 32;
+// The sorted level from the order of the quantised keys (q, v): a candidate
+// alone with its quantised key is in place; a run of equal ones is put in
+// full-key order by its first one's thread (stable insertion sort). A run
+// longer than kLowRunMax marks its node for a full sort, unless its keys are
+// all equal and it is no longer than kEqualRunMax.
+constexpr int kLowRunMax = 32, kEqualRunMax = 256;
 
-__global__ void seg_fix_low_kernel(const LevelNode* __restrict__ nodes, const int32_t* __restrict__ node_of, uint64_t* __restrict__ sk,
-                                   uint32_t* __restrict__ sv, int64_t M, uint8_t* __restrict__ flags) {
+__global__ void __launch_bounds__(256) seg_fix_kernel(const LevelNode* __restrict__ nodes, const uint32_t* __restrict__ q,
+                                                      const uint32_t* __restrict__ v, LevelBuffers lb, uint64_t* __restrict__ sk,
+                                                      uint32_t* __restrict__ sv, uint8_t* __restrict__ ties, uint8_t* __restrict__ redo) {
 	const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-	if (t >= M) return;
-	const int32_t n = node_of[t];
+	if (t >= lb.M) return;
+	const int32_t n = lb.node_of[t];
 	const int64_t co = nodes[n].cand_off, end = co + nodes[n].count;
-	const uint64_t hi = sk[t] >> 32;
-	if (t > co && (sk[t - 1] >> 32) == hi) return;  // not the first of its run
+	const uint64_t* keys = reinterpret_cast<const uint64_t*>(lb.keys) + co;
+	const uint32_t mine = q[t];
+	if (t > co && q[t - 1] == mine) return;  // not the first of its run
+	const uint32_t v0 = v[t];
+	const uint64_t k0 = keys[v0];
+	sk[t] = k0;
+	sv[t] = v0;
+	if (t + 1 >= end || q[t + 1] != mine) {
+		lb.pos[co + v0] = (int32_t)(t - co);
+		return;
+	}
+	bool same = true;
 	int64_t e = t + 1;
-	while (e < end && (sk[e] >> 32) == hi) {
-		e++;
-		if (e - t > kLowRunMax) {
-			flags[n] |= 2;
+	for (; e < end && q[e] == mine; e++) {
+		const uint32_t w = v[e];
+		const uint64_t k = keys[w];
+		same = same && k == k0;
+		if (e - t >= (same ? kEqualRunMax : kLowRunMax)) {
+			redo[n] = 1;
 			return;
 		}
-	}
-	for (int64_t i = t + 1; i < e; i++) {
-		const uint64_t k = sk[i];
-		const uint32_t v = sv[i];
-		int64_t j = i;
+		int64_t j = e;
 		while (j > t && k < sk[j - 1]) {
 			sk[j] = sk[j - 1];
 			sv[j] = sv[j - 1];
 			j--;
 		}
 		sk[j] = k;
-		sv[j] = v;
+		sv[j] = w;
 	}
+	bool tie = false;
+	for (int64_t i = t; i < e; i++) {
+		lb.pos[co + sv[i]] = (int32_t)(i - co);
+		tie |= i > t && sk[i] == sk[i - 1];
+	}
+	if (tie) ties[n] = 1;
 }
 
-__global__ void seg_ties_kernel(const int32_t* __restrict__ node_of, const uint64_t* __restrict__ sk, int64_t M, uint8_t* __restrict__ tie) {
-	const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-	if (t + 1 >= M) return;
-	const int32_t n = node_of[t];
-	if (node_of[t + 1] == n && sk[t] == sk[t + 1]) tie[n] |= 1;
-}
-
-__global__ void seg_finish_kernel(const LevelNode* __restrict__ nodes, const uint8_t* __restrict__ tie, const uint64_t* __restrict__ sk,
-                                  const uint32_t* __restrict__ sv, LevelBuffers lb) {
+// ties and positions of the nodes sorted again
+__global__ void seg_redo_kernel(const LevelNode* __restrict__ nodes, const uint8_t* __restrict__ redo, const uint64_t* __restrict__ sk,
+                                const uint32_t* __restrict__ sv, LevelBuffers lb, uint8_t* __restrict__ ties) {
 	const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
 	if (t >= lb.M) return;
 	const int32_t n = lb.node_of[t];
-	if (tie[n]) return;  // left to the introsort replay
-	const int64_t off = nodes[n].cand_off;
-	const uint32_t local = sv[t];
-	lb.keys[t] = __longlong_as_double((long long)sk[t]);
-	lb.perm[t] = (int32_t)local;
-	lb.pos[off + local] = (int32_t)(t - off);
+	if (!redo[n]) return;
+	const int64_t co = nodes[n].cand_off;
+	lb.pos[co + sv[t]] = (int32_t)(t - co);
+	if (t > co && sk[t] == sk[t - 1]) ties[n] = 1;
 }
 
-}  // namespace
+// the sorted keys of the nodes that are not left to the replay
+__global__ void seg_finish_kernel(const uint8_t* __restrict__ ties, const uint64_t* __restrict__ sk, const uint32_t* __restrict__ sv,
+                                  LevelBuffers lb) {
+	const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+	if (t >= lb.M || ties[lb.node_of[t]]) return;
+	lb.keys[t] = __longlong_as_double((long long)sk[t]);
+	lb.perm[t] = (int32_t)sv[t];
+}
 
-void segmented_sort_pairs(const std::vector<LevelNode>& ln, int64_t M, const uint64_t* keys_in, const uint32_t* vals_in,
-                          uint64_t* keys_out, uint32_t* vals_out, int begin_bit, int end_bit, DeviceMem& mem) {
-	const int K = (int)ln.size();
-	if (M == 0 || K == 0 || end_bit <= begin_bit) return;
+// what takes a node's keys to 24 bits; 0 (all keys alike, so a full sort) for
+// a box without a usable size
+double key_scale(const LevelNode& n) {
+	double r2 = 0.0;
+	for (int a = 0; a < 3; a++) r2 += (n.max[a] - n.min[a]) * (n.max[a] - n.min[a]) * 0.25;
+	const double f = (double)(1 << kQuantBits) / r2;
+	return f > 0.0 && f < 1e300 ? f : 0.0;
+}
+
+// Passes of K over bits [begin, end) of the nodes' keys. The result of the
+// last pass is in (keys[passes & 1], vals[passes & 1]) with pass p
+// writing (keys[(p + 1) & 1], ...).
+template <class K>
+void seg_sort(const std::vector<LevelNode>& ln, const uint64_t* keys_in, K* const* keys, uint32_t* const* vals, int begin_bit, int end_bit,
+              DeviceMem& mem) {
 	cudaStream_t s = mem.stream();
-	std::vector<SegTile> tiles;
-	int64_t mat = 0, before = 0;
-	for (int k = 0; k < K; k++) {
-		const int64_t n = ln[k].count;
-		if (n == 0) continue;
-		const int64_t T = ceil_div(n, kSegTile);
-		if (T > INT32_MAX / kSegDigits) throw PcgError(5, "segmented sort: node too large");
-		for (int64_t i = 0; i < T; i++) {
-			SegTile st;
-			st.start = ln[k].cand_off + i * kSegTile;
-			st.node_off = ln[k].cand_off;
-			st.adjust = ln[k].cand_off - before;
-			st.cnt_base = mat + i;
-			st.count = (int32_t)std::min<int64_t>(kSegTile, n - i * kSegTile);
-			st.stride = (int32_t)T;
-			tiles.push_back(st);
-		}
-		mat += (int64_t)kSegDigits * T;
-		before += n;
+	std::vector<SegNode> nodes(ln.size());
+	int64_t tiles = 0;
+	for (size_t k = 0; k < ln.size(); k++) {
+		const int64_t T = ceil_div(ln[k].count, kSegTile);
+		nodes[k] = SegNode{ln[k].cand_off, ln[k].count, key_scale(ln[k]), (int32_t)tiles, (int32_t)T};
+		tiles += T;
+		if (tiles > INT32_MAX) throw PcgError(5, "segmented sort: level too large");
 	}
-	const int num_tiles = (int)tiles.size();
-	const int passes = (end_bit - begin_bit + 7) / 8;
-	SegTile* d_tiles = mem.alloc<SegTile>(tiles.size());
-	PCG_CUDA(cudaMemcpyAsync(d_tiles, tiles.data(), tiles.size() * sizeof(SegTile), cudaMemcpyHostToDevice, s));
-	// the last pass writes (keys_out, vals_out)
-	uint64_t* kb[2] = {keys_out, passes > 1 ? mem.alloc<uint64_t>(M) : nullptr};
-	uint32_t* vb[2] = {vals_out, passes > 1 ? mem.alloc<uint32_t>(M) : nullptr};
-	uint32_t* counts = mem.alloc<uint32_t>(mat);
-	uint32_t* offsets = mem.alloc<uint32_t>(mat);
-	static_assert(sizeof(SegShared) <= 227 * 1024, "tile does not fit shared memory");
-	PCG_CUDA(cudaFuncSetAttribute(seg_downsweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SegShared)));
-	const uint64_t* kin = keys_in;
-	const uint32_t* vin = vals_in;
-	for (int pass = 0; pass < passes; pass++) {
-		const int shift = begin_bit + 8 * pass;
-		const int dst = (passes - 1 - pass) & 1;
-		uint64_t* kout = kb[dst];
-		uint32_t* vout = vb[dst];
-		seg_upsweep<<<num_tiles, kSegThreads, 0, s>>>(d_tiles, kin, shift, counts);
+	if (tiles == 0) return;
+	SegNode* d_nodes = mem.alloc<SegNode>(nodes.size());
+	PCG_CUDA(cudaMemcpyAsync(d_nodes, nodes.data(), nodes.size() * sizeof(SegNode), cudaMemcpyHostToDevice, s));
+	SegTile* d_tiles = mem.alloc<SegTile>(tiles);
+	seg_tiles_kernel<<<(unsigned)ceil_div(tiles, 256), 256, 0, s>>>(d_nodes, (int)nodes.size(), (int)tiles, d_tiles);
+	PCG_LAUNCHED();
+	uint32_t* counts = mem.alloc<uint32_t>((size_t)tiles * kSegDigits);
+	uint32_t* base = mem.alloc<uint32_t>(nodes.size() * kSegDigits);
+	constexpr int smem = (int)sizeof(SegShared<K>);
+	static_assert(smem <= 48 * 1024, "the tile fits what a kernel may use unasked");
+	const void* kin = keys_in;
+	const uint32_t* vin = nullptr;
+	int pass = 0;
+	for (int shift = begin_bit; shift < end_bit; shift += 8, pass++) {
+		K* kout = keys[(pass + 1) & 1];
+		uint32_t* vout = vals[(pass + 1) & 1];
+		if (pass == 0) seg_count_kernel<K, true><<<(unsigned)tiles, kSegThreads, 0, s>>>(d_tiles, kin, shift, counts);
+		else seg_count_kernel<K, false><<<(unsigned)tiles, kSegThreads, 0, s>>>(d_tiles, kin, shift, counts);
 		PCG_LAUNCHED();
-		exclusive_scan_u32(counts, offsets, mat, false, mem);
-		seg_downsweep<<<num_tiles, kSegThreads, sizeof(SegShared), s>>>(d_tiles, kin, vin, kout, vout, shift, offsets);
+		seg_offsets_kernel<<<(unsigned)nodes.size(), kSegDigits * kParts, 0, s>>>(d_nodes, counts, base);
+		PCG_LAUNCHED();
+		if (pass == 0)
+			seg_scatter_kernel<K, true><<<(unsigned)tiles, kSegThreads, smem, s>>>(d_tiles, kin, vin, kout, vout, shift, counts, base);
+		else seg_scatter_kernel<K, false><<<(unsigned)tiles, kSegThreads, smem, s>>>(d_tiles, kin, vin, kout, vout, shift, counts, base);
 		PCG_LAUNCHED();
 		kin = kout;
 		vin = vout;
 	}
 	mem.free(counts);
-	mem.free(offsets);
-	if (kb[1]) mem.free(kb[1]);
-	if (vb[1]) mem.free(vb[1]);
+	mem.free(base);
 	mem.free(d_tiles);
+	mem.free(d_nodes);
 }
+
+// all 64 bits, into (sk, sv)
+void seg_sort_full(const std::vector<LevelNode>& ln, int64_t M, const uint64_t* keys, uint64_t* sk, uint32_t* sv, DeviceMem& mem) {
+	uint64_t* k1 = mem.alloc<uint64_t>(M);
+	uint32_t* v1 = mem.alloc<uint32_t>(M);
+	uint64_t* const kb[2] = {sk, k1};
+	uint32_t* const vb[2] = {sv, v1};
+	seg_sort<uint64_t>(ln, keys, kb, vb, 0, 64, mem);  // 8 passes: the last writes kb[0]
+	mem.free(k1);
+	mem.free(v1);
+}
+
+}  // namespace
 
 namespace {
 
@@ -298,7 +431,7 @@ void build_sorted_level(const LevelNode* d_nodes, const std::vector<LevelNode>& 
 	cudaStream_t s = mem.stream();
 	uint64_t* sk = mem.alloc<uint64_t>(M);
 	uint32_t* sv = mem.alloc<uint32_t>(M);
-	segmented_sort_pairs(ln, M, keys, nullptr, sk, sv, 0, 64, mem);
+	seg_sort_full(ln, M, keys, sk, sv, mem);
 	const unsigned blocks = (unsigned)ceil_div(M, 256);
 	uint32_t* f = mem.alloc<uint32_t>(M);
 	uint32_t* ex = mem.alloc<uint32_t>(M);
@@ -333,36 +466,51 @@ void sort_level_distinct(const LevelNode* d_nodes, const std::vector<LevelNode>&
 	tie.assign(K, 0);
 	if (M == 0 || K == 0) return;
 	cudaStream_t s = mem.stream();
-	uint64_t* sk = mem.alloc<uint64_t>(M);
-	uint32_t* sv = mem.alloc<uint32_t>(M);
 	const uint64_t* keys = reinterpret_cast<const uint64_t*>(lb.keys);
-	// the high words by radix (four passes), the low words inside the short
-	// runs of equal high words
-	segmented_sort_pairs(ln, M, keys, nullptr, sk, sv, 32, 64, mem);
-	uint8_t* d_flags = mem.alloc<uint8_t>(K);
-	PCG_CUDA(cudaMemsetAsync(d_flags, 0, K, s));
+	uint32_t* const q[2] = {mem.alloc<uint32_t>(M), mem.alloc<uint32_t>(M)};
+	uint32_t* const v[2] = {mem.alloc<uint32_t>(M), mem.alloc<uint32_t>(M)};
+	seg_sort<uint32_t>(ln, keys, q, v, 0, kQuantBits, mem);
+	static_assert(kQuantBits == 24, "three passes end in q[1], v[1]");
+	uint64_t* sk = mem.alloc<uint64_t>(M);
+	uint32_t* sv = v[0];
+	uint8_t* d_ties = mem.alloc<uint8_t>(2 * (size_t)K);
+	uint8_t* d_redo = d_ties + K;
+	PCG_CUDA(cudaMemsetAsync(d_ties, 0, 2 * (size_t)K, s));
 	const unsigned blocks = (unsigned)ceil_div(M, 256);
-	seg_fix_low_kernel<<<blocks, 256, 0, s>>>(d_nodes, lb.node_of, sk, sv, M, d_flags);
+	seg_fix_kernel<<<blocks, 256, 0, s>>>(d_nodes, q[1], v[1], lb, sk, sv, d_ties, d_redo);
 	PCG_LAUNCHED();
-	std::vector<uint8_t> flags(K);
-	PCG_CUDA(cudaMemcpyAsync(flags.data(), d_flags, K, cudaMemcpyDeviceToHost, s));
+	mem.free(q[0]);
+	mem.free(q[1]);
+	mem.free(v[1]);
+	std::vector<uint8_t> marks(2 * (size_t)K);
+	PCG_CUDA(cudaMemcpyAsync(marks.data(), d_ties, marks.size(), cudaMemcpyDeviceToHost, s));
 	PCG_CUDA(cudaStreamSynchronize(s));
-	std::vector<LevelNode> redo;
+	std::vector<LevelNode> again;
 	for (int k = 0; k < K; k++)
-		if (flags[k] & 2) redo.push_back(ln[k]);
-	// nodes with a long run of equal high words: all 64 bits by radix
-	if (!redo.empty()) segmented_sort_pairs(redo, M, keys, nullptr, sk, sv, 0, 64, mem);
-	PCG_CUDA(cudaMemsetAsync(d_flags, 0, K, s));
-	seg_ties_kernel<<<blocks, 256, 0, s>>>(lb.node_of, sk, M, d_flags);
-	PCG_LAUNCHED();
-	seg_finish_kernel<<<blocks, 256, 0, s>>>(d_nodes, d_flags, sk, sv, lb);
-	PCG_LAUNCHED();
-	PCG_CUDA(cudaMemcpyAsync(tie.data(), d_flags, K, cudaMemcpyDeviceToHost, s));
-	PCG_CUDA(cudaStreamSynchronize(s));
-	mem.free(d_flags);
+		if (marks[K + k]) again.push_back(ln[k]);
+	if (!again.empty()) {
+		seg_sort_full(again, M, keys, sk, sv, mem);
+		seg_redo_kernel<<<blocks, 256, 0, s>>>(d_nodes, d_redo, sk, sv, lb, d_ties);
+		PCG_LAUNCHED();
+		PCG_CUDA(cudaMemcpyAsync(marks.data(), d_ties, K, cudaMemcpyDeviceToHost, s));
+		PCG_CUDA(cudaStreamSynchronize(s));
+	}
+	std::copy(marks.begin(), marks.begin() + K, tie.begin());
 	bool any_tie = false;
 	for (uint8_t t : tie) any_tie |= t != 0;
-	if (keep && any_tie) {
+	if (!any_tie) {
+		// the sorted buffers take the place of the gathered ones
+		mem.free(d_ties);
+		mem.free(lb.keys);
+		mem.free(lb.perm);
+		lb.keys = reinterpret_cast<double*>(sk);
+		lb.perm = reinterpret_cast<int32_t*>(sv);
+		return;
+	}
+	seg_finish_kernel<<<blocks, 256, 0, s>>>(d_ties, sk, sv, lb);
+	PCG_LAUNCHED();
+	mem.free(d_ties);
+	if (keep) {
 		uint32_t* f = mem.alloc<uint32_t>(M);
 		uint32_t* ex = mem.alloc<uint32_t>(M);
 		int32_t* ties = mem.alloc<int32_t>(M);
