@@ -13,11 +13,10 @@
 
 #include <algorithm>
 #include <iomanip>
+#include <cstring>
 #include <limits>
-#include <map>
-#include <memory>
 #include <sstream>
-#include <unordered_map>
+#include <utility>
 
 namespace pcg {
 
@@ -28,164 +27,182 @@ constexpr int kRecordBytes = 22;   // type, childMask, numPoints, offset, size
 
 enum NodeType : uint8_t { T_NORMAL = 0, T_LEAF = 1, T_PROXY = 2 };
 
+// A node's name as a number: a 1, then three bits per digit after the "r". The
+// parent is code >> 3, and the order by length, then text, is the order of
+// the codes. 64 bits hold 21 levels, 128 bits 42: a cube of 2^32 units has 33
+// and one round of five more.
+template <class Code>
+Code code_of(const char* name, size_t len) {
+	Code c = 1;
+	for (size_t i = 1; i < len; i++) c = c << 3 | (Code)(name[i] - '0');
+	return c;
+}
+
+template <class Code>
 struct BNode {
-	std::string name;
+	Code code = 0;
 	int32_t num_points = 0;
+	uint32_t order = 0;  // in the file
 	uint8_t child_mask = 0;
-	uint64_t byte_offset = 0, byte_size = 0;
 	uint8_t type = T_LEAF;
+	uint64_t byte_offset = 0, byte_size = 0;
 	uint64_t proxy_offset = 0, proxy_size = 0;
 };
 
+template <class Code>
 struct BChunk {
-	std::string name;
-	std::vector<BNode*> nodes;
-	int64_t byte_offset = 0;
+	Code code = 0;
+	size_t first = 0, count = 0;  // its entries
 };
 
+// The chunks of a batch in order, and their nodes in order.
+template <class Code>
 struct Batch {
-	std::string name;
-	std::vector<std::unique_ptr<BNode>> nodes;
-	std::vector<std::unique_ptr<BChunk>> chunks;
-	std::unordered_map<std::string, BNode*> node_of;
-	std::unordered_map<std::string, BChunk*> chunk_of;
+	Code code = 0;
+	std::vector<BNode<Code>> nodes;                  // by code
+	std::vector<BChunk<Code>> chunks;                // by code
+	std::vector<std::pair<Code, uint32_t>> entries;  // (chunk, node), chunk by chunk
+	std::vector<std::pair<Code, uint32_t>> by_code;  // (node, record)
 	int64_t byte_size = 0;
+
+	BNode<Code>* find(Code c) {
+		auto it = std::lower_bound(nodes.begin(), nodes.end(), c, [](const BNode<Code>& n, Code v) { return n.code < v; });
+		return it != nodes.end() && it->code == c ? &*it : nullptr;
+	}
+	bool has_chunk(Code c) const {
+		auto it = std::lower_bound(chunks.begin(), chunks.end(), c, [](const BChunk<Code>& n, Code v) { return n.code < v; });
+		return it != chunks.end() && it->code == c;
+	}
 };
-
-bool bfs_less(const std::string& a, const std::string& b) {
-	return a.size() != b.size() ? a.size() < b.size() : a < b;
-}
-
-BChunk* chunk_for(Batch& b, const std::string& key) {
-	auto it = b.chunk_of.find(key);
-	if (it != b.chunk_of.end()) return it->second;
-	b.chunks.push_back(std::make_unique<BChunk>());
-	b.chunks.back()->name = key;
-	b.chunk_of[key] = b.chunks.back().get();
-	return b.chunks.back().get();
-}
 
 // HierarchyBuilder::loadBatch (HierarchyBuilder.h:82-197) over the records a
-// flusher file holds, in file order.
-std::unique_ptr<Batch> load_batch(const std::string& name, const std::vector<const HierRecord*>& recs) {
-	auto b = std::make_unique<Batch>();
-	b->name = name;
-	for (const HierRecord* r : recs) {
-		auto n = std::make_unique<BNode>();
-		n->name = r->name;
-		n->num_points = (int32_t)(uint32_t)r->num_points;
-		n->byte_offset = (uint64_t)r->byte_offset;
-		n->byte_size = (uint64_t)(int64_t)(int32_t)(uint32_t)r->byte_size;
-		// chunk key: "r" for names up to 5 chars, then the first 4k+1 chars
-		size_t len = n->name.size();
-		std::string key = len <= 5 ? n->name.substr(0, 1) : n->name.substr(0, kStep * ((len - 2) / 4) + 1);
-		if (n->name == b->name) key = n->name;
-		BNode* np = n.get();
-		chunk_for(*b, key)->nodes.push_back(np);
-		b->node_of[np->name] = np;
-		b->nodes.push_back(std::move(n));
-		if ((len - 1) % kStep == 0 && len > (size_t)kStep + 1) chunk_for(*b, np->name)->nodes.push_back(np);
-	}
-	std::sort(b->chunks.begin(), b->chunks.end(), [](const auto& x, const auto& y) { return bfs_less(x->name, y->name); });
-	for (auto& n : b->nodes) {
-		n->type = T_LEAF;
-		auto it = b->node_of.find(n->name.substr(0, n->name.size() - 1));
-		if (it != b->node_of.end()) {
-			it->second->type = T_NORMAL;
-			it->second->child_mask |= (uint8_t)(1 << (n->name.back() - '0'));
+// flusher file holds.
+template <class Code>
+void load_batch(Batch<Code>& b, Code code, const std::vector<const HierRecord*>& recs) {
+	b.code = code;
+	b.nodes.clear();
+	b.chunks.clear();
+	b.entries.clear();
+	b.by_code.clear();
+	for (uint32_t i = 0; i < recs.size(); i++) b.by_code.push_back({code_of<Code>(recs[i]->name.data(), recs[i]->name.size()), i});
+	std::sort(b.by_code.begin(), b.by_code.end());
+	size_t up = 0;  // the first node not before the parent
+	for (uint32_t i = 0; i < b.by_code.size(); i++) {
+		const HierRecord& r = *recs[b.by_code[i].second];
+		BNode<Code> n;
+		n.code = b.by_code[i].first;
+		n.order = b.by_code[i].second;
+		n.num_points = (int32_t)(uint32_t)r.num_points;
+		n.byte_offset = (uint64_t)r.byte_offset;
+		n.byte_size = (uint64_t)(int64_t)(int32_t)(uint32_t)r.byte_size;
+		// chunk: "r" for names up to 5 chars, then the first 4k+1 chars
+		const int len = (int)r.name.size(), key = len <= 5 ? 1 : kStep * ((len - 2) / 4) + 1;
+		b.entries.push_back({n.code == code ? code : n.code >> (3 * (len - key)), i});
+		if ((len - 1) % kStep == 0 && len > kStep + 1 && n.code != code) b.entries.push_back({n.code, i});
+		while (up < i && b.nodes[up].code < n.code >> 3) up++;
+		if (up < i && b.nodes[up].code == n.code >> 3) {
+			if (n.order > b.nodes[up].order) b.nodes[up].type = T_NORMAL;
+			b.nodes[up].child_mask |= (uint8_t)(1 << (int)(n.code & 7));
 		}
+		b.nodes.push_back(n);
 	}
-	for (auto& c : b->chunks) {
-		auto it = b->node_of.find(c->name);
-		if (it != b->node_of.end()) it->second->type = T_PROXY;
+	std::sort(b.entries.begin(), b.entries.end());
+	for (size_t i = 0; i < b.entries.size(); i++) {
+		if (i == 0 || b.entries[i].first != b.entries[i - 1].first) b.chunks.push_back({b.entries[i].first, i, 0});
+		b.chunks.back().count++;
 	}
-	for (auto& c : b->chunks)
-		std::sort(c->nodes.begin(), c->nodes.end(), [](const BNode* x, const BNode* y) { return bfs_less(x->name, y->name); });
-	return b;
+	for (const auto& c : b.chunks)
+		if (auto* n = b.find(c.code)) n->type = T_PROXY;
 }
 
-bool process_batch(Batch& b, std::string& err) {  // HierarchyBuilder.h:199-238
-	int64_t off = 0;
-	for (auto& c : b.chunks) {
-		c->byte_offset = off;
-		if (c->name != b.name) {
-			std::string parent = c->name.substr(0, c->name.size() - kStep);
-			if (!b.chunk_of.count(parent)) { err = "hierarchy: missing parent chunk " + parent; return false; }
-			auto it = b.node_of.find(c->name);
-			if (it == b.node_of.end()) { err = "hierarchy: missing proxy node " + c->name; return false; }
-			it->second->type = T_PROXY;
-			it->second->proxy_offset = (uint64_t)c->byte_offset;
-			it->second->proxy_size = (uint64_t)kRecordBytes * c->nodes.size();
-		}
-		off += kRecordBytes * (int64_t)c->nodes.size();
+template <class Code>
+bool process_batch(Batch<Code>& b, std::string& err) {  // HierarchyBuilder.h:199-238
+	for (const auto& c : b.chunks) {
+		if (c.code == b.code) continue;
+		if (!b.has_chunk(c.code >> (3 * kStep))) { err = "hierarchy: missing parent chunk"; return false; }
+		auto* n = b.find(c.code);
+		if (!n) { err = "hierarchy: missing proxy node"; return false; }
+		n->proxy_offset = (uint64_t)kRecordBytes * c.first;
+		n->proxy_size = (uint64_t)kRecordBytes * c.count;
 	}
-	b.byte_size = off;
 	return true;
 }
 
-void serialize_batch(Batch& b, int64_t bytes_written, std::vector<uint8_t>& out, size_t at) {  // :240-282
-	size_t k = 0;
-	size_t total = 0;
-	for (auto& c : b.chunks) total += c->nodes.size();
-	if (out.size() < at + kRecordBytes * total) out.resize(at + kRecordBytes * total);
-	for (auto& c : b.chunks) {
-		for (BNode* n : c->nodes) {
-			bool is_proxy = n->type == T_PROXY && n->name != c->name;
-			uint8_t type = (n->type == T_PROXY && !is_proxy) ? (uint8_t)T_NORMAL : n->type;
-			uint64_t size = is_proxy ? n->proxy_size : n->byte_size;
-			uint64_t offset = is_proxy ? (uint64_t)bytes_written + n->proxy_offset : n->byte_offset;
-			uint32_t np = (uint32_t)n->num_points;
-			uint8_t* p = out.data() + at + kRecordBytes * k;
-			p[0] = type;
-			p[1] = n->child_mask;
-			std::memcpy(p + 2, &np, 4);
-			std::memcpy(p + 6, &offset, 8);
-			std::memcpy(p + 14, &size, 8);
-			k++;
-		}
+template <class Code>
+void serialize_batch(Batch<Code>& b, int64_t bytes_written, std::vector<uint8_t>& out, size_t at) {  // :240-282
+	b.byte_size = (int64_t)(kRecordBytes * b.entries.size());
+	if (out.size() < at + (size_t)b.byte_size) out.resize(at + (size_t)b.byte_size);
+	uint8_t* p = out.data() + at;
+	for (const auto& [chunk, i] : b.entries) {
+		const auto& n = b.nodes[i];
+		const bool is_proxy = n.type == T_PROXY && n.code != chunk;
+		const uint8_t type = (n.type == T_PROXY && !is_proxy) ? (uint8_t)T_NORMAL : n.type;
+		const uint64_t size = is_proxy ? n.proxy_size : n.byte_size;
+		const uint64_t offset = is_proxy ? (uint64_t)bytes_written + n.proxy_offset : n.byte_offset;
+		const uint32_t np = (uint32_t)n.num_points;
+		p[0] = type;
+		p[1] = n.child_mask;
+		std::memcpy(p + 2, &np, 4);
+		std::memcpy(p + 6, &offset, 8);
+		std::memcpy(p + 14, &size, 8);
+		p += kRecordBytes;
 	}
-	b.byte_size = (int64_t)(kRecordBytes * total);
+}
+
+template <class Code>
+bool build(const std::vector<HierRecord>& completed, std::vector<uint8_t>& out, int64_t& first_chunk_size, std::string& err) {
+	// flusher files: the root's nodes, and per node of depth 4 its subtree
+	// (indexer.h:171-193); the builder visits files in file-name order, which
+	// equals key order.
+	std::vector<const HierRecord*> top, recs;
+	std::vector<uint64_t> filed;  // file, record
+	for (size_t i = 0; i < completed.size(); i++) {
+		const std::string& name = completed[i].name;
+		if (name.size() <= (size_t)kStep + 1) top.push_back(&completed[i]);
+		if (name.size() > (size_t)kStep) filed.push_back(code_of<uint64_t>(name.data(), kStep + 1) << 32 | i);
+	}
+	std::sort(filed.begin(), filed.end());
+	if (top.empty()) { err = "hierarchy: no root batch"; return false; }
+	Batch<Code> root, b;
+	load_batch(root, Code(1), top);
+	out.assign(kRecordBytes * root.nodes.size(), 0);
+	int64_t written = (int64_t)out.size();
+	for (size_t i = 0; i < filed.size();) {
+		const uint64_t file = filed[i] >> 32;
+		recs.clear();
+		for (; i < filed.size() && filed[i] >> 32 == file; i++) recs.push_back(&completed[filed[i] & 0xffffffffu]);
+		load_batch(b, Code(file), recs);
+		if (!process_batch(b, err)) return false;
+		serialize_batch(b, written, out, out.size());
+		auto* n = root.find(b.code);
+		if (!n) { err = "hierarchy: batch root missing from root batch"; return false; }
+		if (b.nodes.size() > 1) {
+			n->type = T_PROXY;
+			n->proxy_offset = (uint64_t)written;
+			size_t own = 0;
+			for (const auto& c : b.chunks)
+				if (c.code == b.code) own = c.count;
+			n->proxy_size = (uint64_t)kRecordBytes * own;
+		} else {
+			n->type = T_LEAF;
+		}
+		written += b.byte_size;
+	}
+	std::vector<uint8_t> head;
+	serialize_batch(root, 0, head, 0);
+	std::memcpy(out.data(), head.data(), head.size());
+	first_chunk_size = root.byte_size;
+	return true;
 }
 
 }  // namespace
 
 bool build_hierarchy(const std::vector<HierRecord>& completed, std::vector<uint8_t>& out,
                      int64_t& first_chunk_size, std::string& err) {
-	// flusher files: per key, records in completion order (indexer.h:171-193);
-	// the builder visits files in file-name order, which equals key order.
-	std::map<std::string, std::vector<const HierRecord*>> files;
-	for (const auto& r : completed) {
-		const std::string key = r.name.size() <= (size_t)kStep + 1 ? std::string("r") : r.name.substr(0, kStep + 1);
-		files[key].push_back(&r);
-		if (r.name.size() == (size_t)kStep + 1) files[r.name].push_back(&r);
-	}
-	auto rit = files.find("r");
-	if (rit == files.end()) { err = "hierarchy: no root batch"; return false; }
-	auto root = load_batch("r", rit->second);
-	out.assign(kRecordBytes * root->nodes.size(), 0);
-	int64_t written = (int64_t)out.size();
-	for (auto& [key, recs] : files) {
-		if (key == "r") continue;
-		auto b = load_batch(key, recs);
-		if (!process_batch(*b, err)) return false;
-		size_t at = out.size();
-		serialize_batch(*b, written, out, at);
-		auto pit = root->node_of.find(b->name);
-		if (pit == root->node_of.end()) { err = "hierarchy: batch root missing from root batch"; return false; }
-		if (b->nodes.size() > 1) {
-			pit->second->type = T_PROXY;
-			pit->second->proxy_offset = (uint64_t)written;
-			pit->second->proxy_size = (uint64_t)kRecordBytes * b->chunk_of[b->name]->nodes.size();
-		} else {
-			pit->second->type = T_LEAF;
-		}
-		written += b->byte_size;
-	}
-	std::vector<uint8_t> head;
-	serialize_batch(*root, 0, head, 0);
-	std::memcpy(out.data(), head.data(), head.size());
-	first_chunk_size = root->byte_size;
-	return true;
+	size_t longest = 0;
+	for (const auto& r : completed) longest = std::max(longest, r.name.size());
+	if (longest <= 22) return build<uint64_t>(completed, out, first_chunk_size, err);
+	return build<unsigned __int128>(completed, out, first_chunk_size, err);
 }
 
 std::string build_metadata(const std::string& name, const std::string& projection, int64_t points_total,
