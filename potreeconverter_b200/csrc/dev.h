@@ -276,7 +276,6 @@ void radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_tmp, uint32
 // out[i] = sum(in[0..i)) ; returns nothing, total is out[n] when out has n+1
 // elements and write_total is set.
 void exclusive_scan_u32(const uint32_t* in, uint32_t* out, int64_t n, bool write_total, DeviceMem& mem);
-void exclusive_scan_i64(const int64_t* in, int64_t* out, int64_t n, bool write_total, DeviceMem& mem);
 
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 

@@ -420,8 +420,8 @@ __global__ void __launch_bounds__(kBigThreads) sort_single_big_kernel(double* ke
 // Segments longer than kWideMin (the top partitions of large nodes) are
 // partitioned level-synchronously across the whole GPU: every round
 // partitions all pending long segments of all nodes at once -- pivot move,
-// stop counts per 4096-element tile, one scan, stop lists, the pair search,
-// the swaps -- so the first partitions of a node with millions of
+// stop counts per 4096-element tile, stop lists, the pair search, the swaps --
+// so the first partitions of a node with millions of
 // candidates no longer run on a single CTA. Both halves of a partition go on
 // with the decremented depth budget (std::__introsort_loop), so the order in
 // which disjoint segments are processed does not change the result.
@@ -429,16 +429,16 @@ __global__ void __launch_bounds__(kBigThreads) sort_single_big_kernel(double* ke
 // remaining depth budget (a CTA for one whose budget is spent, which is
 // heap-sorted); <= 16-element segments go to the final insertion pass, and
 // segments whose keys became distinct are written from the sorted keys.
-// kWideMin = 1024 measured fastest on the 50M benchmark cloud (sort 36.6 ms
-// per conversion against 40.1 with 4096 and 37.0 with 512): once finished
-// segments leave the rounds, the rounds only carry the segments around
-// equal keys, and the less of them a warp replays in global memory, the
-// better.
+// kWideMin: once finished segments leave the rounds, the rounds only carry the
+// segments around equal keys, and the less of them a warp replays in global
+// memory, the better (an 8M-point lattice: 512 18.5 ms, 1,024 18.7, 2,048
+// 19.5, 4,096 22.0; a 50M-point cloud: no difference).
 constexpr int64_t kWideMin = 1024;
 constexpr int kWideThreads = 256;
 constexpr int kWideWarps = kWideThreads / 32;
 constexpr int kWideSteps = 16;
 constexpr int kWideTile = kWideThreads * kWideSteps;  // 4096
+constexpr int kRoundsAhead = 4;  // even: rounds alternate between two lists
 
 struct WideTile {
 	int64_t p0;          // first element of the tile (after the segment's pivot slot)
@@ -466,7 +466,7 @@ struct FinSeg {          // a segment written from the sorted keys
 };
 
 struct WideLists {       // outputs of a round (device counters)
-	Seg* next; int* n_next;   // still longer than kWideMin
+	Seg* next; int* n_next;   // still longer than kWideMin (n_next: this round's of n_seg[2])
 	SegBounds* next_b;        // their key ranges
 	Seg* cta;  int* n_cta;    // CTA replay (>= kBigSortMin elements, or heapsort)
 	Seg* warp; int* n_warp;   // warp replay
@@ -487,23 +487,49 @@ int64_t wide_min() {
 	return v;
 }
 
-__global__ void wide_pivot_kernel(const Seg* __restrict__ segs, int n, double* key, int32_t* val) {
-	const int s = blockIdx.x * blockDim.x + threadIdx.x;
-	if (s >= n) return;
-	// std::__move_median_to_first(first, first + 1, mid, last - 1)
-	const int64_t f = segs[s].f, l = segs[s].l;
-	const int64_t a = f + 1, b = f + (l - f) / 2, c = l - 1;
-	const double ka = key[a], kb = key[b], kc = key[c];
-	int64_t m;
-	if (ka < kb) {
-		if (kb < kc) m = b;
-		else if (ka < kc) m = c;
-		else m = a;
-	} else if (ka < kc) m = a;
-	else if (kb < kc) m = c;
-	else m = b;
-	const double tk = key[f]; key[f] = key[m]; key[m] = tk;
-	const int32_t tv = val[f]; val[f] = val[m]; val[m] = tv;
+// A round's counters: segments and tiles, by the round's parity. The rounds
+// run without the host, which launches a few of them ahead and then reads the
+// number of segments left: every kernel goes through what the counters say
+// with however many blocks it has, and does nothing when they say nothing.
+// What bounds a round is its chain of five launches, 45 us where 12.6M
+// candidates of 142 nodes take 108 of them. (With the segments read back and
+// the tiles made on the host, a round had four copies up, three down and two
+// waits: 23.0 ms for that conversion, 18.8 now.)
+struct WideCounters {
+	int n_seg[2], n_tiles[2];
+};
+
+// pivots to the front of their segments, and the segments' tiles
+__global__ void wide_pivot_kernel(const Seg* __restrict__ segs, int parity, int cap_seg, int cap_tiles, WideCounters* __restrict__ wc,
+                                  WideTile* __restrict__ tiles, int32_t* __restrict__ seg_tile, double* key, int32_t* val, SampleStats* st) {
+	const int n = min(wc->n_seg[parity], cap_seg);
+	for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
+		const int64_t f = segs[s].f, l = segs[s].l;
+		const int nt = (int)((l - f - 1 + kWideTile - 1) / kWideTile);  // the elements after the pivot slot
+		int first = atomicAdd(&wc->n_tiles[parity], nt);
+		if (first + nt > cap_tiles) {
+			atomicAdd(&st->timeouts, 1ull);
+			first = cap_tiles;
+		}
+		seg_tile[s] = first;
+		for (int j = 0; j < nt && first < cap_tiles; j++) {
+			const int64_t p0 = f + 1 + (int64_t)j * kWideTile;
+			tiles[first + j] = WideTile{p0, (int32_t)min((int64_t)kWideTile, l - p0), s, first, first + nt - 1};
+		}
+		// std::__move_median_to_first(first, first + 1, mid, last - 1)
+		const int64_t a = f + 1, b = f + (l - f) / 2, c = l - 1;
+		const double ka = key[a], kb = key[b], kc = key[c];
+		int64_t m;
+		if (ka < kb) {
+			if (kb < kc) m = b;
+			else if (ka < kc) m = c;
+			else m = a;
+		} else if (ka < kc) m = a;
+		else if (kb < kc) m = c;
+		else m = b;
+		const double tk = key[f]; key[f] = key[m]; key[m] = tk;
+		const int32_t tv = val[f]; val[f] = val[m]; val[m] = tv;
+	}
 }
 
 // stop flags of one tile in warp-contiguous order: warp w covers tile
@@ -522,56 +548,74 @@ __device__ __forceinline__ void wide_flags(const WideTile& t, const double* key,
 	}
 }
 
-__global__ void __launch_bounds__(kWideThreads) wide_count_kernel(const WideTile* __restrict__ tiles, const Seg* __restrict__ segs,
+__global__ void __launch_bounds__(kWideThreads) wide_count_kernel(const WideTile* __restrict__ tiles, int parity, int cap_tiles,
+                                                                WideCounters* wc, const Seg* __restrict__ segs,
                                                                 const double* __restrict__ key, unsigned long long* __restrict__ counts) {
 	__shared__ unsigned long long wsum[kWideWarps];
-	const WideTile t = tiles[blockIdx.x];
-	const double P = key[segs[t.seg].f];
-	uint32_t lb, rb;
-	wide_flags(t, key, P, lb, rb);
-	unsigned long long v = ((unsigned long long)__popc(rb) << 32) | (unsigned long long)__popc(lb);
+	if (blockIdx.x == 0 && threadIdx.x == 0) wc->n_seg[parity ^ 1] = wc->n_tiles[parity ^ 1] = 0;  // the round before is over
+	const int nt = min(wc->n_tiles[parity], cap_tiles);
+	for (int i = blockIdx.x; i < nt; i += gridDim.x) {
+		const WideTile t = tiles[i];
+		const double P = key[segs[t.seg].f];
+		uint32_t lb, rb;
+		wide_flags(t, key, P, lb, rb);
+		unsigned long long v = ((unsigned long long)__popc(rb) << 32) | (unsigned long long)__popc(lb);
 #pragma unroll
-	for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
-	if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = v;
-	__syncthreads();
-	if (threadIdx.x == 0) {
-		unsigned long long tot = 0;
-		for (int w = 0; w < kWideWarps; w++) tot += wsum[w];
-		counts[blockIdx.x] = tot;
+		for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
+		if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = v;
+		__syncthreads();
+		if (threadIdx.x == 0) {
+			unsigned long long tot = 0;
+			for (int w = 0; w < kWideWarps; w++) tot += wsum[w];
+			counts[i] = tot;
+		}
+		__syncthreads();
 	}
 }
 
-__global__ void __launch_bounds__(kWideThreads) wide_write_kernel(const WideTile* __restrict__ tiles, const Seg* __restrict__ segs,
-                                                                const double* __restrict__ key, const unsigned long long* __restrict__ offs,
+// the stop lists; a tile adds up the counts of its segment's tiles before it
+__global__ void __launch_bounds__(kWideThreads) wide_write_kernel(const WideTile* __restrict__ tiles, int parity, int cap_tiles,
+                                                                const WideCounters* wc, const Seg* __restrict__ segs,
+                                                                const double* __restrict__ key, const unsigned long long* __restrict__ counts,
                                                                 int32_t* __restrict__ SL, int32_t* __restrict__ SR) {
-	__shared__ unsigned long long wsum[kWideWarps];
+	__shared__ unsigned long long wsum[kWideWarps], wbefore[kWideWarps];
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-	const WideTile t = tiles[blockIdx.x];
-	const int64_t f = segs[t.seg].f;
-	const double P = key[f];
-	uint32_t lb, rb;
-	wide_flags(t, key, P, lb, rb);
-	// per-warp totals, exclusive over the warps of the tile
-	unsigned long long v = ((unsigned long long)__popc(rb) << 32) | (unsigned long long)__popc(lb);
+	const int nt = min(wc->n_tiles[parity], cap_tiles);
+	for (int i = blockIdx.x; i < nt; i += gridDim.x) {
+		const WideTile t = tiles[i];
+		const int64_t f = segs[t.seg].f;
+		const double P = key[f];
+		uint32_t lb, rb;
+		wide_flags(t, key, P, lb, rb);
+		unsigned long long v = ((unsigned long long)__popc(rb) << 32) | (unsigned long long)__popc(lb), u = 0;
+		for (int j = t.first_tile + (int)threadIdx.x; j < i; j += kWideThreads) u += counts[j];
 #pragma unroll
-	for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
-	if (lane == 0) wsum[warp] = v;
-	__syncthreads();
-	unsigned long long before = offs[blockIdx.x] - offs[t.first_tile];
-	for (int w = 0; w < warp; w++) before += wsum[w];
-	int64_t cl = (int64_t)(before & 0xffffffffull), cr = (int64_t)(before >> 32);
-	const uint32_t lt = lanemask_lt();
-	int32_t* sl = SL + f;
-	int32_t* sr = SR + f;
+		for (int o = 16; o > 0; o >>= 1) {
+			v += __shfl_xor_sync(FULL, v, o);
+			u += __shfl_xor_sync(FULL, u, o);
+		}
+		if (lane == 0) {
+			wsum[warp] = v;
+			wbefore[warp] = u;
+		}
+		__syncthreads();
+		unsigned long long before = 0;
+		for (int w = 0; w < kWideWarps; w++) before += wbefore[w] + (w < warp ? wsum[w] : 0ull);
+		int64_t cl = (int64_t)(before & 0xffffffffull), cr = (int64_t)(before >> 32);
+		const uint32_t lt = lanemask_lt();
+		int32_t* sl = SL + f;
+		int32_t* sr = SR + f;
 #pragma unroll
-	for (int st = 0; st < kWideSteps; st++) {
-		const bool isL = (lb >> st) & 1u, isR = (rb >> st) & 1u;
-		const uint32_t bL = __ballot_sync(FULL, isL), bR = __ballot_sync(FULL, isR);
-		const int32_t rel = (int32_t)(t.p0 + warp * (kWideSteps * 32) + st * 32 + lane - f);
-		if (isL) sl[cl + __popc(bL & lt)] = rel;
-		if (isR) sr[cr + __popc(bR & lt)] = rel;
-		cl += __popc(bL);
-		cr += __popc(bR);
+		for (int st = 0; st < kWideSteps; st++) {
+			const bool isL = (lb >> st) & 1u, isR = (rb >> st) & 1u;
+			const uint32_t bL = __ballot_sync(FULL, isL), bR = __ballot_sync(FULL, isR);
+			const int32_t rel = (int32_t)(t.p0 + warp * (kWideSteps * 32) + st * 32 + lane - f);
+			if (isL) sl[cl + __popc(bL & lt)] = rel;
+			if (isR) sr[cr + __popc(bR & lt)] = rel;
+			cl += __popc(bL);
+			cr += __popc(bR);
+		}
+		__syncthreads();
 	}
 }
 
@@ -648,18 +692,19 @@ __device__ void wide_classify(int64_t f, int64_t l, int d, const SegBounds& b, i
 	}
 }
 
-// one warp per segment: Hoare's pair count K, the cut, the two halves
-__global__ void wide_split_kernel(const Seg* __restrict__ segs, const SegBounds* __restrict__ bounds, int n, const WideTile* __restrict__ tiles,
-                                  const int32_t* __restrict__ seg_tile, const unsigned long long* __restrict__ counts,
-                                  const unsigned long long* __restrict__ offs, const int32_t* __restrict__ SL, const int32_t* __restrict__ SR,
-                                  const double* __restrict__ key, int64_t* __restrict__ segK, int64_t* __restrict__ segCR, WideLists L,
-                                  SampleStats* st) {
-	const int s = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
-	const int lane = threadIdx.x & 31;
-	if (s >= n) return;
+// one warp's segment: Hoare's pair count K, the cut, the two halves
+__device__ void wide_split(int s, int lane, const Seg* __restrict__ segs, const SegBounds* __restrict__ bounds,
+                           const WideTile* __restrict__ tiles, const int32_t* __restrict__ seg_tile, int cap_tiles,
+                           const unsigned long long* __restrict__ counts, const int32_t* __restrict__ SL, const int32_t* __restrict__ SR,
+                           const double* __restrict__ key, int64_t* __restrict__ segK, int64_t* __restrict__ segCR, const WideLists& L,
+                           SampleStats* st) {
 	const Seg g = segs[s];
+	if (seg_tile[s] >= cap_tiles) return;
 	const WideTile ft = tiles[seg_tile[s]];
-	const unsigned long long tot = offs[ft.last_tile] + counts[ft.last_tile] - offs[ft.first_tile];
+	unsigned long long tot = 0;
+	for (int j = ft.first_tile + lane; j <= ft.last_tile; j += 32) tot += counts[j];
+#pragma unroll
+	for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(FULL, tot, o);
 	const int64_t cL = (int64_t)(tot & 0xffffffffull), cR = (int64_t)(tot >> 32);
 	const int32_t* sl = SL + g.f;
 	const int32_t* sr = SR + g.f;
@@ -727,6 +772,17 @@ __global__ void wide_split_kernel(const Seg* __restrict__ segs, const SegBounds*
 	wide_classify(g.f, cut, d, bL, aL, L, st);
 }
 
+__global__ void wide_split_kernel(const Seg* __restrict__ segs, const SegBounds* __restrict__ bounds, int parity, int cap_seg, const WideCounters* wc,
+                                  const WideTile* __restrict__ tiles, const int32_t* __restrict__ seg_tile, int cap_tiles,
+                                  const unsigned long long* __restrict__ counts, const int32_t* __restrict__ SL,
+                                  const int32_t* __restrict__ SR, const double* __restrict__ key, int64_t* __restrict__ segK,
+                                  int64_t* __restrict__ segCR, WideLists L, SampleStats* st) {
+	const int lane = threadIdx.x & 31, warps = (int)((gridDim.x * blockDim.x) >> 5);
+	const int n = min(wc->n_seg[parity], cap_seg);
+	for (int s = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); s < n; s += warps)
+		wide_split(s, lane, segs, bounds, tiles, seg_tile, cap_tiles, counts, SL, SR, key, segK, segCR, L, st);
+}
+
 // the segments with distinct keys get their sorted keys in order; one CTA
 // per tile of kFinTile elements of a segment (tile_seg / tile_off)
 constexpr int64_t kFinTile = 4096;
@@ -740,20 +796,24 @@ __global__ void __launch_bounds__(256) fin_copy_kernel(const FinSeg* __restrict_
 	}
 }
 
-__global__ void __launch_bounds__(kWideThreads) wide_swap_kernel(const WideTile* __restrict__ tiles, const Seg* __restrict__ segs,
+__global__ void __launch_bounds__(kWideThreads) wide_swap_kernel(const WideTile* __restrict__ tiles, int parity, int cap_tiles,
+                                                               const WideCounters* wc, const Seg* __restrict__ segs,
                                                                const int64_t* __restrict__ segK, const int64_t* __restrict__ segCR,
                                                                const int32_t* __restrict__ SL, const int32_t* __restrict__ SR, double* key,
                                                                int32_t* val) {
-	const WideTile t = tiles[blockIdx.x];
-	const int64_t f = segs[t.seg].f;
-	const int64_t K = segK[t.seg], cR = segCR[t.seg];
-	const int64_t k0 = t.p0 - (f + 1);  // the tile's elements double as its share of the pair indices
-	for (int j = threadIdx.x; j < t.count; j += kWideThreads) {
-		const int64_t k = k0 + j;
-		if (k >= K) break;
-		const int64_t a = f + SL[f + k], b = f + SR[f + cR - 1 - k];
-		const double tk = key[a]; key[a] = key[b]; key[b] = tk;
-		const int32_t tv = val[a]; val[a] = val[b]; val[b] = tv;
+	const int nt = min(wc->n_tiles[parity], cap_tiles);
+	for (int i = blockIdx.x; i < nt; i += gridDim.x) {
+		const WideTile t = tiles[i];
+		const int64_t f = segs[t.seg].f;
+		const int64_t K = segK[t.seg], cR = segCR[t.seg];
+		const int64_t k0 = t.p0 - (f + 1);  // the tile's elements double as its share of the pair indices
+		for (int j = threadIdx.x; j < t.count; j += kWideThreads) {
+			const int64_t k = k0 + j;
+			if (k >= K) break;
+			const int64_t a = f + SL[f + k], b = f + SR[f + cR - 1 - k];
+			const double tk = key[a]; key[a] = key[b]; key[b] = tk;
+			const int32_t tv = val[a]; val[a] = val[b]; val[b] = tv;
+		}
 	}
 }
 
@@ -856,8 +916,7 @@ void replay_segments(double* key, int32_t* val, int64_t M, const std::vector<Sor
 	L.warp = mem.alloc<Seg>(L.cap_seg);
 	L.blk = mem.alloc<int32_t>(2 * L.cap_blk);
 	L.fin = mem.alloc<FinSeg>(L.cap_seg);
-	int* counters = mem.alloc<int>(6);  // next, cta, warp, blk, warp-kernel cursor, fin
-	L.n_next = counters;
+	int* counters = mem.alloc<int>(6);  // -, cta, warp, blk, warp-kernel cursor, fin
 	L.n_cta = counters + 1;
 	L.n_warp = counters + 2;
 	L.n_blk = counters + 3;
@@ -885,78 +944,55 @@ void replay_segments(double* key, int32_t* val, int64_t M, const std::vector<Sor
 	if (!warp.empty()) PCG_CUDA(cudaMemcpyAsync(L.warp, warp.data(), warp.size() * sizeof(Seg), cudaMemcpyHostToDevice, s));
 	if (!blk.empty()) PCG_CUDA(cudaMemcpyAsync(L.blk, blk.data(), blk.size() * sizeof(int32_t), cudaMemcpyHostToDevice, s));
 	PCG_CUDA(cudaMemcpyAsync(counters, h_counts, sizeof(h_counts), cudaMemcpyHostToDevice, s));
-	int pp = 0;
-	int64_t* segK = nullptr;
-	int64_t* segCR = nullptr;
-	int64_t seg_cap = 0;
-	for (int round = 0; !cur.empty(); round++) {
-		if (round > 128) throw PcgError(4, "sort replay: partition rounds did not converge");
-		const int n = (int)cur.size();
-		std::vector<WideTile> tiles;
-		std::vector<int32_t> seg_tile(n);
-		for (int i = 0; i < n; i++) {
-			const int64_t f = cur[i].f, len = cur[i].l - cur[i].f - 1;  // elements after the pivot slot
-			const int first = (int)tiles.size();
-			const int nt = (int)ceil_div(len, kWideTile);
-			seg_tile[i] = first;
-			for (int j = 0; j < nt; j++) {
-				WideTile t;
-				t.p0 = f + 1 + (int64_t)j * kWideTile;
-				t.count = (int32_t)std::min<int64_t>(kWideTile, len - (int64_t)j * kWideTile);
-				t.seg = i;
-				t.first_tile = first;
-				t.last_tile = first + nt - 1;
-				tiles.push_back(t);
+	if (!cur.empty()) {
+		const int64_t max_segs = std::min<int64_t>(L.cap_seg, M / L.wide_min + 64);  // disjoint, each longer than wide_min
+		const int64_t max_tiles = M / kWideTile + max_segs;
+		if (max_tiles > INT32_MAX) throw PcgError(5, "sort replay: level too large");
+		const int cap_tiles = (int)max_tiles, cap_seg = (int)max_segs;
+		WideTile* tiles = mem.alloc<WideTile>(cap_tiles);
+		unsigned long long* counts = mem.alloc<unsigned long long>(cap_tiles);
+		int32_t* seg_tile = mem.alloc<int32_t>(cap_seg);
+		int64_t* segK = mem.alloc<int64_t>(cap_seg);
+		int64_t* segCR = mem.alloc<int64_t>(cap_seg);
+		WideCounters* wc = mem.alloc<WideCounters>(1);
+		WideCounters h{{(int)cur.size(), 0}, {0, 0}};
+		PCG_CUDA(cudaMemcpyAsync(wc, &h, sizeof(h), cudaMemcpyHostToDevice, s));
+		PCG_CUDA(cudaMemcpyAsync(ping[0], cur.data(), cur.size() * sizeof(Seg), cudaMemcpyHostToDevice, s));
+		PCG_CUDA(cudaMemcpyAsync(pingb[0], curb.data(), curb.size() * sizeof(SegBounds), cudaMemcpyHostToDevice, s));
+		int64_t first_tiles = 0;
+		for (const Seg& g : cur) first_tiles += ceil_div(g.l - g.f, kWideTile);
+		// segments get shorter than a tile, so later rounds have more tiles
+		const unsigned blocks = (unsigned)std::min<int64_t>(2 * first_tiles + 2, (int64_t)sm_count() * 8);
+		for (int round = 0; h.n_seg[round & 1] != 0; round += kRoundsAhead) {
+			if (round > 128) throw PcgError(4, "sort replay: partition rounds did not converge");
+			for (int r = round; r < round + kRoundsAhead; r++) {
+				const int p = r & 1;
+				const Seg* d_cur = ping[p];
+				L.next = ping[p ^ 1];
+				L.next_b = pingb[p ^ 1];
+				L.n_next = &wc->n_seg[p ^ 1];
+				wide_pivot_kernel<<<blocks, 32, 0, s>>>(d_cur, p, cap_seg, cap_tiles, wc, tiles, seg_tile, key, val, st);
+				PCG_LAUNCHED();
+				wide_count_kernel<<<blocks, kWideThreads, 0, s>>>(tiles, p, cap_tiles, wc, d_cur, key, counts);
+				PCG_LAUNCHED();
+				wide_write_kernel<<<blocks, kWideThreads, 0, s>>>(tiles, p, cap_tiles, wc, d_cur, key, counts, sc.SL, sc.SR);
+				PCG_LAUNCHED();
+				wide_split_kernel<<<blocks, 128, 0, s>>>(d_cur, pingb[p], p, cap_seg, wc, tiles, seg_tile, cap_tiles, counts, sc.SL, sc.SR, key, segK,
+				                                         segCR, L, st);
+				PCG_LAUNCHED();
+				wide_swap_kernel<<<blocks, kWideThreads, 0, s>>>(tiles, p, cap_tiles, wc, d_cur, segK, segCR, sc.SL, sc.SR, key, val);
+				PCG_LAUNCHED();
 			}
+			PCG_CUDA(cudaMemcpyAsync(&h, wc, sizeof(h), cudaMemcpyDeviceToHost, s));
+			PCG_CUDA(cudaStreamSynchronize(s));
+			if (h.n_seg[round & 1] > cap_seg) throw PcgError(5, "sort replay: segment list overflow");
 		}
-		const int nt = (int)tiles.size();
-		Seg* d_cur = ping[pp];
-		SegBounds* d_curb = pingb[pp];
-		L.next = ping[pp ^ 1];
-		L.next_b = pingb[pp ^ 1];
-		PCG_CUDA(cudaMemcpyAsync(d_cur, cur.data(), n * sizeof(Seg), cudaMemcpyHostToDevice, s));
-		PCG_CUDA(cudaMemcpyAsync(d_curb, curb.data(), n * sizeof(SegBounds), cudaMemcpyHostToDevice, s));
-		WideTile* d_tiles = mem.alloc<WideTile>(nt);
-		PCG_CUDA(cudaMemcpyAsync(d_tiles, tiles.data(), nt * sizeof(WideTile), cudaMemcpyHostToDevice, s));
-		int32_t* d_seg_tile = mem.alloc<int32_t>(n);
-		PCG_CUDA(cudaMemcpyAsync(d_seg_tile, seg_tile.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice, s));
-		if (n > seg_cap) {
-			if (segK) { mem.free(segK); mem.free(segCR); }
-			seg_cap = 2 * (int64_t)n;
-			segK = mem.alloc<int64_t>(seg_cap);
-			segCR = mem.alloc<int64_t>(seg_cap);
-		}
-		unsigned long long* counts = mem.alloc<unsigned long long>(nt);
-		unsigned long long* offs = mem.alloc<unsigned long long>(nt);
-		PCG_CUDA(cudaMemsetAsync(L.n_next, 0, sizeof(int), s));
-		wide_pivot_kernel<<<(unsigned)ceil_div(n, 128), 128, 0, s>>>(d_cur, n, key, val);
-		PCG_LAUNCHED();
-		wide_count_kernel<<<nt, kWideThreads, 0, s>>>(d_tiles, d_cur, key, counts);
-		PCG_LAUNCHED();
-		exclusive_scan_i64(reinterpret_cast<const int64_t*>(counts), reinterpret_cast<int64_t*>(offs), nt, false, mem);
-		wide_write_kernel<<<nt, kWideThreads, 0, s>>>(d_tiles, d_cur, key, offs, sc.SL, sc.SR);
-		PCG_LAUNCHED();
-		wide_split_kernel<<<(unsigned)ceil_div((int64_t)n * 32, 128), 128, 0, s>>>(d_cur, d_curb, n, d_tiles, d_seg_tile, counts, offs, sc.SL,
-		                                                                          sc.SR, key, segK, segCR, L, st);
-		PCG_LAUNCHED();
-		wide_swap_kernel<<<nt, kWideThreads, 0, s>>>(d_tiles, d_cur, segK, segCR, sc.SL, sc.SR, key, val);
-		PCG_LAUNCHED();
-		int n_next = 0;
-		PCG_CUDA(cudaMemcpyAsync(&n_next, L.n_next, sizeof(int), cudaMemcpyDeviceToHost, s));
-		PCG_CUDA(cudaStreamSynchronize(s));
-		if (n_next > L.cap_seg) throw PcgError(5, "sort replay: segment list overflow");
-		cur.resize(n_next);
-		curb.resize(n_next);
-		if (n_next) {
-			PCG_CUDA(cudaMemcpyAsync(cur.data(), L.next, n_next * sizeof(Seg), cudaMemcpyDeviceToHost, s));
-			PCG_CUDA(cudaMemcpyAsync(curb.data(), L.next_b, n_next * sizeof(SegBounds), cudaMemcpyDeviceToHost, s));
-		}
-		PCG_CUDA(cudaStreamSynchronize(s));
+		mem.free(tiles);
 		mem.free(counts);
-		mem.free(offs);
-		mem.free(d_tiles);
-		mem.free(d_seg_tile);
-		pp ^= 1;
+		mem.free(seg_tile);
+		mem.free(segK);
+		mem.free(segCR);
+		mem.free(wc);
 	}
 	PCG_CUDA(cudaMemcpyAsync(h_counts, counters, sizeof(h_counts), cudaMemcpyDeviceToHost, s));
 	PCG_CUDA(cudaStreamSynchronize(s));
@@ -998,7 +1034,6 @@ void replay_segments(double* key, int32_t* val, int64_t M, const std::vector<Sor
 		blk_insertion_kernel<<<(unsigned)ceil_div(h_counts[3], 128), 128, 0, s>>>(L.blk, h_counts[3], key, val);
 		PCG_LAUNCHED();
 	}
-	if (segK) { mem.free(segK); mem.free(segCR); }
 	mem.free(ping[0]);
 	mem.free(ping[1]);
 	mem.free(pingb[0]);

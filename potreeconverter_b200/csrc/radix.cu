@@ -193,10 +193,6 @@ void exclusive_scan_u32(const uint32_t* in, uint32_t* out, int64_t n, bool write
 	exclusive_scan_impl<uint32_t>(in, out, n, write_tot, mem);
 }
 
-void exclusive_scan_i64(const int64_t* in, int64_t* out, int64_t n, bool write_tot, DeviceMem& mem) {
-	exclusive_scan_impl<int64_t>(in, out, n, write_tot, mem);
-}
-
 void radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_tmp, uint32_t* vals_tmp, int64_t n,
                       int begin_bit, int end_bit, DeviceMem& mem) {
 	if (n <= 1 || end_bit <= begin_bit) return;
