@@ -351,7 +351,7 @@ __global__ void lut_fill_kernel(const ChunkCell* __restrict__ chunks, int grid_s
 }
 
 __global__ void assign_kernel(const uint32_t* __restrict__ cell, const int32_t* __restrict__ lut, int64_t n, int chunk_base,
-                              uint32_t* __restrict__ chunk_of, uint32_t* __restrict__ ids, int64_t* error) {
+                              uint32_t* __restrict__ chunk_of, int64_t* error) {
 	int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
 	if (i >= n) return;
 	int32_t c = lut[cell[i]];
@@ -361,7 +361,6 @@ __global__ void assign_kernel(const uint32_t* __restrict__ cell, const int32_t* 
 		c = 0;
 	}
 	chunk_of[i] = (uint32_t)c;
-	ids[i] = (uint32_t)i;
 }
 
 // ---------------------------------------------------- parts of a large cloud
@@ -561,10 +560,10 @@ void launch_lut_fill(const ChunkCell* chunks, int num_chunks, int grid_size, int
 	PCG_LAUNCHED();
 }
 
-void launch_assign_chunks(const uint32_t* cell, const int32_t* lut, int64_t n, int chunk_base, uint32_t* chunk_of, uint32_t* ids,
-                          int64_t* error, DeviceMem& mem) {
+void launch_assign_chunks(const uint32_t* cell, const int32_t* lut, int64_t n, int chunk_base, uint32_t* chunk_of, int64_t* error,
+                          DeviceMem& mem) {
 	if (n == 0) return;
-	assign_kernel<<<(unsigned)ceil_div(n, 256), 256, 0, mem.stream()>>>(cell, lut, n, chunk_base, chunk_of, ids, error);
+	assign_kernel<<<(unsigned)ceil_div(n, 256), 256, 0, mem.stream()>>>(cell, lut, n, chunk_base, chunk_of, error);
 	PCG_LAUNCHED();
 }
 

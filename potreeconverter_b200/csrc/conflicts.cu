@@ -41,7 +41,7 @@
 // distance D. The FP64 values the reference compares are themselves within
 // 1.1e-16 |x| of the exact coordinates, below 1.1e-10 s when |x| < 1e6 s
 // (checked per node; beyond it the node uses FP64 alone). So D32 >= s^2 (1 +
-// 1e-3) (rounded up by at most u; fused multiply-adds only drop roundings) implies D64 > s^2, and D32 < s^2 (1 - 1e-3)
+// 1e-3) (rounded up by at most u) implies D64 > s^2, and D32 < s^2 (1 - 1e-3)
 // implies D64 < s^2: the margin is 30x the error.
 //
 // The early-exit bound needs the earlier candidate's key only where it can
@@ -303,7 +303,7 @@ struct PairTest {
 	// qf: the record, u: its sorted position; a wanted one could reject
 	__device__ __forceinline__ bool operator()(const float4& qf, int32_t u, bool wanted, const LevelBuffers& lb, const PosParamsS& pp) {
 		const float fx = qf.x - mf.x, fy = qf.y - mf.y, fz = qf.z - mf.z;
-		const float d2 = __fmaf_rn(fz, fz, __fmaf_rn(fy, fy, fx * fx));
+		const float d2 = fx * fx + fy * fy + fz * fz;
 		bool hit = wanted && !(d2 >= s2hi);
 		const bool inside = d2 < s2lo;
 		if (hit && !(inside && far_from_centre)) hit = exact(lb, pp, u, inside);

@@ -268,10 +268,14 @@ private:
 
 // ---------------------------------------------------------------- launchers
 // Stable LSD radix sort of (key, value) uint32 pairs on bits [begin_bit,
-// end_bit). The sorted pairs end in (keys, vals); tmp buffers are scratch of
-// the same length.
-void radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_tmp, uint32_t* vals_tmp, int64_t n,
-                      int begin_bit, int end_bit, DeviceMem& mem);
+// end_bit). The sorted pairs end in (keys, vals), which change places with the
+// scratch buffers (of the same length) where the passes are odd in number.
+// iota: the values are 0 .. n - 1 and need not be there.
+void radix_sort_pairs(uint32_t*& keys, uint32_t*& vals, uint32_t*& keys_tmp, uint32_t*& vals_tmp, int64_t n, int begin_bit, int end_bit,
+                      DeviceMem& mem, bool iota = false);
+// the same within every (first, count) range by itself
+void radix_sort_segments(uint32_t*& keys, uint32_t*& vals, uint32_t*& keys_tmp, uint32_t*& vals_tmp,
+                         const std::vector<std::pair<int64_t, int64_t>>& segs, int begin_bit, int end_bit, DeviceMem& mem);
 
 // out[i] = sum(in[0..i)) ; returns nothing, total is out[n] when out has n+1
 // elements and write_total is set.

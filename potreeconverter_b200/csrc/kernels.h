@@ -35,10 +35,10 @@ void launch_lut_merge(const uint32_t* grid, int grid_size, int64_t max_points_pe
                       int32_t* num_chunks, int capacity, DeviceMem& mem);
 // Fills the LUT: chunk k owns cells of chunks[k] (already in chunk order).
 void launch_lut_fill(const ChunkCell* chunks, int num_chunks, int grid_size, int32_t* lut, DeviceMem& mem);
-// chunk_of[i] = lut[cell[i]] - chunk_base, ids[i] = i; a cell without a
-// chunk, or one below chunk_base, sets error[1]
-void launch_assign_chunks(const uint32_t* cell, const int32_t* lut, int64_t n, int chunk_base, uint32_t* chunk_of, uint32_t* ids,
-                          int64_t* error, DeviceMem& mem);
+// chunk_of[i] = lut[cell[i]] - chunk_base; a cell without a chunk, or one
+// below chunk_base, sets error[1]
+void launch_assign_chunks(const uint32_t* cell, const int32_t* lut, int64_t n, int chunk_base, uint32_t* chunk_of, int64_t* error,
+                          DeviceMem& mem);
 // Appends the records among recs[0..n) (one source, p.src0's layout) whose
 // count-grid cell lies in chunks k0 .. k1 - 1 to out, in input order, at
 // record index *fill onwards; *fill (device) advances by their count.
@@ -75,7 +75,7 @@ struct PosParams {
 };
 
 void launch_octree_round(uint32_t* ids, const int32_t* X, const int32_t* Y, const int32_t* Z, const PosParams& pp,
-                         const SegmentDesc* d_segs, int num_segs, int64_t total, NodeCand* cands, int32_t* num_cands,
+                         const std::vector<SegmentDesc>& segs, const SegmentDesc* d_segs, int64_t total, NodeCand* cands, int32_t* num_cands,
                          int64_t cand_capacity, DeviceMem& mem);
 // number of distinct (X, Y, Z) among ids[0..n)
 int64_t count_unique_positions(const uint32_t* ids, int64_t n, const int32_t* X, const int32_t* Y, const int32_t* Z, DeviceMem& mem);

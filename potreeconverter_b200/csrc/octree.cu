@@ -2,8 +2,8 @@
 //
 // One round processes every node that must be split, across all chunks at
 // once: each point gets the Morton code of its 32^3 cell inside its node's
-// box (indexer.cpp:851-871), the round's points are stably sorted by
-// (node, Morton code) -- the reference's stable counting sort
+// box (indexer.cpp:851-871), every node's points are stably sorted by
+// Morton code -- the reference's stable counting sort
 // (indexer.cpp:874-909) -- and one CTA per node builds the 5-level sum
 // pyramid in shared memory and walks it (createSumPyramid / createNodes,
 // indexer.cpp:691-817), emitting leaves and nodes that need another round.
@@ -219,8 +219,9 @@ __global__ void count_distinct_kernel(const uint32_t* __restrict__ ids, const ui
 }  // namespace
 
 void launch_octree_round(uint32_t* ids, const int32_t* X, const int32_t* Y, const int32_t* Z, const PosParams& pp,
-                         const SegmentDesc* d_segs, int num_segs, int64_t total, NodeCand* cands, int32_t* num_cands,
+                         const std::vector<SegmentDesc>& segs, const SegmentDesc* d_segs, int64_t total, NodeCand* cands, int32_t* num_cands,
                          int64_t cand_capacity, DeviceMem& mem) {
+	const int num_segs = (int)segs.size();
 	if (total == 0 || num_segs == 0) return;
 	if (num_segs >= (1 << 17)) throw PcgError(5, "octree round: too many segments");
 	cudaStream_t s = mem.stream();
@@ -231,8 +232,11 @@ void launch_octree_round(uint32_t* ids, const int32_t* X, const int32_t* Y, cons
 	unsigned blocks = (unsigned)ceil_div(total, 256);
 	octree_keys_kernel<<<blocks, 256, 0, s>>>(ids, X, Y, Z, pp, d_segs, num_segs, total, keys, vals);
 	PCG_LAUNCHED();
-	int bits = 15 + bits_for((uint64_t)(num_segs - 1));
-	radix_sort_pairs(keys, vals, keys_t, vals_t, total, 0, bits, mem);
+	// the nodes' points lie together, so only the 15 bits of the cells are
+	// sorted, two passes (with the node's number on top, as one range, three)
+	std::vector<std::pair<int64_t, int64_t>> ranges;
+	for (const SegmentDesc& g : segs) ranges.push_back({g.coff, g.count});
+	radix_sort_segments(keys, vals, keys_t, vals_t, ranges, 0, 15, mem);
 	octree_scatter_kernel<<<blocks, 256, 0, s>>>(ids, vals, d_segs, num_segs, total);
 	PCG_LAUNCHED();
 	size_t smem = (size_t)(kCells + kPyr) * sizeof(uint32_t);

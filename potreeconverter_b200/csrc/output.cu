@@ -140,29 +140,68 @@ __global__ void fill_colors_kernel(DecodeParams p, const uint32_t* __restrict__ 
 	with_source<kMulti>(p, id, [&](const SourceDesc& sd) { cols[i] = record_rgb(sd.recs + ((int64_t)id - sd.first) * sd.rec_len, p, sd); });
 }
 
-__global__ void gather_u32_kernel(const uint32_t* __restrict__ src, const int64_t* __restrict__ idx, int64_t n, uint32_t* __restrict__ dst) {
-	int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-	if (i < n) dst[i] = src[idx[i]];
-}
+constexpr int kSplitThreads = 256;
+constexpr int kSplitSteps = kSplitStretch / 32;  // of a warp, which takes a stretch
 
-__global__ void flags_to_u32_kernel(const uint8_t* __restrict__ f, int64_t n, uint32_t* __restrict__ o) {
-	int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-	if (i < n) o[i] = f[i];
-}
-
-__global__ void split_kernel(const uint8_t* __restrict__ accepted, const uint32_t* __restrict__ pre, int64_t n, const uint32_t* __restrict__ ids,
-                             const uint64_t* __restrict__ cols, const int4* __restrict__ rec, uint32_t* __restrict__ acc_ids,
-                             uint64_t* __restrict__ acc_cols, int4* __restrict__ acc_rec, uint32_t* __restrict__ rej_ids) {
-	int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-	if (j >= n) return;
-	uint32_t a = pre[j];
-	if (accepted[j]) {
-		acc_ids[a] = ids[j];
-		if (acc_cols) acc_cols[a] = cols[j];
-		if (acc_rec) acc_rec[a] = rec[j];
-	} else if (rej_ids) {
-		rej_ids[j - a] = ids[j];
+// accepted candidates per stretch, one warp each, 16 flags a lane
+__global__ void __launch_bounds__(kSplitThreads) split_count_kernel(const uint8_t* __restrict__ accepted, int64_t n,
+                                                                    uint32_t* __restrict__ counts) {
+	const int64_t w = ((int64_t)blockIdx.x * kSplitThreads + threadIdx.x) >> 5;
+	const int lane = threadIdx.x & 31;
+	const int64_t at = w * kSplitStretch + lane * 16;
+	uint32_t c = 0;
+	if (at + 16 <= n) {
+		const uint4 v = *reinterpret_cast<const uint4*>(accepted + at);
+		c = __popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w);
+	} else {
+		for (int64_t i = at; i < n; i++) c += accepted[i];
 	}
+	c = __reduce_add_sync(FULL, c);
+	if (lane == 0 && w * kSplitStretch < n) counts[w] = c;
+}
+
+// One warp per stretch: ballots give every candidate its place. Bound by
+// memory, 29 to 45 bytes a candidate. (Flags widened to words, scanned and read
+// again per candidate: 3.3 ms for 162M candidates where this and its
+// counts take 1.3.)
+__global__ void __launch_bounds__(kSplitThreads) split_kernel(const uint8_t* __restrict__ accepted, const uint32_t* __restrict__ before, int64_t n,
+                                                              const uint32_t* __restrict__ ids, const uint64_t* __restrict__ cols,
+                                                              const int4* __restrict__ rec, uint32_t* __restrict__ acc_ids,
+                                                              uint64_t* __restrict__ acc_cols, int4* __restrict__ acc_rec,
+                                                              uint32_t* __restrict__ rej_ids) {
+	const int64_t w = ((int64_t)blockIdx.x * kSplitThreads + threadIdx.x) >> 5;
+	const int lane = threadIdx.x & 31;
+	if (w * kSplitStretch >= n) return;
+	uint32_t a = before[w];
+	const uint32_t lt = (1u << lane) - 1u;
+#pragma unroll 4
+	for (int s = 0; s < kSplitSteps; s++) {
+		const int64_t j = w * kSplitStretch + s * 32 + lane;
+		const bool in = j < n, take = in && accepted[j];
+		const uint32_t b = __ballot_sync(FULL, take);
+		const uint32_t r = a + __popc(b & lt);
+		if (take) {
+			acc_ids[r] = ids[j];
+			if (acc_cols) acc_cols[r] = cols[j];
+			if (acc_rec) acc_rec[r] = rec[j];
+		} else if (in && rej_ids) {
+			rej_ids[j - r] = ids[j];
+		}
+		a += __popc(b);
+	}
+}
+
+// one warp per index
+__global__ void accepted_before_kernel(const uint8_t* __restrict__ accepted, int64_t n, const uint32_t* __restrict__ before,
+                                       const int64_t* __restrict__ idx, int64_t num, uint32_t* __restrict__ dst) {
+	const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+	const int lane = threadIdx.x & 31;
+	if (i >= num) return;
+	const int64_t j = idx[i], w = j / kSplitStretch;
+	uint32_t c = 0;
+	for (int64_t k = w * kSplitStretch + lane; k < j; k += 32) c += accepted[k];
+	c = __reduce_add_sync(FULL, c);
+	if (lane == 0) dst[i] = before[w] + c;
 }
 
 }  // namespace
@@ -199,22 +238,27 @@ void launch_fill_colors(const DecodeParams& p, const uint32_t* ids, int64_t n, u
 	PCG_LAUNCHED();
 }
 
-void launch_gather_u32(const uint32_t* src, const int64_t* idx, int64_t n, uint32_t* dst, DeviceMem& mem) {
-	if (n == 0) return;
-	gather_u32_kernel<<<(unsigned)ceil_div(n, 256), 256, 0, mem.stream()>>>(src, idx, n, dst);
-	PCG_LAUNCHED();
+void launch_split(const uint8_t* accepted, int64_t n, const uint32_t* ids, const uint64_t* cols, const int4* rec, uint32_t* before,
+                  uint32_t* acc_ids, uint64_t* acc_cols, int4* acc_rec, uint32_t* rej_ids, DeviceMem& mem) {
+	const int64_t stretches = split_stretches(n);
+	uint32_t* counts = mem.alloc<uint32_t>(std::max<int64_t>(stretches, 1));
+	const unsigned blocks = (unsigned)ceil_div(stretches * 32, kSplitThreads);
+	if (n > 0) {
+		split_count_kernel<<<blocks, kSplitThreads, 0, mem.stream()>>>(accepted, n, counts);
+		PCG_LAUNCHED();
+	}
+	exclusive_scan_u32(counts, before, stretches, true, mem);
+	if (n > 0) {
+		split_kernel<<<blocks, kSplitThreads, 0, mem.stream()>>>(accepted, before, n, ids, cols, rec, acc_ids, acc_cols, acc_rec, rej_ids);
+		PCG_LAUNCHED();
+	}
+	mem.free(counts);
 }
 
-void launch_split(const uint8_t* accepted, int64_t n, const uint32_t* ids, const uint64_t* cols, const int4* rec, uint32_t* pre,
-                  uint32_t* acc_ids, uint64_t* acc_cols, int4* acc_rec, uint32_t* rej_ids, DeviceMem& mem) {
-	if (n == 0) return;
-	uint32_t* f = mem.alloc<uint32_t>(n);
-	flags_to_u32_kernel<<<(unsigned)ceil_div(n, 256), 256, 0, mem.stream()>>>(accepted, n, f);
-	PCG_LAUNCHED();
-	exclusive_scan_u32(f, pre, n, true, mem);
-	mem.free(f);
-	split_kernel<<<(unsigned)ceil_div(n, 256), 256, 0, mem.stream()>>>(accepted, pre, n, ids, cols, rec, acc_ids, acc_cols, acc_rec,
-	                                                                 rej_ids);
+void launch_accepted_before(const uint8_t* accepted, int64_t n, const uint32_t* before, const int64_t* idx, int64_t num, uint32_t* dst,
+                            DeviceMem& mem) {
+	if (num == 0) return;
+	accepted_before_kernel<<<(unsigned)ceil_div(num * 32, 256), 256, 0, mem.stream()>>>(accepted, n, before, idx, num, dst);
 	PCG_LAUNCHED();
 }
 

@@ -17,12 +17,17 @@ void launch_write_payloads(const DecodeParams& p, const std::vector<PayloadItem>
                            DeviceMem& mem);
 // Packed colour (r | g << 16 | b << 32) of every point's output record.
 void launch_fill_colors(const DecodeParams& p, const uint32_t* ids, int64_t n, uint64_t* cols, DeviceMem& mem);
-void launch_gather_u32(const uint32_t* src, const int64_t* idx, int64_t n, uint32_t* dst, DeviceMem& mem);
-// Stable split of candidates by accepted flag: pre = exclusive prefix of the
-// flags (n + 1 entries), accepted ids (and colours, records) compacted in
-// order into acc_ids (acc_cols, acc_rec), rejected ids into rej_ids (skipped
-// when null).
-void launch_split(const uint8_t* accepted, int64_t n, const uint32_t* ids, const uint64_t* cols, const int4* rec, uint32_t* pre,
+// Stable split of candidates by accepted flag (0 or 1): accepted ids (and
+// colours, records) compacted in order into acc_ids (acc_cols, acc_rec),
+// rejected ids into rej_ids (skipped when null). before: how many are accepted
+// before every stretch of kSplitStretch candidates and, last, in all;
+// split_stretches(n) + 1 entries.
+constexpr int kSplitStretch = 512;
+inline int64_t split_stretches(int64_t n) { return ceil_div(n, kSplitStretch); }
+void launch_split(const uint8_t* accepted, int64_t n, const uint32_t* ids, const uint64_t* cols, const int4* rec, uint32_t* before,
                   uint32_t* acc_ids, uint64_t* acc_cols, int4* acc_rec, uint32_t* rej_ids, DeviceMem& mem);
+// dst[i] = accepted candidates before idx[i] (at most n)
+void launch_accepted_before(const uint8_t* accepted, int64_t n, const uint32_t* before, const int64_t* idx, int64_t num, uint32_t* dst,
+                            DeviceMem& mem);
 
 }  // namespace pcg

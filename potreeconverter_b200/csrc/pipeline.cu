@@ -3,7 +3,7 @@
 // Stage map (reference files relative to the PotreeConverter source tree):
 //   decode + count grid   chunking.cu   chunker_countsort_laszip.cpp:131-361, 749-803
 //   LUT merge             chunking.cu   chunker_countsort_laszip.cpp:1074-1204
-//   stable scatter        radix.cu      chunker_countsort_laszip.cpp:837-904
+//   stable scatter        segsort.cu    chunker_countsort_laszip.cpp:837-904
 //   per-chunk octree      octree.cu     indexer.cpp:691-1109
 //   samplers              sampling.cu   sampler_poisson.h, sampler_poisson_average.h, sampler_random.h
 //   completion order      here          indexer.cpp:1581-1745 (chunks, chunk-root tasks, root)
@@ -938,7 +938,7 @@ struct Converter {
 			}
 			SegmentDesc* d_segs = upload(segs, mem);
 			PCG_CUDA(cudaMemsetAsync(d_ncands, 0, 4, stream));
-			launch_octree_round(ids, X, Y, Z, pp, d_segs, (int)segs.size(), total, d_cands, d_ncands, cand_cap, mem);
+			launch_octree_round(ids, X, Y, Z, pp, segs, d_segs, total, d_cands, d_ncands, cand_cap, mem);
 			int ncand = download(d_ncands, 1, stream)[0];
 			if (ncand > cand_cap) throw PcgError(PCG_INTERNAL, "octree round overflow");
 			auto cands = download(d_cands, (size_t)ncand, stream);
@@ -1031,11 +1031,15 @@ struct Converter {
 	// every chunk starts in ids.
 	void scatter_chunks(const uint32_t* cell, const int32_t* lut, int64_t n, int nchunks, int chunk_base, uint32_t* ids, int64_t* error,
 	                    DeviceMem& mem, int64_t* chunk_start = nullptr) {
+		const int bits = std::max(1, bits_for((uint64_t)std::max(nchunks - 1, 0)));
 		uint32_t* chunk_of = mem.alloc<uint32_t>(std::max<int64_t>(n, 1));
-		launch_assign_chunks(cell, lut, n, chunk_base, chunk_of, ids, error, mem);
+		launch_assign_chunks(cell, lut, n, chunk_base, chunk_of, error, mem);
 		uint32_t* kt = mem.alloc<uint32_t>(std::max<int64_t>(n, 1));
 		uint32_t* vt = mem.alloc<uint32_t>(std::max<int64_t>(n, 1));
-		radix_sort_pairs(chunk_of, ids, kt, vt, n, 0, std::max(1, bits_for((uint64_t)std::max(nchunks - 1, 0))), mem);
+		// the last pass writes ids
+		const bool odd = ((bits + 7) / 8) & 1;
+		uint32_t *v = odd ? vt : ids, *other = odd ? ids : vt;
+		radix_sort_pairs(chunk_of, v, kt, other, n, 0, bits, mem, true);
 		if (chunk_start) launch_segment_starts(chunk_of, n, nchunks, chunk_start, mem);
 		mem.free(kt);
 		mem.free(vt);
@@ -1869,19 +1873,19 @@ struct Converter {
 			mem.free(lb.keys); mem.free(lb.perm); mem.free(lb.pos);
 		}
 		// split candidates into the parents' buffers and the children's payloads
-		uint32_t* pre = mem.alloc<uint32_t>(M + 1);
+		uint32_t* before = mem.alloc<uint32_t>(split_stretches(M) + 1);
 		uint32_t* acc_ids = mem.alloc<uint32_t>(M);
 		uint64_t* acc_cols = lb.cols ? mem.alloc<uint64_t>(M) : nullptr;
 		uint32_t* rej_ids = method == PCG_POISSON_AVERAGE ? nullptr : mem.alloc<uint32_t>(M);
 		int4* acc_rec = lb.rec ? mem.alloc<int4>(M) : nullptr;
-		launch_split(lb.accepted, M, lb.ids, lb.cols, lb.rec, pre, acc_ids, acc_cols, acc_rec, rej_ids, mem);
-		// prefix values at node and child boundaries
+		launch_split(lb.accepted, M, lb.ids, lb.cols, lb.rec, before, acc_ids, acc_cols, acc_rec, rej_ids, mem);
+		// accepted before the node and child boundaries
 		std::vector<int64_t> bidx;
 		for (int k = 0; k < K; k++) { bidx.push_back(ln[k].cand_off); bidx.push_back(ln[k].cand_off + ln[k].count); }
 		for (auto& cs : child_slots) { bidx.push_back(cs.start); bidx.push_back(cs.start + cs.count); }
 		int64_t* d_bidx = upload(bidx, mem);
 		uint32_t* d_bval = mem.alloc<uint32_t>(bidx.size());
-		launch_gather_u32(pre, d_bidx, (int64_t)bidx.size(), d_bval, mem);
+		launch_accepted_before(lb.accepted, M, before, d_bidx, (int64_t)bidx.size(), d_bval, mem);
 		auto bval = download(d_bval, bidx.size(), s);
 		// parents
 		for (int k = 0; k < K; k++) {
@@ -1923,7 +1927,7 @@ struct Converter {
 		}
 		mem.free(d_bidx);
 		mem.free(d_bval);
-		mem.free(pre);
+		mem.free(before);
 		mem.free(d_nodes);
 		mem.free(d_items);
 		mem.free(lb.child);

@@ -1,5 +1,6 @@
-// Exact per-node sort of a level's candidate keys without the introsort
-// replay.
+// Stable LSD radix sorts: of a level's candidates, every node by itself and
+// exact without the introsort replay; of points by chunk, and of the points of
+// the octree's nodes by cell.
 //
 // The samplers order each node's candidates with std::sort by FP64 squared
 // distance to the node centre (sampler_poisson.h:183-203). When a node's keys
@@ -31,10 +32,17 @@
 //
 // Measured, 162M candidates of a 50M-point conversion: counts 1.1 ms (shared
 // atomics: the digits of a tile spread; by peer masks 3.4), positions 0.4,
-// scatters 3.0, fixing 2.1. Four passes over the high 32 bits of the FP64 keys,
+// scatters 3.0, fixing 2.1. (Four passes over the high 32 bits of the FP64 keys,
 // 12 bytes per candidate each, with one scan over the level's counts in
 // digit order, then separate kernels for the low bits, the ties and the
-// results took 14.
+// results took 14.)
+//
+// A range that is sorted as a whole (points by chunk) is cut into groups of
+// kGroupTiles tiles: a block per group, then one over the groups, make its
+// counts positions. The octree's nodes are segments: two passes over the 15
+// bits of their cells. 50M points, by chunk and by cell in two rounds: 1.4 ms
+// (with counts by digit, one scan, and the node's number among the sorted
+// bits 3.8).
 
 #include <cuda_runtime.h>
 
@@ -64,6 +72,7 @@ constexpr int kSegTile = kSegThreads * kSegSteps;
 
 struct SegNode {
 	int64_t off;    // first candidate (level-wide index)
+	int64_t out;    // where its output begins: off, or 0 for a group of a whole range's tiles
 	int64_t count;
 	double scale;   // key -> quantised key
 	int32_t tile0;  // its first tile
@@ -72,7 +81,7 @@ struct SegNode {
 
 struct SegTile {
 	int64_t start;     // first candidate
-	int64_t node_off;  // of the tile's node
+	int64_t out;       // of the tile's node
 	double scale;
 	int32_t count;     // candidates in the tile
 	int32_t node;
@@ -105,21 +114,21 @@ __global__ void seg_tiles_kernel(const SegNode* __restrict__ nodes, int K, int n
 	const int64_t first = (int64_t)(i - n.tile0) * kSegTile;
 	SegTile t;
 	t.start = n.off + first;
-	t.node_off = n.off;
+	t.out = n.out;
 	t.scale = n.scale;
 	t.count = (int32_t)(n.count - first < kSegTile ? n.count - first : kSegTile);
 	t.node = lo;
 	tiles[i] = t;
 }
 
-// FIRST: the keys are the node's, to be quantised when K has 32 bits
-template <class K, bool FIRST>
+// QUANT: 64-bit keys, to be quantised
+template <class K, bool QUANT>
 __device__ __forceinline__ K seg_key(const void* keys, int64_t p, double scale) {
-	if (sizeof(K) == 4 && FIRST) return (K)quantised(static_cast<const uint64_t*>(keys)[p], scale);
+	if (QUANT) return (K)quantised(static_cast<const uint64_t*>(keys)[p], scale);
 	return static_cast<const K*>(keys)[p];
 }
 
-template <class K, bool FIRST>
+template <class K, bool QUANT>
 __global__ void __launch_bounds__(kSegThreads) seg_count_kernel(const SegTile* __restrict__ tiles, const void* __restrict__ keys, int shift,
                                                               uint32_t* __restrict__ counts) {
 	__shared__ uint32_t hist[kSegDigits];
@@ -129,7 +138,7 @@ __global__ void __launch_bounds__(kSegThreads) seg_count_kernel(const SegTile* _
 #pragma unroll
 	for (int s = 0; s < kSegSteps; s++) {
 		const int i = s * kSegThreads + (int)threadIdx.x;
-		if (i < t.count) atomicAdd(&hist[(seg_key<K, FIRST>(keys, t.start + i, t.scale) >> shift) & 0xff], 1u);
+		if (i < t.count) atomicAdd(&hist[(seg_key<K, QUANT>(keys, t.start + i, t.scale) >> shift) & 0xff], 1u);
 	}
 	__syncthreads();
 	counts[(int64_t)blockIdx.x * kSegDigits + threadIdx.x] = hist[threadIdx.x];
@@ -137,9 +146,11 @@ __global__ void __launch_bounds__(kSegThreads) seg_count_kernel(const SegTile* _
 
 // One block per node: a tile's count of a digit becomes the node's count of
 // that digit in the tiles before it; base: where the digit begins in the node.
+// SUMS: only the node's count of each digit instead.
 // kParts threads share a digit's tiles, each its own stretch of them.
 constexpr int kParts = 4;
 
+template <bool SUMS>
 __global__ void __launch_bounds__(kSegDigits* kParts) seg_offsets_kernel(const SegNode* __restrict__ nodes, uint32_t* __restrict__ counts,
                                                                          uint32_t* __restrict__ base) {
 	__shared__ uint32_t part[kParts][kSegDigits];
@@ -160,18 +171,22 @@ __global__ void __launch_bounds__(kSegDigits* kParts) seg_offsets_kernel(const S
 		run += k < p ? part[k][d] : 0;
 		total += part[k][d];
 	}
-	uint32_t x = total;
+	if (SUMS) {
+		if (p == 0) base[(int64_t)blockIdx.x * kSegDigits + d] = total;
+	} else {
+		uint32_t x = total;
 #pragma unroll
-	for (int o = 1; o < 32; o <<= 1) {
-		const uint32_t y = __shfl_up_sync(FULL, x, o);
-		if (lane >= o) x += y;
-	}
-	if (p == 0 && lane == 31) wsum[d >> 5] = x;
-	__syncthreads();
-	if (p == 0) {
-		uint32_t before = 0;
-		for (int w = 0; w < d >> 5; w++) before += wsum[w];
-		base[(int64_t)blockIdx.x * kSegDigits + d] = before + x - total;
+		for (int o = 1; o < 32; o <<= 1) {
+			const uint32_t y = __shfl_up_sync(FULL, x, o);
+			if (lane >= o) x += y;
+		}
+		if (p == 0 && lane == 31) wsum[d >> 5] = x;
+		__syncthreads();
+		if (p == 0) {
+			uint32_t before = 0;
+			for (int w = 0; w < d >> 5; w++) before += wsum[w];
+			base[(int64_t)blockIdx.x * kSegDigits + d] = before + x - total;
+		}
 	}
 #pragma unroll 8
 	for (int t = t0; t < t1; t++) {
@@ -181,17 +196,20 @@ __global__ void __launch_bounds__(kSegDigits* kParts) seg_offsets_kernel(const S
 	}
 }
 
-// vals_in == nullptr: the value is the candidate's index in its node
-template <class K, bool FIRST>
+// vals_in == nullptr: the value is the candidate's index in its node. first:
+// where the digits of a whole range begin, or null.
+template <class K, bool QUANT>
 __global__ void __launch_bounds__(kSegThreads, 4) seg_scatter_kernel(const SegTile* __restrict__ tiles, const void* __restrict__ keys_in,
                                                                      const uint32_t* __restrict__ vals_in, K* __restrict__ keys_out,
                                                                      uint32_t* __restrict__ vals_out, int shift,
-                                                                     const uint32_t* __restrict__ counts, const uint32_t* __restrict__ base) {
+                                                                     const uint32_t* __restrict__ counts, const uint32_t* __restrict__ base,
+                                                                     const uint32_t* __restrict__ first) {
 	extern __shared__ __align__(16) unsigned char seg_smem[];
 	SegShared<K>& sh = *reinterpret_cast<SegShared<K>*>(seg_smem);
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 	const SegTile t = tiles[blockIdx.x];
-	const uint32_t before_tile = counts[(int64_t)blockIdx.x * kSegDigits + tid] + base[(int64_t)t.node * kSegDigits + tid];
+	const uint32_t before_tile =
+	    counts[(int64_t)blockIdx.x * kSegDigits + tid] + base[(int64_t)t.node * kSegDigits + tid] + (first ? first[tid] : 0u);
 	for (int i = tid; i < kSegWarps * kSegDigits; i += kSegThreads) (&sh.whist[0][0])[i] = 0;
 	__syncthreads();
 	K kr[kSegSteps];
@@ -204,8 +222,8 @@ __global__ void __launch_bounds__(kSegThreads, 4) seg_scatter_kernel(const SegTi
 		vr[s] = 0;
 		if (li < t.count) {
 			const int64_t p = t.start + li;
-			kr[s] = seg_key<K, FIRST>(keys_in, p, t.scale);
-			vr[s] = vals_in ? vals_in[p] : (uint32_t)(p - t.node_off);
+			kr[s] = seg_key<K, QUANT>(keys_in, p, t.scale);
+			vr[s] = vals_in ? vals_in[p] : (uint32_t)(p - t.out);
 		}
 	}
 #pragma unroll
@@ -242,7 +260,7 @@ __global__ void __launch_bounds__(kSegThreads, 4) seg_scatter_kernel(const SegTi
 	const uint32_t lbase = wbefore + x - run;  // exclusive over digits
 #pragma unroll
 	for (int w = 0; w < kSegWarps; w++) sh.whist[w][d] += lbase;
-	sh.gbase[d] = t.node_off + (int64_t)before_tile - (int64_t)lbase;
+	sh.gbase[d] = t.out + (int64_t)before_tile - (int64_t)lbase;
 	__syncthreads();
 #pragma unroll
 	for (int s = 0; s < kSegSteps; s++) {
@@ -344,45 +362,61 @@ double key_scale(const LevelNode& n) {
 	return f > 0.0 && f < 1e300 ? f : 0.0;
 }
 
-// Passes of K over bits [begin, end) of the nodes' keys. The result of the
-// last pass is in (keys[passes & 1], vals[passes & 1]) with pass p
-// writing (keys[(p + 1) & 1], ...).
-template <class K>
-void seg_sort(const std::vector<LevelNode>& ln, const uint64_t* keys_in, K* const* keys, uint32_t* const* vals, int begin_bit, int end_bit,
-              DeviceMem& mem) {
-	cudaStream_t s = mem.stream();
-	std::vector<SegNode> nodes(ln.size());
+// The nodes' tiles numbered through.
+int64_t number_tiles(std::vector<SegNode>& nodes) {
 	int64_t tiles = 0;
-	for (size_t k = 0; k < ln.size(); k++) {
-		const int64_t T = ceil_div(ln[k].count, kSegTile);
-		nodes[k] = SegNode{ln[k].cand_off, ln[k].count, key_scale(ln[k]), (int32_t)tiles, (int32_t)T};
+	for (SegNode& n : nodes) {
+		const int64_t T = ceil_div(n.count, kSegTile);
+		n.tile0 = (int32_t)tiles;
+		n.tiles = (int32_t)T;
 		tiles += T;
-		if (tiles > INT32_MAX) throw PcgError(5, "segmented sort: level too large");
+		if (tiles > INT32_MAX) throw PcgError(5, "segmented sort: too large");
 	}
+	return tiles;
+}
+
+// Passes of K over bits [begin, end) of the nodes' keys (keys_in; QUANT:
+// 64-bit keys to be quantised), and of their values (vals_in, or the index in
+// the node). Pass p writes (keys[(p + 1) & 1], vals[(p + 1) & 1]). whole: the
+// nodes are groups of the tiles of one range, which is sorted as a whole.
+template <class K, bool QUANT>
+void seg_sort(std::vector<SegNode>& nodes, bool whole, const void* keys_in, const uint32_t* vals_in, K* const* keys, uint32_t* const* vals,
+              int begin_bit, int end_bit, DeviceMem& mem) {
+	cudaStream_t s = mem.stream();
+	const int64_t tiles = number_tiles(nodes);
 	if (tiles == 0) return;
+	const size_t num = nodes.size();
+	if (whole) nodes.push_back(SegNode{0, 0, 0, 0.0, 0, (int32_t)num});  // the groups, as the tiles of one node
 	SegNode* d_nodes = mem.alloc<SegNode>(nodes.size());
 	PCG_CUDA(cudaMemcpyAsync(d_nodes, nodes.data(), nodes.size() * sizeof(SegNode), cudaMemcpyHostToDevice, s));
 	SegTile* d_tiles = mem.alloc<SegTile>(tiles);
-	seg_tiles_kernel<<<(unsigned)ceil_div(tiles, 256), 256, 0, s>>>(d_nodes, (int)nodes.size(), (int)tiles, d_tiles);
+	seg_tiles_kernel<<<(unsigned)ceil_div(tiles, 256), 256, 0, s>>>(d_nodes, (int)num, (int)tiles, d_tiles);
 	PCG_LAUNCHED();
 	uint32_t* counts = mem.alloc<uint32_t>((size_t)tiles * kSegDigits);
-	uint32_t* base = mem.alloc<uint32_t>(nodes.size() * kSegDigits);
+	uint32_t* base = mem.alloc<uint32_t>((num + 1) * kSegDigits);
+	uint32_t* first = whole ? base + num * kSegDigits : nullptr;
 	constexpr int smem = (int)sizeof(SegShared<K>);
 	static_assert(smem <= 48 * 1024, "the tile fits what a kernel may use unasked");
 	const void* kin = keys_in;
-	const uint32_t* vin = nullptr;
+	const uint32_t* vin = vals_in;
 	int pass = 0;
 	for (int shift = begin_bit; shift < end_bit; shift += 8, pass++) {
 		K* kout = keys[(pass + 1) & 1];
 		uint32_t* vout = vals[(pass + 1) & 1];
-		if (pass == 0) seg_count_kernel<K, true><<<(unsigned)tiles, kSegThreads, 0, s>>>(d_tiles, kin, shift, counts);
+		if (pass == 0) seg_count_kernel<K, QUANT><<<(unsigned)tiles, kSegThreads, 0, s>>>(d_tiles, kin, shift, counts);
 		else seg_count_kernel<K, false><<<(unsigned)tiles, kSegThreads, 0, s>>>(d_tiles, kin, shift, counts);
 		PCG_LAUNCHED();
-		seg_offsets_kernel<<<(unsigned)nodes.size(), kSegDigits * kParts, 0, s>>>(d_nodes, counts, base);
+		if (whole) {
+			seg_offsets_kernel<true><<<(unsigned)num, kSegDigits * kParts, 0, s>>>(d_nodes, counts, base);
+			PCG_LAUNCHED();
+			seg_offsets_kernel<false><<<1, kSegDigits * kParts, 0, s>>>(d_nodes + num, base, first);
+		} else {
+			seg_offsets_kernel<false><<<(unsigned)num, kSegDigits * kParts, 0, s>>>(d_nodes, counts, base);
+		}
 		PCG_LAUNCHED();
 		if (pass == 0)
-			seg_scatter_kernel<K, true><<<(unsigned)tiles, kSegThreads, smem, s>>>(d_tiles, kin, vin, kout, vout, shift, counts, base);
-		else seg_scatter_kernel<K, false><<<(unsigned)tiles, kSegThreads, smem, s>>>(d_tiles, kin, vin, kout, vout, shift, counts, base);
+			seg_scatter_kernel<K, QUANT><<<(unsigned)tiles, kSegThreads, smem, s>>>(d_tiles, kin, vin, kout, vout, shift, counts, base, first);
+		else seg_scatter_kernel<K, false><<<(unsigned)tiles, kSegThreads, smem, s>>>(d_tiles, kin, vin, kout, vout, shift, counts, base, first);
 		PCG_LAUNCHED();
 		kin = kout;
 		vin = vout;
@@ -393,18 +427,59 @@ void seg_sort(const std::vector<LevelNode>& ln, const uint64_t* keys_in, K* cons
 	mem.free(d_nodes);
 }
 
+std::vector<SegNode> seg_nodes(const std::vector<LevelNode>& ln) {
+	std::vector<SegNode> nodes;
+	for (const LevelNode& n : ln) nodes.push_back(SegNode{n.cand_off, n.cand_off, n.count, key_scale(n), 0, 0});
+	return nodes;
+}
+
 // all 64 bits, into (sk, sv)
 void seg_sort_full(const std::vector<LevelNode>& ln, int64_t M, const uint64_t* keys, uint64_t* sk, uint32_t* sv, DeviceMem& mem) {
 	uint64_t* k1 = mem.alloc<uint64_t>(M);
 	uint32_t* v1 = mem.alloc<uint32_t>(M);
 	uint64_t* const kb[2] = {sk, k1};
 	uint32_t* const vb[2] = {sv, v1};
-	seg_sort<uint64_t>(ln, keys, kb, vb, 0, 64, mem);  // 8 passes: the last writes kb[0]
+	std::vector<SegNode> nodes = seg_nodes(ln);
+	seg_sort<uint64_t, false>(nodes, false, keys, nullptr, kb, vb, 0, 64, mem);  // 8 passes: the last writes kb[0]
 	mem.free(k1);
 	mem.free(v1);
 }
 
 }  // namespace
+
+// A group's tiles: the block that adds a group up, then the one that adds the
+// groups up, each go through few enough (50M pairs: 382 groups).
+constexpr int64_t kGroupTiles = 64;
+
+void radix_sort_pairs(uint32_t*& keys, uint32_t*& vals, uint32_t*& keys_tmp, uint32_t*& vals_tmp, int64_t n, int begin_bit, int end_bit,
+                      DeviceMem& mem, bool iota) {
+	if (n >= (int64_t(1) << 32)) throw PcgError(1, "radix sort: more than 2^32 elements");
+	if (n <= 0 || end_bit <= begin_bit) return;
+	std::vector<SegNode> groups;
+	const int64_t per = kGroupTiles * kSegTile;
+	for (int64_t o = 0; o < n; o += per) groups.push_back(SegNode{o, 0, std::min(per, n - o), 0.0, 0, 0});
+	uint32_t* const kb[2] = {keys, keys_tmp};
+	uint32_t* const vb[2] = {vals, vals_tmp};
+	seg_sort<uint32_t, false>(groups, groups.size() > 1, keys, iota ? nullptr : vals, kb, vb, begin_bit, end_bit, mem);
+	if (((end_bit - begin_bit + 7) / 8) & 1) {
+		std::swap(keys, keys_tmp);
+		std::swap(vals, vals_tmp);
+	}
+}
+
+void radix_sort_segments(uint32_t*& keys, uint32_t*& vals, uint32_t*& keys_tmp, uint32_t*& vals_tmp,
+                         const std::vector<std::pair<int64_t, int64_t>>& segs, int begin_bit, int end_bit, DeviceMem& mem) {
+	if (end_bit <= begin_bit) return;
+	std::vector<SegNode> nodes;
+	for (const auto& g : segs) nodes.push_back(SegNode{g.first, g.first, g.second, 0.0, 0, 0});
+	uint32_t* const kb[2] = {keys, keys_tmp};
+	uint32_t* const vb[2] = {vals, vals_tmp};
+	seg_sort<uint32_t, false>(nodes, false, keys, vals, kb, vb, begin_bit, end_bit, mem);
+	if (((end_bit - begin_bit + 7) / 8) & 1) {
+		std::swap(keys, keys_tmp);
+		std::swap(vals, vals_tmp);
+	}
+}
 
 namespace {
 
@@ -469,7 +544,8 @@ void sort_level_distinct(const LevelNode* d_nodes, const std::vector<LevelNode>&
 	const uint64_t* keys = reinterpret_cast<const uint64_t*>(lb.keys);
 	uint32_t* const q[2] = {mem.alloc<uint32_t>(M), mem.alloc<uint32_t>(M)};
 	uint32_t* const v[2] = {mem.alloc<uint32_t>(M), mem.alloc<uint32_t>(M)};
-	seg_sort<uint32_t>(ln, keys, q, v, 0, kQuantBits, mem);
+	std::vector<SegNode> nodes = seg_nodes(ln);
+	seg_sort<uint32_t, true>(nodes, false, keys, nullptr, q, v, 0, kQuantBits, mem);
 	static_assert(kQuantBits == 24, "three passes end in q[1], v[1]");
 	uint64_t* sk = mem.alloc<uint64_t>(M);
 	uint32_t* sv = v[0];
