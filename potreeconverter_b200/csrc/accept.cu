@@ -20,11 +20,16 @@
 // waited for: 1,600 cycles a link.)
 // One block decides a node, a batch of positions after the other: the
 // decisions of the batch lie in shared memory (a byte each, and a bit each once
-// 32 are complete), those before it in global memory as bits.
-// Measured: a 50M-point hot-spot cloud (poisson, 162M candidates) 14.6 ms, in
-// rounds on a block or a cluster of blocks 29.5; one node of 41,054 candidates
-// 0.15 ms (in rounds 0.62 for 47,768); the 31M candidates of a 10M-point cloud
-// (poisson_average) 4.1 ms (14.3).
+// 32 are complete), those before it in global memory as bits. A node that is
+// large for its level gets a cluster of up to eight blocks: all hold all
+// decisions, and a warp writes what it decides into every block's shared
+// memory, so that reading costs what it does in one block. (Issue slots bound a
+// block, 400 instructions a word of 32 candidates at 55 % of the slots; spread
+// through global memory the same took 7 times as long as one block.)
+// Measured: a 50M-point hot-spot cloud (poisson, 162M candidates) 9.6 ms, one
+// block a node 16.1, in rounds with barriers 29.5; the 31M candidates of a
+// 10M-point cloud (poisson_average) 2.7 ms (4.1, 14.3); one node of 41,054
+// candidates 0.15 ms (in rounds 0.62 for 47,768).
 //
 // The 10,001-check cap compares how many points were accepted before the
 // candidate (count) with the rank of its last accepted conflict: it is
@@ -51,6 +56,11 @@ namespace {
 
 constexpr int kWindow = 10000;    // accepted points a conflict may have after it
 constexpr uint32_t kPollLimit = 1u << 24;
+// Blocks of a cluster (162M candidates of 50M points: 512 threads 14.8 ms, 768
+// 9.6, 1,024 10.0; clusters of 16 blocks no faster), and from how many
+// candidates a node may get one (40,000: 0.50 ms in clusters, 0.45 alone).
+constexpr int kClusterThreads = 768, kClusterMost = 8;
+constexpr int64_t kClusterMin = 65536;
 constexpr int64_t kBatchMost = 80 * 1024;  // positions of a batch: two blocks of 1,024 threads fit an SM
 
 // Decisions by sorted position: 0 not yet, 1 rejected, 2 accepted.
@@ -59,28 +69,52 @@ constexpr uint32_t kRejected = 1, kAccepted = 2;
 // shared memory of a block for a batch of that many positions (a multiple of
 // 128), byte offsets
 struct BatchLayout {
-	int32_t bits, prefix, done, bytes, end;  // by words: accepted bits, accepted before, complete; decisions (and one more)
+	int32_t prefix, words, bytes, end;  // by words: accepted before, accepted bits; decisions (and one more)
 };
 __host__ __device__ inline BatchLayout batch_layout(int32_t batch) {
 	BatchLayout l;
-	l.bits = 0;
-	l.prefix = l.bits + batch / 8;
-	l.done = l.prefix + batch / 8;
-	l.bytes = l.done + batch / 32;
+	l.prefix = 0;
+	l.words = l.prefix + batch / 8;
+	l.bytes = l.words + batch / 4;
 	l.end = l.bytes + batch + 4;
 	return l;
 }
 
+constexpr unsigned long long kComplete = 1ull << 32;
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+	uint32_t r;
+	asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+	return r;
+}
+__device__ __forceinline__ uint32_t cluster_blocks() {
+	uint32_t r;
+	asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+	return r;
+}
+// the same shared-memory address in block r of the cluster
+__device__ __forceinline__ uint32_t in_block(uint32_t address, uint32_t r) {
+	uint32_t a;
+	asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(address), "r"(r));
+	return a;
+}
+__device__ __forceinline__ void cluster_barrier() {
+	asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// CLUSTER: the blocks of a cluster decide one node; each holds all decisions,
+// and what a block decides it writes to the others as well.
+template <bool CLUSTER>
 struct State {
 	uint32_t base;          // shared-memory address of the decision of the batch's first position
 	int32_t first, n;       // that position; the node's candidates
-	uint32_t* bits;         // the batch's accepted bits (complete words)
+	uint32_t words;         // shared-memory address of the batch's accepted bits, kComplete added once a word is complete
 	uint32_t* prefix;       // accepted points before each of its words (below the frontier)
-	uint8_t* done;          // whether a word is complete
 	uint32_t* old_bits;     // bits and prefix of the whole node in global memory, for the batches before
 	uint32_t* old_prefix;
 	unsigned long long* frontier;  // word | accepted points before it << 32: every word below is complete
 	uint32_t* stop;                // a wait gave up: everybody leaves
+	uint32_t block, blocks;  // this one's place in the cluster, and how many
 
 	// position u of the batch
 	__device__ __forceinline__ uint32_t ld(int32_t u) const {
@@ -88,12 +122,29 @@ struct State {
 		asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(base + (uint32_t)(u - first)) : "memory");
 		return v;
 	}
+	// word w of the batch
+	__device__ __forceinline__ unsigned long long word(int32_t w) const {
+		unsigned long long v;
+		asm volatile("ld.volatile.shared.u64 %0, [%1];" : "=l"(v) : "r"(words + (uint32_t)w * 8u) : "memory");
+		return v;
+	}
 	// any position before those now taken
 	__device__ __forceinline__ uint32_t any(int32_t u) const {
 		return u < first ? kRejected + (__ldcg(old_bits + (u >> 5)) >> (u & 31) & 1) : ld(u);
 	}
 	__device__ __forceinline__ void st(int32_t u, uint32_t v) const {
-		asm volatile("st.shared.u8 [%0], %1;" ::"r"(base + (uint32_t)(u - first)), "r"(v) : "memory");
+		const uint32_t a = base + (uint32_t)(u - first);
+		asm volatile("st.shared.u8 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+		if (CLUSTER)
+			for (uint32_t r = 0; r < blocks; r++)
+				if (r != block) asm volatile("st.shared::cluster.u8 [%0], %1;" ::"r"(in_block(a, r)), "r"(v) : "memory");
+	}
+	__device__ __forceinline__ void give_up(SampleStats* st) const {
+		const uint32_t a = (uint32_t)__cvta_generic_to_shared(stop);
+		if (CLUSTER)
+			for (uint32_t r = 0; r < blocks; r++) asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(in_block(a, r)), "r"(1u) : "memory");
+		else *(volatile uint32_t*)stop = 1;
+		atomicAdd(&st->timeouts, 1ull);
 	}
 	__device__ __forceinline__ bool stopped() const { return *(volatile uint32_t*)stop != 0; }
 	__device__ __forceinline__ unsigned long long at_frontier() const { return *(volatile unsigned long long*)frontier; }
@@ -102,7 +153,7 @@ struct State {
 		const uint32_t below = (1u << (u & 31)) - 1;
 		if (u < first) return (int32_t)(__ldcg(old_prefix + (u >> 5)) + (uint32_t)__popc(__ldcg(old_bits + (u >> 5)) & below));
 		const int32_t w = (u - first) >> 5;
-		return (int32_t)(*(volatile uint32_t*)(prefix + w) + (uint32_t)__popc(*(volatile uint32_t*)(bits + w) & below));
+		return (int32_t)(*(volatile uint32_t*)(prefix + w) + (uint32_t)__popc((uint32_t)word(w) & below));
 	}
 	// Whether at most `most` points were accepted before t: 0 no, 1 yes, 2 not
 	// known yet. own, open: t's word's accepted and undecided lanes before t.
@@ -116,30 +167,32 @@ struct State {
 	}
 	// word g of 32 candidates is complete (one lane)
 	__device__ __forceinline__ void complete(int32_t g, uint32_t accepted) const {
-		const int32_t w = g - first / 32;
-		*(volatile uint32_t*)(bits + w) = accepted;
-		__threadfence_block();
-		*(volatile uint8_t*)(done + w) = 1;
+		const uint32_t a = words + (uint32_t)(g - first / 32) * 8u;
+		const unsigned long long v = kComplete | accepted;
+		asm volatile("st.volatile.shared.u64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
+		if (CLUSTER)
+			for (uint32_t r = 0; r < blocks; r++)
+				if (r != block) asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(in_block(a, r)), "l"(v) : "memory");
 	}
 	// The frontier's warp: accepted points before the batch's words as they are
 	// completed from its start on. False: a wait gave up.
 	__device__ bool keep_frontier(int32_t nb) const {
 		const int lane = threadIdx.x & 31;
-		const int32_t words = (nb + 31) >> 5;
+		const int32_t end = (nb + 31) >> 5;
 		uint32_t count = (uint32_t)(at_frontier() >> 32);
-		int32_t word = 0;
-		for (uint32_t poll = 0; word < words; poll++) {
-			const int32_t i = word + lane;
-			const bool full = i < words && *(volatile uint8_t*)(done + i) != 0;
+		int32_t at = 0;
+		for (uint32_t poll = 0; at < end; poll++) {
+			const int32_t i = at + lane;
+			const unsigned long long mine = i < end ? word(i) : 0ull;
+			const bool full = mine >= kComplete;
 			const uint32_t votes = __ballot_sync(FULL, full);
-			const int now = votes == FULL ? 32 : __ffs(~votes) - 1;  // complete from `word` on
+			const int now = votes == FULL ? 32 : __ffs(~votes) - 1;  // complete from `at` on
 			if (now == 0) {
 				if (poll >= kPollLimit || ((poll & 255) == 255 && stopped())) return false;
 				continue;
 			}
 			poll = 0;
-			__threadfence_block();
-			const uint32_t c = lane < now ? (uint32_t)__popc(*(volatile uint32_t*)(bits + i)) : 0u;
+			const uint32_t c = lane < now ? (uint32_t)__popc((uint32_t)mine) : 0u;
 			uint32_t x = c;
 #pragma unroll
 			for (int o = 1; o < 32; o <<= 1) {
@@ -148,10 +201,10 @@ struct State {
 			}
 			if (lane < now) *(volatile uint32_t*)(prefix + i) = count + x - c;
 			count += __shfl_sync(FULL, x, 31);
-			word += now;
+			at += now;
 			__threadfence_block();
 			__syncwarp();
-			if (lane == 0) *(volatile unsigned long long*)frontier = (unsigned long long)count << 32 | (uint32_t)(first / 32 + word);
+			if (lane == 0) *(volatile unsigned long long*)frontier = (unsigned long long)count << 32 | (uint32_t)(first / 32 + at);
 		}
 		return true;
 	}
@@ -160,15 +213,16 @@ struct State {
 // A distant accepted conflict u (t - u - 1 > kWindow) leaves t rejected while at
 // most rank(u) + kWindow + 1 points were accepted before t; -1: u's word is
 // not below the frontier yet.
-__device__ __forceinline__ int32_t most_before(const State& S, int32_t u) {
+template <class S_>
+__device__ __forceinline__ int32_t most_before(const S_& S, int32_t u) {
 	return (u >> 5) < (int32_t)(uint32_t)S.at_frontier() ? S.rank(u) + kWindow + 1 : -1;
 }
 
 // The decisions of 32 candidates some of which have a long list or wait for a
 // distant entry: every lane goes through its list from its first undecided entry
 // on. False: a wait gave up.
-template <int MODE>
-__device__ __noinline__ bool decide_any(const State S, int32_t t0, int nl, int4 q, int32_t ovf, bool done, const ConflictLists cl) {
+template <int MODE, class S_>
+__device__ __noinline__ bool decide_any(const S_ S, int32_t t0, int nl, int4 q, int32_t ovf, bool done, const ConflictLists cl) {
 	const int lane = threadIdx.x & 31;
 	const int32_t t = t0 + lane;
 	const bool is_long = nl == kListLong;
@@ -261,8 +315,8 @@ __device__ __noinline__ bool decide_any(const State S, int32_t t0, int nl, int4 
 // batch; `none` reads as rejected), then pool[at .. end) of the batch; most >= 0:
 // rejected too while at most so many points were accepted before t. False:
 // gave up.
-template <int E, bool CAPPED>
-__device__ __forceinline__ bool wait_for_lists(const State& S, int32_t t, bool done, const int32_t (&entry)[8], int32_t none, const int32_t* pool,
+template <int E, bool CAPPED, class S_>
+__device__ __forceinline__ bool wait_for_lists(const S_& S, int32_t t, bool done, const int32_t (&entry)[8], int32_t none, const int32_t* pool,
                                                int32_t at, int32_t end, int32_t most) {
 	int32_t e[E];
 #pragma unroll
@@ -326,8 +380,8 @@ __device__ __forceinline__ bool wait_for_lists(const State& S, int32_t t, bool d
 // The warp decides words w0, w0 + step, ... below w1 of 32 candidates; the next
 // word's lists are on their way meanwhile. `none`: a position whose decision
 // reads as rejected.
-template <int MODE>
-__device__ __forceinline__ void decide(const State& S, int64_t co, int32_t none, int32_t w0, int32_t w1, int32_t step, const ConflictLists& cl,
+template <int MODE, class S_>
+__device__ __forceinline__ void decide(const S_& S, int64_t co, int32_t none, int32_t w0, int32_t w1, int32_t step, const ConflictLists& cl,
                                        SampleStats* st) {
 	const int lane = threadIdx.x & 31;
 	const int32_t n = S.n;
@@ -427,69 +481,69 @@ __device__ __forceinline__ void decide(const State& S, int64_t co, int32_t none,
 		else if (more) ok = wait_for_lists<8, false>(S, t, done, e, none, cl.pool, at, end, -1);
 		else ok = wait_for_lists<4, false>(S, t, done, e, none, nullptr, 0, 0, -1);
 		if (!ok) {
-			if (lane == 0) {
-				*(volatile uint32_t*)S.stop = 1;
-				atomicAdd(&st->timeouts, 1ull);
-			}
+			if (lane == 0) S.give_up(st);
 			return;
 		}
 		const uint32_t acc = __ballot_sync(FULL, valid && S.ld(valid ? t : none) == kAccepted);
-		if (lane == 0) {
-			if (MODE == 0 && n > kWindow) S.complete(g, acc);
-			else S.bits[g - S.first / 32] = acc;
-		}
+		if (lane == 0) S.complete(g, acc);
 	}
 }
 
-// One block per node.
-template <int MODE, int THREADS>
-__global__ void __launch_bounds__(THREADS) accept_kernel(const LevelNode* __restrict__ nodes, const int32_t* __restrict__ set, int32_t batch, int wide,
+// One block per node, or one cluster of blocks.
+template <int MODE, int THREADS, bool CLUSTER>
+__global__ void __launch_bounds__(THREADS) accept_kernel(const LevelNode* __restrict__ nodes, const int32_t* __restrict__ set, int32_t batch, int64_t wide_min,
                                                          ConflictLists cl, uint32_t* accepted_bits, uint32_t* prefixes, SampleStats* st) {
 	extern __shared__ __align__(16) uint8_t accept_smem[];
 	__shared__ uint32_t stop;
 	__shared__ unsigned long long frontier;
-	const int32_t node = set[blockIdx.x];
+	State<CLUSTER> S;
+	S.block = CLUSTER ? cluster_rank() : 0;
+	S.blocks = CLUSTER ? cluster_blocks() : 1;
+	const int32_t node = set[blockIdx.x / S.blocks];
 	const int64_t co = nodes[node].cand_off;
 	const int32_t n = (int32_t)nodes[node].count;
 	const BatchLayout l = batch_layout(batch);
-	State S;
 	S.base = (uint32_t)__cvta_generic_to_shared(accept_smem + l.bytes);
 	S.n = n;
-	S.bits = reinterpret_cast<uint32_t*>(accept_smem + l.bits);
+	S.words = (uint32_t)__cvta_generic_to_shared(accept_smem + l.words);
 	S.prefix = reinterpret_cast<uint32_t*>(accept_smem + l.prefix);
-	S.done = accept_smem + l.done;
 	S.old_bits = accepted_bits + accept_word(co, node);
 	S.old_prefix = prefixes + accept_word(co, node);
 	S.frontier = &frontier;
 	S.stop = &stop;
+	auto barrier = [&] {
+		if (CLUSTER) cluster_barrier();
+		else __syncthreads();
+	};
 	if (threadIdx.x == 0) {
 		stop = 0;
 		frontier = 0;
-		if (wide) atomicAdd(&st->cluster_nodes, 1ull);
+		if (n >= wide_min && S.block == 0) atomicAdd(&st->cluster_nodes, 1ull);
 	}
 	for (int32_t b0 = 0; b0 < n; b0 += batch) {
 		const int32_t nb = n - b0 < batch ? n - b0 : batch;
 		S.first = b0;
-		// no word complete, no decision (done and bytes lie together)
-		uint32_t* word = reinterpret_cast<uint32_t*>(accept_smem + l.done);
-		for (int32_t i = threadIdx.x; i < (batch / 32 + nb + 3) / 4; i += THREADS) word[i] = 0;
+		// no word complete, no decision (words and bytes lie together)
+		uint32_t* zero = reinterpret_cast<uint32_t*>(accept_smem + l.words);
+		for (int32_t i = threadIdx.x; i < (batch / 4 + nb + 3) / 4; i += THREADS) zero[i] = 0;
 		__syncthreads();
 		if (threadIdx.x == 0) accept_smem[l.bytes + batch] = kRejected;
-		__syncthreads();
+		barrier();
 		// with the cap in play the first warp keeps the frontier
-		const int32_t keepers = MODE == 0 && n > kWindow ? 1 : 0, warp = (int32_t)threadIdx.x / 32;
+		const int32_t keepers = MODE == 0 && n > kWindow ? 1 : 0, warp = (int32_t)threadIdx.x / 32, workers = THREADS / 32 - keepers;
 		if (warp >= keepers) {
-			decide<MODE>(S, co, b0 + batch, b0 / 32 + warp - keepers, (b0 + nb + 31) / 32, THREADS / 32 - keepers, cl, st);
+			decide<MODE>(S, co, b0 + batch, b0 / 32 + (int32_t)S.block * workers + warp - keepers, (b0 + nb + 31) / 32,
+			             (int32_t)S.blocks * workers, cl, st);
 		} else if (!S.keep_frontier(nb) && threadIdx.x == 0) {
-			stop = 1;
-			atomicAdd(&st->timeouts, 1ull);
+			S.give_up(st);
 		}
-		__syncthreads();
-		for (int32_t i = threadIdx.x; i < (nb + 31) / 32; i += THREADS) S.old_bits[b0 / 32 + i] = S.bits[i];
-		if (MODE == 0)
-			for (int32_t i = threadIdx.x; i < (nb + 31) / 32; i += THREADS) S.old_prefix[b0 / 32 + i] = S.prefix[i];
+		barrier();
+		for (int32_t i = (int32_t)(S.block * THREADS + threadIdx.x); i < (nb + 31) / 32; i += (int32_t)S.blocks * THREADS) {
+			S.old_bits[b0 / 32 + i] = (uint32_t)S.word(i);
+			if (MODE == 0) S.old_prefix[b0 / 32 + i] = S.prefix[i];
+		}
 		__threadfence();
-		__syncthreads();
+		barrier();
 	}
 }
 
@@ -531,18 +585,35 @@ void launch_accept(int mode, const LevelNode* d_nodes, const std::vector<LevelNo
 		else if (ln[k].count > 0) order.push_back(k);
 	}
 	std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) { return ln[a].count > ln[b].count; });
-	// three sets, largest first
-	size_t n_wide = 0, n_full = 0;
-	while (n_wide < order.size() && ln[order[n_wide]].count >= sch.cluster_min) n_wide++;
-	while (n_wide + n_full < order.size() && ln[order[n_wide + n_full]].count >= full_min) n_full++;
-	const size_t n_small = order.size() - n_wide - n_full;
+	// The sets, largest first. A node that holds more than an SM's share of the
+	// level gets a cluster of about so many blocks: alone on its SM it would be
+	// what the level waits for (50M points: 16.1 ms without clusters, 13.4 where
+	// they only go to the levels of few nodes, 9.6 so; twice as many blocks, or
+	// three quarters, within 2 %).
+	struct Set {
+		size_t first, count;
+		int threads;
+		unsigned cluster;
+	};
+	std::vector<Set> sets;
+	int64_t total = 0;
+	for (int32_t k : order) total += ln[k].count;
+	const int middle = sch.middle >= 32 ? 512 : sch.middle >= 16 ? 256 : 128;
+	for (size_t i = 0; i < order.size(); i++) {
+		const int64_t n = ln[order[i]].count;
+		unsigned c = 1;
+		if (n >= kClusterMin)
+			while (c < kClusterMost && n * sm_count() > total * c) c *= 2;
+		const int threads = c > 1 ? kClusterThreads : n >= sch.cluster_min ? 1024 : n >= full_min ? middle : 128;
+		if (sets.empty() || sets.back().threads != threads || sets.back().cluster != c) sets.push_back(Set{i, 0, threads, c});
+		sets.back().count++;
+	}
 	uint32_t* prefixes = mem.alloc<uint32_t>(mode == 0 ? (size_t)accept_words(lb.M, K) : 1);
 	int32_t* d_order = mem.alloc<int32_t>(std::max<size_t>(order.size(), 1));
 	if (!order.empty()) PCG_CUDA(cudaMemcpyAsync(d_order, order.data(), order.size() * sizeof(int32_t), cudaMemcpyHostToDevice, s));
 	// the sets are independent: the first runs on the job's stream, the others
 	// each on a side stream
-	const int sets = (n_wide ? 1 : 0) + (n_full ? 1 : 0) + (n_small ? 1 : 0);
-	const int nsides = mem.arena() ? std::min(sets - 1, DeviceArena::kSides) : 0;
+	const int nsides = mem.arena() ? std::max(0, std::min((int)sets.size() - 1, DeviceArena::kSides)) : 0;
 	cudaStream_t side[DeviceArena::kSides] = {};
 	cudaEvent_t fork[DeviceArena::kSides] = {}, join[DeviceArena::kSides] = {};
 	for (int k = 0; k < nsides; k++) {
@@ -551,30 +622,39 @@ void launch_accept(int mode, const LevelNode* d_nodes, const std::vector<LevelNo
 		PCG_CUDA(cudaStreamWaitEvent(side[k], fork[k], 0));
 	}
 	int used = 0;
-	auto launch_set = [&](auto kernel, size_t first, size_t count, int threads) {
+	auto launch_set = [&](auto kernel, size_t first, size_t count, int threads, unsigned cluster) {
 		const int i = used++;
 		cudaStream_t cs = i == 0 || nsides == 0 ? s : side[std::min(i, nsides) - 1];
 		const int64_t n = ln[order[first]].count;  // the set's largest
 		const int32_t batch = (int32_t)std::min<int64_t>((n + 127) & ~int64_t(127), kBatchMost);
 		const size_t smem = (size_t)batch_layout(batch).end;
 		if (smem > 48 * 1024) PCG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-		kernel<<<(unsigned)count, threads, smem, cs>>>(d_nodes, d_order + first, batch, first < n_wide, cl, accepted_bits, prefixes, st);
+		cudaLaunchAttribute attr{};
+		attr.id = cudaLaunchAttributeClusterDimension;
+		attr.val.clusterDim.x = cluster;
+		attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+		cudaLaunchConfig_t cfg{};
+		cfg.gridDim = dim3((unsigned)count * cluster);
+		cfg.blockDim = dim3((unsigned)threads);
+		cfg.dynamicSmemBytes = smem;
+		cfg.stream = cs;
+		cfg.attrs = &attr;
+		cfg.numAttrs = cluster > 1 ? 1 : 0;
+		PCG_CUDA(cudaLaunchKernelEx(&cfg, kernel, d_nodes, (const int32_t*)(d_order + first), batch, sch.cluster_min, cl, accepted_bits, prefixes, st));
 		PCG_LAUNCHED();
 	};
-	auto set_of = [&](size_t first, size_t count, int threads) {
-		if (!count) return;
+	auto set_of = [&](size_t first, size_t count, int threads, unsigned cluster) {
 		auto pick = [&](auto poisson, auto average) {
-			if (mode == 0) launch_set(poisson, first, count, threads);
-			else launch_set(average, first, count, threads);
+			if (mode == 0) launch_set(poisson, first, count, threads, cluster);
+			else launch_set(average, first, count, threads, cluster);
 		};
-		if (threads == 1024) pick(accept_kernel<0, 1024>, accept_kernel<1, 1024>);
-		else if (threads == 512) pick(accept_kernel<0, 512>, accept_kernel<1, 512>);
-		else if (threads == 256) pick(accept_kernel<0, 256>, accept_kernel<1, 256>);
-		else pick(accept_kernel<0, 128>, accept_kernel<1, 128>);
+		if (cluster > 1) pick(accept_kernel<0, kClusterThreads, true>, accept_kernel<1, kClusterThreads, true>);
+		else if (threads == 1024) pick(accept_kernel<0, 1024, false>, accept_kernel<1, 1024, false>);
+		else if (threads == 512) pick(accept_kernel<0, 512, false>, accept_kernel<1, 512, false>);
+		else if (threads == 256) pick(accept_kernel<0, 256, false>, accept_kernel<1, 256, false>);
+		else pick(accept_kernel<0, 128, false>, accept_kernel<1, 128, false>);
 	};
-	set_of(0, n_wide, 1024);
-	set_of(n_wide, n_full, sch.middle >= 32 ? 512 : sch.middle >= 16 ? 256 : 128);
-	set_of(n_wide + n_full, n_small, 128);
+	for (const Set& g : sets) set_of(g.first, g.count, g.threads, g.cluster);
 	for (int k = 0; k < nsides; k++) {
 		PCG_CUDA(cudaEventRecord(join[k], side[k]));
 		PCG_CUDA(cudaStreamWaitEvent(s, join[k], 0));

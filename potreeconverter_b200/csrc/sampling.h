@@ -83,7 +83,8 @@ void launch_gather_records(const uint32_t* ids, int64_t n, const int32_t* X, con
 // How many threads decide which node of a level (accept.cu): nodes of at
 // least cluster_min candidates get 1,024, those of at least cta_min
 // (small_level_cta_min on levels with fewer nodes than 2 x SMs) 16 x middle
-// (128, 256 or 512), smaller ones 128. The compiled-in values come from the
+// (128, 256 or 512), smaller ones 128; large ones of their level a cluster of
+// blocks instead. The compiled-in values come from the
 // autotuner's table (tuned_schedule.h, written by
 // potreeconverter_b200/autotune.py); PCG_SCHEDULE="cta_min,
 // small_level_cta_min,cluster_min,middle" in the environment overrides them
