@@ -596,6 +596,7 @@ void launch_accept(int mode, const LevelNode* d_nodes, const std::vector<LevelNo
 		unsigned cluster;
 	};
 	std::vector<Set> sets;
+	const int64_t sms = sm_count();
 	int64_t total = 0;
 	for (int32_t k : order) total += ln[k].count;
 	const int middle = sch.middle >= 32 ? 512 : sch.middle >= 16 ? 256 : 128;
@@ -603,7 +604,7 @@ void launch_accept(int mode, const LevelNode* d_nodes, const std::vector<LevelNo
 		const int64_t n = ln[order[i]].count;
 		unsigned c = 1;
 		if (n >= kClusterMin)
-			while (c < kClusterMost && n * sm_count() > total * c) c *= 2;
+			while (c < kClusterMost && n * sms > total * c) c *= 2;
 		const int threads = c > 1 ? kClusterThreads : n >= sch.cluster_min ? 1024 : n >= full_min ? middle : 128;
 		if (sets.empty() || sets.back().threads != threads || sets.back().cluster != c) sets.push_back(Set{i, 0, threads, c});
 		sets.back().count++;

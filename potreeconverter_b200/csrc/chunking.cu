@@ -339,13 +339,16 @@ __global__ void lut_merge_kernel(const TH* __restrict__ high, int64_t* __restric
 	}
 }
 
+// kLutSlices blocks share a chunk's cells: a coarse chunk has as many as all the
+// others, and one block for it took 42 us of a 128^3 grid.
+constexpr int kLutSlices = 32;
 __global__ void lut_fill_kernel(const ChunkCell* __restrict__ chunks, int grid_size, int level_max, int32_t* __restrict__ lut) {
-	ChunkCell c = chunks[blockIdx.x];
-	int size = 1 << (level_max - c.level);
-	int64_t cells = (int64_t)size * size * size;
-	for (int64_t t = threadIdx.x; t < cells; t += blockDim.x) {
-		int ox = (int)(t % size), oy = (int)((t / size) % size), oz = (int)(t / ((int64_t)size * size));
-		int64_t x = (int64_t)size * c.x + ox, y = (int64_t)size * c.y + oy, z = (int64_t)size * c.z + oz;
+	const ChunkCell c = chunks[blockIdx.x];
+	const int shift = level_max - c.level, size = 1 << shift;
+	const int64_t cells = (int64_t)1 << (3 * shift);
+	for (int64_t t = (int64_t)blockIdx.y * blockDim.x + threadIdx.x; t < cells; t += (int64_t)gridDim.y * blockDim.x) {
+		const int64_t x = ((int64_t)c.x << shift) + (t & (size - 1)), y = ((int64_t)c.y << shift) + (t >> shift & (size - 1)),
+		              z = ((int64_t)c.z << shift) + (t >> (2 * shift));
 		lut[x + y * grid_size + z * (int64_t)grid_size * grid_size] = (int32_t)blockIdx.x;
 	}
 }
@@ -556,7 +559,7 @@ void launch_lut_merge(const uint32_t* grid, int grid_size, int64_t max_points_pe
 void launch_lut_fill(const ChunkCell* chunks, int num_chunks, int grid_size, int32_t* lut, DeviceMem& mem) {
 	if (num_chunks == 0) return;
 	int level_max = bits_for((uint64_t)grid_size) - 1;
-	lut_fill_kernel<<<num_chunks, 256, 0, mem.stream()>>>(chunks, grid_size, level_max, lut);
+	lut_fill_kernel<<<dim3(num_chunks, kLutSlices), 256, 0, mem.stream()>>>(chunks, grid_size, level_max, lut);
 	PCG_LAUNCHED();
 }
 

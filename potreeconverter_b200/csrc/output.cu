@@ -142,17 +142,17 @@ __global__ void fill_colors_kernel(DecodeParams p, const uint32_t* __restrict__ 
 
 constexpr int kSplitThreads = 256;
 constexpr int kSplitSteps = kSplitStretch / 32;  // of a warp, which takes a stretch
+static_assert(kSplitSteps == 4, "a lane counts four flags in one word");
 
-// accepted candidates per stretch, one warp each, 16 flags a lane
+// accepted candidates per stretch, one warp each, four flags a lane
 __global__ void __launch_bounds__(kSplitThreads) split_count_kernel(const uint8_t* __restrict__ accepted, int64_t n,
                                                                     uint32_t* __restrict__ counts) {
 	const int64_t w = ((int64_t)blockIdx.x * kSplitThreads + threadIdx.x) >> 5;
 	const int lane = threadIdx.x & 31;
-	const int64_t at = w * kSplitStretch + lane * 16;
+	const int64_t at = w * kSplitStretch + lane * kSplitSteps;
 	uint32_t c = 0;
-	if (at + 16 <= n) {
-		const uint4 v = *reinterpret_cast<const uint4*>(accepted + at);
-		c = __popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w);
+	if (at + kSplitSteps <= n) {
+		c = __popc(*reinterpret_cast<const uint32_t*>(accepted + at));
 	} else {
 		for (int64_t i = at; i < n; i++) c += accepted[i];
 	}
@@ -161,7 +161,8 @@ __global__ void __launch_bounds__(kSplitThreads) split_count_kernel(const uint8_
 }
 
 // One warp per stretch: ballots give every candidate its place. Bound by
-// memory, 29 to 45 bytes a candidate. (Flags widened to words, scanned and read
+// memory, 29 to 45 bytes a candidate. (Stretches of 512 left a small level to
+// a few warps: 12 us for 3,000 candidates, 4 so.) (Flags widened to words, scanned and read
 // again per candidate: 3.3 ms for 162M candidates where this and its
 // counts take 1.3.)
 __global__ void __launch_bounds__(kSplitThreads) split_kernel(const uint8_t* __restrict__ accepted, const uint32_t* __restrict__ before, int64_t n,
@@ -174,7 +175,7 @@ __global__ void __launch_bounds__(kSplitThreads) split_kernel(const uint8_t* __r
 	if (w * kSplitStretch >= n) return;
 	uint32_t a = before[w];
 	const uint32_t lt = (1u << lane) - 1u;
-#pragma unroll 4
+#pragma unroll
 	for (int s = 0; s < kSplitSteps; s++) {
 		const int64_t j = w * kSplitStretch + s * 32 + lane;
 		const bool in = j < n, take = in && accepted[j];

@@ -22,7 +22,7 @@ void launch_fill_colors(const DecodeParams& p, const uint32_t* ids, int64_t n, u
 // rejected ids into rej_ids (skipped when null). before: how many are accepted
 // before every stretch of kSplitStretch candidates and, last, in all;
 // split_stretches(n) + 1 entries.
-constexpr int kSplitStretch = 512;
+constexpr int kSplitStretch = 128;
 inline int64_t split_stretches(int64_t n) { return ceil_div(n, kSplitStretch); }
 void launch_split(const uint8_t* accepted, int64_t n, const uint32_t* ids, const uint64_t* cols, const int4* rec, uint32_t* before,
                   uint32_t* acc_ids, uint64_t* acc_cols, int4* acc_rec, uint32_t* rej_ids, DeviceMem& mem);
