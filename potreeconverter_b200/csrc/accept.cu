@@ -82,26 +82,6 @@ __host__ __device__ inline BatchLayout batch_layout(int32_t batch) {
 
 constexpr unsigned long long kComplete = 1ull << 32;
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-	uint32_t r;
-	asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-	return r;
-}
-__device__ __forceinline__ uint32_t cluster_blocks() {
-	uint32_t r;
-	asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
-	return r;
-}
-// the same shared-memory address in block r of the cluster
-__device__ __forceinline__ uint32_t in_block(uint32_t address, uint32_t r) {
-	uint32_t a;
-	asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(address), "r"(r));
-	return a;
-}
-__device__ __forceinline__ void cluster_barrier() {
-	asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
-}
-
 // CLUSTER: the blocks of a cluster decide one node; each holds all decisions,
 // and what a block decides it writes to the others as well.
 template <bool CLUSTER>

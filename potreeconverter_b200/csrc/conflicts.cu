@@ -16,22 +16,26 @@
 //  1. cells of one spacing (x 1.000001) over the node box, so every point
 //     closer than the spacing lies in the 3 x 3 x 3 cells around a
 //     candidate's own; a bitmap of the occupied cells, 128 bits per row of
-//     cells along x, and per row how many occupied cells come before it: a
-//     cell's rank among the node's occupied ones is one 16-byte load, one
-//     4-byte load and a few population counts;
+//     cells along x, and beside each of its words how many occupied cells
+//     come before it: a cell's rank among the node's occupied ones is one
+//     8-byte load and a population count;
 //  2. a counting sort of the candidates by that rank (within a cell in any
 //     order: a list is a set). Everything up to here runs in gather order,
 //     in which neighbours in memory are neighbours in space, so the counters
 //     and the scattered records of a warp fall into a few lines. (A stable
 //     radix sort in the order of the distances and a hash table of the cells
-//     took 16.5 ms of a 50M-point conversion where this takes 7.6.)
+//     took 16.5 ms of a 50M-point conversion where this takes 6.2, the scan
+//     included.)
 //  3. one thread per candidate in cell order: the cells x - 1 .. x + 1 of a
 //     row lie together in memory, so the 27 cells are nine runs of records,
 //     whose bounds are loaded at once. The FP32 distance on node-relative
 //     coordinates decides every pair outside the band s^2 (1 -/+ 1e-3);
 //     pairs inside the band are decided by the reference's FP64 test and
 //     counted as escalated; then the early-exit bound. (27 hash probes per
-//     candidate took 30.6 ms of a 50M-point conversion, this 13.3.)
+//     candidate took 30.6 ms of a 50M-point conversion, this 11.9;
+//     with the counts beside the rows 13.3, leaving out the cells that the
+//     ball of a spacing misses or finding a cell's runs once for the warp
+//     gains nothing.)
 //
 // Error bound of the FP32 test (u = 2^-24): a node-relative coordinate v lies
 // in [0, L], L = 128 s, so its float differs from the FP64 value by at most
@@ -73,6 +77,7 @@ namespace {
 constexpr int kAxisBits = 7;
 constexpr int kCellsPerAxis = 1 << kAxisBits;  // node box = 128 spacings
 constexpr int64_t kRows = (int64_t)kCellsPerAxis * kCellsPerAxis;  // of a node
+constexpr int kRowWords = kCellsPerAxis / 32;
 // entries of all long lists of a level (1 GiB)
 constexpr int64_t kLongBudget = int64_t(1) << 28;
 // six blocks an SM: 40 registers, a few spills outside the loop (50M points:
@@ -90,17 +95,6 @@ __device__ __forceinline__ int clamp_cell(double u) {
 	return (int)f;
 }
 
-// occupied cells of a row below x
-__device__ __forceinline__ int row_rank(const uint4& b, int x) {
-	const int w = x >> 5;
-	const uint32_t m = (1u << (x & 31)) - 1;
-	int r = __popc((w == 0 ? b.x : w == 1 ? b.y : w == 2 ? b.z : b.w) & m);
-	if (w > 0) r += __popc(b.x);
-	if (w > 1) r += __popc(b.y);
-	if (w > 2) r += __popc(b.z);
-	return r;
-}
-
 // every candidate's cell (z, y, x, seven bits each) and the occupancy bitmaps
 __global__ void cell_mark_kernel(const LevelNode* __restrict__ nodes, PosParamsS pp, LevelBuffers lb, uint32_t* __restrict__ cell,
                                  uint32_t* __restrict__ rows) {
@@ -115,69 +109,87 @@ __global__ void cell_mark_kernel(const LevelNode* __restrict__ nodes, PosParamsS
 	const int cz = clamp_cell((qcoord(r.z, 2, pp) - nd.min[2]) * inv);
 	const uint32_t row = (uint32_t)(cz << kAxisBits | cy);
 	cell[j] = row << kAxisBits | (uint32_t)cx;
-	uint32_t* word = rows + ((int64_t)node * kRows + row) * 4 + (cx >> 5);
+	uint32_t* word = rows + ((int64_t)node * kRows + row) * kRowWords + (cx >> 5);
 	const uint32_t bit = 1u << (cx & 31);
 	// most candidates find their cell marked already
 	if (!(*(volatile uint32_t*)word & bit)) atomicOr(word, bit);
 }
 
-constexpr int kRowThreads = 1024;
-constexpr int kRowSteps = (int)(kRows / kRowThreads);  // a warp's stretch of rows, 32 a step
+constexpr int kRowThreads = 256, kRowBlocks = 8;
+constexpr int kRowSteps = (int)(kRows / kRowBlocks / kRowThreads);  // a warp's stretch of rows, 32 a step
 
-// Occupied cells of the node before each row; one block per node. Bound by its
-// loads, so a warp's lie side by side (a thread's own 16 rows in a row: 19 us
-// for a few nodes, 6 so).
-__global__ void __launch_bounds__(kRowThreads) row_base_kernel(const uint4* __restrict__ rows, uint32_t* __restrict__ base) {
-	__shared__ uint32_t sums[kRowThreads / 32];
+// The words of a node's rows with the occupied cells before each; a cluster of
+// blocks per node, each with its stretch of rows in registers, which tell one
+// another their counts. Bound by memory (256 KB in, 512 KB out a node), which
+// one block for a node takes 23 us to move; a cluster 6, and 2,743 nodes 0.60 ms.
+__global__ void __cluster_dims__(kRowBlocks) __launch_bounds__(kRowThreads) row_words_kernel(const uint4* __restrict__ rows, uint4* __restrict__ words) {
+	__shared__ uint32_t sums[kRowThreads / 32], parts[kRowBlocks];
+	cluster_barrier();  // all blocks are there
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-	const int64_t r0 = (int64_t)blockIdx.x * kRows + warp * (kRowSteps * 32) + lane;
-	uint32_t c[kRowSteps];
+	const uint32_t rank = cluster_rank();
+	const int64_t r0 = (int64_t)blockIdx.x * (kRows / kRowBlocks) + warp * (kRowSteps * 32) + lane;
+	uint4 b[kRowSteps];
+#pragma unroll
+	for (int i = 0; i < kRowSteps; i++) b[i] = rows[r0 + i * 32];
+	// the count before each in the warp's stretch
+	uint32_t c[kRowSteps], run = 0;
 #pragma unroll
 	for (int i = 0; i < kRowSteps; i++) {
-		const uint4 b = rows[r0 + i * 32];
-		c[i] = (uint32_t)(__popc(b.x) + __popc(b.y) + __popc(b.z) + __popc(b.w));
-	}
-	// each becomes the count before it in the warp's stretch
-	uint32_t run = 0;
-#pragma unroll
-	for (int i = 0; i < kRowSteps; i++) {
-		uint32_t x = c[i];
+		const uint32_t own = (uint32_t)(__popc(b[i].x) + __popc(b[i].y) + __popc(b[i].z) + __popc(b[i].w));
+		uint32_t x = own;
 #pragma unroll
 		for (int o = 1; o < 32; o <<= 1) {
 			const uint32_t y = __shfl_up_sync(FULL, x, o);
 			if (lane >= o) x += y;
 		}
-		c[i] = run + x - c[i];
+		c[i] = run + x - own;
 		run += __shfl_sync(FULL, x, 31);
 	}
 	if (lane == 0) sums[warp] = run;
 	__syncthreads();
-	uint32_t before = lane < warp ? sums[lane] : 0u;
-	before = __reduce_add_sync(FULL, before);
+	uint32_t before = 0, total = 0;
+	for (int w = 0; w < kRowThreads / 32; w++) {
+		before += w < warp ? sums[w] : 0u;
+		total += sums[w];
+	}
+	if (threadIdx.x < kRowBlocks)
+		asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(in_block((uint32_t)__cvta_generic_to_shared(&parts[rank]), threadIdx.x)), "r"(total)
+		             : "memory");
+	cluster_barrier();
+	for (uint32_t r = 0; r < rank; r++) before += parts[r];
 #pragma unroll
-	for (int i = 0; i < kRowSteps; i++) base[r0 + i * 32] = before + c[i];
+	for (int i = 0; i < kRowSteps; i++) {
+		const uint32_t c0 = before + c[i], c1 = c0 + __popc(b[i].x), c2 = c1 + __popc(b[i].y), c3 = c2 + __popc(b[i].z);
+		words[2 * (r0 + i * 32)] = make_uint4(b[i].x, c0, b[i].y, c1);
+		words[2 * (r0 + i * 32) + 1] = make_uint4(b[i].z, c2, b[i].w, c3);
+	}
 }
 
 // (cell index of the level, place within the cell) of every candidate; the
-// node's cells are counted in count[cand_off ..). The lanes of a warp that
-// share a cell count once.
+// node's cells are counted in count[cand_off ..). Neighbouring lanes that share
+// a cell count once (all lanes that do, found by match: 1.9 ms for 162M
+// candidates, 1.65 so).
 __global__ void cell_count_kernel(const LevelNode* __restrict__ nodes, LevelBuffers lb, const uint32_t* __restrict__ cell,
-                                  const uint4* __restrict__ rows, const uint32_t* __restrict__ base, uint32_t* __restrict__ count,
-                                  uint2* __restrict__ place) {
+                                  const uint2* __restrict__ words, uint32_t* __restrict__ count, uint2* __restrict__ place) {
 	const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+	const int lane = threadIdx.x & 31;
 	uint32_t idx = 0xffffffffu;
 	if (j < lb.M) {
 		const int32_t node = lb.node_of[j];
 		const uint32_t c = cell[j];
-		const int64_t row = (int64_t)node * kRows + (c >> kAxisBits);
-		idx = (uint32_t)nodes[node].cand_off + base[row] + (uint32_t)row_rank(rows[row], (int)(c & (kCellsPerAxis - 1)));
+		const uint2 w = words[((int64_t)node * kRows + (c >> kAxisBits)) * kRowWords + (c >> 5 & (kRowWords - 1))];
+		idx = (uint32_t)nodes[node].cand_off + w.y + (uint32_t)__popc(w.x & ((1u << (c & 31)) - 1));
 	}
-	const unsigned peers = __match_any_sync(FULL, idx);
-	const int leader = __ffs(peers) - 1;
+	const uint32_t prev = __shfl_up_sync(FULL, idx, 1);
+	const uint32_t heads = __ballot_sync(FULL, lane == 0 || prev != idx);
+	const uint32_t upto = lanemask_lt() << 1 | 1u;
+	const int leader = 31 - __clz(heads & upto);
+	const uint32_t after = heads & ~upto;
+	const int end = after ? __ffs(after) - 1 : 32;  // the run's, for its leader
 	uint32_t first = 0;
-	if (j < lb.M && (int)(threadIdx.x & 31) == leader) first = atomicAdd(&count[idx], (uint32_t)__popc(peers));
+	if (j < lb.M && lane == leader) first = atomicAdd(&count[idx], (uint32_t)(end - lane));
 	first = __shfl_sync(FULL, first, leader);
-	if (j < lb.M) place[j] = make_uint2(idx, first + (uint32_t)__popc(peers & lanemask_lt()));
+	if (j < lb.M) place[j] = make_uint2(idx, first + (uint32_t)(lane - leader));
 }
 
 // records in cell order: the position relative to the node's minimum corner in
@@ -196,31 +208,38 @@ __global__ void cell_scatter_kernel(const LevelNode* __restrict__ nodes, PosPara
 	if (lc.col) lc.col[at] = lb.cols[j];
 }
 
-// The runs of records around cell c of a node (rows, base: the node's; co: its
+// The runs of records around cell c of a node (words: the node's; co: its
 // cand_off): up to nine, written to runs[0], runs[stride], ... as [first, end).
-// Returns how many.
-__device__ __forceinline__ int find_runs(uint32_t c, uint32_t co, const uint4* __restrict__ rows, const uint32_t* __restrict__ base,
-                                         const uint32_t* __restrict__ start, uint2* runs, int stride) {
+// Returns how many. Candidates lie sparsely, one or two a cell and most rows
+// around it empty, so this is most of a search; it waits for two loads one
+// after the other, of the word that tells both which cells are occupied and
+// how many come before it, and of the bounds.
+__device__ __forceinline__ int find_runs(uint32_t c, uint32_t co, const uint2* __restrict__ words, const uint32_t* __restrict__ start, uint2* runs,
+                                         int stride) {
 	const int cx = (int)(c & (kCellsPerAxis - 1)), cy = (int)(c >> kAxisBits & (kCellsPerAxis - 1)), cz = (int)(c >> (2 * kAxisBits));
 	const int x0 = cx > 0 ? cx - 1 : 0, x1 = cx + 1 < kCellsPerAxis ? cx + 1 : cx;
+	const int w = x0 >> 5, sh = x0 & 31;
+	const bool cross = (x1 >> 5) != w;  // into the next word
+	const uint32_t window = (2u << (x1 - x0)) - 1;
 	int n = 0;
 #pragma unroll
 	for (int q = 0; q < 9; q++) {
 		const int y = cy + q % 3 - 1, z = cz + q / 3 - 1;
-		if (y >= 0 && y < kCellsPerAxis && z >= 0 && z < kCellsPerAxis) {
-			const int row = z << kAxisBits | y;
-			const uint4 b = rows[row];
-			// the occupied ones among x0 .. x1
-			const int w = x0 >> 5;
-			const uint32_t lo = w == 0 ? b.x : w == 1 ? b.y : w == 2 ? b.z : b.w;
-			const uint32_t up = w == 0 ? b.y : w == 1 ? b.z : w == 2 ? b.w : 0u;
-			const uint32_t bits = __funnelshift_r(lo, up, x0 & 31) & ((2u << (x1 - x0)) - 1);
+		if ((unsigned)y < (unsigned)kCellsPerAxis && (unsigned)z < (unsigned)kCellsPerAxis) {
+			const uint2* at = words + (z << kAxisBits | y) * kRowWords + w;
+			const uint2 v = *at;
+			const uint32_t up = cross ? at[1].x : 0u;
+			const uint32_t bits = __funnelshift_r(v.x, up, sh) & window;
 			if (bits) {
-				const uint32_t first = co + base[row] + (uint32_t)row_rank(b, x0);
-				runs[n * stride] = make_uint2(start[first], start[first + __popc(bits)]);
+				const uint32_t first = co + v.y + (uint32_t)__popc(v.x & ((1u << sh) - 1));
+				runs[n * stride] = make_uint2(first, first + __popc(bits));
 				n++;
 			}
 		}
+	}
+	for (int q = 0; q < n; q++) {
+		const uint2 r = runs[q * stride];
+		runs[q * stride] = make_uint2(start[r.x], start[r.y]);
 	}
 	return n;
 }
@@ -228,7 +247,7 @@ __device__ __forceinline__ int find_runs(uint32_t c, uint32_t co, const uint4* _
 // A thread's way through its runs, one record after the other and the next one
 // loaded ahead. (A loop per run costs a warp the longest of its lanes' runs
 // nine times over: 14 of 32 lanes were at work, so it is 20, and the search of
-// 162M candidates' lists fell from 17.4 ms to 13.3.)
+// 162M candidates' lists fell from 17.4 ms to 13.3; 11.9 with all since.)
 struct RunWalk {
 	uint2* runs;
 	const float4* rec;
@@ -323,7 +342,7 @@ __global__ void __launch_bounds__(kListThreads, kListBlocks) conf_lists_kernel(c
 		const int32_t node = lb.node_of[i];  // a node's records keep its range
 		const LevelNode& nd = nodes[node];
 		const int64_t co = nd.cand_off;
-		const int nr = find_runs(lc.cell[i], (uint32_t)co, lc.rows + (int64_t)node * kRows, lc.base + (int64_t)node * kRows, lc.start,
+		const int nr = find_runs(lc.cell[i], (uint32_t)co, lc.words + (int64_t)node * kRows * kRowWords, lc.start,
 		                         &runs[0][threadIdx.x], kListThreads);
 		PairTest<MODE> test(nd, lc.rec[i]);
 		const int32_t t = test.t;
@@ -391,7 +410,7 @@ __global__ void __launch_bounds__(128) conf_long_kernel(const LevelNode* __restr
 	const int32_t node = lb.node_of[i];
 	if (dense[node]) return;
 	const LevelNode& nd = nodes[node];
-	const int nr = find_runs(lc.cell[i], (uint32_t)nd.cand_off, lc.rows + (int64_t)node * kRows, lc.base + (int64_t)node * kRows, lc.start,
+	const int nr = find_runs(lc.cell[i], (uint32_t)nd.cand_off, lc.words + (int64_t)node * kRows * kRowWords, lc.start,
 	                         &runs[0][threadIdx.x], 128);
 	PairTest<MODE> test(nd, lc.rec[i]);
 	int32_t* out = cl.long_pool + l.off;
@@ -463,7 +482,7 @@ __global__ void __launch_bounds__(kCompact) accepted_records_kernel(const LevelN
 // point sums over the records around it (no two accepted points lie within
 // the spacing); colours lie in cell order, beside the records. Bound by the
 // records and colours read; scattered atomics from the rejected side through
-// a hash of the accepted points took 4.04 ms for 31M candidates, this 2.07.
+// a hash of the accepted points took 4.04 ms for 31M candidates, this 1.88.
 __global__ void __launch_bounds__(128) cell_colors_kernel(const LevelNode* __restrict__ nodes, PosParamsS pp, LevelBuffers lb, LevelCells lc,
                                                           const uint32_t* __restrict__ list, const unsigned int* __restrict__ num) {
 	__shared__ uint2 runs[9][128];
@@ -472,7 +491,7 @@ __global__ void __launch_bounds__(128) cell_colors_kernel(const LevelNode* __res
 		const int32_t node = lb.node_of[i];
 		const LevelNode& nd = nodes[node];
 		const int64_t co = nd.cand_off;
-		const int nr = find_runs(lc.cell[i], (uint32_t)co, lc.rows + (int64_t)node * kRows, lc.base + (int64_t)node * kRows, lc.start,
+		const int nr = find_runs(lc.cell[i], (uint32_t)co, lc.words + (int64_t)node * kRows * kRowWords, lc.start,
 		                         &runs[0][threadIdx.x], 128);
 		PairTest<1> test(nd, lc.rec[i]);
 		unsigned long long r = 0, g = 0, b = 0, w = 0;
@@ -512,8 +531,8 @@ void build_level_cells(const LevelNode* d_nodes, const PosParamsS& pp, LevelBuff
 	cudaStream_t s = mem.stream();
 	const unsigned blocks = (unsigned)ceil_div(M, 256);
 	const int64_t rows = (int64_t)lb.K * kRows;
-	lc.rows = mem.alloc<uint4>(rows);
-	lc.base = mem.alloc<uint32_t>(rows);
+	lc.words = mem.alloc<uint2>(rows * kRowWords);
+	uint4* bits = mem.alloc<uint4>(rows);
 	lc.start = mem.alloc<uint32_t>(M + 1);
 	lc.rec = mem.alloc<float4>(M);
 	lc.cell = mem.alloc<uint32_t>(M);
@@ -521,13 +540,14 @@ void build_level_cells(const LevelNode* d_nodes, const PosParamsS& pp, LevelBuff
 	uint32_t* cell = mem.alloc<uint32_t>(M);
 	uint32_t* count = mem.alloc<uint32_t>(M);
 	uint2* place = mem.alloc<uint2>(M);
-	PCG_CUDA(cudaMemsetAsync(lc.rows, 0, rows * sizeof(uint4), s));
+	PCG_CUDA(cudaMemsetAsync(bits, 0, rows * sizeof(uint4), s));
 	PCG_CUDA(cudaMemsetAsync(count, 0, M * sizeof(uint32_t), s));
-	cell_mark_kernel<<<blocks, 256, 0, s>>>(d_nodes, pp, lb, cell, reinterpret_cast<uint32_t*>(lc.rows));
+	cell_mark_kernel<<<blocks, 256, 0, s>>>(d_nodes, pp, lb, cell, reinterpret_cast<uint32_t*>(bits));
 	PCG_LAUNCHED();
-	row_base_kernel<<<(unsigned)lb.K, kRowThreads, 0, s>>>(lc.rows, lc.base);
+	row_words_kernel<<<(unsigned)lb.K * kRowBlocks, kRowThreads, 0, s>>>(bits, reinterpret_cast<uint4*>(lc.words));
 	PCG_LAUNCHED();
-	cell_count_kernel<<<blocks, 256, 0, s>>>(d_nodes, lb, cell, lc.rows, lc.base, count, place);
+	mem.free(bits);
+	cell_count_kernel<<<blocks, 256, 0, s>>>(d_nodes, lb, cell, lc.words, count, place);
 	PCG_LAUNCHED();
 	exclusive_scan_u32(count, lc.start, M, true, mem);
 	cell_scatter_kernel<<<blocks, 256, 0, s>>>(d_nodes, pp, lb, cell, place, lc);
@@ -538,8 +558,7 @@ void build_level_cells(const LevelNode* d_nodes, const PosParamsS& pp, LevelBuff
 }
 
 void free_level_cells(LevelCells& lc, DeviceMem& mem) {
-	if (lc.rows) mem.free(lc.rows);
-	if (lc.base) mem.free(lc.base);
+	if (lc.words) mem.free(lc.words);
 	if (lc.start) mem.free(lc.start);
 	if (lc.rec) mem.free(lc.rec);
 	if (lc.cell) mem.free(lc.cell);

@@ -32,6 +32,27 @@ __device__ __forceinline__ uint32_t digit_peers(int digit) {
 	return p;
 }
 
+// clusters of blocks: this block's place, how many there are, the barrier
+__device__ __forceinline__ uint32_t cluster_rank() {
+	uint32_t r;
+	asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+	return r;
+}
+__device__ __forceinline__ uint32_t cluster_blocks() {
+	uint32_t r;
+	asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+	return r;
+}
+// the same shared-memory address in block r of the cluster
+__device__ __forceinline__ uint32_t in_block(uint32_t address, uint32_t r) {
+	uint32_t a;
+	asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(address), "r"(r));
+	return a;
+}
+__device__ __forceinline__ void cluster_barrier() {
+	asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
 constexpr int kWarpsPerBlock = 4;            // warp-per-node kernels: warps per CTA
 constexpr int kBigThreads = 512;             // CTA-per-node kernels
 constexpr int kBigWarps = kBigThreads / 32;

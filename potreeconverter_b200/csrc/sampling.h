@@ -137,8 +137,7 @@ void launch_node_pos(const LevelNode* nodes, const std::vector<uint8_t>& pick, L
 // The candidates of a level sorted by cell (conflicts.cu): cells of one
 // spacing, a node's records in its own range [cand_off, cand_off + count).
 struct LevelCells {
-	uint4* rows = nullptr;      // [K x 128 x 128] occupied cells of the row (z, y), a bit per x
-	uint32_t* base = nullptr;   // [K x 128 x 128] the node's occupied cells before the row
+	uint2* words = nullptr;     // [K x 128 x 128 x 4] occupied cells of the row (z, y), a bit per x, and the node's before the word
 	uint32_t* start = nullptr;  // [M + 1] first record of occupied cell r of a node, at cand_off + r
 	float4* rec = nullptr;      // [M] position relative to the node's minimum corner, sorted position
 	uint32_t* cell = nullptr;   // [M] the record's cell, z << 14 | y << 7 | x
