@@ -443,14 +443,13 @@ def main():
     rec_len = int.from_bytes(header[105:107], "little")
     bpp = 39
     out_pts = s["output_points"]
-    # roofline: the largest kernel family of a step (ncu launch list, 25 %)
-    # is the acceptance from conflict lists (greedy_list_cluster_kernel for
-    # the largest nodes, greedy_list_kernel, greedy_list_warp_kernel),
-    # launched once per octree level. Algorithmic bytes: per candidate its
-    # record (16 B), list length (1 B) and its decision, rank and flag
-    # (9 B); per list entry the entry (4 B) and that candidate's decision
-    # (4 B). Duration: the acceptance device time of the step (ms_greedy
-    # minus the list builds), all levels.
+    # roofline: the acceptance from conflict lists (accept_kernel, one launch
+    # per set of nodes of an octree level), with the list search the largest
+    # share of a step. Algorithmic bytes: per candidate its inline entries
+    # (16 B), list length (1 B) and its decision, rank and flag (9 B); per
+    # list entry the entry (4 B) and that candidate's decision (4 B).
+    # Duration: the acceptance device time of the step (ms_greedy minus the
+    # list builds), all levels.
     accept_ms = s["ms_greedy"] - s["ms_lists"]
     accept_bytes = s["candidates"] * 26 + s["list_entries"] * 8
     peak, peak_kind = peak_hbm()
@@ -518,7 +517,7 @@ def main():
             "e2e": {"value": e2e, "unit": "Mpts/s", "h2d_bytes_per_step": int(pinned.numel()),
                     "d2h_bytes_per_step": int(octree_bytes)},
             "gpu_launches": int(s["gpu_launches"]) * args.steps,
-            "roofline": {"bound": "hbm", "kernel": "greedy_list_cluster_kernel + greedy_list_kernel + greedy_list_warp_kernel (list acceptance, all levels of a step)",
+            "roofline": {"bound": "hbm", "kernel": "accept_kernel (list acceptance, all levels of a step)",
                          "achieved": achieved, "peak": peak, "peak_kind": peak_kind, "unit": "GB/s", "frac": achieved / peak,
                          "traffic": traffic, "traffic_source": "DRAM bytes per candidate from ncu, profiles/accept_hotspots-5M_poisson.md",
                          "algorithmic_bytes": accept_bytes, "kernel_ms": accept_ms,

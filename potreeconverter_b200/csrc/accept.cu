@@ -471,8 +471,7 @@ __device__ __forceinline__ void decide(const S_& S, int64_t co, int32_t none, in
 
 // One block per node, or one cluster of blocks.
 template <int MODE, int THREADS, bool CLUSTER>
-__global__ void __launch_bounds__(THREADS) accept_kernel(const LevelNode* __restrict__ nodes, const int32_t* __restrict__ set, int32_t batch, int64_t wide_min,
-                                                         ConflictLists cl, uint32_t* accepted_bits, uint32_t* prefixes, SampleStats* st) {
+__global__ void __launch_bounds__(THREADS) accept_kernel(const LevelNode* __restrict__ nodes, const int32_t* __restrict__ set, int32_t batch, ConflictLists cl, uint32_t* accepted_bits, uint32_t* prefixes, SampleStats* st) {
 	extern __shared__ __align__(16) uint8_t accept_smem[];
 	__shared__ uint32_t stop;
 	__shared__ unsigned long long frontier;
@@ -498,7 +497,7 @@ __global__ void __launch_bounds__(THREADS) accept_kernel(const LevelNode* __rest
 	if (threadIdx.x == 0) {
 		stop = 0;
 		frontier = 0;
-		if (n >= wide_min && S.block == 0) atomicAdd(&st->cluster_nodes, 1ull);
+		if (CLUSTER && S.block == 0) atomicAdd(&st->cluster_nodes, 1ull);
 	}
 	for (int32_t b0 = 0; b0 < n; b0 += batch) {
 		const int32_t nb = n - b0 < batch ? n - b0 : batch;
@@ -621,7 +620,7 @@ void launch_accept(int mode, const LevelNode* d_nodes, const std::vector<LevelNo
 		cfg.stream = cs;
 		cfg.attrs = &attr;
 		cfg.numAttrs = cluster > 1 ? 1 : 0;
-		PCG_CUDA(cudaLaunchKernelEx(&cfg, kernel, d_nodes, (const int32_t*)(d_order + first), batch, sch.cluster_min, cl, accepted_bits, prefixes, st));
+		PCG_CUDA(cudaLaunchKernelEx(&cfg, kernel, d_nodes, (const int32_t*)(d_order + first), batch, cl, accepted_bits, prefixes, st));
 		PCG_LAUNCHED();
 	};
 	auto set_of = [&](size_t first, size_t count, int threads, unsigned cluster) {
