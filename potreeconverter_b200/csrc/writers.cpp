@@ -16,6 +16,7 @@
 #include <cstring>
 #include <limits>
 #include <sstream>
+#include <type_traits>
 #include <utility>
 
 namespace pcg {
@@ -29,18 +30,50 @@ enum NodeType : uint8_t { T_NORMAL = 0, T_LEAF = 1, T_PROXY = 2 };
 
 // A node's name as a number: a 1, then three bits per digit after the "r". The
 // parent is code >> 3, and the order by length, then text, is the order of
-// the codes. 64 bits hold 21 levels, 128 bits 42: a cube of 2^32 units has 33
-// and one round of five more.
+// the codes. 64 bits hold 21 levels, 128 bits 42. A cube of 2^32 units of the
+// smallest scale has at most 33 and one round of five more, but every axis has
+// a scale of its own: a header box that is long in one axis only has as many
+// levels as its doubles resolve. Names past 42 levels stay text.
+class TextCode {
+public:
+	TextCode() = default;
+	explicit TextCode(uint64_t code) {
+		for (int b = 63 - __builtin_clzll(code) - 3; b >= 0; b -= 3) digits_ += (char)('0' + (code >> b & 7));
+	}
+	TextCode(const char* name, size_t len) : digits_(name + 1, len - 1) {}
+	friend TextCode operator>>(const TextCode& c, int bits) {  // the root has no parent
+		TextCode up;
+		if ((size_t)bits / 3 > c.digits_.size()) up.none_ = true;
+		else up.digits_ = c.digits_.substr(0, c.digits_.size() - (size_t)bits / 3);
+		return up;
+	}
+	friend int operator&(const TextCode& c, int) { return c.digits_.empty() ? 1 : c.digits_.back() - '0'; }
+	friend bool operator==(const TextCode& a, const TextCode& b) { return a.none_ == b.none_ && a.digits_ == b.digits_; }
+	friend bool operator!=(const TextCode& a, const TextCode& b) { return !(a == b); }
+	friend bool operator<(const TextCode& a, const TextCode& b) {
+		if (a.none_ != b.none_) return a.none_;
+		return a.digits_.size() != b.digits_.size() ? a.digits_.size() < b.digits_.size() : a.digits_ < b.digits_;
+	}
+
+private:
+	std::string digits_;
+	bool none_ = false;  // above the root
+};
+
 template <class Code>
 Code code_of(const char* name, size_t len) {
-	Code c = 1;
-	for (size_t i = 1; i < len; i++) c = c << 3 | (Code)(name[i] - '0');
-	return c;
+	if constexpr (std::is_same_v<Code, TextCode>) {
+		return TextCode(name, len);
+	} else {
+		Code c = 1;
+		for (size_t i = 1; i < len; i++) c = c << 3 | (Code)(name[i] - '0');
+		return c;
+	}
 }
 
 template <class Code>
 struct BNode {
-	Code code = 0;
+	Code code{};
 	int32_t num_points = 0;
 	uint32_t order = 0;  // in the file
 	uint8_t child_mask = 0;
@@ -51,14 +84,14 @@ struct BNode {
 
 template <class Code>
 struct BChunk {
-	Code code = 0;
+	Code code{};
 	size_t first = 0, count = 0;  // its entries
 };
 
 // The chunks of a batch in order, and their nodes in order.
 template <class Code>
 struct Batch {
-	Code code = 0;
+	Code code{};
 	std::vector<BNode<Code>> nodes;                  // by code
 	std::vector<BChunk<Code>> chunks;                // by code
 	std::vector<std::pair<Code, uint32_t>> entries;  // (chunk, node), chunk by chunk
@@ -202,7 +235,8 @@ bool build_hierarchy(const std::vector<HierRecord>& completed, std::vector<uint8
 	size_t longest = 0;
 	for (const auto& r : completed) longest = std::max(longest, r.name.size());
 	if (longest <= 22) return build<uint64_t>(completed, out, first_chunk_size, err);
-	return build<unsigned __int128>(completed, out, first_chunk_size, err);
+	if (longest <= 43) return build<unsigned __int128>(completed, out, first_chunk_size, err);
+	return build<TextCode>(completed, out, first_chunk_size, err);
 }
 
 std::string build_metadata(const std::string& name, const std::string& projection, int64_t points_total,
