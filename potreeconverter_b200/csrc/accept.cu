@@ -96,16 +96,25 @@ struct State {
 	uint32_t* stop;                // a wait gave up: everybody leaves
 	uint32_t block, blocks;  // this one's place in the cluster, and how many
 
+	// What warps wait for is read and written by relaxed operations of the
+	// scope of all who take part, the block or the cluster (weak ones would race,
+	// and need not see what another warp writes). Nothing else follows from a
+	// decision or a word, so they order nothing; the frontier releases and
+	// acquires the prefixes below it.
 	// position u of the batch
 	__device__ __forceinline__ uint32_t ld(int32_t u) const {
 		uint32_t v;
-		asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(base + (uint32_t)(u - first)) : "memory");
+		const uint32_t a = base + (uint32_t)(u - first);
+		if (CLUSTER) asm volatile("ld.relaxed.cluster.shared::cta.u8 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+		else asm volatile("ld.relaxed.cta.shared::cta.u8 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
 		return v;
 	}
 	// word w of the batch
 	__device__ __forceinline__ unsigned long long word(int32_t w) const {
 		unsigned long long v;
-		asm volatile("ld.volatile.shared.u64 %0, [%1];" : "=l"(v) : "r"(words + (uint32_t)w * 8u) : "memory");
+		const uint32_t a = words + (uint32_t)w * 8u;
+		if (CLUSTER) asm volatile("ld.relaxed.cluster.shared::cta.u64 %0, [%1];" : "=l"(v) : "r"(a) : "memory");
+		else asm volatile("ld.relaxed.cta.shared::cta.u64 %0, [%1];" : "=l"(v) : "r"(a) : "memory");
 		return v;
 	}
 	// any position before those now taken
@@ -114,26 +123,40 @@ struct State {
 	}
 	__device__ __forceinline__ void st(int32_t u, uint32_t v) const {
 		const uint32_t a = base + (uint32_t)(u - first);
-		asm volatile("st.shared.u8 [%0], %1;" ::"r"(a), "r"(v) : "memory");
-		if (CLUSTER)
-			for (uint32_t r = 0; r < blocks; r++)
-				if (r != block) asm volatile("st.shared::cluster.u8 [%0], %1;" ::"r"(in_block(a, r)), "r"(v) : "memory");
+		if (!CLUSTER) {
+			asm volatile("st.relaxed.cta.shared::cta.u8 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+			return;
+		}
+		asm volatile("st.relaxed.cluster.shared::cta.u8 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+		for (uint32_t r = 0; r < blocks; r++)
+			if (r != block) asm volatile("st.relaxed.cluster.shared::cluster.u8 [%0], %1;" ::"r"(in_block(a, r)), "r"(v) : "memory");
 	}
 	__device__ __forceinline__ void give_up(SampleStats* st) const {
 		const uint32_t a = (uint32_t)__cvta_generic_to_shared(stop);
 		if (CLUSTER)
-			for (uint32_t r = 0; r < blocks; r++) asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(in_block(a, r)), "r"(1u) : "memory");
-		else *(volatile uint32_t*)stop = 1;
+			for (uint32_t r = 0; r < blocks; r++) asm volatile("st.relaxed.cluster.shared::cluster.u32 [%0], %1;" ::"r"(in_block(a, r)), "r"(1u) : "memory");
+		else asm volatile("st.relaxed.cta.shared::cta.u32 [%0], %1;" ::"r"(a), "r"(1u) : "memory");
 		atomicAdd(&st->timeouts, 1ull);
 	}
-	__device__ __forceinline__ bool stopped() const { return *(volatile uint32_t*)stop != 0; }
-	__device__ __forceinline__ unsigned long long at_frontier() const { return *(volatile unsigned long long*)frontier; }
+	__device__ __forceinline__ bool stopped() const {
+		uint32_t v;
+		const uint32_t a = (uint32_t)__cvta_generic_to_shared(stop);
+		if (CLUSTER) asm volatile("ld.relaxed.cluster.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+		else asm volatile("ld.relaxed.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+		return v != 0;
+	}
+	// (each block keeps its own, so the block is its scope)
+	__device__ __forceinline__ unsigned long long at_frontier() const {
+		unsigned long long v;
+		asm volatile("ld.acquire.cta.shared::cta.u64 %0, [%1];" : "=l"(v) : "r"((uint32_t)__cvta_generic_to_shared(frontier)) : "memory");
+		return v;
+	}
 	// accepted points before position u of a word below the frontier
 	__device__ __forceinline__ int32_t rank(int32_t u) const {
 		const uint32_t below = (1u << (u & 31)) - 1;
 		if (u < first) return (int32_t)(__ldcg(old_prefix + (u >> 5)) + (uint32_t)__popc(__ldcg(old_bits + (u >> 5)) & below));
 		const int32_t w = (u - first) >> 5;
-		return (int32_t)(*(volatile uint32_t*)(prefix + w) + (uint32_t)__popc((uint32_t)word(w) & below));
+		return (int32_t)(prefix[w] + (uint32_t)__popc((uint32_t)word(w) & below));
 	}
 	// Whether at most `most` points were accepted before t: 0 no, 1 yes, 2 not
 	// known yet. own, open: t's word's accepted and undecided lanes before t.
@@ -149,10 +172,13 @@ struct State {
 	__device__ __forceinline__ void complete(int32_t g, uint32_t accepted) const {
 		const uint32_t a = words + (uint32_t)(g - first / 32) * 8u;
 		const unsigned long long v = kComplete | accepted;
-		asm volatile("st.volatile.shared.u64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
-		if (CLUSTER)
-			for (uint32_t r = 0; r < blocks; r++)
-				if (r != block) asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(in_block(a, r)), "l"(v) : "memory");
+		if (!CLUSTER) {
+			asm volatile("st.relaxed.cta.shared::cta.u64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
+			return;
+		}
+		asm volatile("st.relaxed.cluster.shared::cta.u64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
+		for (uint32_t r = 0; r < blocks; r++)
+			if (r != block) asm volatile("st.relaxed.cluster.shared::cluster.u64 [%0], %1;" ::"r"(in_block(a, r)), "l"(v) : "memory");
 	}
 	// The frontier's warp: accepted points before the batch's words as they are
 	// completed from its start on. False: a wait gave up.
@@ -179,12 +205,14 @@ struct State {
 				const uint32_t y = __shfl_up_sync(FULL, x, o);
 				if (lane >= o) x += y;
 			}
-			if (lane < now) *(volatile uint32_t*)(prefix + i) = count + x - c;
+			if (lane < now) prefix[i] = count + x - c;
 			count += __shfl_sync(FULL, x, 31);
 			at += now;
-			__threadfence_block();
 			__syncwarp();
-			if (lane == 0) *(volatile unsigned long long*)frontier = (unsigned long long)count << 32 | (uint32_t)(first / 32 + at);
+			if (lane == 0)
+				asm volatile("st.release.cta.shared::cta.u64 [%0], %1;" ::"r"((uint32_t)__cvta_generic_to_shared(frontier)),
+				             "l"((unsigned long long)count << 32 | (uint32_t)(first / 32 + at))
+				             : "memory");
 		}
 		return true;
 	}
