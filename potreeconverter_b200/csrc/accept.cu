@@ -636,7 +636,7 @@ void launch_accept(int mode, const LevelNode* d_nodes, const std::vector<LevelNo
 		const int64_t n = ln[order[first]].count;  // the set's largest
 		const int32_t batch = (int32_t)std::min<int64_t>((n + 127) & ~int64_t(127), kBatchMost);
 		const size_t smem = (size_t)batch_layout(batch).end;
-		if (smem > 48 * 1024) PCG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+		if (smem > 48 * 1024) allow_shared_memory(kernel, (size_t)batch_layout((int32_t)kBatchMost).end);
 		cudaLaunchAttribute attr{};
 		attr.id = cudaLaunchAttributeClusterDimension;
 		attr.val.clusterDim.x = cluster;

@@ -524,8 +524,7 @@ void launch_decode_count(const DecodeParams& p, uint32_t* grid, ChunkingOut& out
 		decode_count_kernel<true, false><<<(unsigned)blocks, kDecodeThreads, 0, mem.stream()>>>(p, grid, out);
 	} else if (staged) {
 		const size_t smem = 2 * (size_t)kDecodeTile * p.src0.rec_len;
-		if (smem > 48 * 1024)
-			PCG_CUDA(cudaFuncSetAttribute(decode_count_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+		if (smem > 48 * 1024) allow_shared_memory(decode_count_kernel<false, true>, 2 * (size_t)kDecodeTile * kDecodeStageMaxRec);
 		int64_t tb = ceil_div(p.n, kDecodeTile);
 		if (tb > cap) tb = cap;
 		decode_count_kernel<false, true><<<(unsigned)tb, kDecodeThreads, smem, mem.stream()>>>(p, grid, out);

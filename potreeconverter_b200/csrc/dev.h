@@ -35,6 +35,15 @@ struct PcgError : std::runtime_error {
 			throw ::pcg::CudaError(e_, std::string(#call) + ": " + cudaGetErrorString(e_)); \
 	} while (0)
 
+// Lets `kernel` be launched with up to `most` bytes of dynamic shared memory.
+// The limit belongs to the function in its context, not to the calling thread,
+// so `most` is the same at every call for a kernel: with a limit of each
+// launch's own size a thread could lower it between another's call and launch.
+template <class Kernel>
+void allow_shared_memory(Kernel* kernel, size_t most) {
+	PCG_CUDA(cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+}
+
 // Launch bookkeeping: every kernel launch goes through PCG_LAUNCH so the
 // number of launches per job is reported and launch errors surface at once.
 extern thread_local int64_t g_launch_count;

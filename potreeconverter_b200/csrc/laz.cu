@@ -75,7 +75,7 @@ void launch_laz_decode(const uint8_t* d_bytes, uint64_t base, const std::vector<
 	size_t smem_bytes = std::min<size_t>((size_t)per_block, (size_t)per_sm / blocks_per_sm - 1024) & ~size_t(15);
 	smem_bytes = std::max(smem_bytes, least);
 	const uint32_t fast_words = (uint32_t)((smem_bytes - state_bytes) / 4);
-	if (smem_bytes > 48 * 1024) PCG_CUDA(cudaFuncSetAttribute(laz_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes));
+	if (smem_bytes > 48 * 1024) allow_shared_memory(laz_decode_kernel, (size_t)per_block);
 	for (int c0 = 0; c0 < (int)chunks.size(); c0 += wave) {
 		const int n = std::min<int>(wave, (int)chunks.size() - c0);
 		laz_decode_kernel<<<(unsigned)n, 64, smem_bytes, mem.stream()>>>(d_bytes, bytes_end, base, d_chunks, c0, n, L, fast_words, arena, words,

@@ -240,7 +240,7 @@ void launch_octree_round(uint32_t* ids, const int32_t* X, const int32_t* Y, cons
 	octree_scatter_kernel<<<blocks, 256, 0, s>>>(ids, vals, d_segs, num_segs, total);
 	PCG_LAUNCHED();
 	size_t smem = (size_t)(kCells + kPyr) * sizeof(uint32_t);
-	PCG_CUDA(cudaFuncSetAttribute(octree_nodes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+	allow_shared_memory(octree_nodes_kernel, smem);
 	octree_nodes_kernel<<<num_segs, kNodesThreads, smem, s>>>(keys, d_segs, cands, num_cands, cand_capacity);
 	PCG_LAUNCHED();
 	mem.free(keys);

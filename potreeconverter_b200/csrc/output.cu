@@ -69,6 +69,7 @@ __device__ __forceinline__ uint64_t record_rgb(const uint8_t* r, const DecodePar
 }
 
 constexpr int kOutThreads = 256;
+constexpr size_t kOutSharedMost = 200 * 1024;  // for the records and payloads of a block
 
 // words of shared scratch per thread for one LAS record (4-byte aligned
 // cover of rec_len bytes at any offset)
@@ -213,9 +214,9 @@ void launch_write_payloads(const DecodeParams& p, const std::vector<PayloadItem>
 	const int64_t total = items.back().out_offset + items.back().count;
 	if (total == 0) return;
 	size_t smem = (size_t)kOutThreads * (rec_words(p.max_rec_len) * 4 + p.bpp);
-	if (smem > 200 * 1024) throw PcgError(1, "point records too long for the payload writer (record + output > 800 bytes)");
+	if (smem > kOutSharedMost) throw PcgError(1, "point records too long for the payload writer (record + output > 800 bytes)");
 	auto kernel = p.nsrc > 1 ? write_payloads_kernel<true> : write_payloads_kernel<false>;
-	if (smem > 48 * 1024) PCG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+	if (smem > 48 * 1024) allow_shared_memory(kernel, kOutSharedMost);
 	// the payload holding the first point of every 256-point chunk
 	const int64_t chunks = ceil_div(total, kOutThreads);
 	std::vector<int32_t> chunk_item(chunks);

@@ -955,8 +955,8 @@ void launch_greedy(int mode, bool fp32_guard, const LevelNode* nodes, const int3
 		arena.ovf = grid->ovf;
 		arena.link = mem.alloc<int32_t>((size_t)lb.M);
 		arena.accq = mem.alloc<int4>((size_t)lb.M);
-		if (mode == 0) PCG_CUDA(cudaFuncSetAttribute(greedy_big_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-		else PCG_CUDA(cudaFuncSetAttribute(greedy_big_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+		if (mode == 0) allow_shared_memory(greedy_big_kernel<0>, smem);
+		else allow_shared_memory(greedy_big_kernel<1>, smem);
 		for (int b0 = node_begin; b0 < big_end; b0 += slots) {
 			const int cnt = big_end - b0 < slots ? big_end - b0 : slots;
 			if (mode == 0) greedy_big_kernel<0><<<cnt, kBigThreads, smem, s>>>(nodes, order, b0, pp, lb, ga, arena, st);
