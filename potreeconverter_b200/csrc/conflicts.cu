@@ -59,13 +59,18 @@
 // Lists of up to kListCap entries lie in the candidate's slot and a pool; a
 // longer one (points much denser than the spacing, as on a facade) is counted
 // here and written by a warp of its own once its room is known. Nodes whose
-// long lists would take more than kLongBudget entries in all keep the
+// lists find no room -- the pool holds 2^31 entries, the long lists
+// kLongBudget in all, and both no more than the device has left -- keep the
 // lookup kernels (greedy_big_kernel).
 
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
+#include <cstdio>
+#include <cstdlib>
 #include <numeric>
+#include <type_traits>
 
 #include "devutil.cuh"
 #include "sampling.h"
@@ -78,8 +83,6 @@ constexpr int kAxisBits = 7;
 constexpr int kCellsPerAxis = 1 << kAxisBits;  // node box = 128 spacings
 constexpr int64_t kRows = (int64_t)kCellsPerAxis * kCellsPerAxis;  // of a node
 constexpr int kRowWords = kCellsPerAxis / 32;
-// entries of all long lists of a level (1 GiB)
-constexpr int64_t kLongBudget = int64_t(1) << 28;
 // six blocks an SM: 40 registers, a few spills outside the loop (50M points:
 // a loop per run: four blocks 17.0 ms, five 15.1, six 14.6, seven 19.4)
 constexpr int kListThreads = 256, kListBlocks = 6;
@@ -369,6 +372,8 @@ __global__ void __launch_bounds__(kListThreads, kListBlocks) conf_lists_kernel(c
 			if ((int64_t)at < cl.long_cap) {
 				cl.longs[at] = LongList{(int64_t)off, (int32_t)i, n};
 				cl.ovf_off[slot] = (int32_t)at;
+			} else {
+				cl.node_dense[node] = 1;
 			}
 		}
 	}
@@ -387,6 +392,8 @@ __global__ void __launch_bounds__(kListThreads, kListBlocks) conf_lists_kernel(c
 		if (extra && (int64_t)(at + extra) <= cl.pool_cap) {
 			cl.ovf_off[slot] = (int32_t)at;
 			for (uint32_t e = 0; e < extra; e++) cl.pool[at + e] = list[kListInline + e];
+		} else if (extra) {
+			cl.node_dense[lb.node_of[i]] = 1;
 		}
 	}
 	const unsigned entries = __reduce_add_sync(FULL, (unsigned)n);
@@ -523,6 +530,24 @@ __global__ void add_list_stats_kernel(SampleStats* st, const SampleStats* lst) {
 	atomicAdd(&st->escalated, lst->escalated);
 }
 
+// Room for a level's lists, in entries and lists. PCG_LIST_LIMITS="pool,
+// longs,long_entries" lowers it (read at every level): a level whose lists
+// find no room is otherwise one of hundreds of millions of points, or of a
+// device that something else fills.
+struct ListLimits {
+	int64_t pool, longs, long_entries;
+};
+
+ListLimits list_limits() {
+	ListLimits l{INT32_MAX, INT32_MAX, kLongBudget};
+	if (const char* e = std::getenv("PCG_LIST_LIMITS")) {
+		long long a = 0, b = 0, c = 0;
+		if (std::sscanf(e, "%lld,%lld,%lld", &a, &b, &c) == 3 && a > 0 && b > 0 && c > 0)
+			l = ListLimits{std::min<int64_t>(a, l.pool), std::min<int64_t>(b, l.longs), std::min<int64_t>(c, l.long_entries)};
+	}
+	return l;
+}
+
 }  // namespace
 
 void build_level_cells(const LevelNode* d_nodes, const PosParamsS& pp, LevelBuffers& lb, LevelCells& lc, DeviceMem& mem) {
@@ -577,73 +602,95 @@ void build_conflict_lists(int mode, const LevelNode* d_nodes, int K, const PosPa
 	cl.inl = mem.alloc<int4>(M);
 	cl.ovf_off = mem.alloc<int32_t>(M);
 	cl.count = mem.alloc<uint8_t>(M);
+	const ListLimits limits = list_limits();
+	// As much room as the device can hold of what is wanted: every half that
+	// fails is halved again.
+	auto alloc_room = [&](auto*& p, int64_t& cap, int64_t want) {
+		for (cap = std::max<int64_t>(want, 1);; cap /= 2) {
+			try {
+				p = mem.alloc<std::remove_reference_t<decltype(*p)>>(cap);
+				return;
+			} catch (const PcgError& e) {
+				if (e.status != 3 || cap <= 4096) throw;  // 3: PCG_OOM
+			}
+		}
+	};
 	// room for 8 pooled entries per candidate (lists average about one entry)
 	// and one long list in 16; a level that needs more is searched again with
-	// the room it asked for
-	unsigned long long* used = mem.alloc<unsigned long long>(3 + (size_t)K);
+	// the room it asked for, or what there is of it: nodes with a list that
+	// finds none are marked
+	const size_t counters = 3 + (size_t)K, zeroed = counters * sizeof(unsigned long long) + K;
+	unsigned long long* used = mem.alloc<unsigned long long>(counters + ((size_t)K + 7) / 8);
 	cl.pool_used = used;
 	cl.long_used = used + 1;
 	cl.long_entries = used + 2;
 	cl.node_long = used + 3;
-	cl.pool_cap = std::min<int64_t>(M * 2 * kListInline, (int64_t)INT32_MAX);
-	cl.long_cap = std::min<int64_t>(M, M / 16 + 4096);
-	cl.pool = mem.alloc<int32_t>(cl.pool_cap);
-	cl.longs = mem.alloc<LongList>(cl.long_cap);
+	cl.node_dense = reinterpret_cast<uint8_t*>(used + counters);
+	alloc_room(cl.pool, cl.pool_cap, std::min(M * 2 * kListInline, limits.pool));
+	alloc_room(cl.longs, cl.long_cap, std::min({M, M / 16 + 4096, limits.longs}));
 	SampleStats* lst = mem.alloc<SampleStats>(1);
-	std::vector<unsigned long long> h(3 + (size_t)K);
-	for (int attempt = 0; attempt < 2; attempt++) {
-		PCG_CUDA(cudaMemsetAsync(used, 0, (3 + (size_t)K) * sizeof(unsigned long long), s));
+	std::vector<unsigned long long> h(counters);
+	for (int attempt = 0;; attempt++) {
+		PCG_CUDA(cudaMemsetAsync(used, 0, zeroed, s));
 		PCG_CUDA(cudaMemsetAsync(lst, 0, sizeof(SampleStats), s));
 		if (mode == 0) conf_lists_kernel<0><<<list_blocks, kListThreads, 0, s>>>(d_nodes, pp, lb, lc, cl, lst);
 		else conf_lists_kernel<1><<<list_blocks, kListThreads, 0, s>>>(d_nodes, pp, lb, lc, cl, lst);
 		PCG_LAUNCHED();
 		PCG_CUDA(cudaMemcpyAsync(h.data(), used, h.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
 		PCG_CUDA(cudaStreamSynchronize(s));
-		if ((int64_t)h[0] > (int64_t)INT32_MAX) throw PcgError(3, "conflict lists of a level exceed 2^31 entries");
-		const bool fits = (int64_t)h[0] <= cl.pool_cap && (int64_t)h[1] <= cl.long_cap;
-		if (fits) break;
-		if (attempt == 1) throw PcgError(5, "conflict lists changed between two searches");
-		if ((int64_t)h[0] > cl.pool_cap) {
+		const int64_t pool = std::min<int64_t>((int64_t)h[0], limits.pool), longs = std::min<int64_t>((int64_t)h[1], limits.longs);
+		if (attempt || (pool <= cl.pool_cap && longs <= cl.long_cap)) break;
+		if (pool > cl.pool_cap) {
 			mem.free(cl.pool);
-			cl.pool_cap = (int64_t)h[0];
-			cl.pool = mem.alloc<int32_t>(cl.pool_cap);
+			alloc_room(cl.pool, cl.pool_cap, pool);
 		}
-		if ((int64_t)h[1] > cl.long_cap) {
+		if (longs > cl.long_cap) {
 			mem.free(cl.longs);
-			cl.long_cap = (int64_t)h[1];
-			cl.longs = mem.alloc<LongList>(cl.long_cap);
+			alloc_room(cl.longs, cl.long_cap, longs);
 		}
 	}
 	add_list_stats_kernel<<<1, 1, 0, s>>>(st, lst);
 	PCG_LAUNCHED();
+	mem.free(lst);
+	if ((int64_t)h[0] > cl.pool_cap || (int64_t)h[1] > cl.long_cap) {
+		PCG_CUDA(cudaMemcpyAsync(dense.data(), cl.node_dense, K, cudaMemcpyDeviceToHost, s));
+		PCG_CUDA(cudaStreamSynchronize(s));
+	}
 	if (h[1]) {
 		// past the budget the nodes with the most entries go to the lookup kernels
-		int64_t kept = (int64_t)h[2];
-		if (kept > kLongBudget) {
-			std::vector<int> order(K);
-			std::iota(order.begin(), order.end(), 0);
-			std::sort(order.begin(), order.end(), [&](int a, int b) { return h[3 + a] > h[3 + b]; });
+		std::vector<int> order(K);
+		std::iota(order.begin(), order.end(), 0);
+		std::sort(order.begin(), order.end(), [&](int a, int b) { return h[3 + a] > h[3 + b]; });
+		int64_t kept = 0;
+		for (int k = 0; k < K; k++) kept += dense[k] ? 0 : (int64_t)h[3 + k];
+		for (int64_t budget = limits.long_entries;; budget = kept / 2) {
 			for (int k : order) {
-				if (kept <= kLongBudget) break;
+				if (kept <= budget) break;
+				if (dense[k]) continue;
 				dense[k] = 1;
 				kept -= (int64_t)h[3 + k];
+			}
+			try {
+				cl.long_pool = mem.alloc<int32_t>(std::max<int64_t>(kept, 1));
+				break;
+			} catch (const PcgError& e) {
+				if (e.status != 3 || kept <= 4096) throw;
 			}
 		}
 		uint8_t* d_dense = mem.alloc<uint8_t>(K);
 		PCG_CUDA(cudaMemcpyAsync(d_dense, dense.data(), K, cudaMemcpyHostToDevice, s));
-		if ((int64_t)h[2] > kLongBudget) {
+		const int64_t num = std::min<int64_t>((int64_t)h[1], cl.long_cap);
+		if (kept != (int64_t)h[2]) {
 			PCG_CUDA(cudaMemsetAsync(cl.long_entries, 0, sizeof(unsigned long long), s));
-			long_places_kernel<<<(unsigned)ceil_div((int64_t)h[1], 256), 256, 0, s>>>(lb, cl, d_dense, (int64_t)h[1], cl.long_entries);
+			long_places_kernel<<<(unsigned)ceil_div(num, 256), 256, 0, s>>>(lb, cl, d_dense, num, cl.long_entries);
 			PCG_LAUNCHED();
 		}
-		cl.long_pool = mem.alloc<int32_t>(std::max<int64_t>(kept, 1));
-		const unsigned lblocks = (unsigned)ceil_div((int64_t)h[1] * 32, 128);
-		if (mode == 0) conf_long_kernel<0><<<lblocks, 128, 0, s>>>(d_nodes, pp, lb, lc, cl, d_dense, (int64_t)h[1]);
-		else conf_long_kernel<1><<<lblocks, 128, 0, s>>>(d_nodes, pp, lb, lc, cl, d_dense, (int64_t)h[1]);
+		const unsigned lblocks = (unsigned)ceil_div(num * 32, 128);
+		if (mode == 0) conf_long_kernel<0><<<lblocks, 128, 0, s>>>(d_nodes, pp, lb, lc, cl, d_dense, num);
+		else conf_long_kernel<1><<<lblocks, 128, 0, s>>>(d_nodes, pp, lb, lc, cl, d_dense, num);
 		PCG_LAUNCHED();
 		mem.free(d_dense);
 	}
-	mem.free(lst);
 }
 
 void launch_cell_colors(const LevelNode* d_nodes, const std::vector<uint8_t>& dense, const PosParamsS& pp, LevelBuffers& lb,

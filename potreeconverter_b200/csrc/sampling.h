@@ -171,12 +171,15 @@ struct ConflictLists {
 	int64_t long_cap = 0;
 	int32_t* long_pool = nullptr;
 	uint8_t* count = nullptr;       // [M] by sorted position: entries (| kListDistant), or kListLong past kListCap
-	unsigned long long* pool_used = nullptr;  // entries of pool handed out (one allocation with the next three)
+	unsigned long long* pool_used = nullptr;  // entries of pool handed out (one allocation with the next four)
 	unsigned long long* long_used = nullptr;     // long lists
 	unsigned long long* long_entries = nullptr;  // their entries
 	unsigned long long* node_long = nullptr;     // [K] their entries by node
+	uint8_t* node_dense = nullptr;               // [K] 1: one of its lists found no room
 };
-// Nodes flagged in `dense` have no lists (conflicts.cu kLongBudget).
+// entries of all long lists of a level (1 GiB)
+constexpr int64_t kLongBudget = int64_t(1) << 28;
+// Nodes flagged in `dense` have no lists: there was no room for them.
 void build_conflict_lists(int mode, const LevelNode* d_nodes, int K, const PosParamsS& pp, LevelBuffers& lb, const LevelCells& lc,
                           ConflictLists& cl, std::vector<uint8_t>& dense, SampleStats* st, DeviceMem& mem);
 void free_conflict_lists(ConflictLists& cl, DeviceMem& mem);
