@@ -582,11 +582,16 @@ inline size_t device_available(int device) {
 
 // Device memory a job of `points` points and `record_bytes` bytes of point
 // records is expected to hold at its peak (the request loop's admission
-// figure): the records, a per-point working set and the count grid and LUT.
-// Checked against pcg_stats.device_peak_bytes by the request-loop tests.
+// figure): the records, a per-point working set (the 768 KiB of cells that
+// every sampled node has count with it: a level has no more of them than one
+// per 10,000 points and 20 above the chunks), the count grid and LUT, and the
+// long conflict lists of a level of points close to one another (an entry per
+// pair, as far as they are kept). Checked against pcg_stats.device_peak_bytes
+// by the request-loop tests.
 constexpr int64_t kJobBytesPerPoint = 400;
 inline size_t estimate_footprint(int64_t points, int64_t record_bytes) {
-	return (size_t)(record_bytes + points * kJobBytesPerPoint) + (size_t(256) << 20);
+	const int64_t long_lists = points < (int64_t(1) << 15) ? std::min(2 * points * points, kLongListBytes) : kLongListBytes;
+	return (size_t)(record_bytes + points * kJobBytesPerPoint + long_lists) + (size_t(256) << 20);
 }
 
 struct Converter {
@@ -1847,6 +1852,7 @@ struct Converter {
 					launch_cand_records(d_nodes, co.X, co.Y, co.Z, lb, mem);
 					launch_greedy(mode, true, d_nodes, lk.d_order, dense_nodes, co.X, co.Y, co.Z, pps, lb, lk.hkeys, lk.hvals, lk.axyz, lk.akey,
 					              lk.anext, lk.apos, d_st, mem, &grid_arena, 0, -1, big_nodes(dense_order));
+					greedy_arena_free(grid_arena, mem);  // before the next level's lists
 					lookup_end(d_dense);
 					mem.free(d_dense);
 				}

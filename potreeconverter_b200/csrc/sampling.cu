@@ -922,9 +922,14 @@ void launch_cand_records(const LevelNode* nodes, const int32_t* X, const int32_t
 	PCG_LAUNCHED();
 }
 
+void greedy_arena_free(GreedyArena& a, DeviceMem& mem) {
+	if (a.cells) { mem.free(a.cells); mem.free(a.ovf); }
+	a = GreedyArena{};
+}
+
 void greedy_arena_reserve(GreedyArena& a, int slots, DeviceMem& mem) {
 	if (slots <= a.slots) return;
-	if (a.cells) { mem.free(a.cells); mem.free(a.ovf); }
+	greedy_arena_free(a, mem);
 	a.cells = mem.alloc<AccCell>((size_t)slots * kGridCells);
 	a.ovf = mem.alloc<int32_t>((size_t)slots * kGridCells);
 	PCG_CUDA(cudaMemsetAsync(a.cells, 0, (size_t)slots * kGridCells * sizeof(AccCell), mem.stream()));
@@ -945,8 +950,9 @@ void launch_greedy(int mode, bool fp32_guard, const LevelNode* nodes, const int3
 	if (big_end > node_begin) {
 		size_t smem = sizeof(RoundShared);
 		// one dense acceptance grid per resident CTA (kept empty between
-		// nodes); large levels go in batches
-		const int batch = sm_count() * 2;
+		// nodes), 33 MiB each and all together within the room of the long lists,
+		// which the caller has freed; large levels go in batches
+		const int batch = (int)std::min<int64_t>(sm_count() * 2, kLongListBytes / (kGridCells * (int64_t)(sizeof(AccCell) + sizeof(int32_t))));
 		const int nbig = big_end - node_begin;
 		const int slots = nbig < batch ? nbig : batch;
 		greedy_arena_reserve(*grid, slots, mem);

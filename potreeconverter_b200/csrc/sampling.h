@@ -179,6 +179,7 @@ struct ConflictLists {
 };
 // entries of all long lists of a level (1 GiB)
 constexpr int64_t kLongBudget = int64_t(1) << 28;
+constexpr int64_t kLongListBytes = kLongBudget * (int64_t)sizeof(int32_t);
 // Nodes flagged in `dense` have no lists: there was no room for them.
 void build_conflict_lists(int mode, const LevelNode* d_nodes, int K, const PosParamsS& pp, LevelBuffers& lb, const LevelCells& lc,
                           ConflictLists& cl, std::vector<uint8_t>& dense, SampleStats* st, DeviceMem& mem);
@@ -204,6 +205,7 @@ struct GreedyArena {
 	int slots = 0;
 };
 void greedy_arena_reserve(GreedyArena& a, int slots, DeviceMem& mem);
+void greedy_arena_free(GreedyArena& a, DeviceMem& mem);
 // mode 0 = poisson (early exit + 10,001-check window), 1 = poisson_average (pure greedy)
 void launch_greedy(int mode, bool fp32_guard, const LevelNode* nodes, const int32_t* order, int K, const int32_t* X, const int32_t* Y,
                    const int32_t* Z, const PosParamsS& pp, LevelBuffers& lb, uint64_t* hash_keys, int32_t* hash_heads,
