@@ -1784,20 +1784,19 @@ struct Converter {
 			std::vector<int32_t> order(K);
 			for (int k = 0; k < K; k++) order[k] = k;
 			std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return ln[a].count > ln[b].count; });
-			const LevelSchedule sch = level_schedule();
-			const int64_t big_min = K < 2 * sms ? sch.small_level_cta_min : sch.cta_min;
+			const int64_t big_min = K < 2 * sms ? kLookupBlockMinFew : kLookupBlockMin;
 			auto big_nodes = [&](const std::vector<int32_t>& o) {
 				int n = 0;
 				while (n < (int)o.size() && ln[o[n]].count >= big_min) n++;
 				return n;
 			};
-			int dense_nodes = 0;
+			int dense_nodes = 0, lookup_blocks = 0;
 			cudaEvent_t ev[4];  // start, sorted, lists built, accepted
 			for (auto& e : ev) PCG_CUDA(cudaEventCreate(&e));
 			PCG_CUDA(cudaEventRecord(ev[0], s));
 			if (form == PCG_FORM_PLAIN) {
 				lookup_begin(order);
-				const int num_big = big_nodes(order);
+				const int num_big = lookup_blocks = big_nodes(order);
 				for (int k = 0; k < K; k++) launch_node_sort(d_nodes, lk.d_order, K, lb, d_st, mem, k, k + 1, num_big);
 				launch_cand_records(d_nodes, co.X, co.Y, co.Z, lb, mem);
 				PCG_CUDA(cudaEventRecord(ev[1], s));
@@ -1848,10 +1847,11 @@ struct Converter {
 				dense_nodes = (int)dense_order.size();
 				if (dense_nodes) {
 					lookup_begin(dense_order);
+					lookup_blocks = big_nodes(dense_order);
 					uint8_t* d_dense = upload(dense, mem);
 					launch_cand_records(d_nodes, co.X, co.Y, co.Z, lb, mem);
 					launch_greedy(mode, true, d_nodes, lk.d_order, dense_nodes, co.X, co.Y, co.Z, pps, lb, lk.hkeys, lk.hvals, lk.axyz, lk.akey,
-					              lk.anext, lk.apos, d_st, mem, &grid_arena, 0, -1, big_nodes(dense_order));
+					              lk.anext, lk.apos, d_st, mem, &grid_arena, 0, -1, lookup_blocks);
 					greedy_arena_free(grid_arena, mem);  // before the next level's lists
 					lookup_end(d_dense);
 					mem.free(d_dense);
@@ -1870,9 +1870,9 @@ struct Converter {
 				int64_t mx = 0;
 				for (auto& l : ln) mx = std::max<int64_t>(mx, l.count);
 				fprintf(stderr,
-				        "[pcg] level %d: nodes %d (dense %d), candidates %lld, largest %lld, sort %.3f ms, greedy %.3f ms (lists %.3f), "
+				        "[pcg] level %d: nodes %d (dense %d, lookup by blocks %d), candidates %lld, largest %lld, sort %.3f ms, greedy %.3f ms (lists %.3f), "
 				        "host %.3f ms (alloc %.3f)\n",
-				        K ? ln[0].level : -1, K, dense_nodes, (long long)M, (long long)mx, t_sort, t_greedy, t_lists, ms_since(t_level),
+				        K ? ln[0].level : -1, K, dense_nodes, lookup_blocks, (long long)M, (long long)mx, t_sort, t_greedy, t_lists, ms_since(t_level),
 				        mem.alloc_ms() - alloc0);
 			}
 			for (auto& e : ev) cudaEventDestroy(e);

@@ -96,6 +96,13 @@ struct LevelSchedule {
 	int middle;
 };
 LevelSchedule level_schedule();
+// From how many candidates the lookup kernels (launch_node_sort, launch_greedy:
+// the plain form, and nodes without conflict lists) give a node a block of
+// its own instead of a warp: on levels of at least two nodes per SM, and of
+// fewer, where a warp is what the level waits for. (16,384 and 4,096, as the
+// acceptance from lists has it: plain form 3.0 Mpts/s for 3.8 on 50M points,
+// 2.0 for 5.7 on 10M strips.)
+constexpr int64_t kLookupBlockMin = 8192, kLookupBlockMinFew = 1024;
 void launch_node_sort(const LevelNode* nodes, const int32_t* order, int K, LevelBuffers& lb, SampleStats* st, DeviceMem& mem,
                       int node_begin = 0, int node_end = -1, int num_big = 0);
 // Exact ascending sort of every node's keys (segmented LSD radix sort). Nodes whose keys are pairwise distinct end sorted in lb.keys,
