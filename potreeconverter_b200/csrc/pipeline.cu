@@ -28,12 +28,12 @@
 #include <map>
 #include <memory>
 #include <mutex>
-#include <system_error>
 #include <thread>
 #include <unordered_map>
 #include <unistd.h>
 
 #include "../../include/pcgpu.h"
+#include "host_copy.h"
 #include "kernels.h"
 #include "output.h"
 #include "sampling.h"
@@ -270,23 +270,6 @@ struct JobResult {
 	}
 };
 
-// A host copy by several threads, 8 MiB or more each: one thread moves 11 GB/s.
-void parallel_copy(uint8_t* dst, const uint8_t* src, size_t bytes) {
-	const int nt = (int)std::min<size_t>(8, std::max<size_t>(1, bytes >> 23));
-	if (nt == 1) {
-		std::memcpy(dst, src, bytes);
-		return;
-	}
-	std::vector<std::thread> th;
-	const size_t per = (bytes + nt - 1) / nt;
-	for (int k = 0; k < nt; k++) {
-		const size_t o = k * per;
-		if (o >= bytes) break;
-		th.emplace_back([=] { std::memcpy(dst + o, src + o, std::min(per, bytes - o)); });
-	}
-	for (auto& x : th) x.join();
-}
-
 bool page_locked(const void* p) {
 	cudaPointerAttributes a{};
 	const bool r = cudaPointerGetAttributes(&a, p) == cudaSuccess && a.type == cudaMemoryTypeHost;
@@ -316,7 +299,14 @@ void upload_records(const std::vector<HostRecords>& all, cudaStream_t s, int dev
 		locked.push_back(page_locked(r.src));
 		if (!locked.back()) pageable += r.bytes;
 	}
-	uint8_t* stage = pageable >= kStagedMin ? g_pinned.take(2 * kThreads * kPiece) : nullptr;
+	struct Stage {  // goes back to the pool however this ends
+		uint8_t* p;
+		~Stage() {
+			if (p) g_pinned.give(p);
+		}
+	};
+	const Stage held{pageable >= kStagedMin ? g_pinned.take(2 * kThreads * kPiece) : nullptr};
+	uint8_t* const stage = held.p;
 	for (size_t k = 0; k < all.size(); k++) {
 		const HostRecords& r = all[k];
 		if (!stage || locked[k]) {
@@ -349,16 +339,7 @@ void upload_records(const std::vector<HostRecords>& all, cudaStream_t s, int dev
 		}
 		failed[t] = e;
 	};
-	std::vector<std::thread> th;
-	try {
-		for (int t = 1; t < kThreads; t++) th.emplace_back(send, t);
-	} catch (const std::system_error&) {
-		// no thread to be had: its pieces are sent here
-	}
-	send(0);
-	for (int t = (int)th.size() + 1; t < kThreads; t++) send(t);
-	for (auto& x : th) x.join();
-	g_pinned.give(stage);
+	on_threads(kThreads, send);
 	for (cudaError_t e : failed) PCG_CUDA(e);
 }
 
