@@ -15,6 +15,8 @@
 //  * a symbol's count lies in the word of its distribution value, so the
 //    load of the search brings it and the lane of the symbol stores it back;
 //    lane 31 keeps the symbols until the model's next update the same way;
+//    (a lane's word is read by its neighbour too, so a warp barrier lies on
+//    either side of the stores: the two cost 2.4 % of the decode);
 //  * a model update is a warp scan over the counts;
 //  * coded bytes come from a ring in shared memory, refilled once per point.
 // The second warp turns the decoded symbols (32 points at a time, through a
@@ -278,12 +280,15 @@ struct Decoder {
 			length = (s == 30 ? q1 : (s == 31 ? q2 : top)) - x;
 			value -= x;
 			renorm();
+			__syncwarp();
 			if (s > 30 && lane == 0) b.st(W_SLOT + 4 * (s + 1), (s == 31 ? e31 : e32) + 0x10000u);
 		} else {
 			take(p0, p1, s);
 		}
+		__syncwarp();  // every lane has loaded
 		m.st_lane(lane, 31, W_SLOT, w0 - 1);
 		m.st_lane(lane, s < 31 ? s : 32, W_SLOT, w0 + 0x10000u);
+		__syncwarp();  // and the next symbol's loads see this
 		if (votes >> 31) model_update(Near{a}, n);
 		return s;
 	}
@@ -302,8 +307,10 @@ struct Decoder {
 		const uint32_t p0 = (w0 & 0xffff) * part, p1 = i + 1 < n ? (w1 & 0xffff) * part : length;
 		const uint32_t o = ((uint32_t)__popc(__ballot_sync(kAll, lane < size && i < n && p0 <= value)) - 1) & (size - 1);
 		take(p0, p1, o);
+		__syncwarp();
 		m.st_lane(lane, 31, W_UNTIL, start - 1);
 		m.st_lane(lane, o, W_ENTRY + 4 * i, w0 + 0x10000u);
+		__syncwarp();
 		if (votes >> 31) model_update(m, n);
 		return (g << sh) + o;
 	}
