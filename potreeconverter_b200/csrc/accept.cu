@@ -578,9 +578,9 @@ LevelSchedule level_schedule() {
 	return v;
 }
 
-void launch_accept(int mode, const LevelNode* d_nodes, const std::vector<LevelNode>& ln, const std::vector<uint8_t>& dense, LevelBuffers& lb,
+std::vector<AcceptSet> launch_accept(int mode, const LevelNode* d_nodes, const std::vector<LevelNode>& ln, const std::vector<uint8_t>& dense, LevelBuffers& lb,
                    const ConflictLists& cl, uint32_t* accepted_bits, SampleStats* st, DeviceMem& mem) {
-	if (lb.M == 0) return;
+	if (lb.M == 0) return {};
 	cudaStream_t s = mem.stream();
 	const int K = (int)ln.size();
 	const LevelSchedule sch = level_schedule();
@@ -597,12 +597,7 @@ void launch_accept(int mode, const LevelNode* d_nodes, const std::vector<LevelNo
 	// what the level waits for (50M points: 16.1 ms without clusters, 13.4 where
 	// they only go to the levels of few nodes, 9.6 so; twice as many blocks, or
 	// three quarters, within 2 %).
-	struct Set {
-		size_t first, count;
-		int threads;
-		unsigned cluster;
-	};
-	std::vector<Set> sets;
+	std::vector<AcceptSet> sets;
 	const int64_t sms = sm_count();
 	int64_t total = 0;
 	for (int32_t k : order) total += ln[k].count;
@@ -613,7 +608,7 @@ void launch_accept(int mode, const LevelNode* d_nodes, const std::vector<LevelNo
 		if (n >= kClusterMin)
 			while (c < kClusterMost && n * sms > total * c) c *= 2;
 		const int threads = c > 1 ? kClusterThreads : n >= sch.cluster_min ? 1024 : n >= full_min ? middle : 128;
-		if (sets.empty() || sets.back().threads != threads || sets.back().cluster != c) sets.push_back(Set{i, 0, threads, c});
+		if (sets.empty() || sets.back().threads != threads || sets.back().cluster != c) sets.push_back(AcceptSet{i, 0, threads, c});
 		sets.back().count++;
 	}
 	uint32_t* prefixes = mem.alloc<uint32_t>(mode == 0 ? (size_t)accept_words(lb.M, K) : 1);
@@ -662,7 +657,7 @@ void launch_accept(int mode, const LevelNode* d_nodes, const std::vector<LevelNo
 		else if (threads == 256) pick(accept_kernel<0, 256, false>, accept_kernel<1, 256, false>);
 		else pick(accept_kernel<0, 128, false>, accept_kernel<1, 128, false>);
 	};
-	for (const Set& g : sets) set_of(g.first, g.count, g.threads, g.cluster);
+	for (const AcceptSet& g : sets) set_of(g.first, g.count, g.threads, g.cluster);
 	for (int k = 0; k < nsides; k++) {
 		PCG_CUDA(cudaEventRecord(join[k], side[k]));
 		PCG_CUDA(cudaStreamWaitEvent(s, join[k], 0));
@@ -677,6 +672,7 @@ void launch_accept(int mode, const LevelNode* d_nodes, const std::vector<LevelNo
 	if (d_dense) mem.free(d_dense);
 	mem.free(d_order);
 	mem.free(prefixes);
+	return sets;
 }
 
 }  // namespace pcg

@@ -1772,6 +1772,7 @@ struct Converter {
 				return n;
 			};
 			int dense_nodes = 0, lookup_blocks = 0;
+			std::vector<AcceptSet> sets;
 			cudaEvent_t ev[4];  // start, sorted, lists built, accepted
 			for (auto& e : ev) PCG_CUDA(cudaEventCreate(&e));
 			PCG_CUDA(cudaEventRecord(ev[0], s));
@@ -1817,7 +1818,7 @@ struct Converter {
 				build_conflict_lists(mode, d_nodes, K, pps, lb, lc, cl, dense, d_st, mem);
 				PCG_CUDA(cudaEventRecord(ev[2], s));
 				uint32_t* accepted_bits = mem.alloc<uint32_t>((size_t)accept_words(M, K));
-				launch_accept(mode, d_nodes, ln, dense, lb, cl, accepted_bits, d_st, mem);
+				sets = launch_accept(mode, d_nodes, ln, dense, lb, cl, accepted_bits, d_st, mem);
 				free_conflict_lists(cl, mem);
 				if (mode == 1) launch_cell_colors(d_nodes, dense, pps, lb, lc, accepted_bits, mem);
 				mem.free(accepted_bits);
@@ -1850,11 +1851,15 @@ struct Converter {
 			if (trace_levels()) {
 				int64_t mx = 0;
 				for (auto& l : ln) mx = std::max<int64_t>(mx, l.count);
+				std::string with;
+				for (const AcceptSet& g : sets)
+					with += (with.empty() ? ", nodes by threads x blocks " : ", ") + std::to_string(g.count) + " by " + std::to_string(g.threads) +
+					        " x " + std::to_string(g.cluster);
 				fprintf(stderr,
 				        "[pcg] level %d: nodes %d (dense %d, lookup by blocks %d), candidates %lld, largest %lld, sort %.3f ms, greedy %.3f ms (lists %.3f), "
-				        "host %.3f ms (alloc %.3f)\n",
+				        "host %.3f ms (alloc %.3f)%s\n",
 				        K ? ln[0].level : -1, K, dense_nodes, lookup_blocks, (long long)M, (long long)mx, t_sort, t_greedy, t_lists, ms_since(t_level),
-				        mem.alloc_ms() - alloc0);
+				        mem.alloc_ms() - alloc0, with.c_str());
 			}
 			for (auto& e : ev) cudaEventDestroy(e);
 			mem.free(lb.keys); mem.free(lb.perm); mem.free(lb.pos);

@@ -66,7 +66,7 @@ struct SampleStats {
 	unsigned long long passes;     // its parallel decision passes
 	unsigned long long serial;     // its rounds that needed the in-order decision warp
 	unsigned long long list_entries; // conflict-list entries written
-	unsigned long long cluster_nodes; // nodes decided by 1,024 threads
+	unsigned long long cluster_nodes; // nodes decided by clusters of blocks
 	unsigned long long cycles[7];  // CTA greedy: SM cycles of thread 0 in phases A, B, C1, C2, D; cells read past 3 and 7 points
 };
 
@@ -195,8 +195,15 @@ void free_conflict_lists(ConflictLists& cl, DeviceMem& mem);
 // position, node k's words from accept_word(cand_off, k) on (a multiple of 4).
 __host__ __device__ inline int64_t accept_word(int64_t cand_off, int node) { return ((cand_off >> 7) + node) * 4; }
 inline int64_t accept_words(int64_t M, int K) { return ((M >> 7) + K + 1) * 4; }
+// nodes decided by one launch, largest first: blocks of `threads`, clusters of
+// `cluster` blocks
+struct AcceptSet {
+	size_t first, count;
+	int threads;
+	unsigned cluster;
+};
 // decides every node that is not dense; lb.accepted of their candidates
-void launch_accept(int mode, const LevelNode* d_nodes, const std::vector<LevelNode>& ln, const std::vector<uint8_t>& dense, LevelBuffers& lb,
+std::vector<AcceptSet> launch_accept(int mode, const LevelNode* d_nodes, const std::vector<LevelNode>& ln, const std::vector<uint8_t>& dense, LevelBuffers& lb,
                    const ConflictLists& cl, uint32_t* accepted_bits, SampleStats* st, DeviceMem& mem);
 // poisson_average's colours of those nodes, into lb.cols
 void launch_cell_colors(const LevelNode* d_nodes, const std::vector<uint8_t>& dense, const PosParamsS& pp, LevelBuffers& lb,
