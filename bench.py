@@ -60,9 +60,12 @@ WORKLOAD = {"workload": "hotspots-50M", "points": 50_000_000, "las": "1.4", "poi
             "sampler": "poisson", "form": "batched", "l2": "inputs larger than L2 (1.9 GB records)"}
 REF_SAMPLE_POINTS = 2_000_000
 GOLDEN = os.path.join(REPO, "tests", "golden", "golden.json")
-# DRAM bytes (read + write) per candidate of the acceptance kernel, from the
-# ncu capture summarised in profiles/accept_hotspots-5M_poisson.md
-ACCEPT_DRAM_BYTES_PER_CANDIDATE = 22.1
+# DRAM bytes (read + write) per candidate of the acceptance, accept_kernel 22.1
+# and accepted_kernel 8.1, from the ncu captures summarised in
+# profiles/accept_hotspots-5M_poisson.md
+ACCEPT_DRAM_BYTES_PER_CANDIDATE = 30.2
+# of which are written, and may stay in L2: the flag, the bit and the word's count
+ACCEPT_WRITTEN_PER_CANDIDATE = 1.25
 MEASURED_PEAKS = os.path.join(REPO, "MEASURED_PEAKS.json")
 
 
@@ -358,6 +361,16 @@ def serving_leg(local, jobs: int, rate: float, seed: int = 2000):
             "time_compression": f"{rate / 4.0:g}x the configuration's 4 jobs/s, {jobs} of its 2,000 jobs"}
 
 
+def acceptance_bytes(candidates):
+    """Algorithmic bytes of the acceptance from conflict lists. accept_kernel
+    reads a candidate's slot of up to four entries (16 B), its list length
+    (1 B) and where its list goes on (4 B), and writes a bit and, per 32
+    candidates, a count; accepted_kernel reads its sorted position and its node
+    (8 B) and writes its flag (1 B). Decisions stay in shared memory. Entries
+    past the fourth (4 B each, not counted by the library) are left out."""
+    return candidates * (16 + 1 + 4 + 8 + ACCEPT_WRITTEN_PER_CANDIDATE)
+
+
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--gpus", type=int, default=1)
@@ -445,13 +458,10 @@ def main():
     out_pts = s["output_points"]
     # roofline: the acceptance from conflict lists (accept_kernel, one launch
     # per set of nodes of an octree level), with the list search the largest
-    # share of a step. Algorithmic bytes: per candidate its inline entries
-    # (16 B), list length (1 B) and its decision, rank and flag (9 B); per
-    # list entry the entry (4 B) and that candidate's decision (4 B).
-    # Duration: the acceptance device time of the step (ms_greedy minus the
-    # list builds), all levels.
+    # share of a step. Duration: the acceptance device time of the step
+    # (ms_greedy minus the list builds), all levels.
     accept_ms = s["ms_greedy"] - s["ms_lists"]
-    accept_bytes = s["candidates"] * 26 + s["list_entries"] * 8
+    accept_bytes = acceptance_bytes(s["candidates"])
     peak, peak_kind = peak_hbm()
     achieved = accept_bytes / (accept_ms * 1e-3) / 1e9 if accept_ms > 0 else 0.0
     traffic = s["candidates"] * ACCEPT_DRAM_BYTES_PER_CANDIDATE if ACCEPT_DRAM_BYTES_PER_CANDIDATE else None
@@ -517,7 +527,7 @@ def main():
             "e2e": {"value": e2e, "unit": "Mpts/s", "h2d_bytes_per_step": int(pinned.numel()),
                     "d2h_bytes_per_step": int(octree_bytes)},
             "gpu_launches": int(s["gpu_launches"]) * args.steps,
-            "roofline": {"bound": "hbm", "kernel": "accept_kernel (list acceptance, all levels of a step)",
+            "roofline": {"bound": "hbm", "kernel": "accept_kernel + accepted_kernel (list acceptance, all levels of a step)",
                          "achieved": achieved, "peak": peak, "peak_kind": peak_kind, "unit": "GB/s", "frac": achieved / peak,
                          "traffic": traffic, "traffic_source": "DRAM bytes per candidate from ncu, profiles/accept_hotspots-5M_poisson.md",
                          "algorithmic_bytes": accept_bytes, "kernel_ms": accept_ms,
