@@ -31,14 +31,12 @@
 
 #include "devutil.cuh"
 #include "sampling.h"
+#include "shuffle_draw.h"
 
 namespace pcg {
 
 namespace {
 
-constexpr uint32_t kModulus = 2147483647u;     // minstd_rand0
-constexpr uint32_t kFactor = 16807u;
-constexpr uint32_t kRange = 2147483645u;       // largest draw minus the smallest
 constexpr int64_t kLongest = 46340;            // two swaps per draw up to here: kRange / n >= n
 constexpr int kDraws = 1024;                   // draws settled at once
 enum Way { kEven = 0, kOdd, kLong, kWays };
@@ -49,12 +47,6 @@ inline Way way_of(int64_t n) { return n > kLongest ? kLong : (n % 2 == 0 ? kEven
 struct Ways {
 	int64_t n[kWays], base[kWays];
 };
-
-__device__ __forceinline__ uint32_t mul_mod(uint32_t a, uint32_t b) {
-	const uint64_t p = (uint64_t)a * b;  // below 2^62
-	const uint32_t r = (uint32_t)(p & kModulus) + (uint32_t)(p >> 31);
-	return r >= kModulus ? r - kModulus : r;
-}
 
 __device__ uint32_t pow_mod(uint32_t a, uint32_t e) {
 	uint32_t r = 1;
@@ -79,7 +71,9 @@ __global__ void __launch_bounds__(kDraws) shuffle_targets_kernel(uint32_t seed, 
 	int32_t* target = target_all + ways.base[way];
 	if (n > 0 && threadIdx.x == 0) target[0] = 0;
 	if (n < 2) return;
-	const uint32_t steps = (uint32_t)(way == kEven ? n / 2 : (way == kOdd ? (n - 1) / 2 : n - 1));
+	// the last step of 2^31 - 1 elements chooses from more values than a draw has
+	const bool one_more = n > (int64_t)kRange + 1;
+	const uint32_t steps = (uint32_t)(way == kEven ? n / 2 : (way == kOdd ? (n - 1) / 2 : n - 1 - one_more));
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	uint32_t x = seed % kModulus;
 	if (x == 0) x = 1;
@@ -92,7 +86,7 @@ __global__ void __launch_bounds__(kDraws) shuffle_targets_kernel(uint32_t seed, 
 		bool taken = false, changed = false;
 		for (int pass = 0; pass <= kDraws; pass++) {
 			range = step_range(way, step < steps ? step : steps - 1);
-			scaling = kRange / range;
+			scaling = draw_scaling(range);
 			taken = draw < range * scaling;
 			const unsigned votes = __ballot_sync(FULL, taken);
 			if (lane == 0) sums[warp] = (uint32_t)__popc(votes);
@@ -114,6 +108,7 @@ __global__ void __launch_bounds__(kDraws) shuffle_targets_kernel(uint32_t seed, 
 			const uint32_t v = draw / scaling;
 			if (way == kLong) {
 				target[step + 1] = (int32_t)v;
+				if (one_more && step + 1 == steps) target[n - 1] = (int32_t)draw_of_one_more(x);
 			} else if (way == kEven && step == 0) {
 				target[1] = (int32_t)v;
 			} else {
