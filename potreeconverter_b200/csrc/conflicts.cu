@@ -92,11 +92,11 @@ __device__ __forceinline__ double qcoord(int32_t X, int a, const PosParamsS& pp)
 	return ((double)X * pp.scale[a]) + pp.offset[a];
 }
 
-__device__ __forceinline__ int clamp_cell(double u) {
-	double f = floor(u);
-	f = f < 0.0 ? 0.0 : (f > (double)(kCellsPerAxis - 1) ? (double)(kCellsPerAxis - 1) : f);
-	return (int)f;
-}
+// Any cell does where u is NaN (a corner of the box over a spacing whose
+// reciprocal is infinite: nothing is closer than such a spacing), but it has to
+// be one: fmax and fmin leave NaN out, a comparison would keep it and the
+// conversion make a negative index of it.
+__device__ __forceinline__ int clamp_cell(double u) { return (int)fmin(fmax(floor(u), 0.0), (double)(kCellsPerAxis - 1)); }
 
 // every candidate's cell (z, y, x, seven bits each) and the occupancy bitmaps
 __global__ void cell_mark_kernel(const LevelNode* __restrict__ nodes, PosParamsS pp, LevelBuffers lb, uint32_t* __restrict__ cell,
