@@ -43,8 +43,8 @@
 // carries at most 256 s u + |d| u, its square a relative error of 2 (257 u)
 // + u, and the sum of three squares at most 517 u = 3.1e-5 of the squared
 // distance D. The FP64 values the reference compares are themselves within
-// 1.1e-16 |x| of the exact coordinates, below 1.1e-10 s when |x| < 1e6 s
-// (checked per node; beyond it the node uses FP64 alone). So D32 >= s^2 (1 +
+// 1.1e-16 |x| of the exact coordinates, below 1.1e-10 s when |x| < 1e6 s.
+// (Both are checked per node, fp32_decides; otherwise FP64 alone decides.) So D32 >= s^2 (1 +
 // 1e-3) (rounded up by at most u) implies D64 > s^2, and D32 < s^2 (1 - 1e-3)
 // implies D64 < s^2: the margin is 30x the error.
 //
@@ -292,9 +292,7 @@ struct PairTest {
 		t = __float_as_int(rec.w);
 		escalated = 0;
 		const double sp = nd.spacing, s2 = sp * sp;
-		double amax = 0.0;
-		for (int a = 0; a < 3; a++) amax = fmax(amax, fmax(fabs(nd.min[a]), fabs(nd.max[a])));
-		const bool pre32 = s2 > 1e-30 && s2 < 1e30 && amax < 1e6 * sp;
+		const bool pre32 = nd.fp32 != 0;
 		s2hi = pre32 ? (float)(s2 * 1.001) : __int_as_float(0x7fffffff);
 		s2lo = pre32 ? (float)(s2 * 0.999) : -1.0f;
 		// c >= 1.1 s: 1.25 s^2 leaves 3 % for the roundings of FP32

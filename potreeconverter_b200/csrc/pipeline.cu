@@ -1701,7 +1701,7 @@ struct Converter {
 			l.max[0] = n.max.x; l.max[1] = n.max.y; l.max[2] = n.max.z;
 			l.level = n.depth;
 			l.spacing = base_spacing / std::pow(2.0, (double)n.depth);  // sampler_poisson.h:114
-			l.pad = 0;
+			l.fp32 = fp32_decides(l);
 		}
 		res.stats.sampled_nodes += K;
 		res.stats.candidates += M;

@@ -1,6 +1,7 @@
 // Sampler kernels (one octree level across all its nodes per launch).
 #pragma once
 
+#include <cmath>
 #include <vector>
 
 #include "dev.h"
@@ -15,7 +16,7 @@ struct LevelNode {          // one inner node sampled at this level
 	double min[3], max[3];   // node box
 	double spacing;          // baseSpacing / 2^level
 	int32_t level;
-	int32_t pad;
+	int32_t fp32;            // distances may be judged in FP32 (fp32_decides)
 };
 
 struct GatherItem {         // copy `count` ids (and colours, records) of one child buffer
@@ -30,6 +31,18 @@ struct GatherItem {         // copy `count` ids (and colours, records) of one ch
 // the gather launch takes the items cut into pieces of at most this many
 // ids, one CTA each, so a large child buffer does not keep one CTA busy
 constexpr int64_t kGatherPiece = 4096;
+
+// Whether the error bound of the conflict search's FP32 test holds for a node
+// (conflicts.cu): its box measures 128 spacings, as a conversion's always does
+// (a caller of the acceptance alone may ask for another spacing), and the
+// coordinates are below a million of them.
+inline int32_t fp32_decides(const LevelNode& n) {
+	const double sp = n.spacing, s2 = sp * sp;
+	bool ok = s2 > 1e-30 && s2 < 1e30;
+	for (int a = 0; a < 3; a++)
+		ok = ok && n.max[a] - n.min[a] < 128.01 * sp && std::fabs(n.min[a]) < 1e6 * sp && std::fabs(n.max[a]) < 1e6 * sp;
+	return ok ? 1 : 0;
+}
 
 struct LevelBuffers {
 	int64_t M = 0;                 // candidates at this level
