@@ -138,7 +138,9 @@ typedef struct pcg_stats {
 	double ms_total;              /* wall time of pcg_convert               */
 	double ms_h2d, ms_chunking, ms_octree, ms_sampling, ms_output, ms_d2h, ms_host_writers;
 	int64_t gpu_launches;         /* kernels launched for this job          */
-	double ms_sort, ms_greedy;    /* device time of the sampler sort / acceptance kernels */
+	double ms_sort, ms_greedy;    /* device time of the sampler's sorts, and of
+	                                 its conflict lists, acceptance and
+	                                 (poisson_average) averaged colours     */
 	int64_t sampled_nodes;        /* inner nodes sampled                    */
 	int64_t candidates;           /* candidate points over all sampled nodes */
 	int64_t replayed_nodes;       /* nodes with equal keys, sorted by the

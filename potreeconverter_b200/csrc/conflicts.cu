@@ -266,10 +266,9 @@ struct RunWalk {
 		runs[n * stride] = run;  // what is loaded after the last record
 		next = rec[run.x];
 	}
-	// the record, and in k its index; left is above 0
-	__device__ __forceinline__ float4 take(uint32_t& k) {
+	// the record; left is above 0
+	__device__ __forceinline__ float4 take() {
 		const float4 r = next;
-		k = run.x;
 		if (++run.x == run.y) run = *(runs += stride);
 		next = rec[run.x];
 		left--;
@@ -350,8 +349,7 @@ __global__ void __launch_bounds__(kListThreads, kListBlocks) conf_lists_kernel(c
 		RunWalk walk(&runs[0][threadIdx.x], nr, kListThreads, lc.rec);
 #pragma unroll 1
 		while (walk.left) {
-			uint32_t k;
-			const float4 qf = walk.take(k);
+			const float4 qf = walk.take();
 			const int32_t u = __float_as_int(qf.w);
 			const bool hit = test(qf, u, u < t, lb, pp);
 			if (hit) list[n < kListCap ? n : kListCap] = u;

@@ -6,7 +6,7 @@
 // distance to the node centre (sampler_poisson.h:183-203). When a node's keys
 // are pairwise distinct, the ascending order is unique, so any exact sort
 // yields the permutation std::sort yields. Only nodes with equal keys need
-// the element-for-element introsort replay of sampling.cu, because there the
+// the element-for-element introsort replay of introsort.cu, because there the
 // order among equal keys is an artefact of the partitions.
 //
 // This unit sorts every node of a level at once with a segmented LSD radix
