@@ -42,8 +42,8 @@ __global__ void __launch_bounds__(64) laz_decode_kernel(const uint8_t* __restric
 // resident: four per SM, as the models of a chunk take about 40 KB of shared
 // memory. Measured on one B200 (flight lines, format 3), one thread per chunk
 // before, two warps per chunk now: 20 chunks of 50,000 points 417.5 ms and
-// 224.0 ms (8.35 and 4.48 us a point), 400 chunks of 5,000 points 45.2 and
-// 23.7 ms, 800 of them (two waves) 78.7 and 59.0, 1,000 chunks of 1,000 points
+// 223.5 ms (8.35 and 4.47 us a point), 400 chunks of 5,000 points 45.2 and
+// 23.6 ms, 800 of them (two waves) 78.7 and 58.7, 1,000 chunks of 1,000 points
 // 28.8 and 12.4. Of the decoder warp's 8,800 cycles a point the 16 symbols
 // take about 5,000; its instructions issue every 5.5 cycles (dependent
 // arithmetic 2.5, shared memory and shuffles 1.1, instruction fetches 0.6).

@@ -16,7 +16,9 @@
 //    load of the search brings it and the lane of the symbol stores it back;
 //    lane 31 keeps the symbols until the model's next update the same way;
 //    (a lane's word is read by its neighbour too, so a warp barrier lies on
-//    either side of the stores: the two cost 2.4 % of the decode);
+//    either side of the stores: the two cost 1.4 % of chunks of 50,000 points
+//    and 2.5 % of a conversion of 5,000-point chunks, a little more where the
+//    first one stands before the stores and not behind the ballot);
 //  * a model update is a warp scan over the counts;
 //  * coded bytes come from a ring in shared memory, refilled once per point.
 // The second warp turns the decoded symbols (32 points at a time, through a
@@ -267,6 +269,7 @@ struct Decoder {
 		const uint32_t part = length >> laz::kSymShift;
 		const uint32_t p0 = (w0 & 0xffff) * part, p1 = lane + 1 < n ? (w1 & 0xffff) * part : length;
 		const uint32_t votes = __ballot_sync(kAll, lane < 31 ? lane < n && p0 <= value : w0 == 1);
+		__syncwarp();  // every lane has loaded
 		uint32_t s = (uint32_t)__popc(votes & 0x7fffffffu) - 1;  // lane 0's distribution value is 0
 		if (s == 30 && n > 31) {
 			// symbols 30, 31 and 32 (slots 30, 32 and 33), rarely
@@ -285,7 +288,6 @@ struct Decoder {
 		} else {
 			take(p0, p1, s);
 		}
-		__syncwarp();  // every lane has loaded
 		m.st_lane(lane, 31, W_SLOT, w0 - 1);
 		m.st_lane(lane, s < 31 ? s : 32, W_SLOT, w0 + 0x10000u);
 		__syncwarp();  // and the next symbol's loads see this
@@ -306,8 +308,8 @@ struct Decoder {
 		const uint32_t w0 = m.ld(W_ENTRY + 4 * i), w1 = m.ld(W_ENTRY + 4 * i + 4);
 		const uint32_t p0 = (w0 & 0xffff) * part, p1 = i + 1 < n ? (w1 & 0xffff) * part : length;
 		const uint32_t o = ((uint32_t)__popc(__ballot_sync(kAll, lane < size && i < n && p0 <= value)) - 1) & (size - 1);
-		take(p0, p1, o);
 		__syncwarp();
+		take(p0, p1, o);
 		m.st_lane(lane, 31, W_UNTIL, start - 1);
 		m.st_lane(lane, o, W_ENTRY + 4 * i, w0 + 0x10000u);
 		__syncwarp();
