@@ -77,7 +77,9 @@ def write(rows: list, points: int, out_dir: str = CSRC):
         f.write("// Level schedule of the samplers (sampling.h LevelSchedule). Written by\n"
                 "// potreeconverter_b200/autotune.py from a sweep on the target GPU; the\n"
                 "// values below are the sweep's best for the benchmarked workload, or the\n"
-                "// hand-set defaults until a sweep has run.\n#pragma once\n"
+                "// hand-set defaults until a sweep has run. The names are older than what they\n"
+                "// stand for: from how many candidates a node gets a block of 16 x\n"
+                "// WARP_BLOCKS_PER_SM threads, the same on levels of few nodes, a block of 1,024.\n#pragma once\n"
                 f"#define PCG_TUNED_CTA_MIN {cta}\n#define PCG_TUNED_SMALL_LEVEL_CTA_MIN {small}\n"
                 f"#define PCG_TUNED_CLUSTER_MIN {clu}\n#define PCG_TUNED_WARP_BLOCKS_PER_SM {warp}\n")
     with open(os.path.join(out_dir, "tuned_schedule.json"), "w") as f:

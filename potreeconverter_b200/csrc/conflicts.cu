@@ -44,9 +44,9 @@
 // + u, and the sum of three squares at most 517 u = 3.1e-5 of the squared
 // distance D. The FP64 values the reference compares are themselves within
 // 1.1e-16 |x| of the exact coordinates, below 1.1e-10 s when |x| < 1e6 s.
-// (Both are checked per node, fp32_decides; otherwise FP64 alone decides.) So D32 >= s^2 (1 +
-// 1e-3) (rounded up by at most u) implies D64 > s^2, and D32 < s^2 (1 - 1e-3)
-// implies D64 < s^2: the margin is 30x the error.
+// (Both are checked per node, fp32_decides; otherwise FP64 alone decides.) So
+// D32 >= s^2 (1 + 1e-3) (rounded up by at most u) implies D64 > s^2, and D32 <
+// s^2 (1 - 1e-3) implies D64 < s^2: the margin is 30x the error.
 //
 // The early-exit bound needs the earlier candidate's key only where it can
 // fail. With c = sqrt(key(p)) >= 1.1 s and a pair the FP32 test puts inside
