@@ -923,18 +923,29 @@ void launch_cand_records(const LevelNode* nodes, const int32_t* X, const int32_t
 }
 
 void greedy_arena_free(GreedyArena& a, DeviceMem& mem) {
-	if (a.cells) { mem.free(a.cells); mem.free(a.ovf); }
+	if (a.cells) mem.free(a.cells);
+	if (a.ovf) mem.free(a.ovf);
 	a = GreedyArena{};
 }
 
-void greedy_arena_reserve(GreedyArena& a, int slots, DeviceMem& mem) {
-	if (slots <= a.slots) return;
+int greedy_arena_reserve(GreedyArena& a, int slots, DeviceMem& mem) {
+	if (slots <= a.slots) return slots;
 	greedy_arena_free(a, mem);
-	a.cells = mem.alloc<AccCell>((size_t)slots * kGridCells);
-	a.ovf = mem.alloc<int32_t>((size_t)slots * kGridCells);
+	// as many as the device can hold
+	while (!a.ovf) {
+		try {
+			a.cells = mem.alloc<AccCell>((size_t)slots * kGridCells);
+			a.ovf = mem.alloc<int32_t>((size_t)slots * kGridCells);
+		} catch (const PcgError& e) {
+			greedy_arena_free(a, mem);
+			if (e.status != 3 || slots == 1) throw;  // 3: PCG_OOM
+			slots = (slots + 1) / 2;
+		}
+	}
 	PCG_CUDA(cudaMemsetAsync(a.cells, 0, (size_t)slots * kGridCells * sizeof(AccCell), mem.stream()));
 	PCG_CUDA(cudaMemsetAsync(a.ovf, 0xff, (size_t)slots * kGridCells * sizeof(int32_t), mem.stream()));
 	a.slots = slots;
+	return slots;
 }
 
 void launch_greedy(int mode, bool fp32_guard, const LevelNode* nodes, const int32_t* order, int K, const int32_t* X, const int32_t* Y,
@@ -954,13 +965,12 @@ void launch_greedy(int mode, bool fp32_guard, const LevelNode* nodes, const int3
 		// which the caller has freed; large levels go in batches
 		const int batch = (int)std::min<int64_t>(sm_count() * 2, kLongListBytes / (kGridCells * (int64_t)(sizeof(AccCell) + sizeof(int32_t))));
 		const int nbig = big_end - node_begin;
-		const int slots = nbig < batch ? nbig : batch;
-		greedy_arena_reserve(*grid, slots, mem);
 		GridArena arena;
-		arena.cells = static_cast<AccCell*>(grid->cells);
-		arena.ovf = grid->ovf;
 		arena.link = mem.alloc<int32_t>((size_t)lb.M);
 		arena.accq = mem.alloc<int4>((size_t)lb.M);
+		const int slots = greedy_arena_reserve(*grid, nbig < batch ? nbig : batch, mem);
+		arena.cells = static_cast<AccCell*>(grid->cells);
+		arena.ovf = grid->ovf;
 		if (mode == 0) allow_shared_memory(greedy_big_kernel<0>, smem);
 		else allow_shared_memory(greedy_big_kernel<1>, smem);
 		for (int b0 = node_begin; b0 < big_end; b0 += slots) {

@@ -231,7 +231,7 @@ struct GreedyArena {
 	int32_t* ovf = nullptr;
 	int slots = 0;
 };
-void greedy_arena_reserve(GreedyArena& a, int slots, DeviceMem& mem);
+int greedy_arena_reserve(GreedyArena& a, int slots, DeviceMem& mem);  // returns how many there are, at most `slots`
 void greedy_arena_free(GreedyArena& a, DeviceMem& mem);
 // mode 0 = poisson (early exit + 10,001-check window), 1 = poisson_average (pure greedy)
 void launch_greedy(int mode, bool fp32_guard, const LevelNode* nodes, const int32_t* order, int K, const int32_t* X, const int32_t* Y,

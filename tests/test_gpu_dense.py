@@ -87,3 +87,30 @@ def test_clouds_with_less_room(oracle, method, limits):
     assert any(d > 0 for n, d in levels)
     if limits != "1,1,1":
         assert any(0 < d < n for n, d in levels), levels
+
+
+FULL = """
+import hashlib, sys
+import torch
+import potreeconverter_b200 as pc
+from tests.test_gpu_estimate import clumps
+las = clumps(1_000_000, 250)
+leave = float(sys.argv[1])
+torch.zeros(1, device="cuda")
+with pc.Context() as ctx:
+    held = torch.empty(int(torch.cuda.mem_get_info()[0] - leave * 2 ** 30), dtype=torch.uint8, device="cuda") if leave else None
+    c = ctx.convert(las, method="poisson", name="full")
+    print(hashlib.md5(c.octree + c.hierarchy).hexdigest())
+"""
+
+
+def test_device_that_something_else_fills():
+    # 1.2 GiB are left for a conversion that takes 1.2 when it can have them:
+    # neither the long lists nor the grids of the nodes without any find the
+    # room they ask for
+    def convert(leave):
+        r = subprocess.run([sys.executable, "-c", FULL, str(leave)], cwd=REPO, capture_output=True, text=True, timeout=300)
+        assert r.returncode == 0, r.stderr[-500:]
+        return r.stdout
+
+    assert convert(1.2) == convert(0)
